@@ -66,6 +66,7 @@
 #include "layered_mixers3.cuh"
 #include "layered_mixers4.cuh"
 #include "layered_mixers5.cuh"
+#include "layered_tc.h"
 #include "modeldir.h"
 #include "sample_host.h"
 
@@ -208,6 +209,7 @@ struct LayeredEngine : nb::EngineBase {
     // generation on the implicit sequence
     int gen_seq = -1;
     void *samp_ws = nullptr; size_t samp_cub = 0; uint32_t *samp_host = nullptr;
+    TcState tc;              // products of long portions on the tensor cores' own memory (layered_tc.cu)
     std::vector<void *> allocs;
 };
 
@@ -881,6 +883,8 @@ uint32_t gemv_blocks(const LayeredEngine *e, uint32_t N, uint32_t groups) {
     return std::min((N + 7u) / 8u, std::max(1u, (uint32_t)e->num_sms * 8u / groups));
 }
 
+uint32_t ew_grid(size_t n) { return (uint32_t)std::min<size_t>((n + 255) / 256, 148 * 16); }
+
 // one matrix product; maxM = the most rows any group can have.  wf32: the weights are fp32 whatever the engine's mode (router).
 // active: how many of the groups can have rows at all (routed products: tokens x top); the matrix-vector grid is sized for those
 int gemm(LayeredEngine *e, GemmArgs a, uint32_t groups, uint32_t maxM, bool wf32 = false, uint32_t active = 0) {
@@ -903,6 +907,11 @@ int gemm(LayeredEngine *e, GemmArgs a, uint32_t groups, uint32_t maxM, bool wf32
         return f32 ? launch<GemmArgs>(e, k_gemv<float>, dim3(gx, groups), dim3(256), 0, a) : launch<GemmArgs>(e, k_gemv<__nv_bfloat16>, dim3(gx, groups), dim3(256), 0, a);
     }
     if (a.glu) return fail(NB200_EINVAL, "the gated-pair product is a matrix-vector instance (portions of at most %u tokens)", kGemvMaxM);
+    const uint32_t rows = a.g_off && active ? active : a.M;
+    if (!f32 && (!a.g_off || active) && tc_fits(&e->tc, a, rows)) {
+        e->launches += 2;
+        return tc_gemm(&e->tc, a, groups, maxM, rows, a.g_off ? std::max(1u, (active + groups - 1u) / groups) : maxM, e->cur == e->side ? 1u : e->cur == e->side2 ? 2u : 0u, e->cur, e->use_pdl);
+    }
     const dim3 grid((a.N + 63u) / 64u, (maxM + 63u) / 64u, groups);
     return f32 ? launch<GemmArgs>(e, k_gemm_f32<float>, grid, dim3(256), 0, a) : launch<GemmArgs>(e, k_gemm_bf16, grid, dim3(128), 0, a);
 }
@@ -913,8 +922,6 @@ GemmArgs plain(const float *A, uint32_t lda, const Weight &w, float *C, uint32_t
     a.epi = bias && epi == EPI_NONE ? EPI_BIAS : epi; a.split = split; a.a_gmod = 1;
     return a;
 }
-
-uint32_t ew_grid(size_t n) { return (uint32_t)std::min<size_t>((n + 255) / 256, 148 * 16); }
 
 constexpr int kAttnQT = 8;      // query tokens per attention block in a prefill portion (4 where the latent is wider than 256)
 size_t attn_smem(uint32_t R, int qt) { return ((size_t)qt * kAttnWarps * R + (size_t)kPage * (R + 4)) * 4; }
@@ -1897,7 +1904,7 @@ int lm_step(nb200_engine *h, uint32_t seq, const uint32_t *tokens, uint32_t n, c
         if ((r = step_dev(e, seq, e->ids_dev, m, done.data(), (uint32_t)done.size(), logits ? logits + (size_t)w0 * e->V : nullptr))) return r;
     }
     CK(cudaStreamSynchronize(e->stream));
-    return 0;
+    return tc_check(&e->tc);
 }
 
 int lm_step_timed(nb200_engine *h, uint32_t seq, const uint32_t *tokens, uint32_t n, uint32_t reps, float *ms) {
@@ -1927,7 +1934,7 @@ int lm_step_timed(nb200_engine *h, uint32_t seq, const uint32_t *tokens, uint32_
     cudaEventDestroy(ev[0]); cudaEventDestroy(ev[1]);
     if (r) return r;
     *ms = total / (float)reps;
-    return 0;
+    return tc_check(&e->tc);
 }
 
 int lm_read_residual(nb200_engine *h, uint32_t run, float *dst, uint32_t count) {
@@ -1989,7 +1996,7 @@ int lm_forward(nb200_engine *h, uint32_t token, uint32_t pos, uint32_t is_causal
     int r;
     if ((r = gen_seek(e, nullptr, pos)) || (r = gen_token(e, token))) return r;
     CK(cudaStreamSynchronize(e->stream));
-    return 0;
+    return tc_check(&e->tc);
 }
 
 int lm_read_logits(nb200_engine *h, float *out) {
@@ -2028,7 +2035,7 @@ int lm_next_greedy(nb200_engine *h, const uint32_t *ids, uint32_t pos, int is_pr
     CK(cudaMemcpyAsync(e->tok_host, e->next_dev, 4, cudaMemcpyDeviceToHost, e->stream));
     CK(cudaStreamSynchronize(e->stream));
     *next = is_prefilling ? ids[pos + 1] : *e->tok_host;
-    return 0;
+    return tc_check(&e->tc);
 }
 
 int lm_next_sampled(nb200_engine *h, const uint32_t *ids, uint32_t pos, float penalty, float temperature, float top_p, float coin, uint32_t *next, uint32_t *top6) {
@@ -2055,7 +2062,7 @@ int lm_next_sampled(nb200_engine *h, const uint32_t *ids, uint32_t pos, float pe
     CK(cudaStreamSynchronize(e->stream));
     *next = e->samp_host[0];
     if (top6) for (int i = 0; i < 6; i++) top6[i] = e->samp_host[1 + i];
-    return 0;
+    return tc_check(&e->tc);
 }
 
 // prompt ids[0..n_prompt) -> greedy ids[n_prompt..n_total); positions 0..n_prompt-2 run as one prefill portion, the rest token by
@@ -2100,7 +2107,7 @@ int lm_decode_greedy(nb200_engine *h, uint32_t *ids, uint32_t n_prompt, uint32_t
     CK(cudaEventElapsedTime(&b, evs.ev[1], evs.ev[2]));
     if (prefill_ms) *prefill_ms = a;
     if (device_ms) *device_ms = b;
-    return 0;
+    return tc_check(&e->tc);
 }
 
 int lm_get_config(const nb200_engine *h, nb200_config *c) {
@@ -2120,6 +2127,7 @@ void lm_destroy(nb200_engine *h) {
     for (void *p : e->allocs) cudaFree(p);
     if (e->tok_host) cudaFreeHost(e->tok_host);
     if (e->samp_host) cudaFreeHost(e->samp_host);
+    tc_free(&e->tc);
     if (e->ev_fork) cudaEventDestroy(e->ev_fork);
     if (e->ev_join) cudaEventDestroy(e->ev_join);
     if (e->ev_join2) cudaEventDestroy(e->ev_join2);
@@ -2541,6 +2549,11 @@ int create(LayeredEngine *e, const nb::ModelDir *dir, uint32_t max_tokens) {
         if (mSFF) { DM(e->b_sh, T * std::max(mSFF, mSFF2) * 4); DM(e->b_so, T * E * 4); }
         if (mFF2) { DM(e->b_hg, T * mFF2 * 4); DM(e->b_wrow, T * mTop * 4); DM(e->b_sg, T * 4); }
         if (mSFF2) DM(e->b_sh2, T * mSFF * 4);
+    }
+    if (!e->f32) {      // the widest rows any product reads (a routed product: one row per token and choice)
+        size_t w = std::max<size_t>(E, mTop * E);
+        for (uint32_t v : {2 * mC, mZ, mQR, mQ, mHR, mOV, sP, sQK, sXC, sA, sRO, sDBC, sF, sF2, sXC2, sY, dV, dSp, dGt, mMO, mFF, mFF2, mSFF, mSFF2}) w = std::max<size_t>(w, v);
+        if ((r = tc_setup(&e->tc, std::max<size_t>(T, kWantBatch) * ((w + 7u) & ~(size_t)7u), (uint32_t)e->num_sms))) return r;
     }
     DM(e->dpos, 64); DM(e->zero_dev, 64);
     CK(cudaMemset(e->dpos, 0, 64)); CK(cudaMemset(e->zero_dev, 0, 64));

@@ -1,0 +1,29 @@
+// layered_tc.h -- host side of layered_tc.cu: matrix products of long portions on tcgen05
+#pragma once
+#include <cuda.h>
+#include <stddef.h>
+
+#include "layered_common.cuh"
+
+namespace nb {
+namespace lm {
+
+// what an engine keeps for these products: rounded activation rows (one buffer for each of its three streams), the driver's tensor-map encoder,
+// the word a bounded wait reports to
+struct TcState {
+    __nv_bfloat16 *rows[3] = {nullptr, nullptr, nullptr}; size_t elems = 0;
+    decltype(&cuTensorMapEncodeTiled) encode = nullptr;
+    uint32_t *err_host = nullptr, *err_dev = nullptr, sms = 148;
+};
+int tc_setup(TcState *t, size_t elems, uint32_t sms);
+void tc_free(TcState *t);
+// after a synchronisation: did a bounded wait of a kernel run out
+int tc_check(TcState *t);
+// whether the product's layout allows it.  rows: all rows of A it reads (a routed product: tokens x choices)
+bool tc_fits(const TcState *t, const GemmArgs &a, uint32_t rows);
+// two launches on `stream` (with programmatic serialization when pdl).  buf: which of the row buffers is the stream's; maxM: the most rows of a group, each:
+// how many a group has on average
+int tc_gemm(TcState *t, GemmArgs a, uint32_t groups, uint32_t maxM, uint32_t rows, uint32_t each, uint32_t buf, cudaStream_t stream, bool pdl);
+
+}  // namespace lm
+}  // namespace nb
