@@ -39,8 +39,9 @@ def _newer(target: str, sources) -> bool:
 UNITS = {
     "api.cu": ["family.h", "modeldir.h", "../../include/nano_b200.h"],
     "modeldir.cu": ["modeldir.h"],
-    "layered.cu": ["layered_kernels.cuh", "layered_common.cuh", "layered_tc.h", "layered_mixers.cuh", "layered_mixers2.cuh", "layered_mixers3.cuh", "layered_mixers4.cuh", "layered_mixers5.cuh", "family.h", "modeldir.h", "sample_host.h", "../../include/nano_b200.h"],
+    "layered.cu": ["layered_kernels.cuh", "layered_common.cuh", "layered_tc.h", "attn_tc.h", "layered_mixers.cuh", "layered_mixers2.cuh", "layered_mixers3.cuh", "layered_mixers4.cuh", "layered_mixers5.cuh", "family.h", "modeldir.h", "sample_host.h", "../../include/nano_b200.h"],
     "layered_tc.cu": ["layered_common.cuh", "layered_tc.h", "tc_ptx.cuh", "family.h"],
+    "attn_tc.cu": ["attn_tc.h", "tc_ptx.cuh", "family.h"],
     "engine.cu": ["kernels.cuh", "expf_ref.cuh", "stream_args.h", "stream_host.h", "sample_host.h", "family.h", "../../include/nano_b200.h"],
     "stream.cu": ["kernels.cuh", "expf_ref.cuh", "stream_args.h", "stream_host.h", "stream.cuh"],
     "sample.cu": ["kernels.cuh", "expf_ref.cuh", "sample_host.h"],
@@ -49,7 +50,7 @@ UNITS = {
 
 # the units a model FOLDER (config.json + model.safetensors) needs: registry, folder reader, layered runtime, device sampler.
 # The model-file family (engine.cu, stream.cu: minutes of nvcc) is not among them.
-LAYERED_UNITS = ["api.cu", "modeldir.cu", "layered.cu", "layered_tc.cu", "sample.cu"]
+LAYERED_UNITS = ["api.cu", "modeldir.cu", "layered.cu", "layered_tc.cu", "attn_tc.cu", "sample.cu"]
 LAYERED_SO = os.path.join(LIB, "libnano_b200_layered.so")
 
 
@@ -58,7 +59,7 @@ def build_engine(force: bool = False, verbose: bool = False, units=None, target:
     units / target: a library of a subset of the families (build_layered)."""
     os.makedirs(LIB, exist_ok=True)
     target = target or ENGINE_SO
-    base = [NVCC, "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "--split-compile", "0", "-Xcompiler", "-fPIC"]
+    base = [NVCC, "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC"]
     if verbose:
         base.insert(1, "-Xptxas=-v")
     objs, procs = [], []

@@ -59,6 +59,7 @@
 #include <string>
 #include <vector>
 
+#include "attn_tc.h"
 #include "family.h"
 #include "layered_kernels.cuh"
 #include "layered_mixers.cuh"
@@ -210,6 +211,7 @@ struct LayeredEngine : nb::EngineBase {
     int gen_seq = -1;
     void *samp_ws = nullptr; size_t samp_cub = 0; uint32_t *samp_host = nullptr;
     TcState tc;              // products of long portions on the tensor cores' own memory (layered_tc.cu)
+    nb::TcAttnState ta;      // and their attention (attn_tc.cu)
     std::vector<void *> allocs;
 };
 
@@ -1358,6 +1360,7 @@ template <int VJ>
 int gqa_attn_launch(LayeredEngine *e, const GqaArgs &a) {
     return launch<GqaArgs>(e, k_gqa_attn<VJ>, dim3((a.T * (a.H / a.G) + kGqaM - 1u) / kGqaM, a.G), dim3(256), gqa_attn_smem(a.D, VJ), a);
 }
+constexpr uint64_t kTcAttnWork = 128 * 128;      // tokens x keys from which a portion's attention goes to the tensor cores
 uint32_t gqa_hb(const Layer &L) { return std::min(L.H / L.G, kGqaHeads); }
 // from the rows of the joint product (q, k, v from column 0) to dst [T][E]
 int gqa_branch(LayeredEngine *e, const Layer &L, const Run &run, const Ctx &cx, float *dst) {
@@ -1378,6 +1381,16 @@ int gqa_branch(LayeredEngine *e, const Layer &L, const Run &run, const Ctx &cx, 
 #undef GQA_DECODE
     } else {
         if ((r = launch<GqaArgs>(e, k_qk_norm_rope, dim3(T), dim3(256), 0, a))) return r;
+        nb::TcAttn ta{};      // (queries carry the scale already)
+        ta.q = e->b_p; ta.ldq = P; ta.q_head = D; ta.k = run.cache; ta.v = run.cache + G * D; ta.ldk = ta.ldv = L.RL; ta.k_head = D; ta.v_head = VD; ta.table = cx.table;
+        ta.out = e->b_a; ta.T = T; ta.H = H; ta.G = G; ta.D = D; ta.VD = VD; ta.pos0 = cx.pos0; ta.block = L.block_size; ta.scale = 1.0f; ta.softcap = L.softcap; ta.sink = L.sink;
+        if (L.has_gate) { ta.gate = e->b_p + L.c_hg; ta.ldg = P; }
+        // its two launches cost some 20 us however little there is to do: 5 x 8 (tokens x keys) 20 us against 11, 128 x 128 equal, 333 x 410 36 against 60
+        if (nb::attn_tc_fits(&e->ta, ta) && (uint64_t)T * (cx.pos0 + T - nb::attn_tc_first(ta)) >= kTcAttnWork) {
+            e->launches += 2;
+            if ((r = nb::attn_tc_launch(&e->ta, ta, e->cur, e->use_pdl))) return r;
+            return gemm(e, plain(e->b_a, H * VD, L.o, dst, e->E, T), 1, T);
+        }
         const int vj = gqa_vj(VD);
         r = vj == 1 ? gqa_attn_launch<1>(e, a) : vj == 2 ? gqa_attn_launch<2>(e, a) : gqa_attn_launch<4>(e, a);
     }
@@ -2127,6 +2140,7 @@ void lm_destroy(nb200_engine *h) {
     for (void *p : e->allocs) cudaFree(p);
     if (e->tok_host) cudaFreeHost(e->tok_host);
     if (e->samp_host) cudaFreeHost(e->samp_host);
+    nb::attn_tc_free(&e->ta);
     tc_free(&e->tc);
     if (e->ev_fork) cudaEventDestroy(e->ev_fork);
     if (e->ev_join) cudaEventDestroy(e->ev_join);
@@ -2553,7 +2567,13 @@ int create(LayeredEngine *e, const nb::ModelDir *dir, uint32_t max_tokens) {
     if (!e->f32) {      // the widest rows any product reads (a routed product: one row per token and choice)
         size_t w = std::max<size_t>(E, mTop * E);
         for (uint32_t v : {2 * mC, mZ, mQR, mQ, mHR, mOV, sP, sQK, sXC, sA, sRO, sDBC, sF, sF2, sXC2, sY, dV, dSp, dGt, mMO, mFF, mFF2, mSFF, mSFF2}) w = std::max<size_t>(w, v);
-        if ((r = tc_setup(&e->tc, std::max<size_t>(T, kWantBatch) * ((w + 7u) & ~(size_t)7u), (uint32_t)e->num_sms))) return r;
+        // images of every key a sequence can hold, up to 1 GB (longer contexts of many heads go through the fp32 kernels)
+        size_t bytes = 0, tiles = 0;
+        const uint32_t keys = e->n_pages * kPage;
+        for (const Layer &L : e->layers)
+            if (L.type == MIX_ATTN_DELTA || L.type == MIX_GQA) { bytes = std::max(bytes, nb::attn_tc_bytes(keys, L.G, L.dim, L.vdim)); tiles = std::max(tiles, nb::attn_tc_tiles(keys, L.G)); }
+        if ((r = tc_setup(&e->tc, std::max<size_t>(T, kWantBatch) * ((w + 7u) & ~(size_t)7u), (uint32_t)e->num_sms)) ||
+            (r = nb::attn_tc_setup(&e->ta, std::min<size_t>(bytes, (size_t)1 << 30), tiles, e->tc.err_dev))) return r;
     }
     DM(e->dpos, 64); DM(e->zero_dev, 64);
     CK(cudaMemset(e->dpos, 0, 64)); CK(cudaMemset(e->zero_dev, 0, 64));

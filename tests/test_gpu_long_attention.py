@@ -1,0 +1,40 @@
+"""Attention of long portions on the tensor cores (csrc/attn_tc.cu) at the edges of its tiles: tiles of 128 keys and of 128 (token, head) rows, head sizes
+around 64 and 128, blocks of positions that start inside a tile, a context before the portion, sharp scores.
+
+The portion is held against the same tokens one at a time, whose kernels sum in fp32.  Every product's operands are rounded to bfloat16 the same way
+on both sides; the attention differs by its own error of about 1e-6, which turns last bits (2^-9) of later operands here and there: under
+1.2e-2 of a row's norm through one layer, of which sharp scores (a factor of 6 on the logits of the softmax) may multiply the part before
+them."""
+import numpy as np
+import pytest
+
+from nano_b200 import engine as E, modeldir as md
+import fidatar_oracle as F
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("heads,kv,dim,vdim,size,scale", [(4, 1, 32, 32, None, 0.2), (8, 8, 64, 64, None, 0.125), (6, 2, 68, 60, 200, 0.12), (4, 2, 128, 128, None, 0.6), (2, 1, 48, 128, 130, 0.15), (4, 4, 4, 4, 128, 0.5)])
+def test_portions_against_single_tokens(tmp_path, heads, kv, dim, vdim, size, scale):
+    mixer = {"heads": heads, "kv_heads": kv, "dim": dim, "vdim": vdim, "scale": scale, "rot": {"dims": 4, "base": 100.0}}
+    if size:
+        mixer["mask"] = {"size": size}
+    cfg = md.fidatar_config(64, 96, [("attention", mixer, None)], alpha=0.5, scale=2.0, softcap=None)
+    w = md.fidatar_random(cfg, 5)
+    eng = E.Engine(md.write_model_dir(str(tmp_path / "m"), cfg, w), 1024)
+    toks = np.random.default_rng(2).integers(0, 64, size=600).astype(np.uint32)
+    ref = F.forward(cfg, w, toks)
+    s = eng.seq_open()
+    one = np.concatenate([eng.step(s, toks[i:i + 1], [0]) for i in range(toks.size)])
+    eng.seq_close(s)
+    for cuts in ([600], [127, 129, 128, 130], [128, 256, 1, 215], [40, 300, 260], [513, 64]):
+        s, at, out = eng.seq_open(), 0, []
+        for n in cuts:
+            out.append(eng.step(s, toks[at:at + n], range(len(toks[at:at + n]))))
+            at += n
+        eng.seq_close(s)
+        got = np.concatenate(out)
+        d = np.sqrt(((got - one[:at]) ** 2).mean(-1) / (one[:at] ** 2).mean(-1))
+        assert d.max() < 1.2e-2, (cuts, int(d.argmax()))
+        assert np.linalg.norm(got - ref[:at]) < 2e-2 * np.linalg.norm(ref[:at]), cuts
+    eng.close()
