@@ -100,7 +100,7 @@ struct Layer {
     float *yx_b = nullptr, *conv = nullptr, *conv_b = nullptr, *gates_b = nullptr, *lam = nullptr;
     // latent attention
     uint32_t H = 0, dim = 0, vdim = 0, R = 0, QR = 0; float scale = 0.0f;
-    Weight dqkv, uq, ukT, uv;
+    Weight dqkv, uq, ukT, uv, ukv;      // ukv: [keys' | values' up-projection], for portions that multiply the latents out
     float *dq_norm = nullptr, *dkv_norm = nullptr;
     // latent attention with direct queries (QR == 0): proj = [q | down-projection | gate]; RD rotated key columns beside the latent
     // (rot_dims of them turn, table rot_tab), RS the length of a cache row, window (kAttnNoWindow: causal), sink per head (optional),
@@ -212,6 +212,7 @@ struct LayeredEngine : nb::EngineBase {
     void *samp_ws = nullptr; size_t samp_cub = 0; uint32_t *samp_host = nullptr;
     TcState tc;              // products of long portions on the tensor cores' own memory (layered_tc.cu)
     nb::TcAttnState ta;      // and their attention (attn_tc.cu)
+    float *b_kv = nullptr; size_t kv_floats = 0;      // keys and values multiplied out of the latents
     std::vector<void *> allocs;
 };
 
@@ -329,6 +330,8 @@ int load_rglru(Loader &ld, const nb::Json *m, const std::string &p, Layer *L, ui
     return ld.stacked({p + "o"}, {E}, C, &L->o);
 }
 
+// whether long portions can multiply the latents out to keys and values (mix_latent_attn): shapes of attn_tc.cu, no key columns beside the latent
+bool latent_up(const LayeredEngine *e, const Layer &L) { return !e->f32 && !L.RD && L.dim <= 128u && L.vdim <= 128u && ((L.dim | L.vdim) & 3u) == 0 && L.R % 8u == 0; }
 int load_latent_attn(Loader &ld, const nb::Json *m, const std::string &p, Layer *L, uint32_t E) {
     double sc;
     if (!u32_of(m, "heads", &L->H) || !u32_of(m, "dim", &L->dim) || !u32_of(m, "vdim", &L->vdim) || !u32_of(m, "kv_rank", &L->R) || !u32_of(m, "q_rank", &L->QR) ||
@@ -346,6 +349,7 @@ int load_latent_attn(Loader &ld, const nb::Json *m, const std::string &p, Layer 
     for (uint64_t h = 0; h < H; h++)          // [H*dim, R] -> per head [R, dim]: absorbed query = q_h W_uk,h
         for (uint64_t dd = 0; dd < D; dd++)
             for (uint64_t k = 0; k < R; k++) t[(h * R + k) * D + dd] = uk[(h * D + dd) * R + k];
+    if (latent_up(ld.e, *L) && (r = ld.stacked({p + "uk", p + "uv"}, {H * D, H * VD}, R, &L->ukv))) return r;
     return ld.put_w(t, (uint32_t)(H * R), (uint32_t)D, &L->ukT);
 }
 
@@ -686,6 +690,7 @@ int load_latent_attn_direct(Loader &ld, const nb::Json *m, const std::string &p,
     for (uint64_t h = 0; h < H; h++)          // [H*dim, R] -> per head [R, dim]: absorbed query = q_h W_uk,h
         for (uint64_t dd = 0; dd < D; dd++)
             for (uint64_t k = 0; k < R; k++) t[(h * R + k) * D + dd] = uk[(h * D + dd) * R + k];
+    if (latent_up(ld.e, *L) && (r = ld.stacked({p + "uk", p + "uv"}, {H * D, H * VD}, R, &L->ukv))) return r;
     return ld.put_w(t, (uint32_t)(H * R), (uint32_t)D, &L->ukT);
 }
 
@@ -965,6 +970,9 @@ int attn_optin(int smem) {
 // ---------------- mixers: e->hm [T][E] -> e->d [T][E], from the cache pages and the state slot of the sequence ----------------
 struct Ctx { float *st; const uint32_t *table; uint32_t T, pos0; const uint32_t *pos_ptr; };
 
+constexpr uint64_t kTcAttnWork = 128 * 128;      // tokens x keys, or keys, from which a portion's grouped-query attention goes to the tensor cores
+constexpr uint32_t kTcAttnKeys = 512, kTcLatentKeys = 128;      // ... and keys from which latents are multiplied out
+
 int mix_rglru(LayeredEngine *e, const Layer &L, const Run &run, const Ctx &cx) {
     const uint32_t E = e->E, T = cx.T; float *st = cx.st; int r;
     const uint32_t C = L.C, bs = C / L.blocks;
@@ -996,6 +1004,20 @@ int mix_rglru(LayeredEngine *e, const Layer &L, const Run &run, const Ctx &cx) {
 int mix_latent_attn(LayeredEngine *e, const Layer &L, const Run &run, const Ctx &cx) {
     const uint32_t E = e->E, T = cx.T, pos0 = cx.pos0; const uint32_t *table = cx.table, *pos_ptr = cx.pos_ptr; int r;
     const uint32_t H = L.H, R = L.R, QR = L.QR, RS = L.RS;
+    // Long portions multiply the latents out: keys and values of every position in sight, in 32-bit precision, then attention over head sizes instead of
+    // the latent's rank.  Per token and key that is 2 (dim + vdim) multiply-adds a head instead of 4 R, for 3 R (dim + vdim) a head and key
+    // once: the larger part of a short portion, but the absorbed kernel has a block per 4 or 8 queries then, which walks the keys alone (8 tokens behind
+    // 2000, four layers of 16 heads: 4283 us; 64 tokens with the keys multiplied out: 1369).
+    const uint32_t QW0 = H * (L.dim + L.RD);
+    nb::TcAttn ta{};
+    ta.q = QR ? e->b_q : e->b_z; ta.ldq = QR ? H * L.dim : QW0 + R + L.RD + (L.has_gate ? H * L.vdim : 0u); ta.q_head = L.dim;
+    ta.k = e->b_kv; ta.v = e->b_kv ? e->b_kv + H * L.dim : nullptr; ta.ldk = ta.ldv = H * (L.dim + L.vdim); ta.k_head = L.dim; ta.v_head = L.vdim;
+    ta.out = e->b_ov; ta.T = T; ta.H = ta.G = H; ta.D = L.dim; ta.VD = L.vdim; ta.pos0 = pos0; ta.window = L.window < kAttnNoWindow ? L.window : 0u; ta.scale = L.scale; ta.sink = L.sink;
+    if (!QR && L.has_gate) { ta.mul = e->b_z + QW0 + R; ta.ldm = ta.ldq; }
+    ta.first_row = nb::attn_tc_first(ta);
+    const uint32_t seen = pos0 + T - ta.first_row;
+    const bool up = L.ukv.p && T > kGemvMaxM && seen >= kTcLatentKeys && (size_t)seen * ta.ldk <= e->kv_floats && nb::attn_tc_fits(&e->ta, ta) &&
+                    tc_split_fits(&e->tc, H * (L.dim + L.vdim), R, seen, L.ukv.p, run.cache, RS);
     GemmArgs g{};      // absorb: qa[t][h][0..R) = q[t][h] W_uk,h
     g.W = L.ukT.p; g.ldw = L.dim; g.C = e->b_qa; g.ldc = H * RS; g.M = T; g.N = R; g.K = L.dim;
     g.a_gmod = H; g.c_gcols = RS; g.w_gstride = (uint64_t)R * L.dim;
@@ -1013,7 +1035,7 @@ int mix_latent_attn(LayeredEngine *e, const Layer &L, const Run &run, const Ctx 
             if ((r = gemm(e, plain(e->b_cq, QR, L.uq, e->b_q, H * L.dim, T), 1, T))) return r;
         }
         g.A = e->b_q; g.lda = H * L.dim; g.a_gcols = L.dim;
-        if ((r = gemm(e, g, H, T))) return r;
+        if (!up && (r = gemm(e, g, H, T))) return r;
     } else {
         // one product gives [q | down-projection | gate]; the latent's norm, both rotations and the cache write are one kernel, for
         // short portions the last block of the absorb product
@@ -1025,7 +1047,13 @@ int mix_latent_attn(LayeredEngine *e, const Layer &L, const Run &run, const Ctx 
             ga.g.round_a = e->f32 ? 0u : 1u;
             const dim3 grid(gemv_blocks(e, g.N, H), H), block(256);
             if ((r = e->f32 ? launch<GemvLatentRopeArgs>(e, k_gemv_latent_rope<float>, grid, block, 0, ga) : launch<GemvLatentRopeArgs>(e, k_gemv_latent_rope<__nv_bfloat16>, grid, block, 0, ga))) return r;
-        } else if ((r = launch<LatentRopeArgs>(e, k_latent_rope, dim3(T), dim3(128), 0, ra)) || (r = gemm(e, g, H, T))) return r;
+        } else if ((r = launch<LatentRopeArgs>(e, k_latent_rope, dim3(T), dim3(128), 0, ra)) || (!up && (r = gemm(e, g, H, T)))) return r;
+    }
+    if (up) {
+        e->launches += 4;
+        if ((r = tc_gemm_split(&e->tc, run.cache, table, RS, ta.first_row, seen, L.ukv.p, H * (L.dim + L.vdim), R, e->b_kv, H * (L.dim + L.vdim), e->cur, e->use_pdl)) ||
+            (r = nb::attn_tc_launch(&e->ta, ta, e->cur, e->use_pdl))) return r;
+        return gemm(e, plain(e->b_ov, H * L.vdim, L.o, e->d, E, T), 1, T);
     }
     AttnArgs aa{e->b_qa, run.cache, table, e->b_ol, e->b_part, T, H, R, pos0, 1u, L.scale, pos_ptr, e->b_tick, RS - R, L.window, L.sink};
     if (T <= kGemvMaxM) {      // short portions: the key pages in sight are dealt out to several blocks (two pages each at least)
@@ -1360,7 +1388,6 @@ template <int VJ>
 int gqa_attn_launch(LayeredEngine *e, const GqaArgs &a) {
     return launch<GqaArgs>(e, k_gqa_attn<VJ>, dim3((a.T * (a.H / a.G) + kGqaM - 1u) / kGqaM, a.G), dim3(256), gqa_attn_smem(a.D, VJ), a);
 }
-constexpr uint64_t kTcAttnWork = 128 * 128;      // tokens x keys from which a portion's attention goes to the tensor cores
 uint32_t gqa_hb(const Layer &L) { return std::min(L.H / L.G, kGqaHeads); }
 // from the rows of the joint product (q, k, v from column 0) to dst [T][E]
 int gqa_branch(LayeredEngine *e, const Layer &L, const Run &run, const Ctx &cx, float *dst) {
@@ -1385,8 +1412,10 @@ int gqa_branch(LayeredEngine *e, const Layer &L, const Run &run, const Ctx &cx, 
         ta.q = e->b_p; ta.ldq = P; ta.q_head = D; ta.k = run.cache; ta.v = run.cache + G * D; ta.ldk = ta.ldv = L.RL; ta.k_head = D; ta.v_head = VD; ta.table = cx.table;
         ta.out = e->b_a; ta.T = T; ta.H = H; ta.G = G; ta.D = D; ta.VD = VD; ta.pos0 = cx.pos0; ta.block = L.block_size; ta.scale = 1.0f; ta.softcap = L.softcap; ta.sink = L.sink;
         if (L.has_gate) { ta.gate = e->b_p + L.c_hg; ta.ldg = P; }
-        // its two launches cost some 20 us however little there is to do: 5 x 8 (tokens x keys) 20 us against 11, 128 x 128 equal, 333 x 410 36 against 60
-        if (nb::attn_tc_fits(&e->ta, ta) && (uint64_t)T * (cx.pos0 + T - nb::attn_tc_first(ta)) >= kTcAttnWork) {
+        // its two launches cost some 20 us however little there is to do: 5 x 8 (tokens x keys) 20 us against 11, 128 x 128 equal, 333 x 410 36 against 60; a
+        // few tokens behind many keys are few blocks of the fp32 kernel, each of which walks the keys 64 at a time
+        const uint32_t seen = cx.pos0 + T - nb::attn_tc_first(ta);
+        if (nb::attn_tc_fits(&e->ta, ta) && ((uint64_t)T * seen >= kTcAttnWork || seen >= kTcAttnKeys)) {
             e->launches += 2;
             if ((r = nb::attn_tc_launch(&e->ta, ta, e->cur, e->use_pdl))) return r;
             return gemm(e, plain(e->b_a, H * VD, L.o, dst, e->E, T), 1, T);
@@ -2572,6 +2601,15 @@ int create(LayeredEngine *e, const nb::ModelDir *dir, uint32_t max_tokens) {
         const uint32_t keys = e->n_pages * kPage;
         for (const Layer &L : e->layers)
             if (L.type == MIX_ATTN_DELTA || L.type == MIX_GQA) { bytes = std::max(bytes, nb::attn_tc_bytes(keys, L.G, L.dim, L.vdim)); tiles = std::max(tiles, nb::attn_tc_tiles(keys, L.G)); }
+        size_t kv = 0, planes = 0;
+        for (const Layer &L : e->layers)
+            if (L.ukv.p) {
+                const size_t row = (size_t)L.H * (L.dim + L.vdim), n = std::min<size_t>(keys, ((size_t)1 << 28) / row);
+                kv = std::max(kv, n * row); planes = std::max(planes, n * tc_split_width(L.R));
+                bytes = std::max(bytes, nb::attn_tc_bytes((uint32_t)n, L.H, L.dim, L.vdim)); tiles = std::max(tiles, nb::attn_tc_tiles((uint32_t)n, L.H));
+            }
+        e->kv_floats = kv;
+        if (kv) { DM(e->b_kv, kv * 4); if ((r = tc_split_setup(&e->tc, planes))) return r; }
         if ((r = tc_setup(&e->tc, std::max<size_t>(T, kWantBatch) * ((w + 7u) & ~(size_t)7u), (uint32_t)e->num_sms)) ||
             (r = nb::attn_tc_setup(&e->ta, std::min<size_t>(bytes, (size_t)1 << 30), tiles, e->tc.err_dev))) return r;
     }

@@ -50,9 +50,40 @@ __global__ void __launch_bounds__(256) k_rows_bf16(const RowsArgs a) {
     }
 }
 
+struct PlaneArgs { const float *cache; const uint32_t *table; uint32_t ld, first, rows, K, Kp; __nv_bfloat16 *dst; };
+// dst[r] = [x3 | x2 | x1], x = x1 + x2 + x3 to 2^-26: the small parts first, so that the sum's large part is added last; each part padded to Kp with zeros
+__global__ void __launch_bounds__(256) k_rows_split(const PlaneArgs a) {
+    pdl_enter();
+    const uint32_t k8 = a.Kp >> 3;
+    const size_t total = (size_t)a.rows * k8;
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
+        const uint32_t r = (uint32_t)(i / k8), c = (uint32_t)(i % k8) * 8u, j = a.first + r;
+        const float *s = a.cache + ((size_t)a.table[j / 32u] * 32u + j % 32u) * a.ld + c;
+        float v[8];
+#pragma unroll
+        for (uint32_t q = 0; q < 2; q++) {          // K is a multiple of 8
+            const float4 p = c < a.K ? *reinterpret_cast<const float4 *>(s + 4u * q) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            v[4 * q] = p.x; v[4 * q + 1] = p.y; v[4 * q + 2] = p.z; v[4 * q + 3] = p.w;
+        }
+#pragma unroll
+        for (int part = 2; part >= 0; part--) {
+            uint4 o;
+            __nv_bfloat162 *ob = reinterpret_cast<__nv_bfloat162 *>(&o);
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                ob[q] = __floats2bfloat162_rn(v[2 * q], v[2 * q + 1]);
+                const float2 b = __bfloat1622float2(ob[q]);
+                v[2 * q] -= b.x; v[2 * q + 1] -= b.y;
+            }
+            *reinterpret_cast<uint4 *>(a.dst + (size_t)r * 3u * a.Kp + part * a.Kp + c) = o;
+        }
+    }
+}
+
 // g: the product (A and a_rows unused: the rows are in `amap`, gathered); wmap: [groups][N][K], amap: [rows][a_gmod][K], boxes of 128 weight rows / TN
-// tokens x 64; ks: blocks of a cluster that share one tile's depth (grid.z = groups * ks)
-struct alignas(64) TcArgs { CUtensorMap wmap, amap; GemmArgs g; uint32_t ks; uint32_t *err; };
+// tokens x 64; ks: blocks of a cluster that share one tile's depth (grid.z = groups * ks); wsteps: the stages after which W starts over (rows in several
+// parts; the whole depth otherwise)
+struct alignas(64) TcArgs { CUtensorMap wmap, amap; GemmArgs g; uint32_t ks, wsteps; uint32_t *err; };
 
 // Epilogue of NJ tokens of one output column: every option is looked at once for the NJ values (inside the loop over tokens the switch alone made a
 // tile's epilogue 44 instructions per value, most of them instruction-cache misses: 1024 x 2048 x 128 took 38 us, the same as at a depth of
@@ -152,14 +183,14 @@ __global__ void __launch_bounds__(192) k_gemm_tc(const __grid_constant__ TcArgs 
     pdl_launch_next();
     const uint32_t tmem = tmem_s, npre = a.g_off ? 0u : min(ST, ns);
     if (warp == 0 && lane == 0)          // weights do not depend on the kernel before: their first tiles are on the way while it ends
-        for (uint32_t i = 0; i < npre; i++) { mbar_expect(full + i * 8u, SB); tma_3d(ring + i * SB, &ta.wmap, (s0 + i) * kTcK, n0, group, full + i * 8u); }
+        for (uint32_t i = 0; i < npre; i++) { mbar_expect(full + i * 8u, SB); tma_3d(ring + i * SB, &ta.wmap, (s0 + i) % ta.wsteps * kTcK, n0, group, full + i * 8u); }
     pdl_wait();
     const GroupView gv = group_view(a, group);
     if (warp == 0 && lane == 0) {
         for (uint32_t i = 0; i < ns; i++) {
             const uint32_t st = i % ST, bar = full + st * 8u, dst = ring + st * SB;
             if (i >= ST && !mbar_wait(empty + st * 8u, ((i / ST) - 1u) & 1u)) { bad_s = 1; break; }
-            if (i >= npre) { mbar_expect(bar, SB); tma_3d(dst, &ta.wmap, (s0 + i) * kTcK, n0, group, bar); }
+            if (i >= npre) { mbar_expect(bar, SB); tma_3d(dst, &ta.wmap, (s0 + i) % ta.wsteps * kTcK, n0, group, bar); }
             tma_3d(dst + kTcRows * kTcK * 2u, &ta.amap, (s0 + i) * kTcK, group % a.a_gmod, gv.r0 + m0, bar);
         }
     } else if (warp == 1 && lane == 0) {
@@ -282,6 +313,8 @@ int tc_setup(TcState *t, size_t elems, uint32_t sms) {
 }
 void tc_free(TcState *t) {
     for (auto &p : t->rows) { if (p) cudaFree(p); p = nullptr; }
+    if (t->planes) cudaFree(t->planes);
+    t->planes = nullptr;
     if (t->err_host) cudaFreeHost(t->err_host);
     t->err_host = nullptr; t->encode = nullptr;
 }
@@ -315,11 +348,33 @@ int tc_gemm(TcState *t, GemmArgs a, uint32_t groups, uint32_t maxM, uint32_t row
     const uint32_t tiles = (a.N + kTcRows - 1u) / kTcRows * ((each + tn - 1u) / tn) * groups, steps = (a.K + kTcK - 1u) / kTcK;
     uint32_t ks = 1;
     while (ks < 8u && tiles * ks * 10u <= t->sms * 7u && steps >= ks * 4u) ks *= 2u;
-    ta.ks = ks;
+    ta.ks = ks; ta.wsteps = steps;
     const dim3 grid((a.N + kTcRows - 1u) / kTcRows, (maxM + tn - 1u) / tn, groups * ks), block(192);
     if (tn == 32) return launch<TcArgs>(k_gemm_tc<32>, grid, block, tc_smem(32), stream, pdl, ta, ks);
     if (tn == 64) return launch<TcArgs>(k_gemm_tc<64>, grid, block, tc_smem(64), stream, pdl, ta, ks);
     return launch<TcArgs>(k_gemm_tc<128>, grid, block, tc_smem(128), stream, pdl, ta, ks);
+}
+
+int tc_split_setup(TcState *t, size_t elems) {
+    if (cudaMalloc(&t->planes, elems * 2) != cudaSuccess) return fail(NB200_ENOMEM, "cudaMalloc(%zu) failed", elems * 2);
+    t->plane_elems = elems;
+    return 0;
+}
+bool tc_split_fits(const TcState *t, uint32_t N, uint32_t K, uint32_t rows, const void *W, const float *cache, uint32_t ld) {
+    return t->encode && t->planes && N && K % 8u == 0 && ld % 4u == 0 && ((reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(cache)) & 15u) == 0 && (size_t)rows * tc_split_width(K) <= t->plane_elems;
+}
+int tc_gemm_split(TcState *t, const float *cache, const uint32_t *table, uint32_t ld, uint32_t first, uint32_t rows, const void *W, uint32_t N, uint32_t K, float *C, uint32_t ldc, cudaStream_t stream, bool pdl) {
+    const uint32_t width = tc_split_width(K);
+    int r;
+    const PlaneArgs pa{cache, table, ld, first, rows, K, width / 3u, t->planes};
+    const size_t threads = (size_t)rows * (width / 24u);
+    if ((r = launch<PlaneArgs>(k_rows_split, dim3((uint32_t)((threads + 255u) / 256u < t->sms * 16u ? (threads + 255u) / 256u : t->sms * 16u)), dim3(256), 0, stream, pdl, pa))) return r;
+    TcArgs ta{};
+    ta.g.C = C; ta.g.ldc = ldc; ta.g.M = rows; ta.g.N = N; ta.g.K = width; ta.g.a_gmod = 1;
+    ta.err = t->err_dev; ta.ks = 1; ta.wsteps = width / 3u / kTcK;
+    if (!tensor_map(t, &ta.wmap, W, K, N, 1, (uint64_t)K * 2u, (uint64_t)K * 2u * N, kTcK, kTcRows, 1) || !tensor_map(t, &ta.amap, t->planes, width, 1, rows, (uint64_t)width * 2u, (uint64_t)width * 2u, kTcK, 1, 128))
+        return fail(NB200_ECUDA, "cuTensorMapEncodeTiled refused a product of %u x %u x %u", rows, N, width);
+    return launch<TcArgs>(k_gemm_tc<128>, dim3((N + kTcRows - 1u) / kTcRows, (rows + 127u) / 128u, 1), dim3(192), tc_smem(128), stream, pdl, ta);
 }
 
 }  // namespace lm
