@@ -1,0 +1,473 @@
+// prefill.cu -- the prompt of a model file in portions of up to 1024 positions (F32 and Q80 files, one GPU, fast mode).
+//
+// A decode step streams every weight for one position; here a weight tile meets 64 or 128 positions.  The arithmetic is the decode path's: RMS norm and
+// Q80 activation codes by the same expressions, exact integer group dots, their fp32 terms summed per group; only the order of fp32 sums
+// differs, as it does between the decode paths.  What a prompt leaves behind is its K and V rows, so the last layer stops there.
+//
+//   k_prompt_embed     token rows
+//   k_prompt_prep      a position's activation: RMS norm with gain, plain, or SwiGLU of interleaved pairs; then Q80 codes + group scales, or
+//                      (F32) two f16 parts of the row scaled by a power of two
+//   k_prompt_gemm      C[t][n] (+)= sum over groups: tcgen05.mma on 128 weight rows x TN positions, the accumulator of a GROUP in tensor memory (two
+//                      buffers), added to fp32 registers by the threads that own the rows while the next group multiplies.
+//                      Q80: kind::i8, int32 exact, times weight scale x activation scale.  F32: kind::f16 on two parts of both
+//                      operands (small x large, large x small, large x large: 2^-23 of a product) over 128 of the depth; the
+//                      tensor cores' own additions stay that short.
+//   k_prompt_rope      head norm (Qwen3), rotary positions, K and V rows into the cache
+//   attention          attn_tc.cu
+#include "prefill.h"
+
+#include <cuda_fp16.h>
+
+#include <algorithm>
+
+#include "family.h"
+#define NB_K static
+#include "kernels.cuh"
+#include "tc_ptx.cuh"
+
+namespace nb {
+namespace {
+
+constexpr uint32_t kChunk = 1024, kRows = 128;
+enum { PREP_NORM = 0, PREP_PLAIN = 1, PREP_SWIGLU = 2 };
+
+__device__ __forceinline__ void dep_enter() { asm volatile("griddepcontrol.launch_dependents;\ngriddepcontrol.wait;" ::: "memory"); }
+
+struct PromptEmbedArgs { const void *w, *aux; float *x; const uint32_t *ids; uint32_t E, gs, quant; };
+__global__ void __launch_bounds__(256) k_prompt_embed(const PromptEmbedArgs a) {
+    dep_enter();
+    const size_t tok = a.ids[blockIdx.x];
+    float *x = a.x + (size_t)blockIdx.x * a.E;
+    for (uint32_t i = threadIdx.x; i < a.E; i += 256u) {
+        if (a.quant == 0x00u) x[i] = static_cast<const float *>(a.w)[tok * a.E + i];
+        else x[i] = __fmul_rn((float)static_cast<const int8_t *>(a.w)[tok * a.E + i], static_cast<const float *>(a.aux)[(tok * a.E + i) / a.gs]);
+    }
+}
+
+// codes [T][n] and scales [n / gs][lds] (Q80), or parts [T][2][np] and the inverse of the row's scale (F32)
+struct PromptPrepArgs { const float *src; uint32_t ld; const float *gain; uint32_t n, gs, mode; int8_t *codes; float *scales; uint32_t lds; __half *parts; uint32_t np; float *rinv; };
+__device__ __forceinline__ float prep_value(const PromptPrepArgs &a, const float *s, float inv, uint32_t i) {
+    if (a.mode == PREP_NORM) return __fmul_rn(a.gain[i], __fmul_rn(inv, s[i]));
+    if (a.mode == PREP_PLAIN) return s[i];
+    const float2 v = *reinterpret_cast<const float2 *>(s + 2u * i);
+    return __fmul_rn(__fmul_rn(v.x, __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-v.x)))), v.y);
+}
+// a power of two that brings `big` to [2^14, 2^15)
+__device__ __forceinline__ float power_scale(float big) {
+    const int e = (int)(__float_as_uint(big) >> 23) - 127;
+    if (!(big > 0.0f) || e > 127) return 1.0f;
+    return __uint_as_float((uint32_t)(127 + max(-113, min(100, 14 - e))) << 23);
+}
+template <bool Q80>
+__global__ void __launch_bounds__(256) k_prompt_prep(const PromptPrepArgs a) {
+    dep_enter();
+    __shared__ float red[32];
+    extern __shared__ float val[];
+    const uint32_t t = blockIdx.x, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const float *s = a.src + (size_t)t * a.ld;
+    float inv = 1.0f;
+    if (a.mode == PREP_NORM) {
+        float acc = 0.0f;
+        for (uint32_t i = threadIdx.x; i < a.n; i += 256u) acc = fmaf(s[i], s[i], acc);
+        acc = block_sum<256>(acc, red);
+        inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(acc, (float)a.n), 1e-5f)));
+    }
+    if (Q80) {
+        const uint32_t G = a.n / a.gs, epl = a.gs / 32u;      // gs in {32, 64, 128, 256}
+        for (uint32_t g = warp; g < G; g += 8u) {
+            float v[8], amax = 0.0f;
+#pragma unroll
+            for (uint32_t j = 0; j < 8; j++) if (j < epl) { v[j] = prep_value(a, s, inv, g * a.gs + j * 32u + lane); amax = fmaxf(amax, fabsf(v[j])); }
+            amax = warp_max(amax);
+            const float sc = __fdiv_rn(amax, 127.0f), rinv = __frcp_rn(sc);
+#pragma unroll
+            for (uint32_t j = 0; j < 8; j++) if (j < epl) a.codes[(size_t)t * a.n + g * a.gs + j * 32u + lane] = (int8_t)((sc == 0.0f) ? 0 : q80_code(v[j], sc, rinv));
+            if (lane == 0) a.scales[(size_t)g * a.lds + t] = sc;
+        }
+    } else {
+        float m = 0.0f;
+        for (uint32_t i = threadIdx.x; i < a.n; i += 256u) { const float v = prep_value(a, s, inv, i); val[i] = v; m = fmaxf(m, fabsf(v)); }
+        m = block_max<256>(m, red);
+        const float sc = power_scale(m);
+        __half *hi = a.parts + (size_t)t * 2u * a.np, *lo = hi + a.np;
+        for (uint32_t i = threadIdx.x; i < a.np; i += 256u) {
+            const float v = i < a.n ? val[i] * sc : 0.0f;
+            const __half h = __float2half_rn(v);
+            hi[i] = h; lo[i] = __float2half_rn(v - __half2float(h));
+        }
+        if (threadIdx.x == 0) a.rinv[t] = 1.0f / sc;
+    }
+}
+
+// F32 weights: the largest magnitude (as float bits), then two f16 parts [rows][2][np] under one scale for the matrix
+__global__ void k_weight_max(const float *w, size_t n, uint32_t *bits) {
+    float m = 0.0f;
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) m = fmaxf(m, fabsf(w[i]));
+    m = warp_max(m);
+    if ((threadIdx.x & 31u) == 0) atomicMax(bits, __float_as_uint(m));
+}
+__global__ void k_weight_parts(const float *w, uint32_t rows, uint32_t n, uint32_t np, const uint32_t *bits, __half *parts, float *inv) {
+    const float sc = power_scale(__uint_as_float(*bits));
+    const size_t total = (size_t)rows * np;
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
+        const uint32_t r = (uint32_t)(i / np), c = (uint32_t)(i % np);
+        const float v = c < n ? w[(size_t)r * n + c] * sc : 0.0f;
+        const __half h = __float2half_rn(v);
+        parts[(size_t)r * 2u * np + c] = h; parts[(size_t)r * 2u * np + np + c] = __float2half_rn(v - __half2float(h));
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) *inv = 1.0f / sc;
+}
+
+// add: C += (the residual stream), else C =
+struct alignas(64) PromptGemmArgs {
+    CUtensorMap wmap, amap; const float *ws, *xs; uint32_t ldx; const float *winv, *xinv;
+    uint32_t N, T, n, gs, np; float *C; uint32_t ldc, add; uint32_t *err;
+};
+__device__ __forceinline__ void tma_2d(uint32_t dst, const CUtensorMap *map, uint32_t x, uint32_t y, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void tc_mma_i8(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, bool add) {
+    asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n}" ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"((uint32_t)add) : "memory");
+}
+// a stage holds 128 bytes of the depth of 128 weight rows and TN positions: 128 int8, or 64 f16 of both parts
+template <bool Q80, int TN> __host__ __device__ constexpr uint32_t gemm_stage() { return (kRows + (uint32_t)TN) * 128u * (Q80 ? 1u : 2u); }
+template <bool Q80, int TN> __host__ __device__ constexpr uint32_t gemm_stages() { return Q80 ? (TN == 64 ? 4u : 6u) : (TN == 64 ? 4u : 3u); }
+template <bool Q80, int TN> constexpr size_t gemm_smem() { return (size_t)gemm_stages<Q80, TN>() * gemm_stage<Q80, TN>() + 1024u; }
+
+template <bool Q80, int TN>
+__global__ void __launch_bounds__(192, Q80 && TN == 64 ? 2 : 1) k_prompt_gemm(const __grid_constant__ PromptGemmArgs a) {
+    constexpr uint32_t ST = gemm_stages<Q80, TN>(), SB = gemm_stage<Q80, TN>(), WB = kRows * 128u, XB = TN * 128u;
+    extern __shared__ uint8_t tc_raw[];
+    __shared__ __align__(8) uint64_t bars[2 * ST + 4];
+    __shared__ uint32_t tmem_s, bad_s;
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, ring = (smem_u32(tc_raw) + 1023u) & ~1023u;
+    const uint32_t n0 = blockIdx.x * kRows, m0 = blockIdx.y * TN;
+    const uint32_t full = smem_u32(bars), empty = full + ST * 8u, tfull = empty + ST * 8u, tfree = tfull + 16u;
+    const uint32_t steps = Q80 ? (a.n + 127u) / 128u : a.np / 64u;
+    // groups: the depth that one tensor-memory accumulator takes before it is added up in fp32
+    const uint32_t groups = Q80 ? a.n / a.gs : (steps + 1u) / 2u;
+    if (threadIdx.x == 0) {
+        for (uint32_t i = 0; i < ST; i++) { mbar_init(full + i * 8u, 1); mbar_init(empty + i * 8u, 1); }
+        for (uint32_t i = 0; i < 2; i++) { mbar_init(tfull + i * 8u, 1); mbar_init(tfree + i * 8u, 4); }
+        bad_s = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) { tc_alloc(smem_u32(&tmem_s), 2 * TN); tc_relinquish(); }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    // Only now may the next kernels' blocks come: one that waits for this grid while it holds tensor memory must not be in the way of an allocation here
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const uint32_t tmem = tmem_s, npre = min(ST, steps);
+    auto weights = [&](uint32_t i) {
+        const uint32_t dst = ring + (i % ST) * SB, bar = full + (i % ST) * 8u;
+        mbar_expect(bar, SB);
+        if (Q80) tma_2d(dst, &a.wmap, i * 128u, n0, bar);
+        else { tma_2d(dst, &a.wmap, i * 64u, n0, bar); tma_2d(dst + WB, &a.wmap, a.np + i * 64u, n0, bar); }
+    };
+    if (warp == 0 && lane == 0) for (uint32_t i = 0; i < npre; i++) weights(i);          // weights do not depend on the kernel before
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (warp == 0 && lane == 0) {
+        for (uint32_t i = 0; i < steps; i++) {
+            const uint32_t st = i % ST, bar = full + st * 8u, dst = ring + st * SB + (Q80 ? WB : 2u * WB);
+            if (i >= ST && !mbar_wait(empty + st * 8u, ((i / ST) - 1u) & 1u)) { bad_s = 1; break; }
+            if (i >= npre) weights(i);
+            if (Q80) tma_2d(dst, &a.amap, i * 128u, m0, bar);
+            else { tma_2d(dst, &a.amap, i * 64u, m0, bar); tma_2d(dst + XB, &a.amap, a.np + i * 64u, m0, bar); }
+        }
+    } else if (warp == 1 && lane == 0) {
+        constexpr uint32_t shape = ((uint32_t)(TN >> 3) << 17) | ((kRows >> 4) << 24);
+        constexpr uint32_t idesc = Q80 ? ((2u << 4) | (1u << 7) | (1u << 10) | shape) : ((1u << 4) | shape);          // int32 += int8 x int8; fp32 += f16 x f16
+        bool ok = true;
+        uint32_t gi = 0;
+        auto open = [&]() { const bool w = gi < 2u || mbar_wait(tfree + (gi & 1u) * 8u, ((gi >> 1) - 1u) & 1u); tc_fence_after(); return w; };
+        auto close = [&]() { tc_commit(tfull + (gi & 1u) * 8u); gi++; };
+        for (uint32_t i = 0; i < steps && ok; i++) {
+            ok = mbar_wait(full + (i % ST) * 8u, (i / ST) & 1u);
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t base = ring + (i % ST) * SB;
+            if (Q80) {
+                const uint64_t wd = tc_desc(base), xd = tc_desc(base + WB);
+                const uint32_t depth = min(128u, a.n - i * 128u);
+                if (a.gs >= 128u) {
+                    const uint32_t per = a.gs / 128u, at = i % per;          // stages of a group
+                    if (at == 0 && !(ok = open())) break;
+                    for (uint32_t k = 0; k < depth / 32u; k++) tc_mma_i8(tmem + (gi & 1u) * TN, wd + 2u * k, xd + 2u * k, idesc, at > 0 || k > 0);
+                    if (at + 1u == per) close();
+                } else {
+                    const uint32_t per = a.gs / 32u;
+                    for (uint32_t k0 = 0; k0 < depth / 32u && ok; k0 += per) {
+                        if (!(ok = open())) break;
+                        for (uint32_t k = 0; k < per; k++) tc_mma_i8(tmem + (gi & 1u) * TN, wd + 2u * (k0 + k), xd + 2u * (k0 + k), idesc, k > 0);
+                        close();
+                    }
+                }
+            } else {
+                if ((i & 1u) == 0 && !(ok = open())) break;
+                const uint32_t xb = base + 2u * WB, d = tmem + (gi & 1u) * TN;
+#pragma unroll
+                for (uint32_t p = 0; p < 3; p++)          // small x large, large x small, large x large
+#pragma unroll
+                    for (uint32_t k = 0; k < 4; k++)
+                        tc_mma_ss(d, tc_desc(base + (p == 0 ? WB : 0u)) + 2u * k, tc_desc(xb + (p == 1 ? XB : 0u)) + 2u * k, idesc, (i & 1u) || p > 0 || k > 0);
+                if ((i & 1u) || i + 1u == steps) close();
+            }
+            if (ok) tc_commit(empty + (i % ST) * 8u);
+        }
+        if (!ok) bad_s = 2;
+    } else if (warp >= 2) {
+        const uint32_t quad = warp & 3u, n = n0 + quad * 32u + lane, nr = min(n, a.N - 1u), lanes = (quad * 32u) << 16;
+        float acc[TN];
+#pragma unroll
+        for (int j = 0; j < TN; j++) acc[j] = 0.0f;
+        bool ok = true;
+        const float *ws = Q80 ? a.ws + (size_t)nr * groups : nullptr;
+        float w_next = Q80 ? __ldg(ws) : 1.0f;
+        for (uint32_t g = 0; g < groups; g++) {
+            const float w = w_next;
+            if (Q80 && g + 1u < groups) w_next = __ldg(ws + g + 1u);
+            const float *xs = Q80 ? a.xs + (size_t)g * a.ldx + m0 : nullptr;
+            ok = __all_sync(0xffffffffu, mbar_wait(tfull + (g & 1u) * 8u, (g >> 1) & 1u));
+            if (!ok) break;
+            tc_fence_after();
+#pragma unroll
+            for (int c = 0; c < TN; c += 32) {
+                uint32_t v[32];
+                tc_ld32(tmem + lanes + (g & 1u) * TN + c, v);
+#pragma unroll
+                for (int j = 0; j < 32; j += 4) {
+                    if (Q80) {
+                        const float4 x = __ldcg(reinterpret_cast<const float4 *>(xs + c + j));
+                        acc[c + j] = fmaf((float)(int)v[j], w * x.x, acc[c + j]); acc[c + j + 1] = fmaf((float)(int)v[j + 1], w * x.y, acc[c + j + 1]);
+                        acc[c + j + 2] = fmaf((float)(int)v[j + 2], w * x.z, acc[c + j + 2]); acc[c + j + 3] = fmaf((float)(int)v[j + 3], w * x.w, acc[c + j + 3]);
+                    } else {
+#pragma unroll
+                        for (int q = 0; q < 4; q++) acc[c + j + q] += __uint_as_float(v[j + q]);
+                    }
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(tfree + (g & 1u) * 8u);
+        }
+        if (!ok) bad_s = 3;
+        else if (n < a.N) {
+            const float wi = Q80 ? 1.0f : *a.winv;
+            float *dst = a.C + (size_t)m0 * a.ldc + n;
+            const uint32_t live = min((uint32_t)TN, a.T - m0);
+#pragma unroll
+            for (int j = 0; j < TN; j++) {
+                if ((uint32_t)j < live) {
+                    const float v = Q80 ? acc[j] : acc[j] * (wi * __ldcg(a.xinv + m0 + j));
+                    dst[(size_t)j * a.ldc] = a.add ? dst[(size_t)j * a.ldc] + v : v;
+                }
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (bad_s) {
+        if (threadIdx.x == 0) {
+            *a.err = 0x300u + bad_s;
+            __threadfence_system();
+            const long long t0 = clock64();
+            while (clock64() - t0 < 20000000ll) __nanosleep(1000);          // copies still in flight land in this block's shared memory before it is given back
+        }
+        __syncthreads();
+    }
+    if (warp == 1) tc_dealloc(tmem, 2 * TN);
+}
+
+// head norm (Qwen3) and rotary positions of the rows [q | k | v] of a portion: q to its own buffer, k and v into the cache rows of their positions
+struct PromptRopeArgs { const float *p; uint32_t ld, H, KV, pos0; float *q, *kc, *vc; const float *qn, *kn, *cos_, *sin_; Dims d; };
+__global__ void __launch_bounds__(256) k_prompt_rope(const PromptRopeArgs a) {
+    dep_enter();
+    __shared__ float buf[8][128];
+    const uint32_t t = blockIdx.x, pos = a.pos0 + t, hd = a.d.hd, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const float *row = a.p + (size_t)t * a.ld, *cr = a.cos_ + (size_t)pos * (hd / 2u), *ci = a.sin_ + (size_t)pos * (hd / 2u);
+    for (uint32_t h = warp; h < a.H + 2u * a.KV; h += 8u) {
+        const bool isq = h < a.H, isk = !isq && h < a.H + a.KV;
+        const uint32_t g = isq ? 0u : (h - a.H) % a.KV;
+        float *dst = isq ? a.q + (size_t)t * a.H * hd + (size_t)h * hd : (isk ? a.kc : a.vc) + ((size_t)g * a.d.max_seq + pos) * hd;
+        for (uint32_t i = lane; i < hd; i += 32u) buf[warp][i] = row[(size_t)h * hd + i];
+        __syncwarp();
+        if (isq || isk) head_norm_rope(buf[warp], isq ? a.qn : a.kn, cr, ci, a.d, false);
+        for (uint32_t i = lane; i < hd; i += 32u) dst[i] = buf[warp][i];
+        __syncwarp();
+    }
+}
+
+template <typename A>
+int launch(void (*k)(const A), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, const A &args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr; cfg.numAttrs = 1;
+    NB_CK(cudaLaunchKernelEx(&cfg, k, args));
+    return 0;
+}
+template <bool Q80, int TN>
+int optin() { NB_CK(cudaFuncSetAttribute((const void *)k_prompt_gemm<Q80, TN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_smem<Q80, TN>())); return 0; }
+}  // namespace
+
+struct Product { PrefillMat m; CUtensorMap wmap; const float *winv = nullptr; uint32_t np = 0; };      // np: F32 depth padded to 64
+struct PrefillState {
+    PrefillModel m; uint32_t sms = 148;
+    decltype(&cuTensorMapEncodeTiled) encode = nullptr;
+    std::vector<Product> qkv, wo, w13, w2;
+    float *x = nullptr, *p = nullptr, *q = nullptr, *o = nullptr;      // residual rows, products, turned queries, attention output
+    unsigned char *act = nullptr; float *scales = nullptr;             // codes or parts; group scales [G][kChunk] or row scales
+    struct AMap { uint32_t n, tn; CUtensorMap map; };
+    std::vector<AMap> amaps;
+    TcAttnState attn; uint32_t *err_host = nullptr, *err_dev = nullptr;
+    std::vector<void *> allocs;
+};
+
+namespace {
+int dmalloc(PrefillState *s, void **p, size_t bytes) {
+    if (cudaMalloc(p, bytes ? bytes : 16) != cudaSuccess) return fail(NB200_ENOMEM, "cudaMalloc(%zu) failed", bytes);
+    s->allocs.push_back(*p);
+    return 0;
+}
+#define PM(ptr, bytes) do { int r_ = dmalloc(s, (void **)&(ptr), (bytes)); if (r_) return r_; } while (0)
+bool map_2d(const PrefillState *s, CUtensorMap *m, bool q80, const void *base, uint64_t width, uint64_t rows, uint32_t box) {
+    const cuuint64_t dims[2] = {width, rows}, strides[1] = {width * (q80 ? 1u : 2u)};
+    const cuuint32_t b[2] = {q80 ? 128u : 64u, box}, step[2] = {1, 1};
+    return s->encode(m, q80 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(base), dims, strides, b, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                     CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+int add_product(PrefillState *s, std::vector<Product> *list, const PrefillMat &m) {
+    Product p;
+    p.m = m;
+    const bool q80 = s->m.quant == 0x80u;
+    const void *base = m.w;
+    uint32_t width = m.n;
+    if (!q80) {
+        p.np = (m.n + 63u) & ~63u; width = 2u * p.np;
+        __half *parts = nullptr; uint32_t *bits = nullptr; float *inv = nullptr;
+        PM(parts, (size_t)m.rows * width * 2u); PM(bits, 16); PM(inv, 16);
+        NB_CK(cudaMemset(bits, 0, 16));
+        k_weight_max<<<s->sms * 8u, 256>>>(static_cast<const float *>(m.w), (size_t)m.rows * m.n, bits);
+        k_weight_parts<<<s->sms * 8u, 256>>>(static_cast<const float *>(m.w), m.rows, m.n, p.np, bits, parts, inv);
+        NB_CK(cudaGetLastError());
+        base = parts; p.winv = inv;
+    }
+    if (!map_2d(s, &p.wmap, q80, base, width, m.rows, kRows)) return fail(NB200_ECUDA, "cuTensorMapEncodeTiled refused a matrix of %u x %u", m.rows, m.n);
+    list->push_back(p);
+    return 0;
+}
+int create(PrefillState *s, const PrefillModel &m) {
+    const bool q80 = m.quant == 0x80u;
+    void *fn = nullptr;
+    cudaDriverEntryPointQueryResult got;
+    NB_CK(cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &got));
+    if (got != cudaDriverEntryPointSuccess || !fn) return fail(NB200_ECUDA, "the driver has no cuTensorMapEncodeTiled");
+    s->encode = reinterpret_cast<decltype(s->encode)>(fn);
+    int r;
+    for (uint32_t l = 0; l < m.L; l++) {
+        if ((r = add_product(s, &s->qkv, m.qkv[l]))) return r;
+        if (l + 1u < m.L && ((r = add_product(s, &s->wo, m.wo[l])) || (r = add_product(s, &s->w13, m.w13[l])) || (r = add_product(s, &s->w2, m.w2[l])))) return r;
+    }
+    const uint32_t C = std::min(kChunk, (m.max_seq + 127u) & ~127u), wide = std::max(std::max(m.E, m.q_dim), m.F);
+    PM(s->x, (size_t)C * m.E * 4); PM(s->p, (size_t)C * std::max(m.q_dim + 2 * m.kv_dim, 2 * m.F) * 4); PM(s->q, (size_t)C * m.q_dim * 4); PM(s->o, (size_t)C * m.q_dim * 4);
+    const size_t act = (size_t)C * (q80 ? wide : ((wide + 63u) & ~63u) * 4u), scales = q80 ? (size_t)(wide / m.gs) * kChunk : (size_t)kChunk;
+    PM(s->act, act); PM(s->scales, scales * 4);
+    NB_CK(cudaMemset(s->act, 0, act)); NB_CK(cudaMemset(s->scales, 0, scales * 4));
+    for (uint32_t n : {m.E, m.q_dim, m.F})
+        for (uint32_t tn : {64u, 128u}) {
+            PrefillState::AMap a{n, tn, {}};
+            if (!map_2d(s, &a.map, q80, s->act, q80 ? n : 2u * ((n + 63u) & ~63u), C, tn)) return fail(NB200_ECUDA, "cuTensorMapEncodeTiled refused rows of %u", n);
+            s->amaps.push_back(a);
+        }
+    NB_CK(cudaHostAlloc(&s->err_host, 64, cudaHostAllocMapped));
+    *s->err_host = 0;
+    NB_CK(cudaHostGetDevicePointer(&s->err_dev, s->err_host, 0));
+    if ((r = attn_tc_setup(&s->attn, std::min<size_t>(attn_tc_bytes(m.max_seq, m.KV, m.hd, m.hd), (size_t)1 << 30), attn_tc_tiles(m.max_seq, m.KV), s->err_dev))) return r;
+    if (q80 ? ((r = optin<true, 64>()) || (r = optin<true, 128>())) : ((r = optin<false, 64>()) || (r = optin<false, 128>()))) return r;
+    if (!q80 && (size_t)wide * 4u > 48u * 1024u) NB_CK(cudaFuncSetAttribute((const void *)k_prompt_prep<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(wide * 4u)));
+    NB_CK(cudaDeviceSynchronize());
+    return 0;
+}
+int prep(PrefillState *s, const float *src, uint32_t ld, const float *gain, uint32_t n, uint32_t mode, uint32_t T, cudaStream_t stream) {
+    PromptPrepArgs a{src, ld, gain, n, s->m.gs, mode, reinterpret_cast<int8_t *>(s->act), s->scales, kChunk, reinterpret_cast<__half *>(s->act), (n + 63u) & ~63u, s->scales};
+    return s->m.quant == 0x80u ? launch<PromptPrepArgs>(k_prompt_prep<true>, dim3(T), dim3(256), 0, stream, a) : launch<PromptPrepArgs>(k_prompt_prep<false>, dim3(T), dim3(256), (size_t)n * 4, stream, a);
+}
+int product(PrefillState *s, const Product &w, float *C, uint32_t ldc, bool add, uint32_t T, cudaStream_t stream) {
+    // 64 positions per tile where tiles of 128 leave SMs without a block (1024 rows of the O product: 8 blocks for 128 positions)
+    const uint32_t rt = (w.m.rows + kRows - 1u) / kRows, tn = T <= 64u || rt * ((T + 127u) / 128u) < s->sms ? 64u : 128u;
+    PromptGemmArgs a{};
+    a.wmap = w.wmap;
+    for (const auto &m : s->amaps) if (m.n == w.m.n && m.tn == tn) a.amap = m.map;
+    a.ws = static_cast<const float *>(w.m.aux); a.xs = s->scales; a.ldx = kChunk; a.winv = w.winv; a.xinv = s->scales;
+    a.N = w.m.rows; a.T = T; a.n = w.m.n; a.gs = s->m.gs; a.np = w.np; a.C = C; a.ldc = ldc; a.add = add ? 1u : 0u; a.err = s->err_dev;
+    const dim3 grid(rt, (T + tn - 1u) / tn), block(192);
+    if (s->m.quant == 0x80u)
+        return tn == 64u ? launch<PromptGemmArgs>(k_prompt_gemm<true, 64>, grid, block, gemm_smem<true, 64>(), stream, a) : launch<PromptGemmArgs>(k_prompt_gemm<true, 128>, grid, block, gemm_smem<true, 128>(), stream, a);
+    return tn == 64u ? launch<PromptGemmArgs>(k_prompt_gemm<false, 64>, grid, block, gemm_smem<false, 64>(), stream, a) : launch<PromptGemmArgs>(k_prompt_gemm<false, 128>, grid, block, gemm_smem<false, 128>(), stream, a);
+}
+}  // namespace
+
+int prefill_create(PrefillState **out, const PrefillModel &m, uint32_t sms) {
+    *out = nullptr;
+    const bool q80 = m.quant == 0x80u;
+    if (!q80 && m.quant != 0x00u) return 0;
+    if (q80 && (m.gs != 32u && m.gs != 64u && m.gs != 128u && m.gs != 256u)) return 0;
+    if (m.hd > 128u || m.hd % 4u || m.E % 8u || m.q_dim % 8u || m.F % 8u || m.q_dim != m.H * m.hd || m.kv_dim != m.KV * m.hd || m.H % m.KV || std::max(std::max(m.E, m.q_dim), m.F) > 32768u) return 0;
+    if (q80 && (m.E % 16u || m.q_dim % 16u || m.F % 16u || m.E % m.gs || m.q_dim % m.gs || m.F % m.gs)) return 0;
+    PrefillState *s = new PrefillState();
+    s->m = m; s->sms = sms;
+    const int r = create(s, m);
+    if (r) { prefill_destroy(s); return r; }
+    *out = s;
+    return 0;
+}
+void prefill_destroy(PrefillState *s) {
+    if (!s) return;
+    attn_tc_free(&s->attn);
+    for (void *p : s->allocs) cudaFree(p);
+    if (s->err_host) cudaFreeHost(s->err_host);
+    delete s;
+}
+int prefill_check(PrefillState *s) {
+    if (!s || !s->err_host || !*static_cast<volatile uint32_t *>(s->err_host)) return 0;
+    const uint32_t code = *s->err_host;
+    *s->err_host = 0;
+    return fail(NB200_ECUDA, "a wait inside a prompt kernel ran out (code 0x%x): the results of this call are not valid", code);
+}
+int prefill_run(PrefillState *s, const uint32_t *ids, uint32_t n, cudaStream_t stream, uint64_t *launches) {
+    const PrefillModel &m = s->m;
+    const uint32_t W = m.q_dim + 2 * m.kv_dim;
+    const size_t kvl = (size_t)m.KV * m.max_seq * m.hd;
+    Dims d{};
+    d.arch = m.arch; d.hd = m.hd; d.max_seq = m.max_seq;
+    int r;
+    for (uint32_t p0 = 0; p0 < n; p0 += kChunk) {
+        const uint32_t T = std::min(kChunk, n - p0);
+        if ((r = launch<PromptEmbedArgs>(k_prompt_embed, dim3(T), dim3(256), 0, stream, PromptEmbedArgs{m.emb.w, m.emb.aux, s->x, ids + p0, m.E, m.gs, m.quant}))) return r;
+        (*launches)++;
+        for (uint32_t l = 0; l < m.L; l++) {
+            const PromptRopeArgs ra{s->p, W, m.H, m.KV, p0, s->q, m.kc + l * kvl, m.vc + l * kvl, m.qnorm ? m.qnorm + (size_t)l * m.hd : nullptr, m.knorm ? m.knorm + (size_t)l * m.hd : nullptr, m.rope_cos, m.rope_sin, d};
+            if ((r = prep(s, s->x, m.E, m.norm_attn + (size_t)l * m.E, m.E, PREP_NORM, T, stream)) || (r = product(s, s->qkv[l], s->p, W, false, T, stream)) ||
+                (r = launch<PromptRopeArgs>(k_prompt_rope, dim3(T), dim3(256), 0, stream, ra))) return r;
+            *launches += 3;
+            if (l + 1u == m.L) break;          // nothing reads what the last layer would make of these positions
+            TcAttn a{};
+            a.q = s->q; a.ldq = m.q_dim; a.q_head = m.hd; a.k = m.kc + l * kvl; a.v = m.vc + l * kvl; a.ldk = a.ldv = m.hd; a.k_head = a.v_head = (uint64_t)m.max_seq * m.hd;
+            a.out = s->o; a.T = T; a.H = m.H; a.G = m.KV; a.D = a.VD = m.hd; a.pos0 = p0; a.scale = (float)(1.0 / sqrt((double)m.hd));
+            if (!attn_tc_fits(&s->attn, a)) return fail(NB200_EINVAL, "a prompt of %u positions does not fit the attention's buffers", n);
+            if ((r = attn_tc_launch(&s->attn, a, stream, true)) || (r = prep(s, s->o, m.q_dim, nullptr, m.q_dim, PREP_PLAIN, T, stream)) || (r = product(s, s->wo[l], s->x, m.E, true, T, stream)) ||
+                (r = prep(s, s->x, m.E, m.norm_ffn + (size_t)l * m.E, m.E, PREP_NORM, T, stream)) || (r = product(s, s->w13[l], s->p, 2 * m.F, false, T, stream)) ||
+                (r = prep(s, s->p, 2 * m.F, nullptr, m.F, PREP_SWIGLU, T, stream)) || (r = product(s, s->w2[l], s->x, m.E, true, T, stream))) return r;
+            *launches += 8;
+        }
+    }
+    return 0;
+}
+// whether a prompt of n positions fits
+bool prefill_fits(const PrefillState *s, uint32_t n) { return s && attn_tc_bytes(n, s->m.KV, s->m.hd, s->m.hd) <= s->attn.bytes; }
+
+}  // namespace nb
