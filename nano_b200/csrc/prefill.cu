@@ -10,8 +10,8 @@
 //   k_prompt_gemm      C[t][n] (+)= sum over groups: tcgen05.mma on 128 weight rows x TN positions, the accumulator of a GROUP in tensor memory (two
 //                      buffers), added to fp32 registers by the threads that own the rows while the next group multiplies.
 //                      Q80: kind::i8, int32 exact, times weight scale x activation scale.  F32: kind::f16 on two parts of both
-//                      operands (small x large, large x small, large x large: 2^-23 of a product) over 128 of the depth; the
-//                      tensor cores' own additions stay that short.
+//                      operands (small x large, large x small, large x large: 2^-23 of a product) over 64 of the depth; the
+//                      tensor cores cut what they add, so their own additions stay that short.
 //   k_prompt_rope      head norm (Qwen3), rotary positions, K and V rows into the cache
 //   attention          attn_tc.cu
 #include "prefill.h"
@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(192, Q80 && TN == 64 ? 2 : 1) k_prompt_gemm(co
     const uint32_t full = smem_u32(bars), empty = full + ST * 8u, tfull = empty + ST * 8u, tfree = tfull + 16u;
     const uint32_t steps = Q80 ? (a.n + 127u) / 128u : a.np / 64u;
     // groups: the depth that one tensor-memory accumulator takes before it is added up in fp32
-    const uint32_t groups = Q80 ? a.n / a.gs : (steps + 1u) / 2u;
+    const uint32_t groups = Q80 ? a.n / a.gs : steps;
     if (threadIdx.x == 0) {
         for (uint32_t i = 0; i < ST; i++) { mbar_init(full + i * 8u, 1); mbar_init(empty + i * 8u, 1); }
         for (uint32_t i = 0; i < 2; i++) { mbar_init(tfull + i * 8u, 1); mbar_init(tfree + i * 8u, 4); }
@@ -204,14 +204,14 @@ __global__ void __launch_bounds__(192, Q80 && TN == 64 ? 2 : 1) k_prompt_gemm(co
                     }
                 }
             } else {
-                if ((i & 1u) == 0 && !(ok = open())) break;
+                if (!(ok = open())) break;
                 const uint32_t xb = base + 2u * WB, d = tmem + (gi & 1u) * TN;
 #pragma unroll
                 for (uint32_t p = 0; p < 3; p++)          // small x large, large x small, large x large
 #pragma unroll
                     for (uint32_t k = 0; k < 4; k++)
-                        tc_mma_ss(d, tc_desc(base + (p == 0 ? WB : 0u)) + 2u * k, tc_desc(xb + (p == 1 ? XB : 0u)) + 2u * k, idesc, (i & 1u) || p > 0 || k > 0);
-                if ((i & 1u) || i + 1u == steps) close();
+                        tc_mma_ss(d, tc_desc(base + (p == 0 ? WB : 0u)) + 2u * k, tc_desc(xb + (p == 1 ? XB : 0u)) + 2u * k, idesc, p > 0 || k > 0);
+                close();
             }
             if (ok) tc_commit(empty + (i % ST) * 8u);
         }

@@ -1,0 +1,72 @@
+"""Prompts of model files in portions (csrc/prefill.cu): the K and V rows and the next logits against the same positions one call at a time, at the
+edges of the kernels' tiles (64 and 128 positions, 1024 to a portion, rows of weights that no tile of 128 divides) and for every group size.
+
+Bounds.  The rows of layer 0 come from the same activation codes (Q80) or the same rounding-free products (F32): 32-bit sums in another order,
+2e-6 of a row's norm.  Deeper Q80 rows and the logits: a change in the last place turns a code here and there, which settles at 1 to
+2 % after two to four layers whatever its size; 4e-2.  F32 logits: 1e-5."""
+import dataclasses
+
+import numpy as np
+import pytest
+
+from nano_b200 import engine as E, modelfile as mf
+
+pytestmark = pytest.mark.gpu
+
+
+def rel(a, b):
+    return float(np.linalg.norm(a - b) / np.linalg.norm(b))
+
+
+def rows(eng, spec, layer, pos):
+    return np.concatenate([eng.read(E.F_KROW, spec.kv_dim, layer, pos), eng.read(E.F_VROW, spec.kv_dim, layer, pos)])
+
+
+CASES = [("toy-nano", mf.QUANT_F32, 128), ("toy-qwen3", mf.QUANT_F32, 128), ("toy-nano", mf.QUANT_Q80, 32), ("toy-qwen3", mf.QUANT_Q80, 64), ("toy-nano", mf.QUANT_Q80, 128), ("toy-nano", mf.QUANT_Q80, 256),
+         ("mini-qwen3", mf.QUANT_Q80, 128), ("mini-nano", mf.QUANT_F32, 128), ("toy-nano-odd", mf.QUANT_F32, 128)]
+
+
+@pytest.mark.parametrize("name,quant,gs", CASES)
+def test_portions_against_single_positions(name, quant, gs):
+    spec = dataclasses.replace(mf.PRESETS[name], name=name + "-prompts", block_size=2048)
+    eng = E.Engine(mf.cached_model(spec, quant, gs), 1200)
+    toks = mf.teacher_tokens(1160, spec.vocab)
+    lengths = (33, 65, 129, 130, 257) if name != "toy-qwen3" else (34, 64, 1025, 1154)
+    n = max(lengths)
+    last, want, keep = spec.n_layer - 1, {}, {}
+    for p in range(n):
+        eng.forward_nolog(int(toks[p]), p)
+        if p + 1 in lengths:
+            want[p + 1] = eng.logits()
+    at = lambda m: (0, 1, m // 2, m - 2)          # noqa: E731
+    for m in lengths:
+        for p in at(m):
+            keep[p] = [rows(eng, spec, l, p) for l in (0, last)]
+    tol = 1e-5 if quant == mf.QUANT_F32 else 4e-2
+    for m in lengths:
+        ids = np.zeros(m + 2, np.uint32)
+        ids[:33] = toks[:33][::-1]
+        eng.decode_greedy(ids, 33, 34)          # leaves rows of another prompt behind
+        ids[:m] = toks[:m]
+        eng.decode_greedy(ids, m, m + 1)
+        assert rel(eng.logits(), want[m]) < tol, m
+        for p in at(m):
+            assert rel(rows(eng, spec, 0, p), keep[p][0]) < 2e-6, (m, p)
+            assert rel(rows(eng, spec, last, p), keep[p][1]) < tol, (m, p)
+    eng.close()
+
+
+def test_penalty_sees_the_prompt_and_short_prompts_stay_as_they_were():
+    spec = dataclasses.replace(mf.PRESETS["toy-nano"], name="toy-nano-prompts", block_size=2048)
+    path = mf.cached_model(spec, mf.QUANT_F32, 128, cls_gain=4.0)
+    eng = E.Engine(path, 200)
+    toks = mf.teacher_tokens(64, spec.vocab)
+    for n in (20, 64):
+        a = np.zeros(101, np.uint32)
+        a[:n] = toks[:n]
+        b = a.copy()
+        for pos in range(99):
+            a[pos + 1] = eng.next_greedy(a, pos, 1 if pos < n - 1 else 0, 1.3)
+        eng.decode_greedy(b, n, 100, 1.3)
+        assert a[:100].tolist() == b[:100].tolist(), n
+    eng.close()
