@@ -1234,7 +1234,7 @@ static int nano_next_sampled(nb200_engine *e, const uint32_t *ids, uint32_t pos,
     return 0;
 }
 
-constexpr uint32_t kPortionMin = 32;
+constexpr uint32_t kPortionMin = 8;
 
 static int nano_decode_greedy(nb200_engine *e, uint32_t *ids, uint32_t n_prompt, uint32_t n_total, float penalty,
                         float *prefill_ms, float *device_ms) {
