@@ -58,8 +58,9 @@ __device__ __forceinline__ float power_scale(float big) {
     if (!(big > 0.0f) || e > 127) return 1.0f;
     return __uint_as_float((uint32_t)(127 + max(-113, min(100, 14 - e))) << 23);
 }
+constexpr uint32_t kPrepThreads = 512;
 template <bool Q80>
-__global__ void __launch_bounds__(256) k_prompt_prep(const PromptPrepArgs a) {
+__global__ void __launch_bounds__(kPrepThreads) k_prompt_prep(const PromptPrepArgs a) {
     dep_enter();
     __shared__ float red[32];
     extern __shared__ float val[];
@@ -68,13 +69,13 @@ __global__ void __launch_bounds__(256) k_prompt_prep(const PromptPrepArgs a) {
     float inv = 1.0f;
     if (a.mode == PREP_NORM) {
         float acc = 0.0f;
-        for (uint32_t i = threadIdx.x; i < a.n; i += 256u) acc = fmaf(s[i], s[i], acc);
-        acc = block_sum<256>(acc, red);
+        for (uint32_t i = threadIdx.x; i < a.n; i += kPrepThreads) acc = fmaf(s[i], s[i], acc);
+        acc = block_sum<kPrepThreads>(acc, red);
         inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(acc, (float)a.n), 1e-5f)));
     }
     if (Q80) {
         const uint32_t G = a.n / a.gs, epl = a.gs / 32u;      // gs in {32, 64, 128, 256}
-        for (uint32_t g = warp; g < G; g += 8u) {
+        for (uint32_t g = warp; g < G; g += kPrepThreads / 32u) {
             float v[8], amax = 0.0f;
 #pragma unroll
             for (uint32_t j = 0; j < 8; j++) if (j < epl) { v[j] = prep_value(a, s, inv, g * a.gs + j * 32u + lane); amax = fmaxf(amax, fabsf(v[j])); }
@@ -86,11 +87,11 @@ __global__ void __launch_bounds__(256) k_prompt_prep(const PromptPrepArgs a) {
         }
     } else {
         float m = 0.0f;
-        for (uint32_t i = threadIdx.x; i < a.n; i += 256u) { const float v = prep_value(a, s, inv, i); val[i] = v; m = fmaxf(m, fabsf(v)); }
-        m = block_max<256>(m, red);
+        for (uint32_t i = threadIdx.x; i < a.n; i += kPrepThreads) { const float v = prep_value(a, s, inv, i); val[i] = v; m = fmaxf(m, fabsf(v)); }
+        m = block_max<kPrepThreads>(m, red);
         const float sc = power_scale(m);
         __half *hi = a.parts + (size_t)t * 2u * a.np, *lo = hi + a.np;
-        for (uint32_t i = threadIdx.x; i < a.np; i += 256u) {
+        for (uint32_t i = threadIdx.x; i < a.np; i += kPrepThreads) {
             const float v = i < a.n ? val[i] * sc : 0.0f;
             const __half h = __float2half_rn(v);
             hi[i] = h; lo[i] = __float2half_rn(v - __half2float(h));
@@ -139,7 +140,9 @@ __global__ void __launch_bounds__(192, Q80 && TN == 64 ? 2 : 1) k_prompt_gemm(co
     constexpr uint32_t ST = gemm_stages<Q80, TN>(), SB = gemm_stage<Q80, TN>(), WB = kRows * 128u, XB = TN * 128u;
     extern __shared__ uint8_t tc_raw[];
     __shared__ __align__(8) uint64_t bars[2 * ST + 4];
-    __shared__ uint32_t tmem_s, bad_s;
+    __shared__ uint32_t tmem_s;
+    __shared__ volatile uint32_t bad_s;
+    __shared__ __align__(16) float xs_s[Q80 ? 3 : 1][TN];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, ring = (smem_u32(tc_raw) + 1023u) & ~1023u;
     const uint32_t n0 = blockIdx.x * kRows, m0 = blockIdx.y * TN;
     const uint32_t full = smem_u32(bars), empty = full + ST * 8u, tfull = empty + ST * 8u, tfree = tfull + 16u;
@@ -222,14 +225,25 @@ __global__ void __launch_bounds__(192, Q80 && TN == 64 ? 2 : 1) k_prompt_gemm(co
 #pragma unroll
         for (int j = 0; j < TN; j++) acc[j] = 0.0f;
         bool ok = true;
+        // the scales of a group are fetched two groups ahead: the row's own into a register, the positions' into shared memory (a global load per group
+        // between a full accumulator and its sums cost 2.5 us a group: 250 x 1024 x 3072 took 62 us)
         const float *ws = Q80 ? a.ws + (size_t)nr * groups : nullptr;
-        float w_next = Q80 ? __ldg(ws) : 1.0f;
+        const uint32_t et = threadIdx.x - 64u;
+        auto weight_scale = [&](uint32_t g) { return Q80 && g < groups ? __ldg(ws + g) : 0.0f; };
+        auto act_scale = [&](uint32_t g) { return Q80 && g < groups && et < (uint32_t)TN ? __ldcg(a.xs + (size_t)g * a.ldx + m0 + et) : 0.0f; };
+        auto meet = []() { asm volatile("bar.sync 1, 128;" ::: "memory"); };
+        float w0 = weight_scale(0), w1 = weight_scale(1);
+        if (Q80) {
+            const float x0 = act_scale(0), x1 = act_scale(1);
+            if (et < (uint32_t)TN) { xs_s[0][et] = x0; xs_s[1][et] = x1; }
+            meet();
+        }
+        uint32_t slot = 0;
         for (uint32_t g = 0; g < groups; g++) {
-            const float w = w_next;
-            if (Q80 && g + 1u < groups) w_next = __ldg(ws + g + 1u);
-            const float *xs = Q80 ? a.xs + (size_t)g * a.ldx + m0 : nullptr;
+            const float w = w0, x2 = act_scale(g + 2u);
+            w0 = w1; w1 = weight_scale(g + 2u);
             ok = __all_sync(0xffffffffu, mbar_wait(tfull + (g & 1u) * 8u, (g >> 1) & 1u));
-            if (!ok) break;
+            if (!ok) bad_s = 3;          // (the warps stay together for the barrier below; what they add up is not used)
             tc_fence_after();
 #pragma unroll
             for (int c = 0; c < TN; c += 32) {
@@ -238,7 +252,7 @@ __global__ void __launch_bounds__(192, Q80 && TN == 64 ? 2 : 1) k_prompt_gemm(co
 #pragma unroll
                 for (int j = 0; j < 32; j += 4) {
                     if (Q80) {
-                        const float4 x = __ldcg(reinterpret_cast<const float4 *>(xs + c + j));
+                        const float4 x = *reinterpret_cast<const float4 *>(&xs_s[slot][c + j]);
                         acc[c + j] = fmaf((float)(int)v[j], w * x.x, acc[c + j]); acc[c + j + 1] = fmaf((float)(int)v[j + 1], w * x.y, acc[c + j + 1]);
                         acc[c + j + 2] = fmaf((float)(int)v[j + 2], w * x.z, acc[c + j + 2]); acc[c + j + 3] = fmaf((float)(int)v[j + 3], w * x.w, acc[c + j + 3]);
                     } else {
@@ -250,19 +264,29 @@ __global__ void __launch_bounds__(192, Q80 && TN == 64 ? 2 : 1) k_prompt_gemm(co
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(tfree + (g & 1u) * 8u);
+            if (Q80) {
+                if (et < (uint32_t)TN) xs_s[slot == 0 ? 2 : slot - 1][et] = x2;          // the buffer of the group before this one
+                meet();
+                slot = slot == 2 ? 0 : slot + 1;
+                ok = bad_s == 0;
+            }
+            if (!ok) break;
         }
         if (!ok) bad_s = 3;
         else if (n < a.N) {
             const float wi = Q80 ? 1.0f : *a.winv;
             float *dst = a.C + (size_t)m0 * a.ldc + n;
             const uint32_t live = min((uint32_t)TN, a.T - m0);
+            if (!Q80) {
 #pragma unroll
-            for (int j = 0; j < TN; j++) {
-                if ((uint32_t)j < live) {
-                    const float v = Q80 ? acc[j] : acc[j] * (wi * __ldcg(a.xinv + m0 + j));
-                    dst[(size_t)j * a.ldc] = a.add ? dst[(size_t)j * a.ldc] + v : v;
-                }
+                for (int j = 0; j < TN; j++) acc[j] *= wi * __ldcg(a.xinv + m0 + j);
             }
+            if (a.add) {          // all loads before the first store: one after the other they were 30 us of a product
+#pragma unroll
+                for (int j = 0; j < TN; j++) if ((uint32_t)j < live) acc[j] += __ldcg(dst + (size_t)j * a.ldc);
+            }
+#pragma unroll
+            for (int j = 0; j < TN; j++) if ((uint32_t)j < live) dst[(size_t)j * a.ldc] = acc[j];
         }
     }
     tc_fence_before();
@@ -394,7 +418,7 @@ int create(PrefillState *s, const PrefillModel &m) {
 }
 int prep(PrefillState *s, const float *src, uint32_t ld, const float *gain, uint32_t n, uint32_t mode, uint32_t T, cudaStream_t stream) {
     PromptPrepArgs a{src, ld, gain, n, s->m.gs, mode, reinterpret_cast<int8_t *>(s->act), s->scales, kChunk, reinterpret_cast<__half *>(s->act), (n + 63u) & ~63u, s->scales};
-    return s->m.quant == 0x80u ? launch<PromptPrepArgs>(k_prompt_prep<true>, dim3(T), dim3(256), 0, stream, a) : launch<PromptPrepArgs>(k_prompt_prep<false>, dim3(T), dim3(256), (size_t)n * 4, stream, a);
+    return s->m.quant == 0x80u ? launch<PromptPrepArgs>(k_prompt_prep<true>, dim3(T), dim3(kPrepThreads), 0, stream, a) : launch<PromptPrepArgs>(k_prompt_prep<false>, dim3(T), dim3(kPrepThreads), (size_t)n * 4, stream, a);
 }
 int product(PrefillState *s, const Product &w, float *C, uint32_t ldc, bool add, uint32_t T, cudaStream_t stream) {
     // 64 positions per tile where tiles of 128 leave SMs without a block (1024 rows of the O product: 8 blocks for 128 positions)
