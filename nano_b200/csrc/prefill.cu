@@ -122,7 +122,7 @@ __global__ void k_weight_parts(const float *w, uint32_t rows, uint32_t n, uint32
 // add: C += (the residual stream), else C =
 struct alignas(64) PromptGemmArgs {
     CUtensorMap wmap, amap; const float *ws, *xs; uint32_t ldx; const float *winv, *xinv;
-    uint32_t N, T, n, gs, np; float *C; uint32_t ldc, add; uint32_t *err;
+    uint32_t N, T, n, gs, np; float *C; uint32_t ldc, add, ks; uint32_t *err;      // ks: blocks of a cluster (along z) that share a tile's depth
 };
 __device__ __forceinline__ void tma_2d(uint32_t dst, const CUtensorMap *map, uint32_t x, uint32_t y, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
@@ -146,9 +146,11 @@ __global__ void __launch_bounds__(192, Q80 && TN == 64 ? 2 : 1) k_prompt_gemm(co
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, ring = (smem_u32(tc_raw) + 1023u) & ~1023u;
     const uint32_t n0 = blockIdx.x * kRows, m0 = blockIdx.y * TN;
     const uint32_t full = smem_u32(bars), empty = full + ST * 8u, tfull = empty + ST * 8u, tfree = tfull + 16u;
-    const uint32_t steps = Q80 ? (a.n + 127u) / 128u : a.np / 64u;
-    // groups: the depth that one tensor-memory accumulator takes before it is added up in fp32
-    const uint32_t groups = Q80 ? a.n / a.gs : steps;
+    // this block's share of the depth, in whole units of stages and groups; groups: the depth that one tensor-memory accumulator takes before it is added
+    // up in fp32
+    const uint32_t us = Q80 && a.gs > 128u ? a.gs / 128u : 1u, units = ((Q80 ? (a.n + 127u) / 128u : a.np / 64u) + us - 1u) / us, per_part = (units + a.ks - 1u) / a.ks;
+    const uint32_t u0 = min(units, blockIdx.z * per_part), s0 = u0 * us, steps = min(per_part, units - u0) * us;
+    const uint32_t g0 = Q80 ? s0 * 128u / a.gs : s0, groups = Q80 ? min(a.n, (s0 + steps) * 128u) / a.gs - g0 : steps, all_groups = Q80 ? a.n / a.gs : 0u;
     if (threadIdx.x == 0) {
         for (uint32_t i = 0; i < ST; i++) { mbar_init(full + i * 8u, 1); mbar_init(empty + i * 8u, 1); }
         for (uint32_t i = 0; i < 2; i++) { mbar_init(tfull + i * 8u, 1); mbar_init(tfree + i * 8u, 4); }
@@ -165,18 +167,19 @@ __global__ void __launch_bounds__(192, Q80 && TN == 64 ? 2 : 1) k_prompt_gemm(co
     auto weights = [&](uint32_t i) {
         const uint32_t dst = ring + (i % ST) * SB, bar = full + (i % ST) * 8u;
         mbar_expect(bar, SB);
-        if (Q80) tma_2d(dst, &a.wmap, i * 128u, n0, bar);
-        else { tma_2d(dst, &a.wmap, i * 64u, n0, bar); tma_2d(dst + WB, &a.wmap, a.np + i * 64u, n0, bar); }
+        if (Q80) tma_2d(dst, &a.wmap, (s0 + i) * 128u, n0, bar);
+        else { tma_2d(dst, &a.wmap, (s0 + i) * 64u, n0, bar); tma_2d(dst + WB, &a.wmap, a.np + (s0 + i) * 64u, n0, bar); }
     };
     if (warp == 0 && lane == 0) for (uint32_t i = 0; i < npre; i++) weights(i);          // weights do not depend on the kernel before
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    float *mine = reinterpret_cast<float *>(tc_raw + (ring - smem_u32(tc_raw)));          // [TN][128]: a part's sums, once the ring is free
     if (warp == 0 && lane == 0) {
         for (uint32_t i = 0; i < steps; i++) {
             const uint32_t st = i % ST, bar = full + st * 8u, dst = ring + st * SB + (Q80 ? WB : 2u * WB);
             if (i >= ST && !mbar_wait(empty + st * 8u, ((i / ST) - 1u) & 1u)) { bad_s = 1; break; }
             if (i >= npre) weights(i);
-            if (Q80) tma_2d(dst, &a.amap, i * 128u, m0, bar);
-            else { tma_2d(dst, &a.amap, i * 64u, m0, bar); tma_2d(dst + XB, &a.amap, a.np + i * 64u, m0, bar); }
+            if (Q80) tma_2d(dst, &a.amap, (s0 + i) * 128u, m0, bar);
+            else { tma_2d(dst, &a.amap, (s0 + i) * 64u, m0, bar); tma_2d(dst + XB, &a.amap, a.np + (s0 + i) * 64u, m0, bar); }
         }
     } else if (warp == 1 && lane == 0) {
         constexpr uint32_t shape = ((uint32_t)(TN >> 3) << 17) | ((kRows >> 4) << 24);
@@ -192,7 +195,7 @@ __global__ void __launch_bounds__(192, Q80 && TN == 64 ? 2 : 1) k_prompt_gemm(co
             const uint32_t base = ring + (i % ST) * SB;
             if (Q80) {
                 const uint64_t wd = tc_desc(base), xd = tc_desc(base + WB);
-                const uint32_t depth = min(128u, a.n - i * 128u);
+                const uint32_t depth = min(128u, a.n - (s0 + i) * 128u);
                 if (a.gs >= 128u) {
                     const uint32_t per = a.gs / 128u, at = i % per;          // stages of a group
                     if (at == 0 && !(ok = open())) break;
@@ -227,10 +230,10 @@ __global__ void __launch_bounds__(192, Q80 && TN == 64 ? 2 : 1) k_prompt_gemm(co
         bool ok = true;
         // the scales of a group are fetched two groups ahead: the row's own into a register, the positions' into shared memory (a global load per group
         // between a full accumulator and its sums cost 2.5 us a group: 250 x 1024 x 3072 took 62 us)
-        const float *ws = Q80 ? a.ws + (size_t)nr * groups : nullptr;
+        const float *ws = Q80 ? a.ws + (size_t)nr * all_groups + g0 : nullptr;
         const uint32_t et = threadIdx.x - 64u;
         auto weight_scale = [&](uint32_t g) { return Q80 && g < groups ? __ldg(ws + g) : 0.0f; };
-        auto act_scale = [&](uint32_t g) { return Q80 && g < groups && et < (uint32_t)TN ? __ldcg(a.xs + (size_t)g * a.ldx + m0 + et) : 0.0f; };
+        auto act_scale = [&](uint32_t g) { return Q80 && g < groups && et < (uint32_t)TN ? __ldcg(a.xs + (size_t)(g0 + g) * a.ldx + m0 + et) : 0.0f; };
         auto meet = []() { asm volatile("bar.sync 1, 128;" ::: "memory"); };
         float w0 = weight_scale(0), w1 = weight_scale(1);
         if (Q80) {
@@ -273,7 +276,10 @@ __global__ void __launch_bounds__(192, Q80 && TN == 64 ? 2 : 1) k_prompt_gemm(co
             if (!ok) break;
         }
         if (!ok) bad_s = 3;
-        else if (n < a.N) {
+        else if (a.ks > 1u) {
+#pragma unroll
+            for (int j = 0; j < TN; j++) mine[j * kRows + quad * 32u + lane] = acc[j];
+        } else if (n < a.N) {
             const float wi = Q80 ? 1.0f : *a.winv;
             float *dst = a.C + (size_t)m0 * a.ldc + n;
             const uint32_t live = min((uint32_t)TN, a.T - m0);
@@ -288,6 +294,38 @@ __global__ void __launch_bounds__(192, Q80 && TN == 64 ? 2 : 1) k_prompt_gemm(co
 #pragma unroll
             for (int j = 0; j < TN; j++) if ((uint32_t)j < live) dst[(size_t)j * a.ldc] = acc[j];
         }
+    }
+    if (a.ks > 1u) {          // every block of the cluster finishes TN / ks positions: its own and its peers' parts, added in the order of the depth
+        cluster_sync_all();
+        const uint32_t quad = warp & 3u, n = n0 + quad * 32u + lane, span = TN / a.ks, j0 = blockIdx.z * span, j1 = min(j0 + span, a.T - m0);
+        if (warp >= 2 && n < a.N && !bad_s) {
+            const float wi = Q80 ? 1.0f : *a.winv;
+            const uint32_t at = smem_u32(mine + quad * 32u + lane);
+            float *dst = a.C + (size_t)m0 * a.ldc + n;
+            for (uint32_t j = j0; j < j1; j += 8u) {
+                float f[8];
+#pragma unroll
+                for (int i = 0; i < 8; i++) f[i] = 0.0f;
+#pragma unroll 2
+                for (uint32_t p = 0; p < a.ks; p++) {
+                    uint32_t peer;
+                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(at + j * kRows * 4u), "r"(p));
+#pragma unroll
+                    for (uint32_t i = 0; i < 8; i++) f[i] += ld_cluster_f32(peer + i * kRows * 4u);
+                }
+                if (!Q80) {
+#pragma unroll
+                    for (uint32_t i = 0; i < 8; i++) f[i] *= wi * __ldcg(a.xinv + m0 + j + i);
+                }
+                if (a.add) {
+#pragma unroll
+                    for (uint32_t i = 0; i < 8; i++) if (j + i < j1) f[i] += __ldcg(dst + (size_t)(j + i) * a.ldc);
+                }
+#pragma unroll
+                for (uint32_t i = 0; i < 8; i++) if (j + i < j1) dst[(size_t)(j + i) * a.ldc] = f[i];
+            }
+        }
+        cluster_sync_all();          // no block leaves while another reads its part
     }
     tc_fence_before();
     __syncthreads();
@@ -324,13 +362,15 @@ __global__ void __launch_bounds__(256) k_prompt_rope(const PromptRopeArgs a) {
 }
 
 template <typename A>
-int launch(void (*k)(const A), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, const A &args) {
+int launch(void (*k)(const A), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, const A &args, uint32_t cluster_z = 1) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr; cfg.numAttrs = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 1; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = cluster_z;
+    cfg.attrs = attr; cfg.numAttrs = cluster_z > 1u ? 2 : 1;
     NB_CK(cudaLaunchKernelEx(&cfg, k, args));
     return 0;
 }
@@ -428,10 +468,16 @@ int product(PrefillState *s, const Product &w, float *C, uint32_t ldc, bool add,
     for (const auto &m : s->amaps) if (m.n == w.m.n && m.tn == tn) a.amap = m.map;
     a.ws = static_cast<const float *>(w.m.aux); a.xs = s->scales; a.ldx = kChunk; a.winv = w.winv; a.xinv = s->scales;
     a.N = w.m.rows; a.T = T; a.n = w.m.n; a.gs = s->m.gs; a.np = w.np; a.C = C; a.ldc = ldc; a.add = add ? 1u : 0u; a.err = s->err_dev;
-    const dim3 grid(rt, (T + tn - 1u) / tn), block(192);
-    if (s->m.quant == 0x80u)
-        return tn == 64u ? launch<PromptGemmArgs>(k_prompt_gemm<true, 64>, grid, block, gemm_smem<true, 64>(), stream, a) : launch<PromptGemmArgs>(k_prompt_gemm<true, 128>, grid, block, gemm_smem<true, 128>(), stream, a);
-    return tn == 64u ? launch<PromptGemmArgs>(k_prompt_gemm<false, 64>, grid, block, gemm_smem<false, 64>(), stream, a) : launch<PromptGemmArgs>(k_prompt_gemm<false, 128>, grid, block, gemm_smem<false, 128>(), stream, a);
+    // clusters share a tile's depth while fewer than half of the SMs have a block, down to two units of 128 (Q80) or 64 (F32) each
+    const uint32_t tiles = rt * ((T + tn - 1u) / tn), units = s->m.quant == 0x80u ? w.m.n / std::max(128u, s->m.gs) : w.np / 64u;
+    uint32_t ks = 1;
+    while (ks < 8u && tiles * ks * 2u <= s->sms && units >= ks * 4u) ks *= 2u;
+    a.ks = ks;
+    const dim3 grid(rt, (T + tn - 1u) / tn, ks), block(192);
+#define GEMM(q, t) launch<PromptGemmArgs>(k_prompt_gemm<q, t>, grid, block, gemm_smem<q, t>(), stream, a, ks)
+    if (s->m.quant == 0x80u) return tn == 64u ? GEMM(true, 64) : GEMM(true, 128);
+    return tn == 64u ? GEMM(false, 64) : GEMM(false, 128);
+#undef GEMM
 }
 }  // namespace
 
