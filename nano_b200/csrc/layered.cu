@@ -201,6 +201,9 @@ struct LayeredEngine : nb::EngineBase {
     double *b_mfa = nullptr, *b_mfb = nullptr, *b_mfc = nullptr; float *b_mmt = nullptr, *b_mme = nullptr, *b_mS = nullptr, *b_mn = nullptr, *b_mo = nullptr;
     float *b_gpart = nullptr; uint32_t *b_gtick = nullptr;      // grouped-query attention: partials and tickets of the key splits
     uint32_t *ids_dev = nullptr, *want_dev = nullptr, *next_dev = nullptr, *tok_host = nullptr; uint8_t *seen = nullptr;
+    // pinned host memory that copies go through without a wait: a call's token ids and wanted places, the sequences' page tables, logits rows.
+    // Every entry point synchronises before it returns, so a call finds the first and the last free
+    uint32_t *stage_ids = nullptr, *stage_want = nullptr, *stage_pages = nullptr; float *stage_logits = nullptr; uint32_t stage_rows = 0;
     uint32_t last_T = 0;
     float alpha = 1.0f, logit_cap = 0.0f;      // norms of the sum: the residual's factor; soft cap of the logits (0: none)
     uint32_t S = 1; float res_mult = 1.0f; float *xs = nullptr;      // hyper-connected form: streams, the model's residual multiplier, the streams [S][chunk][E]
@@ -1820,6 +1823,14 @@ int decode_launches(LayeredEngine *e, uint32_t slot) {
     return head_rows(e, 1, e->zero_dev);
 }
 
+// the captured step's position and its token: one launch that carries both (two copies from pageable memory were 12 us of a 114 us step)
+int set_step(LayeredEngine *e, uint32_t pos, uint32_t token) {
+    k_set_step<<<1, 1, 0, e->stream>>>(e->ids_dev, e->dpos, pos, token);
+    CK(cudaGetLastError());
+    e->launches++;
+    return 0;
+}
+
 int decode_step(LayeredEngine *e, uint32_t slot) {
     if (!e->use_graph || e->keep) return decode_launches(e, slot);
     if (!e->graphs[slot]) {
@@ -1854,9 +1865,9 @@ int reserve_pages(LayeredEngine *e, uint32_t seq, uint32_t tokens) {
     if (e->max_pos && tokens > e->max_pos) return fail(NB200_EINVAL, "sequence %u would reach %u tokens; the model has %u positions", seq, tokens, e->max_pos);
     if (need <= have) return 0;
     if (need - have > e->free_pages.size()) return fail(NB200_ENOMEM, "the cache is full: %u tokens asked for sequence %u, %zu pages free", tokens, seq, e->free_pages.size());
-    for (size_t i = have; i < need; i++) { s.pages.push_back(e->free_pages.back()); e->free_pages.pop_back(); }
-    CK(cudaMemcpyAsync(e->table + (size_t)seq * e->n_pages + have, s.pages.data() + have, (need - have) * 4, cudaMemcpyHostToDevice, e->stream));
-    CK(cudaStreamSynchronize(e->stream));      // the source is pageable host memory owned by the vector
+    uint32_t *row = e->stage_pages + (size_t)seq * e->n_pages;
+    for (size_t i = have; i < need; i++) { s.pages.push_back(e->free_pages.back()); e->free_pages.pop_back(); row[i] = s.pages[i]; }
+    CK(cudaMemcpyAsync(e->table + (size_t)seq * e->n_pages + have, row + have, (need - have) * 4, cudaMemcpyHostToDevice, e->stream));
     return 0;
 }
 
@@ -1886,24 +1897,33 @@ int lm_seq_close(nb200_engine *h, uint32_t seq) {
 }
 
 // ---------------- step ----------------
+// the first nw rows of e->logits to the caller, and a wait for everything before them
+int fetch_logits(LayeredEngine *e, uint32_t nw, float *dst) {
+    const bool staged = nw <= e->stage_rows;
+    CK(cudaMemcpyAsync(staged ? e->stage_logits : dst, e->logits, (size_t)nw * e->V * 4, cudaMemcpyDeviceToHost, e->stream));
+    CK(cudaStreamSynchronize(e->stream));
+    if (staged) memcpy(dst, e->stage_logits, (size_t)nw * e->V * 4);
+    return 0;
+}
+
 // tokens already on the device at tok_dev[0..n); want (host, ascending, may be null) -> logits_host [n_want][V]
 int step_dev(LayeredEngine *e, uint32_t seq, const uint32_t *tok_dev, uint32_t n, const uint32_t *want, uint32_t n_want, float *logits_host) {
     int r;
     Seq &s = e->seqs[seq];
     if ((r = reserve_pages(e, seq, s.len + n))) return r;
+    if (n_want) {          // places inside their chunks
+        for (uint32_t i = 0; i < n_want; i++) e->stage_want[i] = want[i] % e->chunk_cap;
+        CK(cudaMemcpyAsync(e->want_dev, e->stage_want, (size_t)n_want * 4, cudaMemcpyHostToDevice, e->stream));
+    }
     uint32_t wi = 0;
     for (uint32_t c0 = 0; c0 < n; c0 += e->chunk_cap) {
         const uint32_t T = std::min(e->chunk_cap, n - c0);
         if ((r = embed_tokens(e, seq, tok_dev + c0, T, nullptr, s.len)) || (r = run_layers(e, seq, T, s.len))) return r;
         s.len += T;
         while (wi < n_want && want[wi] < c0 + T) {
-            uint32_t idx[kWantBatch], nw = 0;
-            while (nw < kWantBatch && wi + nw < n_want && want[wi + nw] < c0 + T) { idx[nw] = want[wi + nw] - c0; nw++; }
-            CK(cudaMemcpyAsync(e->want_dev, idx, nw * 4, cudaMemcpyHostToDevice, e->stream));
-            CK(cudaStreamSynchronize(e->stream));
-            if ((r = head_rows(e, nw))) return r;
-            CK(cudaMemcpyAsync(logits_host + (size_t)wi * e->V, e->logits, (size_t)nw * e->V * 4, cudaMemcpyDeviceToHost, e->stream));
-            CK(cudaStreamSynchronize(e->stream));
+            uint32_t nw = 0;
+            while (nw < kWantBatch && wi + nw < n_want && want[wi + nw] < c0 + T) nw++;
+            if ((r = head_rows(e, nw, e->want_dev + wi)) || (r = fetch_logits(e, nw, logits_host + (size_t)wi * e->V))) return r;
             wi += nw;
         }
     }
@@ -1925,19 +1945,18 @@ int lm_step(nb200_engine *h, uint32_t seq, const uint32_t *tokens, uint32_t n, c
     if (n == 1) {          // a single token: the captured decode step
         Seq &s = e->seqs[seq];
         if ((r = reserve_pages(e, seq, s.len + 1))) return r;
-        CK(cudaMemcpyAsync(e->ids_dev + s.len, tokens, 4, cudaMemcpyHostToDevice, e->stream));
-        CK(cudaMemcpyAsync(e->dpos, &s.len, 4, cudaMemcpyHostToDevice, e->stream));
-        if ((r = decode_step(e, seq))) return r;
+        if ((r = set_step(e, s.len, tokens[0])) || (r = decode_step(e, seq))) return r;
         s.len += 1;
-        if (n_want) CK(cudaMemcpyAsync(logits, e->logits, (size_t)e->V * 4, cudaMemcpyDeviceToHost, e->stream));
+        if (n_want) return fetch_logits(e, 1, logits);
         CK(cudaStreamSynchronize(e->stream));
         return 0;
     }
     std::vector<uint32_t> done;
     for (uint32_t c0 = 0; c0 < n; c0 += e->max_tokens) {          // the staging buffer holds max_tokens ids
         const uint32_t m = std::min(e->max_tokens, n - c0);
-        CK(cudaMemcpyAsync(e->ids_dev, tokens + c0, (size_t)m * 4, cudaMemcpyHostToDevice, e->stream));
-        CK(cudaStreamSynchronize(e->stream));
+        if (c0) CK(cudaStreamSynchronize(e->stream));          // the portion before has been read
+        memcpy(e->stage_ids, tokens + c0, (size_t)m * 4);
+        CK(cudaMemcpyAsync(e->ids_dev, e->stage_ids, (size_t)m * 4, cudaMemcpyHostToDevice, e->stream));
         uint32_t w0 = 0, w1 = 0;
         while (w0 < n_want && want[w0] < c0) w0++;
         w1 = w0;
@@ -2024,9 +2043,7 @@ int gen_token(LayeredEngine *e, uint32_t token) {
     const uint32_t seq = (uint32_t)e->gen_seq;
     Seq &s = e->seqs[seq];
     if ((r = reserve_pages(e, seq, s.len + 1))) return r;
-    CK(cudaMemcpyAsync(e->ids_dev + s.len, &token, 4, cudaMemcpyHostToDevice, e->stream));
-    CK(cudaMemcpyAsync(e->dpos, &s.len, 4, cudaMemcpyHostToDevice, e->stream));
-    if ((r = decode_step(e, seq))) return r;
+    if ((r = set_step(e, s.len, token)) || (r = decode_step(e, seq))) return r;
     s.len += 1;
     return 0;
 }
@@ -2045,9 +2062,7 @@ int lm_read_logits(nb200_engine *h, float *out) {
     LayeredEngine *e = self(h);
     if (!out) return fail(NB200_EINVAL, "null argument");
     CK(cudaSetDevice(e->device));
-    CK(cudaMemcpyAsync(out, e->logits, (size_t)e->V * 4, cudaMemcpyDeviceToHost, e->stream));
-    CK(cudaStreamSynchronize(e->stream));
-    return 0;
+    return fetch_logits(e, 1, out);
 }
 
 int mark_seen(LayeredEngine *e, const uint32_t *ids, uint32_t pos) {
@@ -2167,7 +2182,7 @@ void lm_destroy(nb200_engine *h) {
     if (e->stream) cudaStreamSynchronize(e->stream);
     for (cudaGraphExec_t g : e->graphs) if (g) cudaGraphExecDestroy(g);
     for (void *p : e->allocs) cudaFree(p);
-    if (e->tok_host) cudaFreeHost(e->tok_host);
+    for (void *p : {(void *)e->tok_host, (void *)e->stage_ids, (void *)e->stage_want, (void *)e->stage_pages, (void *)e->stage_logits}) if (p) cudaFreeHost(p);
     if (e->samp_host) cudaFreeHost(e->samp_host);
     nb::attn_tc_free(&e->ta);
     tc_free(&e->tc);
@@ -2618,11 +2633,15 @@ int create(LayeredEngine *e, const nb::ModelDir *dir, uint32_t max_tokens) {
     e->graphs.assign(e->max_seqs, nullptr);
     DM(e->b_xn, (size_t)kWantBatch * E * 4); DM(e->logits, (size_t)kWantBatch * e->V * 4);
     const size_t n_ids = (size_t)e->n_pages * kPage + 16;          // a single-token step stores its token at the sequence's position: every position the pages can hold
-    DM(e->ids_dev, n_ids * 4); DM(e->want_dev, kWantBatch * 4); DM(e->next_dev, 64); DM(e->seen, e->V);
+    DM(e->ids_dev, n_ids * 4); DM(e->want_dev, n_ids * 4); DM(e->next_dev, 64); DM(e->seen, e->V);
     CK(cudaMemset(e->ids_dev, 0, n_ids * 4));
     CK(cudaMemset(e->seen, 0, e->V));
     if (env_u32("NB200_KEEP_RESIDUALS", 0)) DM(e->keep, e->runs.size() * T * E * 4);
     CK(cudaHostAlloc(&e->tok_host, 64, cudaHostAllocDefault));
+    CK(cudaHostAlloc(&e->stage_ids, n_ids * 4, cudaHostAllocDefault)); CK(cudaHostAlloc(&e->stage_want, n_ids * 4, cudaHostAllocDefault));
+    CK(cudaHostAlloc(&e->stage_pages, (size_t)e->max_seqs * e->n_pages * 4, cudaHostAllocDefault));
+    e->stage_rows = (uint32_t)std::max<size_t>(1, std::min<size_t>(kWantBatch, ((size_t)4 << 20) / ((size_t)e->V * 4)));
+    CK(cudaHostAlloc(&e->stage_logits, (size_t)e->stage_rows * e->V * 4, cudaHostAllocDefault));
     CK(cudaDeviceSynchronize());
     return 0;
 }

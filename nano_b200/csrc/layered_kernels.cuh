@@ -477,6 +477,9 @@ __global__ void k_embed(const uint32_t *__restrict__ tokens, const uint32_t *__r
     }
 }
 
+// what a captured decode step reads: the token at its position, and the position
+__global__ void k_set_step(uint32_t *ids, uint32_t *dpos, uint32_t pos, uint32_t token) { ids[pos] = token; *dpos = pos; }
+
 __global__ void k_add(float *__restrict__ x, const float *__restrict__ y, size_t n) {
     pdl_enter();
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) x[i] += y[i];
