@@ -162,7 +162,8 @@ int nb200_next_sampled(nb200_engine *e, const uint32_t *ids, uint32_t pos, float
 
 /* Device-resident greedy loop: ids[0..n_prompt) is the prompt; positions 0..n_total-2 are run and
  * ids[n_prompt..n_total) are filled with greedy tokens (prompt positions are teacher-forced exactly like
- * llm_session_step).  device_ms (optional) receives the CUDA-event time of the decode segment
+ * llm_session_step; prompts of eight positions and more of F32 and Q80 files run in portions, whose fp32 sums come in another order
+ * than those of one call per position: K / V rows and logits agree as two execution paths do).  device_ms (optional) receives the CUDA-event time of the decode segment
  * (positions >= n_prompt-1); prefill_ms the prompt segment. */
 int nb200_decode_greedy(nb200_engine *e, uint32_t *ids, uint32_t n_prompt, uint32_t n_total,
                         float repetition_penalty, float *prefill_ms, float *device_ms);

@@ -371,7 +371,8 @@ int attn_tc_setup(TcAttnState *s, size_t bytes, size_t tiles, uint32_t *err_dev)
     int r;
     s->err_dev = err_dev;
     if (!bytes) return 0;
-    if (cudaMalloc(&s->images, bytes) != cudaSuccess || cudaMalloc(&s->scales, tiles * 8u) != cudaSuccess) return fail(NB200_ENOMEM, "cudaMalloc(%zu) failed", bytes);
+    if (cudaMalloc(&s->images, bytes) != cudaSuccess) { s->images = nullptr; return fail(NB200_ENOMEM, "cudaMalloc(%zu) failed", bytes); }
+    if (cudaMalloc(&s->scales, tiles * 8u) != cudaSuccess) { s->scales = nullptr; return fail(NB200_ENOMEM, "cudaMalloc(%zu) failed", tiles * 8u); }
     s->bytes = bytes; s->tiles = tiles;
     if ((r = optin<64, 64>()) || (r = optin<64, 128>()) || (r = optin<128, 64>()) || (r = optin<128, 128>())) return r;
     return 0;

@@ -1247,21 +1247,25 @@ static int nano_decode_greedy(nb200_engine *e, uint32_t *ids, uint32_t n_prompt,
     cudaEvent_t (&ev)[3] = evs.ev;
     for (auto &v : ev) CK(cudaEventCreate(&v));
     // A prompt of kPortionMin positions or more runs in portions; a shorter one position by position, which gives bit for bit what one call per
-    // token gives (15 positions of Nano-168M 9 ms; 32 positions 20 ms, in one portion 2)
+    // token gives (8 positions of Nano-168M Q80 5 ms one by one and 1.5 in a portion, 15 positions 9.3 and 1.5)
     const uint32_t first = n_prompt - 1;
-    const bool portion = first >= kPortionMin && !e->lora.active && nb::prefill_fits(e->prefill, first);
-    if ((r = push_state(e, portion ? first : 0u, 1, n_prompt, 1, penalty, 0, 0))) return r;
+    // a call that decodes nothing leaves the last prompt position's vectors and logits to be read: that one runs by itself
+    const uint32_t rows = n_total > n_prompt ? first : first ? first - 1u : 0u;
+    const bool portion = rows >= kPortionMin && !e->lora.active && nb::prefill_fits(e->prefill, rows);
+    const uint32_t start = portion ? rows : 0u;
+    if ((r = push_state(e, start, 1, n_prompt, 1, penalty, 0, 0))) return r;
     CK(cudaMemcpyAsync(e->ids_dev, ids, (size_t)n_prompt * 4, cudaMemcpyHostToDevice, e->stream));
     CK(cudaMemsetAsync(e->seen, 0, e->d.V, e->stream));
     e->seen_valid = false; e->seen_mirror.clear();
     CK(cudaEventRecord(ev[0], e->stream));
     if (portion) {
-        if ((r = nb::prefill_run(e->prefill, e->ids_dev, first, e->stream, &e->launches))) return r;
-        k_mark_seen<<<1, 256, 0, e->stream>>>(e->seen, e->ids_dev, 0, first);
+        if ((r = nb::prefill_run(e->prefill, e->ids_dev, rows, e->stream, e->use_pdl, &e->launches))) return r;
+        k_mark_seen<<<1, 256, 0, e->stream>>>(e->seen, e->ids_dev, 0, rows);
         CK(cudaGetLastError());
         e->launches++;
-    } else if (e->use_stream) { if ((r = launch_stream(e, first))) return r; }
-    else for (uint32_t p = 0; p < first; p++) if ((r = launch_token(e))) return r;
+    }
+    if (e->use_stream) { if ((r = launch_stream(e, first - start))) return r; }
+    else for (uint32_t p = start; p < first; p++) if ((r = launch_token(e))) return r;
     CK(cudaEventRecord(ev[1], e->stream));
     if (e->use_stream) { if ((r = launch_stream(e, n_total - n_prompt))) return r; }
     else for (uint32_t p = n_prompt - 1; p + 1 < n_total; p++) if ((r = launch_token(e))) return r;

@@ -352,7 +352,7 @@ int load_latent_attn(Loader &ld, const nb::Json *m, const std::string &p, Layer 
     for (uint64_t h = 0; h < H; h++)          // [H*dim, R] -> per head [R, dim]: absorbed query = q_h W_uk,h
         for (uint64_t dd = 0; dd < D; dd++)
             for (uint64_t k = 0; k < R; k++) t[(h * R + k) * D + dd] = uk[(h * D + dd) * R + k];
-    if (latent_up(ld.e, *L) && (r = ld.stacked({p + "uk", p + "uv"}, {H * D, H * VD}, R, &L->ukv))) return r;
+    if (latent_up(ld.e, *L) && ld.stacked({p + "uk", p + "uv"}, {H * D, H * VD}, R, &L->ukv)) { L->ukv = Weight{}; cudaGetLastError(); }      // (no room: portions stay absorbed)
     return ld.put_w(t, (uint32_t)(H * R), (uint32_t)D, &L->ukT);
 }
 
@@ -693,7 +693,7 @@ int load_latent_attn_direct(Loader &ld, const nb::Json *m, const std::string &p,
     for (uint64_t h = 0; h < H; h++)          // [H*dim, R] -> per head [R, dim]: absorbed query = q_h W_uk,h
         for (uint64_t dd = 0; dd < D; dd++)
             for (uint64_t k = 0; k < R; k++) t[(h * R + k) * D + dd] = uk[(h * D + dd) * R + k];
-    if (latent_up(ld.e, *L) && (r = ld.stacked({p + "uk", p + "uv"}, {H * D, H * VD}, R, &L->ukv))) return r;
+    if (latent_up(ld.e, *L) && ld.stacked({p + "uk", p + "uv"}, {H * D, H * VD}, R, &L->ukv)) { L->ukv = Weight{}; cudaGetLastError(); }      // (no room: portions stay absorbed)
     return ld.put_w(t, (uint32_t)(H * R), (uint32_t)D, &L->ukT);
 }
 
@@ -2608,6 +2608,20 @@ int create(LayeredEngine *e, const nb::ModelDir *dir, uint32_t max_tokens) {
         if (mFF2) { DM(e->b_hg, T * mFF2 * 4); DM(e->b_wrow, T * mTop * 4); DM(e->b_sg, T * 4); }
         if (mSFF2) DM(e->b_sh2, T * mSFF * 4);
     }
+    DM(e->dpos, 64); DM(e->zero_dev, 64);
+    CK(cudaMemset(e->dpos, 0, 64)); CK(cudaMemset(e->zero_dev, 0, 64));
+    e->graphs.assign(e->max_seqs, nullptr);
+    DM(e->b_xn, (size_t)kWantBatch * E * 4); DM(e->logits, (size_t)kWantBatch * e->V * 4);
+    const size_t n_ids = (size_t)e->n_pages * kPage + 16;          // a single-token step stores its token at the sequence's position: every position the pages can hold
+    DM(e->ids_dev, n_ids * 4); DM(e->want_dev, n_ids * 4); DM(e->next_dev, 64); DM(e->seen, e->V);
+    CK(cudaMemset(e->ids_dev, 0, n_ids * 4));
+    CK(cudaMemset(e->seen, 0, e->V));
+    if (env_u32("NB200_KEEP_RESIDUALS", 0)) DM(e->keep, e->runs.size() * T * E * 4);
+    CK(cudaHostAlloc(&e->tok_host, 64, cudaHostAllocDefault));
+    CK(cudaHostAlloc(&e->stage_ids, n_ids * 4, cudaHostAllocDefault)); CK(cudaHostAlloc(&e->stage_want, n_ids * 4, cudaHostAllocDefault));
+    CK(cudaHostAlloc(&e->stage_pages, (size_t)e->max_seqs * e->n_pages * 4, cudaHostAllocDefault));
+    e->stage_rows = (uint32_t)std::max<size_t>(1, std::min<size_t>(kWantBatch, ((size_t)4 << 20) / ((size_t)e->V * 4)));
+    CK(cudaHostAlloc(&e->stage_logits, (size_t)e->stage_rows * e->V * 4, cudaHostAllocDefault));
     if (!e->f32) {      // the widest rows any product reads (a routed product: one row per token and choice)
         size_t w = std::max<size_t>(E, mTop * E);
         for (uint32_t v : {2 * mC, mZ, mQR, mQ, mHR, mOV, sP, sQK, sXC, sA, sRO, sDBC, sF, sF2, sXC2, sY, dV, dSp, dGt, mMO, mFF, mFF2, mSFF, mSFF2}) w = std::max<size_t>(w, v);
@@ -2623,25 +2637,14 @@ int create(LayeredEngine *e, const nb::ModelDir *dir, uint32_t max_tokens) {
                 kv = std::max(kv, n * row); planes = std::max(planes, n * tc_split_width(L.R));
                 bytes = std::max(bytes, nb::attn_tc_bytes((uint32_t)n, L.H, L.dim, L.vdim)); tiles = std::max(tiles, nb::attn_tc_tiles((uint32_t)n, L.H));
             }
-        e->kv_floats = kv;
-        if (kv) { DM(e->b_kv, kv * 4); if ((r = tc_split_setup(&e->tc, planes))) return r; }
-        if ((r = tc_setup(&e->tc, std::max<size_t>(T, kWantBatch) * ((w + 7u) & ~(size_t)7u), (uint32_t)e->num_sms)) ||
-            (r = nb::attn_tc_setup(&e->ta, std::min<size_t>(bytes, (size_t)1 << 30), tiles, e->tc.err_dev))) return r;
+        // All of this makes long portions faster and nothing else: allocated last, and where the memory does not reach, they go through the kernels that need none of it
+        if (tc_setup(&e->tc, std::max<size_t>(T, kWantBatch) * ((w + 7u) & ~(size_t)7u), (uint32_t)e->num_sms)) tc_free(&e->tc);
+        else {
+            if (bytes && nb::attn_tc_setup(&e->ta, std::min<size_t>(bytes, (size_t)1 << 30), tiles, e->tc.err_dev)) nb::attn_tc_free(&e->ta);
+            if (kv && e->ta.images && cudaMalloc(&e->b_kv, kv * 4) == cudaSuccess) { e->allocs.push_back(e->b_kv); if (!tc_split_setup(&e->tc, planes)) e->kv_floats = kv; }
+        }
+        cudaGetLastError();
     }
-    DM(e->dpos, 64); DM(e->zero_dev, 64);
-    CK(cudaMemset(e->dpos, 0, 64)); CK(cudaMemset(e->zero_dev, 0, 64));
-    e->graphs.assign(e->max_seqs, nullptr);
-    DM(e->b_xn, (size_t)kWantBatch * E * 4); DM(e->logits, (size_t)kWantBatch * e->V * 4);
-    const size_t n_ids = (size_t)e->n_pages * kPage + 16;          // a single-token step stores its token at the sequence's position: every position the pages can hold
-    DM(e->ids_dev, n_ids * 4); DM(e->want_dev, n_ids * 4); DM(e->next_dev, 64); DM(e->seen, e->V);
-    CK(cudaMemset(e->ids_dev, 0, n_ids * 4));
-    CK(cudaMemset(e->seen, 0, e->V));
-    if (env_u32("NB200_KEEP_RESIDUALS", 0)) DM(e->keep, e->runs.size() * T * E * 4);
-    CK(cudaHostAlloc(&e->tok_host, 64, cudaHostAllocDefault));
-    CK(cudaHostAlloc(&e->stage_ids, n_ids * 4, cudaHostAllocDefault)); CK(cudaHostAlloc(&e->stage_want, n_ids * 4, cudaHostAllocDefault));
-    CK(cudaHostAlloc(&e->stage_pages, (size_t)e->max_seqs * e->n_pages * 4, cudaHostAllocDefault));
-    e->stage_rows = (uint32_t)std::max<size_t>(1, std::min<size_t>(kWantBatch, ((size_t)4 << 20) / ((size_t)e->V * 4)));
-    CK(cudaHostAlloc(&e->stage_logits, (size_t)e->stage_rows * e->V * 4, cudaHostAllocDefault));
     CK(cudaDeviceSynchronize());
     return 0;
 }

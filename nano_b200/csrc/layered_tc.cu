@@ -302,7 +302,7 @@ int tc_setup(TcState *t, size_t elems, uint32_t sms) {
     if (got != cudaDriverEntryPointSuccess || !fn) return fail(NB200_ECUDA, "the driver has no cuTensorMapEncodeTiled");
     t->encode = reinterpret_cast<decltype(t->encode)>(fn);
     t->sms = sms;
-    for (auto &p : t->rows) if (cudaMalloc(&p, elems * 2) != cudaSuccess) return fail(NB200_ENOMEM, "cudaMalloc(%zu) failed", elems * 2);
+    for (auto &p : t->rows) if (cudaMalloc(&p, elems * 2) != cudaSuccess) { p = nullptr; return fail(NB200_ENOMEM, "cudaMalloc(%zu) failed", elems * 2); }
     t->elems = elems;
     NB_CK(cudaHostAlloc(&t->err_host, 64, cudaHostAllocMapped));
     *t->err_host = 0;
@@ -316,7 +316,7 @@ void tc_free(TcState *t) {
     if (t->planes) cudaFree(t->planes);
     t->planes = nullptr;
     if (t->err_host) cudaFreeHost(t->err_host);
-    t->err_host = nullptr; t->encode = nullptr;
+    t->err_host = t->err_dev = nullptr; t->encode = nullptr; t->elems = t->plane_elems = 0;
 }
 int tc_check(TcState *t) {
     if (!t->err_host || !*static_cast<volatile uint32_t *>(t->err_host)) return 0;
@@ -356,7 +356,7 @@ int tc_gemm(TcState *t, GemmArgs a, uint32_t groups, uint32_t maxM, uint32_t row
 }
 
 int tc_split_setup(TcState *t, size_t elems) {
-    if (cudaMalloc(&t->planes, elems * 2) != cudaSuccess) return fail(NB200_ENOMEM, "cudaMalloc(%zu) failed", elems * 2);
+    if (cudaMalloc(&t->planes, elems * 2) != cudaSuccess) { t->planes = nullptr; return fail(NB200_ENOMEM, "cudaMalloc(%zu) failed", elems * 2); }
     t->plane_elems = elems;
     return 0;
 }

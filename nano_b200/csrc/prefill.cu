@@ -362,15 +362,19 @@ __global__ void __launch_bounds__(256) k_prompt_rope(const PromptRopeArgs a) {
 }
 
 template <typename A>
-int launch(void (*k)(const A), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, const A &args, uint32_t cluster_z = 1) {
+int launch(void (*k)(const A), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, bool pdl, const A &args, uint32_t cluster_z = 1) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
     cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = 1; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = cluster_z;
-    cfg.attrs = attr; cfg.numAttrs = cluster_z > 1u ? 2 : 1;
+    cfg.attrs = attr;
+    if (pdl) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster_z > 1u) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attr[cfg.numAttrs].val.clusterDim.x = 1; attr[cfg.numAttrs].val.clusterDim.y = 1; attr[cfg.numAttrs++].val.clusterDim.z = cluster_z;
+    }
     NB_CK(cudaLaunchKernelEx(&cfg, k, args));
     return 0;
 }
@@ -380,7 +384,7 @@ int optin() { NB_CK(cudaFuncSetAttribute((const void *)k_prompt_gemm<Q80, TN>, c
 
 struct Product { PrefillMat m; CUtensorMap wmap; const float *winv = nullptr; uint32_t np = 0; };      // np: F32 depth padded to 64
 struct PrefillState {
-    PrefillModel m; uint32_t sms = 148;
+    PrefillModel m; uint32_t sms = 148; bool pdl = true;
     decltype(&cuTensorMapEncodeTiled) encode = nullptr;
     std::vector<Product> qkv, wo, w13, w2;
     float *x = nullptr, *p = nullptr, *q = nullptr, *o = nullptr;      // residual rows, products, turned queries, attention output
@@ -458,7 +462,7 @@ int create(PrefillState *s, const PrefillModel &m) {
 }
 int prep(PrefillState *s, const float *src, uint32_t ld, const float *gain, uint32_t n, uint32_t mode, uint32_t T, cudaStream_t stream) {
     PromptPrepArgs a{src, ld, gain, n, s->m.gs, mode, reinterpret_cast<int8_t *>(s->act), s->scales, kChunk, reinterpret_cast<__half *>(s->act), (n + 63u) & ~63u, s->scales};
-    return s->m.quant == 0x80u ? launch<PromptPrepArgs>(k_prompt_prep<true>, dim3(T), dim3(kPrepThreads), 0, stream, a) : launch<PromptPrepArgs>(k_prompt_prep<false>, dim3(T), dim3(kPrepThreads), (size_t)n * 4, stream, a);
+    return s->m.quant == 0x80u ? launch<PromptPrepArgs>(k_prompt_prep<true>, dim3(T), dim3(kPrepThreads), 0, stream, s->pdl, a) : launch<PromptPrepArgs>(k_prompt_prep<false>, dim3(T), dim3(kPrepThreads), (size_t)n * 4, stream, s->pdl, a);
 }
 int product(PrefillState *s, const Product &w, float *C, uint32_t ldc, bool add, uint32_t T, cudaStream_t stream) {
     // 64 positions per tile where tiles of 128 leave SMs without a block (1024 rows of the O product: 8 blocks for 128 positions)
@@ -474,7 +478,7 @@ int product(PrefillState *s, const Product &w, float *C, uint32_t ldc, bool add,
     while (ks < 8u && tiles * ks * 2u <= s->sms && units >= ks * 4u) ks *= 2u;
     a.ks = ks;
     const dim3 grid(rt, (T + tn - 1u) / tn, ks), block(192);
-#define GEMM(q, t) launch<PromptGemmArgs>(k_prompt_gemm<q, t>, grid, block, gemm_smem<q, t>(), stream, a, ks)
+#define GEMM(q, t) launch<PromptGemmArgs>(k_prompt_gemm<q, t>, grid, block, gemm_smem<q, t>(), stream, s->pdl, a, ks)
     if (s->m.quant == 0x80u) return tn == 64u ? GEMM(true, 64) : GEMM(true, 128);
     return tn == 64u ? GEMM(false, 64) : GEMM(false, 128);
 #undef GEMM
@@ -508,7 +512,8 @@ int prefill_check(PrefillState *s) {
     *s->err_host = 0;
     return fail(NB200_ECUDA, "a wait inside a prompt kernel ran out (code 0x%x): the results of this call are not valid", code);
 }
-int prefill_run(PrefillState *s, const uint32_t *ids, uint32_t n, cudaStream_t stream, uint64_t *launches) {
+int prefill_run(PrefillState *s, const uint32_t *ids, uint32_t n, cudaStream_t stream, bool pdl, uint64_t *launches) {
+    s->pdl = pdl;
     const PrefillModel &m = s->m;
     const uint32_t W = m.q_dim + 2 * m.kv_dim;
     const size_t kvl = (size_t)m.KV * m.max_seq * m.hd;
@@ -517,19 +522,19 @@ int prefill_run(PrefillState *s, const uint32_t *ids, uint32_t n, cudaStream_t s
     int r;
     for (uint32_t p0 = 0; p0 < n; p0 += kChunk) {
         const uint32_t T = std::min(kChunk, n - p0);
-        if ((r = launch<PromptEmbedArgs>(k_prompt_embed, dim3(T), dim3(256), 0, stream, PromptEmbedArgs{m.emb.w, m.emb.aux, s->x, ids + p0, m.E, m.gs, m.quant}))) return r;
+        if ((r = launch<PromptEmbedArgs>(k_prompt_embed, dim3(T), dim3(256), 0, stream, pdl, PromptEmbedArgs{m.emb.w, m.emb.aux, s->x, ids + p0, m.E, m.gs, m.quant}))) return r;
         (*launches)++;
         for (uint32_t l = 0; l < m.L; l++) {
             const PromptRopeArgs ra{s->p, W, m.H, m.KV, p0, s->q, m.kc + l * kvl, m.vc + l * kvl, m.qnorm ? m.qnorm + (size_t)l * m.hd : nullptr, m.knorm ? m.knorm + (size_t)l * m.hd : nullptr, m.rope_cos, m.rope_sin, d};
             if ((r = prep(s, s->x, m.E, m.norm_attn + (size_t)l * m.E, m.E, PREP_NORM, T, stream)) || (r = product(s, s->qkv[l], s->p, W, false, T, stream)) ||
-                (r = launch<PromptRopeArgs>(k_prompt_rope, dim3(T), dim3(256), 0, stream, ra))) return r;
+                (r = launch<PromptRopeArgs>(k_prompt_rope, dim3(T), dim3(256), 0, stream, pdl, ra))) return r;
             *launches += 3;
             if (l + 1u == m.L) break;          // nothing reads what the last layer would make of these positions
             TcAttn a{};
             a.q = s->q; a.ldq = m.q_dim; a.q_head = m.hd; a.k = m.kc + l * kvl; a.v = m.vc + l * kvl; a.ldk = a.ldv = m.hd; a.k_head = a.v_head = (uint64_t)m.max_seq * m.hd;
             a.out = s->o; a.T = T; a.H = m.H; a.G = m.KV; a.D = a.VD = m.hd; a.pos0 = p0; a.scale = (float)(1.0 / sqrt((double)m.hd));
             if (!attn_tc_fits(&s->attn, a)) return fail(NB200_EINVAL, "a prompt of %u positions does not fit the attention's buffers", n);
-            if ((r = attn_tc_launch(&s->attn, a, stream, true)) || (r = prep(s, s->o, m.q_dim, nullptr, m.q_dim, PREP_PLAIN, T, stream)) || (r = product(s, s->wo[l], s->x, m.E, true, T, stream)) ||
+            if ((r = attn_tc_launch(&s->attn, a, stream, pdl)) || (r = prep(s, s->o, m.q_dim, nullptr, m.q_dim, PREP_PLAIN, T, stream)) || (r = product(s, s->wo[l], s->x, m.E, true, T, stream)) ||
                 (r = prep(s, s->x, m.E, m.norm_ffn + (size_t)l * m.E, m.E, PREP_NORM, T, stream)) || (r = product(s, s->w13[l], s->p, 2 * m.F, false, T, stream)) ||
                 (r = prep(s, s->p, 2 * m.F, nullptr, m.F, PREP_SWIGLU, T, stream)) || (r = product(s, s->w2[l], s->x, m.E, true, T, stream))) return r;
             *launches += 8;

@@ -22,8 +22,8 @@ struct PrefillState;
 // *out stays null (and 0 is returned) when the model's shapes have no portion kernels; F32 models get a second copy of their weights in two f16 parts
 int prefill_create(PrefillState **out, const PrefillModel &m, uint32_t sms);
 void prefill_destroy(PrefillState *p);
-// K and V rows of the positions [0, n) of the tokens ids[0..n) on the device; n <= max_seq.  launches: how many kernels were put on the stream
-int prefill_run(PrefillState *p, const uint32_t *ids, uint32_t n, cudaStream_t stream, uint64_t *launches);
+// K and V rows of the positions [0, n) of the tokens ids[0..n) on the device; n <= max_seq.  pdl: with programmatic dependent launch; launches: how many kernels were put on the stream
+int prefill_run(PrefillState *p, const uint32_t *ids, uint32_t n, cudaStream_t stream, bool pdl, uint64_t *launches);
 bool prefill_fits(const PrefillState *p, uint32_t n);      // whether the attention has room for that many positions
 // after a synchronisation: did a bounded wait of a kernel run out
 int prefill_check(PrefillState *p);

@@ -9,7 +9,9 @@ import numpy as np
 import pytest
 
 from nano_b200 import engine as E, modeldir as md
+import famudra_oracle as A
 import fidatar_oracle as F
+import vumunex_oracle as V
 
 pytestmark = pytest.mark.gpu
 
@@ -31,6 +33,37 @@ def test_portions_against_single_tokens(tmp_path, heads, kv, dim, vdim, size, sc
         s, at, out = eng.seq_open(), 0, []
         for n in cuts:
             out.append(eng.step(s, toks[at:at + n], range(len(toks[at:at + n]))))
+            at += n
+        eng.seq_close(s)
+        got = np.concatenate(out)
+        d = np.sqrt(((got - one[:at]) ** 2).mean(-1) / (one[:at] ** 2).mean(-1))
+        assert d.max() < 1.2e-2, (cuts, int(d.argmax()))
+        assert np.linalg.norm(got - ref[:at]) < 2e-2 * np.linalg.norm(ref[:at]), cuts
+    eng.close()
+
+
+@pytest.mark.parametrize("design,heads,dim,vdim,rank,size", [("famudra", 3, 24, 40, 48, None), ("famudra", 2, 128, 128, 256, None), ("famudra", 5, 64, 68, 8, None), ("vumunex", 3, 20, 12, 40, None), ("vumunex", 4, 64, 64, 128, 130),
+                                                            ("vumunex", 2, 128, 60, 72, 200)])
+def test_latents_multiplied_out(tmp_path, design, heads, dim, vdim, rank, size):
+    """Portions that see 128 keys and more against single tokens (absorbed): the query and the weighted latents are rounded to bfloat16 (2^-9 each) on the
+    absorbed side only, so the bound of one layer above stands; plain softmax, window, sink and gate."""
+    mixer = {"heads": heads, "dim": dim, "vdim": vdim, "kv_rank": rank, "scale": dim ** -0.5}
+    if design == "famudra":
+        cfg, make, oracle = md.famudra_config(64, 96, [("latent_attention", dict(mixer, q_rank=56), None)]), md.famudra_random, A.forward
+    else:
+        cfg = md.vumunex_config(64, 96, [("latent_attention", dict(mixer, mask={"size": size}) if size else mixer, None)], streams=2)
+        make, oracle = md.vumunex_random, V.forward
+    w = make(cfg, 5)
+    eng = E.Engine(md.write_model_dir(str(tmp_path / "m"), cfg, w), 1024)
+    toks = np.random.default_rng(2).integers(0, 64, size=600).astype(np.uint32)
+    ref = oracle(cfg, w, toks)
+    s = eng.seq_open()
+    one = np.concatenate([eng.step(s, toks[i:i + 1], [0]) for i in range(toks.size)])
+    eng.seq_close(s)
+    for cuts in ([600], [127, 5, 129, 128, 130], [130, 6, 464]):
+        s, at, out = eng.seq_open(), 0, []
+        for n in cuts:
+            out.append(eng.step(s, toks[at:at + n], range(n)))
             at += n
         eng.seq_close(s)
         got = np.concatenate(out)

@@ -70,3 +70,17 @@ def test_penalty_sees_the_prompt_and_short_prompts_stay_as_they_were():
         eng.decode_greedy(b, n, 100, 1.3)
         assert a[:100].tolist() == b[:100].tolist(), n
     eng.close()
+
+
+@pytest.mark.parametrize("n", [2, 9, 10, 33, 130])
+def test_a_call_that_decodes_nothing_leaves_the_last_prompt_position(n):
+    spec = dataclasses.replace(mf.PRESETS["toy-nano"], name="toy-nano-prompts", block_size=2048)
+    eng = E.Engine(mf.cached_model(spec, mf.QUANT_F32, 128), 200)
+    ids = mf.teacher_tokens(n, spec.vocab).astype(np.uint32)
+    for p in range(n - 1):
+        eng.forward_nolog(int(ids[p]), p)
+    want = eng.logits()          # (the streaming path keeps no residual vector that could be read)
+    eng.forward_nolog(3, 150)
+    eng.decode_greedy(ids.copy(), n, n)
+    assert rel(eng.logits(), want) < 1e-5
+    eng.close()
