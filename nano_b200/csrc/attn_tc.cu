@@ -187,7 +187,10 @@ __global__ void __launch_bounds__(192, 1) k_attn_tc(const AttnTcArgs ta) {
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
     }
-    constexpr uint32_t SCOL = 0, PCOL = 256, OCOL = 384;          // tensor memory: scores (two buffers of 128), weights (two planes of 64), a tile's weighted values
+    // tensor memory: scores (two buffers of 128), weights (two planes of 64), a tile's weighted values.  Heads of 64 values have room for a sum per half of
+    // the tile: the tensor cores cut what they add, and half as many additions cut half as much (four layers of width 768 behind 200 / 487 positions, logits
+    // against 64 bits by those of fp32 attention: 1.09 / 1.08 with one sum, 1.05 / 1.04 with two)
+    constexpr uint32_t SCOL = 0, PCOL = 256, OCOL = 384, HCOL = VP == 64 ? 64 : 0;
     if (warp == 0 && lane == 0) {
         for (uint32_t i = 0; i < n; i++) {
             if (i && !mbar_wait(bar(KFREE), (i - 1u) & 1u)) { bad_s = 1; break; }
@@ -220,14 +223,12 @@ __global__ void __launch_bounds__(192, 1) k_attn_tc(const AttnTcArgs ta) {
             ok = mbar_wait(bar(PREADY), i & 1u) && mbar_wait(bar(VFULL), i & 1u);
             if (!ok) break;
             tc_fence_after();
-            bool add = false;
 #pragma unroll
             for (uint32_t p = 0; p < 3; p++)
 #pragma unroll
                 for (uint32_t ks = 0; ks < kTile / 16; ks++) {
                     const uint32_t off = (ks >> 2) * VP * 128u + (ks & 3u) * 32u;
-                    tc_mma_ts(tmem + OCOL, tmem + PCOL + (p == 0 ? 64u : 0u) + ks * 8u, tc_desc(vsm + (p == 1 ? VP * 256u : 0u) + off), id_o, add);
-                    add = true;
+                    tc_mma_ts(tmem + OCOL + (ks >> 2) * HCOL, tmem + PCOL + (p == 0 ? 64u : 0u) + ks * 8u, tc_desc(vsm + (p == 1 ? VP * 256u : 0u) + off), id_o, p > 0 || (HCOL ? ks & 3u : ks) > 0);
                 }
             tc_commit(bar(VFREE)); tc_commit(bar(OREADY));
             if (i + 2u < n) ok = scores(i + 2u);          // its buffer's scores have been read: the weights of tile i are there
@@ -253,6 +254,11 @@ __global__ void __launch_bounds__(192, 1) k_attn_tc(const AttnTcArgs ta) {
                 tc_ld32(tmem + lane_base + OCOL + c, w);
 #pragma unroll
                 for (int j = 0; j < 32; j++) o[c + j] = fmaf(__uint_as_float(w[j]), f, o[c + j] * corr);
+                if (HCOL) {
+                    tc_ld32(tmem + lane_base + OCOL + HCOL + c, w);
+#pragma unroll
+                    for (int j = 0; j < 32; j++) o[c + j] = fmaf(__uint_as_float(w[j]), f, o[c + j]);
+                }
             }
         };
         for (uint32_t i = 0; i < n; i++) {
@@ -362,7 +368,7 @@ int launch(void (*k)(const A), dim3 grid, dim3 block, size_t smem, cudaStream_t 
     return 0;
 }
 template <int DP, int VP>
-int optin() { NB_CK(cudaFuncSetAttribute((const void *)k_attn_tc<DP, VP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)attn_smem<DP, VP>())); return 0; }
+int optin() { NB_CK(nb::smem_at_least((const void *)k_attn_tc<DP, VP>, (int)attn_smem<DP, VP>())); return 0; }
 bool aligned16(const float *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 }  // namespace
 

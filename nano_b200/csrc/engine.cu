@@ -145,7 +145,7 @@ int launch(nb200_engine *e, void (*kern)(const Args), dim3 grid, dim3 block, siz
         attr[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr; cfg.numAttrs = 1;
     }
-    if (smem > 48 * 1024) CK(cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 48 * 1024) CK(nb::smem_at_least((const void *)kern, (int)smem));
     if (e && e->prof_on) {
         nb200_engine::ProfRec r{e->prof_tag, nullptr, nullptr};
         CK(cudaEventCreate(&r.a)); CK(cudaEventCreate(&r.b));
@@ -565,7 +565,7 @@ int setup_stream(nb200_engine *e) {
     g.cta_stride = (g.cls_off + (uint64_t)ntl[SK_CLS] * g.kind[SK_CLS].tile_stride + 127u) & ~(uint64_t)127u;
 
     const uint32_t smem = region0 + nst * stage_bytes;
-    cudaError_t ce = cudaFuncSetAttribute((const void *)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t ce = nb::smem_at_least((const void *)k, (int)smem);
     int occ = 0;
     if (ce == cudaSuccess) ce = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, (const void *)k, kThreads, smem);
     if (ce != cudaSuccess || occ < 1) { cudaGetLastError(); return 0; }
@@ -1423,7 +1423,7 @@ int op_prep(uint32_t quant, const float *x, const float *gain, uint32_t n, uint3
     CK(cudaMemcpy(dx.p, x, (size_t)n * 4, cudaMemcpyHostToDevice));
     if (gain) CK(cudaMemcpy(dg.p, gain, (size_t)n * 4, cudaMemcpyHostToDevice));
     const uint32_t smem = act_smem_bytes(quant, n, gs ? gs : 1);
-    if (smem > 48 * 1024) CK(cudaFuncSetAttribute((const void *)k_op_prep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 48 * 1024) CK(nb::smem_at_least((const void *)k_op_prep, (int)smem));
     k_op_prep<<<1, kThreads, smem>>>(dx.as<float>(), gain ? dg.as<float>() : nullptr, n, gs, quant, exact, dout.as<float>(),
                                      dcodes.as<int8_t>(), dscales.as<float>());
     CK(cudaGetLastError());

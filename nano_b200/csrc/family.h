@@ -7,7 +7,10 @@
 //     nb_family_nano_create     engine.cu    BD4SURLM model-file images (Nano / Qwen2 / Qwen3 decoders, F32 / Q80 / Q4K)
 //     nb_family_layered_create  layered.cu   config.json + model.safetensors folders whose config lists its layers (Famudra, Rakarax, Gokinex, Vumunex, Kadesun, Fidatar)
 #pragma once
+#include <cuda_runtime.h>
 #include <stdint.h>
+
+#include <mutex>
 
 #include "../../include/nano_b200.h"
 
@@ -22,6 +25,17 @@ int fail(int code, const char *fmt, ...);
         if (e_ != cudaSuccess)                                                                                            \
             return ::nb::fail(NB200_ECUDA, "%s failed: %s (%s:%d)", #call, cudaGetErrorString(e_), __FILE__, __LINE__); \
     } while (0)
+
+// A kernel's limit of dynamic shared memory belongs to the process, not to an engine: it is only ever raised, so that a smaller model opened later does
+// not take it from a larger one.
+inline cudaError_t smem_at_least(const void *kernel, int bytes) {
+    static std::mutex m;
+    std::lock_guard<std::mutex> hold(m);
+    cudaFuncAttributes fa;
+    const cudaError_t e = cudaFuncGetAttributes(&fa, kernel);
+    if (e != cudaSuccess || fa.maxDynamicSharedSizeBytes >= bytes) return e;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+}
 
 struct EngineOps {
     void (*destroy)(nb200_engine *);

@@ -957,10 +957,10 @@ int attn_launch(LayeredEngine *e, const AttnArgs &a, uint32_t rch) {
 }
 template <int RCH, int QT>
 int attn_optin_r(int smem) {
-    CK(cudaFuncSetAttribute((const void *)k_latent_attn<RCH, QT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    CK(cudaFuncSetAttribute((const void *)k_latent_attn<RCH, QT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    CK(cudaFuncSetAttribute((const void *)k_latent_attn<RCH, QT, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    CK(cudaFuncSetAttribute((const void *)k_latent_attn<RCH, QT, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    CK(nb::smem_at_least((const void *)k_latent_attn<RCH, QT, true>, smem));
+    CK(nb::smem_at_least((const void *)k_latent_attn<RCH, QT, false>, smem));
+    CK(nb::smem_at_least((const void *)k_latent_attn<RCH, QT, true, true>, smem));
+    CK(nb::smem_at_least((const void *)k_latent_attn<RCH, QT, false, true>, smem));
     return 0;
 }
 template <int QT>
@@ -1134,11 +1134,11 @@ int win_attn_launch_v(LayeredEngine *e, const WinAttnArgs &a, uint32_t qt, uint3
 }
 template <int VCH>
 int win_attn_optin_v(int smem) {
-    CK(cudaFuncSetAttribute((const void *)k_window_attn<VCH, 8, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    CK(cudaFuncSetAttribute((const void *)k_window_attn<VCH, 4, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    CK(cudaFuncSetAttribute((const void *)k_window_attn<VCH, 1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    CK(cudaFuncSetAttribute((const void *)k_window_attn<VCH, 4, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    CK(cudaFuncSetAttribute((const void *)k_window_attn<VCH, 1, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    CK(nb::smem_at_least((const void *)k_window_attn<VCH, 8, 1>, smem));
+    CK(nb::smem_at_least((const void *)k_window_attn<VCH, 4, 1>, smem));
+    CK(nb::smem_at_least((const void *)k_window_attn<VCH, 1, 1>, smem));
+    CK(nb::smem_at_least((const void *)k_window_attn<VCH, 4, 2>, smem));
+    CK(nb::smem_at_least((const void *)k_window_attn<VCH, 1, 2>, smem));
     return 0;
 }
 constexpr size_t kWinSmemMax = 200 * 1024;
@@ -1159,7 +1159,7 @@ int win_attn_launch(LayeredEngine *e, const Layer &L, const WinAttnArgs &a) {
 constexpr size_t kSelStageMax = 160 * 1024;      // dynamic shared memory the time-parallel scan may stage its inputs in (32 KB of maps are static)
 template <int LG>
 int sel_scan_optin() {
-    CK(cudaFuncSetAttribute((const void *)k_selective_scan_par<LG, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSelStageMax));
+    CK(nb::smem_at_least((const void *)k_selective_scan_par<LG, true>, (int)kSelStageMax));
     return 0;
 }
 template <int LG>
@@ -1250,8 +1250,8 @@ int diff_attn_launch_v(LayeredEngine *e, const DiffAttnArgs &a, uint32_t qt, uin
 }
 template <int VCH>
 int diff_attn_optin_v(int smem) {
-    CK(cudaFuncSetAttribute((const void *)k_diff_attn<VCH, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    CK(cudaFuncSetAttribute((const void *)k_diff_attn<VCH, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    CK(nb::smem_at_least((const void *)k_diff_attn<VCH, 4>, smem));
+    CK(nb::smem_at_least((const void *)k_diff_attn<VCH, 1>, smem));
     return 0;
 }
 inline int diff_vch(uint32_t vdim) { return vdim <= 32 ? 0 : vdim <= 64 ? 1 : vdim <= 128 ? 2 : 3; }
@@ -2526,14 +2526,14 @@ int create(LayeredEngine *e, const nb::ModelDir *dir, uint32_t max_tokens) {
         const size_t chunks = (T + kMemChunk - 1) / kMemChunk;
         DM(e->b_mfa, mMH * T * 8); DM(e->b_mfb, mMH * T * 8); DM(e->b_mfc, mMH * chunks * 8); DM(e->b_mmt, mMH * T * 4); DM(e->b_mme, mMH * (chunks + 1) * 4);
         DM(e->b_mS, chunks * mMS * 4); DM(e->b_mn, chunks * mMD * 4); DM(e->b_mo, T * mMO * 4);
-        CK(cudaFuncSetAttribute((const void *)k_memory_out<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)memory_out_smem(2)));
+        CK(nb::smem_at_least((const void *)k_memory_out<2>, (int)memory_out_smem(2)));
     }
     if (dPart) {
         if (dC) DM(e->d2, T * E * 4); DM(e->b_gpart, (size_t)kGemvMaxM * kGqaSplitMax * dPart * 4); DM(e->b_gtick, (size_t)kGemvMaxM * dTick * 4);
         CK(cudaMemset(e->b_gtick, 0, (size_t)kGemvMaxM * dTick * 4));
-        if (gqa_smem[1] > 48 * 1024) CK(cudaFuncSetAttribute((const void *)k_gqa_attn<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gqa_smem[1]));
-        if (gqa_smem[2] > 48 * 1024) CK(cudaFuncSetAttribute((const void *)k_gqa_attn<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gqa_smem[2]));
-        if (gqa_smem[4] > 48 * 1024) CK(cudaFuncSetAttribute((const void *)k_gqa_attn<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gqa_smem[4]));
+        if (gqa_smem[1] > 48 * 1024) CK(nb::smem_at_least((const void *)k_gqa_attn<1>, (int)gqa_smem[1]));
+        if (gqa_smem[2] > 48 * 1024) CK(nb::smem_at_least((const void *)k_gqa_attn<2>, (int)gqa_smem[2]));
+        if (gqa_smem[4] > 48 * 1024) CK(nb::smem_at_least((const void *)k_gqa_attn<4>, (int)gqa_smem[4]));
     }
     if (sSS) DM(e->b_sseg, (size_t)kRetSegs * sSS * 4);
     if (sXC2) DM(e->b_sdx, T * sXC2 * 4);

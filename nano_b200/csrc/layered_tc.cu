@@ -292,7 +292,7 @@ int launch(void (*k)(const A), dim3 grid, dim3 block, size_t smem, cudaStream_t 
     return 0;
 }
 template <int TN>
-int optin() { NB_CK(cudaFuncSetAttribute((const void *)k_gemm_tc<TN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_smem(TN))); return 0; }
+int optin() { NB_CK(nb::smem_at_least((const void *)k_gemm_tc<TN>, (int)tc_smem(TN))); return 0; }
 }  // namespace
 
 int tc_setup(TcState *t, size_t elems, uint32_t sms) {

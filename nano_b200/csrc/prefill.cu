@@ -10,8 +10,11 @@
 //   k_prompt_gemm      C[t][n] (+)= sum over groups: tcgen05.mma on 128 weight rows x TN positions, the accumulator of a GROUP in tensor memory (two
 //                      buffers), added to fp32 registers by the threads that own the rows while the next group multiplies.
 //                      Q80: kind::i8, int32 exact, times weight scale x activation scale.  F32: kind::f16 on two parts of both
-//                      operands (small x large, large x small, large x large: 2^-23 of a product) over 64 of the depth; the
-//                      tensor cores cut what they add, so their own additions stay that short.
+//                      operands, all four products, over 16 of the depth; the tensor cores cut what they add, so they add four
+//                      times only, and what they leave is added up with its rounding error carried along.  Logits against 64
+//                      bits by those of single positions, 40 / 200 positions and four layers of width 768: 1.14 / 1.16 with
+//                      three products, 64 of the depth and a plain sum, 1.06 / 1.09 with 32 and the error carried, 1.02 / 1.04 so
+//                      (attn_tc.cu's shorter sums included).
 //   k_prompt_rope      head norm (Qwen3), rotary positions, K and V rows into the cache
 //   attention          attn_tc.cu
 #include "prefill.h"
@@ -132,7 +135,7 @@ __device__ __forceinline__ void tc_mma_i8(uint32_t d, uint64_t a, uint64_t b, ui
 }
 // a stage holds 128 bytes of the depth of 128 weight rows and TN positions: 128 int8, or 64 f16 of both parts
 template <bool Q80, int TN> __host__ __device__ constexpr uint32_t gemm_stage() { return (kRows + (uint32_t)TN) * 128u * (Q80 ? 1u : 2u); }
-template <bool Q80, int TN> __host__ __device__ constexpr uint32_t gemm_stages() { return Q80 ? (TN == 64 ? 4u : 6u) : (TN == 64 ? 4u : 3u); }
+template <bool Q80, int TN> __host__ __device__ constexpr uint32_t gemm_stages() { return Q80 && TN == 128 ? 6u : 4u; }
 template <bool Q80, int TN> constexpr size_t gemm_smem() { return (size_t)gemm_stages<Q80, TN>() * gemm_stage<Q80, TN>() + 1024u; }
 
 template <bool Q80, int TN>
@@ -150,7 +153,7 @@ __global__ void __launch_bounds__(192, Q80 && TN == 64 ? 2 : 1) k_prompt_gemm(co
     // up in fp32
     const uint32_t us = Q80 && a.gs > 128u ? a.gs / 128u : 1u, units = ((Q80 ? (a.n + 127u) / 128u : a.np / 64u) + us - 1u) / us, per_part = (units + a.ks - 1u) / a.ks;
     const uint32_t u0 = min(units, blockIdx.z * per_part), s0 = u0 * us, steps = min(per_part, units - u0) * us;
-    const uint32_t g0 = Q80 ? s0 * 128u / a.gs : s0, groups = Q80 ? min(a.n, (s0 + steps) * 128u) / a.gs - g0 : steps, all_groups = Q80 ? a.n / a.gs : 0u;
+    const uint32_t g0 = Q80 ? s0 * 128u / a.gs : s0, groups = Q80 ? min(a.n, (s0 + steps) * 128u) / a.gs - g0 : steps * 4u, all_groups = Q80 ? a.n / a.gs : 0u;
     if (threadIdx.x == 0) {
         for (uint32_t i = 0; i < ST; i++) { mbar_init(full + i * 8u, 1); mbar_init(empty + i * 8u, 1); }
         for (uint32_t i = 0; i < 2; i++) { mbar_init(tfull + i * 8u, 1); mbar_init(tfree + i * 8u, 4); }
@@ -210,23 +213,27 @@ __global__ void __launch_bounds__(192, Q80 && TN == 64 ? 2 : 1) k_prompt_gemm(co
                     }
                 }
             } else {
-                if (!(ok = open())) break;
-                const uint32_t xb = base + 2u * WB, d = tmem + (gi & 1u) * TN;
+                const uint32_t xb = base + 2u * WB;
+                for (uint32_t k = 0; k < 4u; k++) {
+                    if (!(ok = open())) break;
 #pragma unroll
-                for (uint32_t p = 0; p < 3; p++)          // small x large, large x small, large x large
-#pragma unroll
-                    for (uint32_t k = 0; k < 4; k++)
-                        tc_mma_ss(d, tc_desc(base + (p == 0 ? WB : 0u)) + 2u * k, tc_desc(xb + (p == 1 ? XB : 0u)) + 2u * k, idesc, p > 0 || k > 0);
-                close();
+                    for (uint32_t p = 0; p < 4; p++)          // small x small, small x large, large x small, large x large
+                        tc_mma_ss(tmem + (gi & 1u) * TN, tc_desc(base + (p < 2 ? WB : 0u)) + 2u * k, tc_desc(xb + (p == 0 || p == 2 ? XB : 0u)) + 2u * k, idesc, p > 0);
+                    close();
+                }
             }
             if (ok) tc_commit(empty + (i % ST) * 8u);
         }
         if (!ok) bad_s = 2;
     } else if (warp >= 2) {
         const uint32_t quad = warp & 3u, n = n0 + quad * 32u + lane, nr = min(n, a.N - 1u), lanes = (quad * 32u) << 16;
-        float acc[TN];
+        float acc[TN], low[Q80 ? 1 : TN];          // low: what acc is too large by (F32)
 #pragma unroll
         for (int j = 0; j < TN; j++) acc[j] = 0.0f;
+        if (!Q80) {
+#pragma unroll
+            for (int j = 0; j < TN; j++) low[Q80 ? 0 : j] = 0.0f;
+        }
         bool ok = true;
         // the scales of a group are fetched two groups ahead: the row's own into a register, the positions' into shared memory (a global load per group
         // between a full accumulator and its sums cost 2.5 us a group: 250 x 1024 x 3072 took 62 us)
@@ -260,7 +267,12 @@ __global__ void __launch_bounds__(192, Q80 && TN == 64 ? 2 : 1) k_prompt_gemm(co
                         acc[c + j + 2] = fmaf((float)(int)v[j + 2], w * x.z, acc[c + j + 2]); acc[c + j + 3] = fmaf((float)(int)v[j + 3], w * x.w, acc[c + j + 3]);
                     } else {
 #pragma unroll
-                        for (int q = 0; q < 4; q++) acc[c + j + q] += __uint_as_float(v[j + q]);
+                        for (int q = 0; q < 4; q++) {
+                            float &lo = low[Q80 ? 0 : c + j + q];
+                            const float y = __fsub_rn(__uint_as_float(v[j + q]), lo), sum = __fadd_rn(acc[c + j + q], y);
+                            lo = __fsub_rn(__fsub_rn(sum, acc[c + j + q]), y);
+                            acc[c + j + q] = sum;
+                        }
                     }
                 }
             }
@@ -379,7 +391,7 @@ int launch(void (*k)(const A), dim3 grid, dim3 block, size_t smem, cudaStream_t 
     return 0;
 }
 template <bool Q80, int TN>
-int optin() { NB_CK(cudaFuncSetAttribute((const void *)k_prompt_gemm<Q80, TN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_smem<Q80, TN>())); return 0; }
+int optin() { NB_CK(nb::smem_at_least((const void *)k_prompt_gemm<Q80, TN>, (int)gemm_smem<Q80, TN>())); return 0; }
 }  // namespace
 
 struct Product { PrefillMat m; CUtensorMap wmap; const float *winv = nullptr; uint32_t np = 0; };      // np: F32 depth padded to 64
@@ -455,8 +467,8 @@ int create(PrefillState *s, const PrefillModel &m) {
     *s->err_host = 0;
     NB_CK(cudaHostGetDevicePointer(&s->err_dev, s->err_host, 0));
     if ((r = attn_tc_setup(&s->attn, std::min<size_t>(attn_tc_bytes(m.max_seq, m.KV, m.hd, m.hd), (size_t)1 << 30), attn_tc_tiles(m.max_seq, m.KV), s->err_dev))) return r;
-    if (q80 ? ((r = optin<true, 64>()) || (r = optin<true, 128>())) : ((r = optin<false, 64>()) || (r = optin<false, 128>()))) return r;
-    if (!q80 && (size_t)wide * 4u > 48u * 1024u) NB_CK(cudaFuncSetAttribute((const void *)k_prompt_prep<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(wide * 4u)));
+    if (q80 ? ((r = optin<true, 64>()) || (r = optin<true, 128>())) : (r = optin<false, 64>())) return r;
+    if (!q80 && (size_t)wide * 4u > 48u * 1024u) NB_CK(nb::smem_at_least((const void *)k_prompt_prep<false>, (int)(wide * 4u)));
     NB_CK(cudaDeviceSynchronize());
     return 0;
 }
@@ -465,8 +477,9 @@ int prep(PrefillState *s, const float *src, uint32_t ld, const float *gain, uint
     return s->m.quant == 0x80u ? launch<PromptPrepArgs>(k_prompt_prep<true>, dim3(T), dim3(kPrepThreads), 0, stream, s->pdl, a) : launch<PromptPrepArgs>(k_prompt_prep<false>, dim3(T), dim3(kPrepThreads), (size_t)n * 4, stream, s->pdl, a);
 }
 int product(PrefillState *s, const Product &w, float *C, uint32_t ldc, bool add, uint32_t T, cudaStream_t stream) {
-    // 64 positions per tile where tiles of 128 leave SMs without a block (1024 rows of the O product: 8 blocks for 128 positions)
-    const uint32_t rt = (w.m.rows + kRows - 1u) / kRows, tn = T <= 64u || rt * ((T + 127u) / 128u) < s->sms ? 64u : 128u;
+    // 64 positions per tile where tiles of 128 leave SMs without a block (1024 rows of the O product: 8 blocks for 128 positions), and in F32, whose
+    // sums take two registers each
+    const uint32_t rt = (w.m.rows + kRows - 1u) / kRows, tn = s->m.quant != 0x80u || T <= 64u || rt * ((T + 127u) / 128u) < s->sms ? 64u : 128u;
     PromptGemmArgs a{};
     a.wmap = w.wmap;
     for (const auto &m : s->amaps) if (m.n == w.m.n && m.tn == tn) a.amap = m.map;
@@ -480,7 +493,7 @@ int product(PrefillState *s, const Product &w, float *C, uint32_t ldc, bool add,
     const dim3 grid(rt, (T + tn - 1u) / tn, ks), block(192);
 #define GEMM(q, t) launch<PromptGemmArgs>(k_prompt_gemm<q, t>, grid, block, gemm_smem<q, t>(), stream, s->pdl, a, ks)
     if (s->m.quant == 0x80u) return tn == 64u ? GEMM(true, 64) : GEMM(true, 128);
-    return tn == 64u ? GEMM(false, 64) : GEMM(false, 128);
+    return GEMM(false, 64);
 #undef GEMM
 }
 }  // namespace

@@ -84,3 +84,18 @@ def test_a_call_that_decodes_nothing_leaves_the_last_prompt_position(n):
     eng.decode_greedy(ids.copy(), n, n)
     assert rel(eng.logits(), want) < 1e-5
     eng.close()
+
+
+def test_a_smaller_model_opened_later_leaves_the_larger_one_working():
+    """The limit of dynamic shared memory belongs to a kernel, not to an engine."""
+    big = E.Engine(mf.cached_model(dataclasses.replace(mf.PRESETS["mini-nano"], name="mini-nano-two", block_size=2048), mf.QUANT_F32, 128), 600)
+    ids = np.zeros(60, np.uint32)
+    ids[:40] = mf.teacher_tokens(40, 512)
+    want = ids.copy()
+    big.decode_greedy(want, 40, 60)
+    small = E.Engine(mf.cached_model(dataclasses.replace(mf.PRESETS["toy-nano"], name="toy-nano-two", block_size=2048), mf.QUANT_F32, 128), 100)
+    got = ids.copy()
+    big.decode_greedy(got, 40, 60)
+    assert got.tolist() == want.tolist()
+    small.close()
+    big.close()
