@@ -26,6 +26,7 @@
 #include "family.h"
 #define NB_K static
 #include "kernels.cuh"
+#include "prompt_split.h"
 #include "tc_ptx.cuh"
 
 namespace nb {
@@ -149,11 +150,9 @@ __global__ void __launch_bounds__(192, Q80 && TN == 64 ? 2 : 1) k_prompt_gemm(co
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, ring = (smem_u32(tc_raw) + 1023u) & ~1023u;
     const uint32_t n0 = blockIdx.x * kRows, m0 = blockIdx.y * TN;
     const uint32_t full = smem_u32(bars), empty = full + ST * 8u, tfull = empty + ST * 8u, tfree = tfull + 16u;
-    // this block's share of the depth, in whole units of stages and groups; groups: the depth that one tensor-memory accumulator takes before it is added
-    // up in fp32
-    const uint32_t us = Q80 && a.gs > 128u ? a.gs / 128u : 1u, units = ((Q80 ? (a.n + 127u) / 128u : a.np / 64u) + us - 1u) / us, per_part = (units + a.ks - 1u) / a.ks;
-    const uint32_t u0 = min(units, blockIdx.z * per_part), s0 = u0 * us, steps = min(per_part, units - u0) * us;
-    const uint32_t g0 = Q80 ? s0 * 128u / a.gs : s0, groups = Q80 ? min(a.n, (s0 + steps) * 128u) / a.gs - g0 : steps * 4u, all_groups = Q80 ? a.n / a.gs : 0u;
+    // this block's share of the depth; groups: the depth that one tensor-memory accumulator takes before it is added up in fp32
+    const PromptPart part = prompt_part(Q80, a.n, a.np, a.gs, a.ks, blockIdx.z);
+    const uint32_t s0 = part.s0, steps = part.steps, g0 = part.g0, groups = Q80 ? part.groups : steps * 4u, all_groups = Q80 ? a.n / a.gs : 0u;
     if (threadIdx.x == 0) {
         for (uint32_t i = 0; i < ST; i++) { mbar_init(full + i * 8u, 1); mbar_init(empty + i * 8u, 1); }
         for (uint32_t i = 0; i < 2; i++) { mbar_init(tfull + i * 8u, 1); mbar_init(tfree + i * 8u, 4); }
@@ -485,10 +484,8 @@ int product(PrefillState *s, const Product &w, float *C, uint32_t ldc, bool add,
     for (const auto &m : s->amaps) if (m.n == w.m.n && m.tn == tn) a.amap = m.map;
     a.ws = static_cast<const float *>(w.m.aux); a.xs = s->scales; a.ldx = kChunk; a.winv = w.winv; a.xinv = s->scales;
     a.N = w.m.rows; a.T = T; a.n = w.m.n; a.gs = s->m.gs; a.np = w.np; a.C = C; a.ldc = ldc; a.add = add ? 1u : 0u; a.err = s->err_dev;
-    // clusters share a tile's depth while fewer than half of the SMs have a block, down to two units of 128 (Q80) or 64 (F32) each
-    const uint32_t tiles = rt * ((T + tn - 1u) / tn), units = s->m.quant == 0x80u ? w.m.n / std::max(128u, s->m.gs) : w.np / 64u;
-    uint32_t ks = 1;
-    while (ks < 8u && tiles * ks * 2u <= s->sms && units >= ks * 4u) ks *= 2u;
+    // clusters share a tile's depth while fewer than half of the SMs have a block
+    const uint32_t tiles = rt * ((T + tn - 1u) / tn), ks = prompt_parts(prompt_units(s->m.quant == 0x80u, w.m.n, w.np, s->m.gs), tiles, s->sms);
     a.ks = ks;
     const dim3 grid(rt, (T + tn - 1u) / tn, ks), block(192);
 #define GEMM(q, t) launch<PromptGemmArgs>(k_prompt_gemm<q, t>, grid, block, gemm_smem<q, t>(), stream, s->pdl, a, ks)

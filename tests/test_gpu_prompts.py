@@ -26,12 +26,10 @@ CASES = [("toy-nano", mf.QUANT_F32, 128), ("toy-qwen3", mf.QUANT_F32, 128), ("to
          ("mini-qwen3", mf.QUANT_Q80, 128), ("mini-nano", mf.QUANT_F32, 128), ("toy-nano-odd", mf.QUANT_F32, 128)]
 
 
-@pytest.mark.parametrize("name,quant,gs", CASES)
-def test_portions_against_single_positions(name, quant, gs):
-    spec = dataclasses.replace(mf.PRESETS[name], name=name + "-prompts", block_size=2048)
-    eng = E.Engine(mf.cached_model(spec, quant, gs), 1200)
+def check(spec, quant, gs, lengths, room=1200):
+    """Prompts of these lengths in portions against the same positions one call at a time."""
+    eng = E.Engine(mf.cached_model(spec, quant, gs), room)
     toks = mf.teacher_tokens(1160, spec.vocab)
-    lengths = (33, 65, 129, 130, 257) if name != "toy-qwen3" else (34, 64, 1025, 1154)
     n = max(lengths)
     last, want, keep = spec.n_layer - 1, {}, {}
     for p in range(n):
@@ -44,7 +42,7 @@ def test_portions_against_single_positions(name, quant, gs):
             keep[p] = [rows(eng, spec, l, p) for l in (0, last)]
     tol = 1e-5 if quant == mf.QUANT_F32 else 4e-2
     for m in lengths:
-        ids = np.zeros(m + 2, np.uint32)
+        ids = np.zeros(max(m, 33) + 2, np.uint32)
         ids[:33] = toks[:33][::-1]
         eng.decode_greedy(ids, 33, 34)          # leaves rows of another prompt behind
         ids[:m] = toks[:m]
@@ -54,6 +52,18 @@ def test_portions_against_single_positions(name, quant, gs):
             assert rel(rows(eng, spec, 0, p), keep[p][0]) < 2e-6, (m, p)
             assert rel(rows(eng, spec, last, p), keep[p][1]) < tol, (m, p)
     eng.close()
+
+
+@pytest.mark.parametrize("name,quant,gs", CASES)
+def test_portions_against_single_positions(name, quant, gs):
+    check(dataclasses.replace(mf.PRESETS[name], name=name + "-prompts", block_size=2048), quant, gs, (33, 65, 129, 130, 257) if name != "toy-qwen3" else (34, 64, 1025, 1154))
+
+
+@pytest.mark.parametrize("width,ff,gs", [(1088, 2240, 32), (1088, 2240, 64), (544, 1120, 32), (320, 4160, 64)])
+def test_depths_that_no_stage_of_128_divides(width, ff, gs):
+    """The last stage of a depth is a short one, and where 2, 4 or 8 blocks share the depth the last of them may have none (9 stages over 4 blocks, 18 over 8)."""
+    spec = mf.ModelSpec("prompts-%d-%d" % (width, ff), mf.ARCH_NANO, 2048, 512, 2, width, 8 if width == 544 else 16, 8, ff)
+    check(spec, mf.QUANT_Q80, gs, (10, 65, 66, 130), 400)
 
 
 def test_penalty_sees_the_prompt_and_short_prompts_stay_as_they_were():
