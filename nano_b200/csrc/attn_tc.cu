@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(192, 1) k_attn_tc(const AttnTcArgs ta) {
         float vinv = 0.0f;
         // the values of the tile before join the sum, which then moves to the new maximum
         auto collect = [&](uint32_t i, float corr) {
-            ok = mbar_wait(bar(OREADY), i & 1u);
+            ok = mbar_wait_warp(bar(OREADY), i & 1u);
             if (!ok) return;
             tc_fence_after();
             const float f = vinv * corr;
@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(192, 1) k_attn_tc(const AttnTcArgs ta) {
             const uint32_t key0 = (lo + i) * kTile, s_at = tmem + lane_base + SCOL + (i & 1u) * kTile;
             const float kc = qinv * scales[2u * i] * (a.softcap > 0.0f ? a.scale / a.softcap : a.scale);
             const bool whole = key0 + kTile <= first_pos + 1u && key0 >= low_last;          // every row of the block sees every key of the tile
-            ok = __all_sync(0xffffffffu, mbar_wait(bar(SFULL0 + (i & 1u)), (i >> 1) & 1u));
+            ok = mbar_wait_warp(bar(SFULL0 + (i & 1u)), (i >> 1) & 1u);
             if (!ok) break;
             tc_fence_after();
             const uint32_t j0 = low > key0 ? low - key0 : 0u, j1 = pos < key0 ? 0u : min(kTile, pos - key0 + 1u);          // the keys this row sees
@@ -286,7 +286,6 @@ __global__ void __launch_bounds__(192, 1) k_attn_tc(const AttnTcArgs ta) {
             if (a.softcap > 0.0f && top != -INFINITY) top = a.softcap * tanhf(top);
             const float mn = fmaxf(m, top), corr = mn == -INFINITY ? 1.0f : expf(m - mn);
             if (i) collect(i - 1u, corr);
-            ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             vinv = scales[2u * i + 1u] / kWeightScale;
             float sum = 0.0f;
@@ -323,7 +322,7 @@ __global__ void __launch_bounds__(192, 1) k_attn_tc(const AttnTcArgs ta) {
             __syncwarp();
             if (lane == 0) mbar_arrive(bar(PREADY));
         }
-        if (ok) { collect(n - 1u, 1.0f); ok = __all_sync(0xffffffffu, ok); }
+        if (ok) collect(n - 1u, 1.0f);
         if (!ok) bad_s = 4;
         if (ok && r0 + r <= last) {
             float f = 1.0f / l;

@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(192) k_gemm_tc(const __grid_constant__ TcArgs 
     bool live = true;
     const uint32_t quad = warp & 3u, n = n0 + quad * 32u + lane, rows = gv.rows;
     if (warp >= 2) {
-        live = mbar_wait(done, 0);
+        live = mbar_wait_warp(done, 0);
         if (!live) bad_s = 3;
         tc_fence_after();
     }

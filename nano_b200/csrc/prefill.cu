@@ -240,19 +240,17 @@ __global__ void __launch_bounds__(192, Q80 && TN == 64 ? 2 : 1) k_prompt_gemm(co
         const uint32_t et = threadIdx.x - 64u;
         auto weight_scale = [&](uint32_t g) { return Q80 && g < groups ? __ldg(ws + g) : 0.0f; };
         auto act_scale = [&](uint32_t g) { return Q80 && g < groups && et < (uint32_t)TN ? __ldcg(a.xs + (size_t)(g0 + g) * a.ldx + m0 + et) : 0.0f; };
-        auto meet = []() { asm volatile("bar.sync 1, 128;" ::: "memory"); };
         float w0 = weight_scale(0), w1 = weight_scale(1);
         if (Q80) {
             const float x0 = act_scale(0), x1 = act_scale(1);
             if (et < (uint32_t)TN) { xs_s[0][et] = x0; xs_s[1][et] = x1; }
-            meet();
+            bar_any(1, 128, false);
         }
         uint32_t slot = 0;
         for (uint32_t g = 0; g < groups; g++) {
             const float w = w0, x2 = act_scale(g + 2u);
             w0 = w1; w1 = weight_scale(g + 2u);
-            ok = __all_sync(0xffffffffu, mbar_wait(tfull + (g & 1u) * 8u, (g >> 1) & 1u));
-            if (!ok) bad_s = 3;          // (the warps stay together for the barrier below; what they add up is not used)
+            ok = mbar_wait_warp(tfull + (g & 1u) * 8u, (g >> 1) & 1u);          // (when it ran out: what is added up below is not used)
             tc_fence_after();
 #pragma unroll
             for (int c = 0; c < TN; c += 32) {
@@ -280,9 +278,8 @@ __global__ void __launch_bounds__(192, Q80 && TN == 64 ? 2 : 1) k_prompt_gemm(co
             if (lane == 0) mbar_arrive(tfree + (g & 1u) * 8u);
             if (Q80) {
                 if (et < (uint32_t)TN) xs_s[slot == 0 ? 2 : slot - 1][et] = x2;          // the buffer of the group before this one
-                meet();
+                ok = !bar_any(1, 128, !ok);          // the four warps leave together: none is left at this barrier
                 slot = slot == 2 ? 0 : slot + 1;
-                ok = bad_s == 0;
             }
             if (!ok) break;
         }
@@ -306,6 +303,7 @@ __global__ void __launch_bounds__(192, Q80 && TN == 64 ? 2 : 1) k_prompt_gemm(co
             for (int j = 0; j < TN; j++) if ((uint32_t)j < live) dst[(size_t)j * a.ldc] = acc[j];
         }
     }
+    __syncwarp();
     if (a.ks > 1u) {          // every block of the cluster finishes TN / ks positions: its own and its peers' parts, added in the order of the depth
         cluster_sync_all();
         const uint32_t quad = warp & 3u, n = n0 + quad * 32u + lane, span = TN / a.ks, j0 = blockIdx.z * span, j1 = min(j0 + span, a.T - m0);

@@ -22,6 +22,14 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
         if (clock64() - t0 > 4000000000ll) return false;
     return true;
 }
+// The same for a whole warp, one verdict for all of it: a warp that goes on to .sync.aligned instructions (tcgen05.ld, barriers) must not part over a wait
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)); }
+// named barrier `id` of `threads` threads that hands every one of them the same answer: does `p` hold for any
+__device__ __forceinline__ bool bar_any(uint32_t id, uint32_t threads, bool p) {
+    uint32_t any;
+    asm volatile("{\n.reg .pred p, q;\nsetp.ne.u32 p, %3, 0;\nbarrier.cta.red.or.pred q, %1, %2, p;\nselp.u32 %0, 1, 0, q;\n}" : "=r"(any) : "r"(id), "r"(threads), "r"((uint32_t)p) : "memory");
+    return any != 0;
+}
 __device__ __forceinline__ void tma_3d(uint32_t dst, const CUtensorMap *map, uint32_t x, uint32_t y, uint32_t z, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
                  ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar) : "memory");
