@@ -174,8 +174,9 @@ __global__ void __launch_bounds__(192, 1) k_attn_tc(const AttnTcArgs ta) {
             load8(a.q + (size_t)(rr / rep) * a.ldq + (size_t)(g * rep + rr % rep) * a.q_head + c, a.D - c, x);
             m = fmaxf(m, max8(x));
         }
-        const float s = tile_scale(block_max<192>(m, red));
+        float s = tile_scale(block_max<192>(m, red));
         qinv = 1.0f / s;
+        if (a.scale < 0.0f) s = -s;          // the largest raw score is to be the largest score: the sign of a negative scale goes with the query
         for (uint32_t i = tid; i < kTile * d8; i += 192u) {
             const uint32_t r = i / d8, c = i % d8, rr = min(r0 + r, last);
             load8(a.q + (size_t)(rr / rep) * a.ldq + (size_t)(g * rep + rr % rep) * a.q_head + c * 8u, c * 8u < a.D ? a.D - c * 8u : 0u, x);
@@ -263,7 +264,7 @@ __global__ void __launch_bounds__(192, 1) k_attn_tc(const AttnTcArgs ta) {
         };
         for (uint32_t i = 0; i < n; i++) {
             const uint32_t key0 = (lo + i) * kTile, s_at = tmem + lane_base + SCOL + (i & 1u) * kTile;
-            const float kc = qinv * scales[2u * i] * (a.softcap > 0.0f ? a.scale / a.softcap : a.scale);
+            const float kc = qinv * scales[2u * i] * (a.softcap > 0.0f ? fabsf(a.scale) / a.softcap : fabsf(a.scale));
             const bool whole = key0 + kTile <= first_pos + 1u && key0 >= low_last;          // every row of the block sees every key of the tile
             ok = mbar_wait_warp(bar(SFULL0 + (i & 1u)), (i >> 1) & 1u);
             if (!ok) break;

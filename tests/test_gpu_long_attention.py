@@ -71,3 +71,25 @@ def test_latents_multiplied_out(tmp_path, design, heads, dim, vdim, rank, size):
         assert d.max() < 1.2e-2, (cuts, int(d.argmax()))
         assert np.linalg.norm(got - ref[:at]) < 2e-2 * np.linalg.norm(ref[:at]), cuts
     eng.close()
+
+
+@pytest.mark.parametrize("design", ["famudra", "vumunex"])
+def test_negative_scale(tmp_path, design):
+    """A folder may state any number: the most negative product is then the largest score, in portions as in single tokens (bound as above)."""
+    mixer = {"heads": 3, "dim": 64, "vdim": 40, "kv_rank": 48, "scale": -0.5}
+    if design == "famudra":
+        cfg, make, oracle = md.famudra_config(64, 96, [("latent_attention", dict(mixer, q_rank=56), None)]), md.famudra_random, A.forward
+    else:
+        cfg, make, oracle = md.vumunex_config(64, 96, [("latent_attention", mixer, None)], streams=2), md.vumunex_random, V.forward
+    w = make(cfg, 5)
+    eng = E.Engine(md.write_model_dir(str(tmp_path / "m"), cfg, w), 512)
+    toks = np.random.default_rng(2).integers(0, 64, size=300).astype(np.uint32)
+    ref = oracle(cfg, w, toks)
+    s = eng.seq_open()
+    one = np.concatenate([eng.step(s, toks[i:i + 1], [0]) for i in range(toks.size)])
+    eng.seq_close(s)
+    s = eng.seq_open()
+    got = eng.step(s, toks, range(toks.size))
+    eng.close()
+    assert np.sqrt(((got - one) ** 2).mean(-1) / (one ** 2).mean(-1)).max() < 1.2e-2
+    assert np.linalg.norm(got - ref) < 2e-2 * np.linalg.norm(ref)
