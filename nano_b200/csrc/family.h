@@ -33,8 +33,11 @@ inline cudaError_t smem_at_least(const void *kernel, int bytes) {
     std::lock_guard<std::mutex> hold(m);
     cudaFuncAttributes fa;
     const cudaError_t e = cudaFuncGetAttributes(&fa, kernel);
-    if (e != cudaSuccess || fa.maxDynamicSharedSizeBytes >= bytes) return e;
-    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e != cudaSuccess) return e;
+    // what a kernel may use without being asked is 48 KB with its static shared memory counted in: 12288 floats and one word more are too much
+    const size_t usual = 48u * 1024u;
+    if (bytes + fa.sharedSizeBytes <= usual || (fa.maxDynamicSharedSizeBytes >= bytes && (size_t)fa.maxDynamicSharedSizeBytes > usual)) return e;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, fa.maxDynamicSharedSizeBytes > bytes ? fa.maxDynamicSharedSizeBytes : bytes);
 }
 
 struct EngineOps {

@@ -465,7 +465,7 @@ int create(PrefillState *s, const PrefillModel &m) {
     NB_CK(cudaHostGetDevicePointer(&s->err_dev, s->err_host, 0));
     if ((r = attn_tc_setup(&s->attn, std::min<size_t>(attn_tc_bytes(m.max_seq, m.KV, m.hd, m.hd), (size_t)1 << 30), attn_tc_tiles(m.max_seq, m.KV), s->err_dev))) return r;
     if (q80 ? ((r = optin<true, 64>()) || (r = optin<true, 128>())) : (r = optin<false, 64>())) return r;
-    if (!q80 && (size_t)wide * 4u > 48u * 1024u) NB_CK(nb::smem_at_least((const void *)k_prompt_prep<false>, (int)(wide * 4u)));
+    if (!q80) NB_CK(nb::smem_at_least((const void *)k_prompt_prep<false>, (int)(wide * 4u)));
     NB_CK(cudaDeviceSynchronize());
     return 0;
 }

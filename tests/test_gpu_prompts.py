@@ -109,3 +109,9 @@ def test_a_smaller_model_opened_later_leaves_the_larger_one_working():
     assert got.tolist() == want.tolist()
     small.close()
     big.close()
+
+
+@pytest.mark.parametrize("ff", [12256, 12288, 12320])
+def test_rows_around_the_shared_memory_that_needs_no_asking(ff):
+    """A 32-bit row of 12288 hidden units (Qwen3-8B's) is 48 KB, to which a kernel's static shared memory comes on top."""
+    check(mf.ModelSpec("prompts-64-%d" % ff, mf.ARCH_NANO, 512, 512, 2, 64, 2, 2, ff), mf.QUANT_F32, 128, (10, 65), 200)
