@@ -6,20 +6,19 @@
 //
 //   k_prompt_embed     token rows
 //   k_prompt_prep      a position's activation: RMS norm with gain, plain, or SwiGLU of interleaved pairs; then Q80 codes + group scales, or
-//                      (F32) two f16 parts of the row scaled by a power of two
+//                      (F32) three bfloat16 parts
+//   k_weight_parts     F32: a matrix in three bfloat16 parts, into one workspace for all of them (its bytes pass through memory two and a half times
+//                      more for that; a copy that stays would hold half again as much as the file)
 //   k_prompt_gemm      C[t][n] (+)= sum over groups: tcgen05.mma on 128 weight rows x TN positions, the accumulator of a GROUP in tensor memory (two
 //                      buffers), added to fp32 registers by the threads that own the rows while the next group multiplies.
-//                      Q80: kind::i8, int32 exact, times weight scale x activation scale.  F32: kind::f16 on two parts of both
-//                      operands, all four products, over 16 of the depth; the tensor cores cut what they add, so they add four
-//                      times only, and what they leave is added up with its rounding error carried along.  Logits against 64
-//                      bits by those of single positions, 40 / 200 positions and four layers of width 768: 1.14 / 1.16 with
-//                      three products, 64 of the depth and a plain sum, 1.06 / 1.09 with 32 and the error carried, 1.02 / 1.04 so
-//                      (attn_tc.cu's shorter sums included).
+//                      Q80: kind::i8, int32 exact, times weight scale x activation scale.  F32: kind::f16 on three bfloat16 parts of both
+//                      operands, which are all of their 24 bits, all nine products, over 16 of the depth; the tensor cores cut what they add, so they
+//                      add nine times only, the small products first, and what they leave is added up with its rounding error carried along.
 //   k_prompt_rope      head norm (Qwen3), rotary positions, K and V rows into the cache
 //   attention          attn_tc.cu
 #include "prefill.h"
 
-#include <cuda_fp16.h>
+#include <cuda_bf16.h>
 
 #include <algorithm>
 
@@ -48,26 +47,31 @@ __global__ void __launch_bounds__(256) k_prompt_embed(const PromptEmbedArgs a) {
     }
 }
 
-// codes [T][n] and scales [n / gs][lds] (Q80), or parts [T][2][np] and the inverse of the row's scale (F32)
-struct PromptPrepArgs { const float *src; uint32_t ld; const float *gain; uint32_t n, gs, mode; int8_t *codes; float *scales; uint32_t lds; __half *parts; uint32_t np; float *rinv; };
+// x = p[0] + p[1] + p[2], three times 8 bits: exact as long as the last part is no smaller than 2^-133.  A number that has no neighbour in bfloat16 (the
+// largest ones would round to infinity) is cut; infinities and NaN stay in the first part
+__device__ __forceinline__ void split3(float x, __nv_bfloat16 (&p)[3]) {
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        __nv_bfloat16 h = __float2bfloat16_rn(x);
+        if (fabsf(__bfloat162float(h)) == INFINITY && fabsf(x) < INFINITY) h = __float2bfloat16_rz(x);
+        p[i] = h;
+        x = fabsf(x) < INFINITY ? x - __bfloat162float(h) : 0.0f;
+    }
+}
+
+// codes [T][n] and scales [n / gs][lds] (Q80), or parts [T][3][np] (F32)
+struct PromptPrepArgs { const float *src; uint32_t ld; const float *gain; uint32_t n, gs, mode; int8_t *codes; float *scales; uint32_t lds; __nv_bfloat16 *parts; uint32_t np; };
 __device__ __forceinline__ float prep_value(const PromptPrepArgs &a, const float *s, float inv, uint32_t i) {
     if (a.mode == PREP_NORM) return __fmul_rn(a.gain[i], __fmul_rn(inv, s[i]));
     if (a.mode == PREP_PLAIN) return s[i];
     const float2 v = *reinterpret_cast<const float2 *>(s + 2u * i);
     return __fmul_rn(__fmul_rn(v.x, __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-v.x)))), v.y);
 }
-// a power of two that brings `big` to [2^14, 2^15)
-__device__ __forceinline__ float power_scale(float big) {
-    const int e = (int)(__float_as_uint(big) >> 23) - 127;
-    if (!(big > 0.0f) || e > 127) return 1.0f;
-    return __uint_as_float((uint32_t)(127 + max(-113, min(100, 14 - e))) << 23);
-}
 constexpr uint32_t kPrepThreads = 512;
 template <bool Q80>
 __global__ void __launch_bounds__(kPrepThreads) k_prompt_prep(const PromptPrepArgs a) {
     dep_enter();
     __shared__ float red[32];
-    extern __shared__ float val[];
     const uint32_t t = blockIdx.x, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const float *s = a.src + (size_t)t * a.ld;
     float inv = 1.0f;
@@ -90,42 +94,44 @@ __global__ void __launch_bounds__(kPrepThreads) k_prompt_prep(const PromptPrepAr
             if (lane == 0) a.scales[(size_t)g * a.lds + t] = sc;
         }
     } else {
-        float m = 0.0f;
-        for (uint32_t i = threadIdx.x; i < a.n; i += kPrepThreads) { const float v = prep_value(a, s, inv, i); val[i] = v; m = fmaxf(m, fabsf(v)); }
-        m = block_max<kPrepThreads>(m, red);
-        const float sc = power_scale(m);
-        __half *hi = a.parts + (size_t)t * 2u * a.np, *lo = hi + a.np;
+        __nv_bfloat16 *to = a.parts + (size_t)t * 3u * a.np;
         for (uint32_t i = threadIdx.x; i < a.np; i += kPrepThreads) {
-            const float v = i < a.n ? val[i] * sc : 0.0f;
-            const __half h = __float2half_rn(v);
-            hi[i] = h; lo[i] = __float2half_rn(v - __half2float(h));
+            __nv_bfloat16 p[3];
+            split3(i < a.n ? prep_value(a, s, inv, i) : 0.0f, p);
+            to[i] = p[0]; to[a.np + i] = p[1]; to[2u * a.np + i] = p[2];
         }
-        if (threadIdx.x == 0) a.rinv[t] = 1.0f / sc;
     }
 }
 
-// F32 weights: the largest magnitude (as float bits), then two f16 parts [rows][2][np] under one scale for the matrix
-__global__ void k_weight_max(const float *w, size_t n, uint32_t *bits) {
-    float m = 0.0f;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) m = fmaxf(m, fabsf(w[i]));
-    m = warp_max(m);
-    if ((threadIdx.x & 31u) == 0) atomicMax(bits, __float_as_uint(m));
-}
-__global__ void k_weight_parts(const float *w, uint32_t rows, uint32_t n, uint32_t np, const uint32_t *bits, __half *parts, float *inv) {
-    const float sc = power_scale(__uint_as_float(*bits));
-    const size_t total = (size_t)rows * np;
+// F32 weights [rows][n] in parts [rows][3][np]; n and np are multiples of 8, a thread makes 8 columns
+struct WeightPartsArgs { const float *w; uint32_t rows, n, np; __nv_bfloat16 *parts; };
+__global__ void __launch_bounds__(256) k_weight_parts(const WeightPartsArgs a) {
+    dep_enter();
+    const uint32_t n8 = a.np / 8u;
+    const size_t total = (size_t)a.rows * n8;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const uint32_t r = (uint32_t)(i / np), c = (uint32_t)(i % np);
-        const float v = c < n ? w[(size_t)r * n + c] * sc : 0.0f;
-        const __half h = __float2half_rn(v);
-        parts[(size_t)r * 2u * np + c] = h; parts[(size_t)r * 2u * np + np + c] = __float2half_rn(v - __half2float(h));
+        const uint32_t r = (uint32_t)(i / n8), c = (uint32_t)(i % n8) * 8u;
+        __align__(16) __nv_bfloat16 o[3][8];
+#pragma unroll
+        for (uint32_t q = 0; q < 2; q++) {
+            const float4 v = c < a.n ? __ldcs(reinterpret_cast<const float4 *>(a.w + (size_t)r * a.n + c) + q) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            const float x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (uint32_t j = 0; j < 4; j++) {
+                __nv_bfloat16 p[3];
+                split3(x[j], p);
+#pragma unroll
+                for (int k = 0; k < 3; k++) o[k][q * 4u + j] = p[k];
+            }
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < 3; k++) *reinterpret_cast<uint4 *>(a.parts + (size_t)r * 3u * a.np + k * a.np + c) = *reinterpret_cast<const uint4 *>(o[k]);
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) *inv = 1.0f / sc;
 }
 
 // add: C += (the residual stream), else C =
 struct alignas(64) PromptGemmArgs {
-    CUtensorMap wmap, amap; const float *ws, *xs; uint32_t ldx; const float *winv, *xinv;
+    CUtensorMap wmap, amap; const float *ws, *xs; uint32_t ldx;
     uint32_t N, T, n, gs, np; float *C; uint32_t ldc, add, ks; uint32_t *err;      // ks: blocks of a cluster (along z) that share a tile's depth
 };
 __device__ __forceinline__ void tma_2d(uint32_t dst, const CUtensorMap *map, uint32_t x, uint32_t y, uint32_t bar) {
@@ -134,9 +140,9 @@ __device__ __forceinline__ void tma_2d(uint32_t dst, const CUtensorMap *map, uin
 __device__ __forceinline__ void tc_mma_i8(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, bool add) {
     asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n}" ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"((uint32_t)add) : "memory");
 }
-// a stage holds 128 bytes of the depth of 128 weight rows and TN positions: 128 int8, or 64 f16 of both parts
-template <bool Q80, int TN> __host__ __device__ constexpr uint32_t gemm_stage() { return (kRows + (uint32_t)TN) * 128u * (Q80 ? 1u : 2u); }
-template <bool Q80, int TN> __host__ __device__ constexpr uint32_t gemm_stages() { return Q80 && TN == 128 ? 6u : 4u; }
+// a stage holds 128 bytes of the depth of 128 weight rows and TN positions: 128 int8, or 64 bfloat16 of all three parts
+template <bool Q80, int TN> __host__ __device__ constexpr uint32_t gemm_stage() { return (kRows + (uint32_t)TN) * 128u * (Q80 ? 1u : 3u); }
+template <bool Q80, int TN> __host__ __device__ constexpr uint32_t gemm_stages() { return !Q80 ? 3u : TN == 128 ? 6u : 4u; }
 template <bool Q80, int TN> constexpr size_t gemm_smem() { return (size_t)gemm_stages<Q80, TN>() * gemm_stage<Q80, TN>() + 1024u; }
 
 template <bool Q80, int TN>
@@ -165,27 +171,27 @@ __global__ void __launch_bounds__(192, Q80 && TN == 64 ? 2 : 1) k_prompt_gemm(co
     tc_fence_after();
     // Only now may the next kernels' blocks come: one that waits for this grid while it holds tensor memory must not be in the way of an allocation here
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    const uint32_t tmem = tmem_s, npre = min(ST, steps);
+    const uint32_t tmem = tmem_s, npre = Q80 ? min(ST, steps) : 0u;
     auto weights = [&](uint32_t i) {
         const uint32_t dst = ring + (i % ST) * SB, bar = full + (i % ST) * 8u;
         mbar_expect(bar, SB);
         if (Q80) tma_2d(dst, &a.wmap, (s0 + i) * 128u, n0, bar);
-        else { tma_2d(dst, &a.wmap, (s0 + i) * 64u, n0, bar); tma_2d(dst + WB, &a.wmap, a.np + (s0 + i) * 64u, n0, bar); }
+        else for (uint32_t p = 0; p < 3; p++) tma_2d(dst + p * WB, &a.wmap, p * a.np + (s0 + i) * 64u, n0, bar);
     };
-    if (warp == 0 && lane == 0) for (uint32_t i = 0; i < npre; i++) weights(i);          // weights do not depend on the kernel before
+    if (warp == 0 && lane == 0) for (uint32_t i = 0; i < npre; i++) weights(i);          // Q80 weights do not depend on the kernels before
     asm volatile("griddepcontrol.wait;" ::: "memory");
     float *mine = reinterpret_cast<float *>(tc_raw + (ring - smem_u32(tc_raw)));          // [TN][128]: a part's sums, once the ring is free
     if (warp == 0 && lane == 0) {
         for (uint32_t i = 0; i < steps; i++) {
-            const uint32_t st = i % ST, bar = full + st * 8u, dst = ring + st * SB + (Q80 ? WB : 2u * WB);
+            const uint32_t st = i % ST, bar = full + st * 8u, dst = ring + st * SB + (Q80 ? WB : 3u * WB);
             if (i >= ST && !mbar_wait(empty + st * 8u, ((i / ST) - 1u) & 1u)) { bad_s = 1; break; }
-            if (i >= npre) weights(i);
+            if (!Q80 || i >= npre) weights(i);
             if (Q80) tma_2d(dst, &a.amap, (s0 + i) * 128u, m0, bar);
-            else { tma_2d(dst, &a.amap, (s0 + i) * 64u, m0, bar); tma_2d(dst + XB, &a.amap, a.np + (s0 + i) * 64u, m0, bar); }
+            else for (uint32_t p = 0; p < 3; p++) tma_2d(dst + p * XB, &a.amap, p * a.np + (s0 + i) * 64u, m0, bar);
         }
     } else if (warp == 1 && lane == 0) {
         constexpr uint32_t shape = ((uint32_t)(TN >> 3) << 17) | ((kRows >> 4) << 24);
-        constexpr uint32_t idesc = Q80 ? ((2u << 4) | (1u << 7) | (1u << 10) | shape) : ((1u << 4) | shape);          // int32 += int8 x int8; fp32 += f16 x f16
+        constexpr uint32_t idesc = Q80 ? ((2u << 4) | (1u << 7) | (1u << 10) | shape) : ((1u << 4) | (1u << 7) | (1u << 10) | shape);          // int32 += int8 x int8; fp32 += bf16 x bf16
         bool ok = true;
         uint32_t gi = 0;
         auto open = [&]() { const bool w = gi < 2u || mbar_wait(tfree + (gi & 1u) * 8u, ((gi >> 1) - 1u) & 1u); tc_fence_after(); return w; };
@@ -212,12 +218,14 @@ __global__ void __launch_bounds__(192, Q80 && TN == 64 ? 2 : 1) k_prompt_gemm(co
                     }
                 }
             } else {
-                const uint32_t xb = base + 2u * WB;
+                const uint32_t xb = base + 3u * WB;
                 for (uint32_t k = 0; k < 4u; k++) {
                     if (!(ok = open())) break;
 #pragma unroll
-                    for (uint32_t p = 0; p < 4; p++)          // small x small, small x large, large x small, large x large
-                        tc_mma_ss(tmem + (gi & 1u) * TN, tc_desc(base + (p < 2 ? WB : 0u)) + 2u * k, tc_desc(xb + (p == 0 || p == 2 ? XB : 0u)) + 2u * k, idesc, p > 0);
+                    for (uint32_t p = 0; p < 9; p++) {          // the smallest products first, large x large last
+                        constexpr uint32_t wp[9] = {2, 1, 2, 0, 2, 1, 0, 1, 0}, xp[9] = {2, 2, 1, 2, 0, 1, 1, 0, 0};
+                        tc_mma_ss(tmem + (gi & 1u) * TN, tc_desc(base + wp[p] * WB) + 2u * k, tc_desc(xb + xp[p] * XB) + 2u * k, idesc, p > 0);
+                    }
                     close();
                 }
             }
@@ -288,13 +296,8 @@ __global__ void __launch_bounds__(192, Q80 && TN == 64 ? 2 : 1) k_prompt_gemm(co
 #pragma unroll
             for (int j = 0; j < TN; j++) mine[j * kRows + quad * 32u + lane] = acc[j];
         } else if (n < a.N) {
-            const float wi = Q80 ? 1.0f : *a.winv;
             float *dst = a.C + (size_t)m0 * a.ldc + n;
             const uint32_t live = min((uint32_t)TN, a.T - m0);
-            if (!Q80) {
-#pragma unroll
-                for (int j = 0; j < TN; j++) acc[j] *= wi * __ldcg(a.xinv + m0 + j);
-            }
             if (a.add) {          // all loads before the first store: one after the other they were 30 us of a product
 #pragma unroll
                 for (int j = 0; j < TN; j++) if ((uint32_t)j < live) acc[j] += __ldcg(dst + (size_t)j * a.ldc);
@@ -308,7 +311,6 @@ __global__ void __launch_bounds__(192, Q80 && TN == 64 ? 2 : 1) k_prompt_gemm(co
         cluster_sync_all();
         const uint32_t quad = warp & 3u, n = n0 + quad * 32u + lane, span = TN / a.ks, j0 = blockIdx.z * span, j1 = min(j0 + span, a.T - m0);
         if (warp >= 2 && n < a.N && !bad_s) {
-            const float wi = Q80 ? 1.0f : *a.winv;
             const uint32_t at = smem_u32(mine + quad * 32u + lane);
             float *dst = a.C + (size_t)m0 * a.ldc + n;
             for (uint32_t j = j0; j < j1; j += 8u) {
@@ -321,10 +323,6 @@ __global__ void __launch_bounds__(192, Q80 && TN == 64 ? 2 : 1) k_prompt_gemm(co
                     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(at + j * kRows * 4u), "r"(p));
 #pragma unroll
                     for (uint32_t i = 0; i < 8; i++) f[i] += ld_cluster_f32(peer + i * kRows * 4u);
-                }
-                if (!Q80) {
-#pragma unroll
-                    for (uint32_t i = 0; i < 8; i++) f[i] *= wi * __ldcg(a.xinv + m0 + j + i);
                 }
                 if (a.add) {
 #pragma unroll
@@ -391,13 +389,14 @@ template <bool Q80, int TN>
 int optin() { NB_CK(nb::smem_at_least((const void *)k_prompt_gemm<Q80, TN>, (int)gemm_smem<Q80, TN>())); return 0; }
 }  // namespace
 
-struct Product { PrefillMat m; CUtensorMap wmap; const float *winv = nullptr; uint32_t np = 0; };      // np: F32 depth padded to 64
+struct Product { PrefillMat m; CUtensorMap wmap; uint32_t np = 0; };      // np: F32 depth padded to 64
 struct PrefillState {
     PrefillModel m; uint32_t sms = 148; bool pdl = true;
     decltype(&cuTensorMapEncodeTiled) encode = nullptr;
     std::vector<Product> qkv, wo, w13, w2;
     float *x = nullptr, *p = nullptr, *q = nullptr, *o = nullptr;      // residual rows, products, turned queries, attention output
-    unsigned char *act = nullptr; float *scales = nullptr;             // codes or parts; group scales [G][kChunk] or row scales
+    unsigned char *act = nullptr; float *scales = nullptr;             // codes or parts; group scales [G][kChunk]
+    __nv_bfloat16 *parts = nullptr;                                    // F32: the matrix that is multiplied by, in parts
     struct AMap { uint32_t n, tn; CUtensorMap map; };
     std::vector<AMap> amaps;
     TcAttnState attn; uint32_t *err_host = nullptr, *err_dev = nullptr;
@@ -414,25 +413,16 @@ int dmalloc(PrefillState *s, void **p, size_t bytes) {
 bool map_2d(const PrefillState *s, CUtensorMap *m, bool q80, const void *base, uint64_t width, uint64_t rows, uint32_t box) {
     const cuuint64_t dims[2] = {width, rows}, strides[1] = {width * (q80 ? 1u : 2u)};
     const cuuint32_t b[2] = {q80 ? 128u : 64u, box}, step[2] = {1, 1};
-    return s->encode(m, q80 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(base), dims, strides, b, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    return s->encode(m, q80 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(base), dims, strides, b, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
                      CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 int add_product(PrefillState *s, std::vector<Product> *list, const PrefillMat &m) {
     Product p;
     p.m = m;
     const bool q80 = s->m.quant == 0x80u;
-    const void *base = m.w;
-    uint32_t width = m.n;
-    if (!q80) {
-        p.np = (m.n + 63u) & ~63u; width = 2u * p.np;
-        __half *parts = nullptr; uint32_t *bits = nullptr; float *inv = nullptr;
-        PM(parts, (size_t)m.rows * width * 2u); PM(bits, 16); PM(inv, 16);
-        NB_CK(cudaMemset(bits, 0, 16));
-        k_weight_max<<<s->sms * 8u, 256>>>(static_cast<const float *>(m.w), (size_t)m.rows * m.n, bits);
-        k_weight_parts<<<s->sms * 8u, 256>>>(static_cast<const float *>(m.w), m.rows, m.n, p.np, bits, parts, inv);
-        NB_CK(cudaGetLastError());
-        base = parts; p.winv = inv;
-    }
+    p.np = q80 ? 0u : (m.n + 63u) & ~63u;
+    const void *base = q80 ? m.w : s->parts;
+    const uint32_t width = q80 ? m.n : 3u * p.np;
     if (!map_2d(s, &p.wmap, q80, base, width, m.rows, kRows)) return fail(NB200_ECUDA, "cuTensorMapEncodeTiled refused a matrix of %u x %u", m.rows, m.n);
     list->push_back(p);
     return 0;
@@ -445,19 +435,25 @@ int create(PrefillState *s, const PrefillModel &m) {
     if (got != cudaDriverEntryPointSuccess || !fn) return fail(NB200_ECUDA, "the driver has no cuTensorMapEncodeTiled");
     s->encode = reinterpret_cast<decltype(s->encode)>(fn);
     int r;
+    if (!q80) {      // the largest matrix
+        size_t most = 0;
+        for (const auto *list : {&m.qkv, &m.wo, &m.w13, &m.w2}) for (const PrefillMat &a : *list) most = std::max(most, (size_t)a.rows * ((a.n + 63u) & ~63u) * 6u);
+        PM(s->parts, most);
+    }
     for (uint32_t l = 0; l < m.L; l++) {
         if ((r = add_product(s, &s->qkv, m.qkv[l]))) return r;
         if (l + 1u < m.L && ((r = add_product(s, &s->wo, m.wo[l])) || (r = add_product(s, &s->w13, m.w13[l])) || (r = add_product(s, &s->w2, m.w2[l])))) return r;
     }
     const uint32_t C = std::min(kChunk, (m.max_seq + 127u) & ~127u), wide = std::max(std::max(m.E, m.q_dim), m.F);
     PM(s->x, (size_t)C * m.E * 4); PM(s->p, (size_t)C * std::max(m.q_dim + 2 * m.kv_dim, 2 * m.F) * 4); PM(s->q, (size_t)C * m.q_dim * 4); PM(s->o, (size_t)C * m.q_dim * 4);
-    const size_t act = (size_t)C * (q80 ? wide : ((wide + 63u) & ~63u) * 4u), scales = q80 ? (size_t)(wide / m.gs) * kChunk : (size_t)kChunk;
+    const size_t act = (size_t)C * (q80 ? wide : ((wide + 63u) & ~63u) * 6u), scales = q80 ? (size_t)(wide / m.gs) * kChunk : 0u;
     PM(s->act, act); PM(s->scales, scales * 4);
-    NB_CK(cudaMemset(s->act, 0, act)); NB_CK(cudaMemset(s->scales, 0, scales * 4));
+    NB_CK(cudaMemset(s->act, 0, act));
+    if (q80) NB_CK(cudaMemset(s->scales, 0, scales * 4));
     for (uint32_t n : {m.E, m.q_dim, m.F})
         for (uint32_t tn : {64u, 128u}) {
             PrefillState::AMap a{n, tn, {}};
-            if (!map_2d(s, &a.map, q80, s->act, q80 ? n : 2u * ((n + 63u) & ~63u), C, tn)) return fail(NB200_ECUDA, "cuTensorMapEncodeTiled refused rows of %u", n);
+            if (!map_2d(s, &a.map, q80, s->act, q80 ? n : 3u * ((n + 63u) & ~63u), C, tn)) return fail(NB200_ECUDA, "cuTensorMapEncodeTiled refused rows of %u", n);
             s->amaps.push_back(a);
         }
     NB_CK(cudaHostAlloc(&s->err_host, 64, cudaHostAllocMapped));
@@ -465,13 +461,12 @@ int create(PrefillState *s, const PrefillModel &m) {
     NB_CK(cudaHostGetDevicePointer(&s->err_dev, s->err_host, 0));
     if ((r = attn_tc_setup(&s->attn, std::min<size_t>(attn_tc_bytes(m.max_seq, m.KV, m.hd, m.hd), (size_t)1 << 30), attn_tc_tiles(m.max_seq, m.KV), s->err_dev))) return r;
     if (q80 ? ((r = optin<true, 64>()) || (r = optin<true, 128>())) : (r = optin<false, 64>())) return r;
-    if (!q80) NB_CK(nb::smem_at_least((const void *)k_prompt_prep<false>, (int)(wide * 4u)));
     NB_CK(cudaDeviceSynchronize());
     return 0;
 }
 int prep(PrefillState *s, const float *src, uint32_t ld, const float *gain, uint32_t n, uint32_t mode, uint32_t T, cudaStream_t stream) {
-    PromptPrepArgs a{src, ld, gain, n, s->m.gs, mode, reinterpret_cast<int8_t *>(s->act), s->scales, kChunk, reinterpret_cast<__half *>(s->act), (n + 63u) & ~63u, s->scales};
-    return s->m.quant == 0x80u ? launch<PromptPrepArgs>(k_prompt_prep<true>, dim3(T), dim3(kPrepThreads), 0, stream, s->pdl, a) : launch<PromptPrepArgs>(k_prompt_prep<false>, dim3(T), dim3(kPrepThreads), (size_t)n * 4, stream, s->pdl, a);
+    const PromptPrepArgs a{src, ld, gain, n, s->m.gs, mode, reinterpret_cast<int8_t *>(s->act), s->scales, kChunk, reinterpret_cast<__nv_bfloat16 *>(s->act), (n + 63u) & ~63u};
+    return launch<PromptPrepArgs>(s->m.quant == 0x80u ? k_prompt_prep<true> : k_prompt_prep<false>, dim3(T), dim3(kPrepThreads), 0, stream, s->pdl, a);
 }
 int product(PrefillState *s, const Product &w, float *C, uint32_t ldc, bool add, uint32_t T, cudaStream_t stream) {
     // 64 positions per tile where tiles of 128 leave SMs without a block (1024 rows of the O product: 8 blocks for 128 positions), and in F32, whose
@@ -480,7 +475,7 @@ int product(PrefillState *s, const Product &w, float *C, uint32_t ldc, bool add,
     PromptGemmArgs a{};
     a.wmap = w.wmap;
     for (const auto &m : s->amaps) if (m.n == w.m.n && m.tn == tn) a.amap = m.map;
-    a.ws = static_cast<const float *>(w.m.aux); a.xs = s->scales; a.ldx = kChunk; a.winv = w.winv; a.xinv = s->scales;
+    a.ws = static_cast<const float *>(w.m.aux); a.xs = s->scales; a.ldx = kChunk;
     a.N = w.m.rows; a.T = T; a.n = w.m.n; a.gs = s->m.gs; a.np = w.np; a.C = C; a.ldc = ldc; a.add = add ? 1u : 0u; a.err = s->err_dev;
     // clusters share a tile's depth while fewer than half of the SMs have a block
     const uint32_t tiles = rt * ((T + tn - 1u) / tn), ks = prompt_parts(prompt_units(s->m.quant == 0x80u, w.m.n, w.np, s->m.gs), tiles, s->sms);
@@ -488,6 +483,10 @@ int product(PrefillState *s, const Product &w, float *C, uint32_t ldc, bool add,
     const dim3 grid(rt, (T + tn - 1u) / tn, ks), block(192);
 #define GEMM(q, t) launch<PromptGemmArgs>(k_prompt_gemm<q, t>, grid, block, gemm_smem<q, t>(), stream, s->pdl, a, ks)
     if (s->m.quant == 0x80u) return tn == 64u ? GEMM(true, 64) : GEMM(true, 128);
+    int r;
+    const WeightPartsArgs wa{static_cast<const float *>(w.m.w), w.m.rows, w.m.n, w.np, s->parts};
+    const size_t blocks = ((size_t)w.m.rows * (w.np / 8u) + 255u) / 256u;
+    if ((r = launch<WeightPartsArgs>(k_weight_parts, dim3((uint32_t)std::min<size_t>(blocks, s->sms * 8u)), dim3(256), 0, stream, s->pdl, wa))) return r;
     return GEMM(false, 64);
 #undef GEMM
 }
@@ -523,7 +522,7 @@ int prefill_check(PrefillState *s) {
 int prefill_run(PrefillState *s, const uint32_t *ids, uint32_t n, cudaStream_t stream, bool pdl, uint64_t *launches) {
     s->pdl = pdl;
     const PrefillModel &m = s->m;
-    const uint32_t W = m.q_dim + 2 * m.kv_dim;
+    const uint32_t W = m.q_dim + 2 * m.kv_dim, extra = m.quant == 0x80u ? 0u : 1u;
     const size_t kvl = (size_t)m.KV * m.max_seq * m.hd;
     Dims d{};
     d.arch = m.arch; d.hd = m.hd; d.max_seq = m.max_seq;
@@ -536,7 +535,7 @@ int prefill_run(PrefillState *s, const uint32_t *ids, uint32_t n, cudaStream_t s
             const PromptRopeArgs ra{s->p, W, m.H, m.KV, p0, s->q, m.kc + l * kvl, m.vc + l * kvl, m.qnorm ? m.qnorm + (size_t)l * m.hd : nullptr, m.knorm ? m.knorm + (size_t)l * m.hd : nullptr, m.rope_cos, m.rope_sin, d};
             if ((r = prep(s, s->x, m.E, m.norm_attn + (size_t)l * m.E, m.E, PREP_NORM, T, stream)) || (r = product(s, s->qkv[l], s->p, W, false, T, stream)) ||
                 (r = launch<PromptRopeArgs>(k_prompt_rope, dim3(T), dim3(256), 0, stream, pdl, ra))) return r;
-            *launches += 3;
+            *launches += 3u + extra;
             if (l + 1u == m.L) break;          // nothing reads what the last layer would make of these positions
             TcAttn a{};
             a.q = s->q; a.ldq = m.q_dim; a.q_head = m.hd; a.k = m.kc + l * kvl; a.v = m.vc + l * kvl; a.ldk = a.ldv = m.hd; a.k_head = a.v_head = (uint64_t)m.max_seq * m.hd;
@@ -545,7 +544,7 @@ int prefill_run(PrefillState *s, const uint32_t *ids, uint32_t n, cudaStream_t s
             if ((r = attn_tc_launch(&s->attn, a, stream, pdl)) || (r = prep(s, s->o, m.q_dim, nullptr, m.q_dim, PREP_PLAIN, T, stream)) || (r = product(s, s->wo[l], s->x, m.E, true, T, stream)) ||
                 (r = prep(s, s->x, m.E, m.norm_ffn + (size_t)l * m.E, m.E, PREP_NORM, T, stream)) || (r = product(s, s->w13[l], s->p, 2 * m.F, false, T, stream)) ||
                 (r = prep(s, s->p, 2 * m.F, nullptr, m.F, PREP_SWIGLU, T, stream)) || (r = product(s, s->w2[l], s->x, m.E, true, T, stream))) return r;
-            *launches += 8;
+            *launches += 8u + 3u * extra;
         }
     }
     return 0;

@@ -19,7 +19,7 @@ struct PrefillModel {
     float *kc, *vc;
 };
 struct PrefillState;
-// *out stays null (and 0 is returned) when the model's shapes have no portion kernels; F32 models get a second copy of their weights in two f16 parts
+// *out stays null (and 0 is returned) when the model's shapes have no portion kernels
 int prefill_create(PrefillState **out, const PrefillModel &m, uint32_t sms);
 void prefill_destroy(PrefillState *p);
 // K and V rows of the positions [0, n) of the tokens ids[0..n) on the device; n <= max_seq.  pdl: with programmatic dependent launch; launches: how many kernels were put on the stream

@@ -1,13 +1,14 @@
 """Prompts of model files in portions (csrc/prefill.cu): the K and V rows and the next logits against the same positions one call at a time, at the
 edges of the kernels' tiles (64 and 128 positions, 1024 to a portion, rows of weights that no tile of 128 divides) and for every group size.
 
-Bounds.  The rows of layer 0 come from the same activation codes (Q80) or the same rounding-free products (F32): 32-bit sums in another order,
+Bounds.  The rows of layer 0 come from the same activation codes (Q80) or exact products (F32): 32-bit sums in another order,
 2e-6 of a row's norm.  Deeper Q80 rows and the logits: a change in the last place turns a code here and there, which settles at 1 to
 2 % after two to four layers whatever its size; 4e-2.  F32 logits: 1e-5."""
 import dataclasses
 
 import numpy as np
 import pytest
+import torch
 
 from nano_b200 import engine as E, modelfile as mf
 
@@ -27,8 +28,12 @@ CASES = [("toy-nano", mf.QUANT_F32, 128), ("toy-qwen3", mf.QUANT_F32, 128), ("to
 
 
 def check(spec, quant, gs, lengths, room=1200):
+    check_file(mf.cached_model(spec, quant, gs), spec, quant, lengths, room)
+
+
+def check_file(path, spec, quant, lengths, room):
     """Prompts of these lengths in portions against the same positions one call at a time."""
-    eng = E.Engine(mf.cached_model(spec, quant, gs), room)
+    eng = E.Engine(path, room)
     toks = mf.teacher_tokens(1160, spec.vocab)
     n = max(lengths)
     last, want, keep = spec.n_layer - 1, {}, {}
@@ -115,3 +120,32 @@ def test_a_smaller_model_opened_later_leaves_the_larger_one_working():
 def test_rows_around_the_shared_memory_that_needs_no_asking(ff):
     """A 32-bit row of 12288 hidden units (Qwen3-8B's) is 48 KB, to which a kernel's static shared memory comes on top."""
     check(mf.ModelSpec("prompts-64-%d" % ff, mf.ARCH_NANO, 512, 512, 2, 64, 2, 2, ff), mf.QUANT_F32, 128, (10, 65), 200)
+
+
+def test_a_wide_range_inside_a_matrix_and_a_row(tmp_path):
+    """One hidden unit is 2^30 times the others and its outgoing weights 2^-30 times: the same model, number for number in fp32, and portions must not lose
+    the small numbers beside the large ones (bounds as above)."""
+    spec = dataclasses.replace(mf.PRESETS["toy-nano"], name="range-prompts", block_size=512)
+    rng = np.random.default_rng(7)
+    L, W, F, Q, K = spec.n_layer, spec.n_embd, spec.n_hidden, spec.q_dim, spec.kv_dim
+    shapes = {"attn_norm": (L, W), "ffn_norm": (L, W), "final_norm": (W,), "emb": (spec.vocab, W), "wq": (L, Q, W), "wk": (L, K, W), "wv": (L, K, W), "wo": (L, W, Q), "w1": (L, F, W), "w2": (L, W, F), "w3": (L, F, W)}
+    w = {k: (1.0 if "norm" in k else 0.0) + rng.standard_normal(s).astype(np.float32) * np.float32(0.05) for k, s in shapes.items()}
+    w["w3"][:, 5] *= np.float32(2.0 ** 30)
+    w["w2"][:, :, 5] *= np.float32(2.0 ** -30)
+    path = str(tmp_path / "range-prompts.bin")
+    mf.write_model_from_weights(path, spec, mf.QUANT_F32, 128, w)
+    check_file(path, spec, mf.QUANT_F32, (10, 65, 130), 300)
+
+
+def test_portions_keep_no_copy_of_the_weights():
+    """What prompts in portions need beside the model does not grow with its layers: an F32 file opened with them (fast mode) and without (exact mode)."""
+    spec = dataclasses.replace(mf.PRESETS["mini-nano"], name="mini-nano-deep", n_layer=12, block_size=512)
+    path = mf.cached_model(spec, mf.QUANT_F32, 128)
+    used = []
+    for flags in (E.FLAG_NO_STREAM | E.FLAG_EXACT, E.FLAG_NO_STREAM | E.FLAG_EXACT, E.FLAG_NO_STREAM):          # (the first: what a first engine loads for good)
+        before = torch.cuda.mem_get_info()[0]
+        eng = E.Engine(path, 300, flags=flags)
+        used.append(before - torch.cuda.mem_get_info()[0])
+        eng.close()
+    layer = 4 * (spec.q_dim * 2 + 2 * spec.kv_dim + 3 * spec.n_hidden) * spec.n_embd
+    assert used[2] - used[1] < 4 * layer, (used, layer)          # one matrix in parts and the activations of a portion; a copy is twelve layers and more
