@@ -188,10 +188,11 @@ __global__ void __launch_bounds__(192, 1) k_attn_tc(const AttnTcArgs ta) {
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
     }
-    // tensor memory: scores (two buffers of 128), weights (two planes of 64), a tile's weighted values.  Heads of 64 values have room for a sum per half of
-    // the tile: the tensor cores cut what they add, and half as many additions cut half as much (four layers of width 768 behind 200 / 487 positions, logits
-    // against 64 bits by those of fp32 attention: 1.09 / 1.08 with one sum, 1.05 / 1.04 with two)
-    constexpr uint32_t SCOL = 0, PCOL = 256, OCOL = 384, HCOL = VP == 64 ? 64 : 0;
+    // tensor memory: scores (two buffers of 128), where a tile's weights take the place of its scores (32 columns of scores: 16 of the large parts, 16 of the
+    // small), and a tile's weighted values.  Heads of 64 values have room for a sum per 32 keys: the tensor cores cut what they add, always towards zero, and a
+    // quarter of the additions cut a quarter as much (four layers of width 768 behind 200 / 487 positions, logits against 64 bits by those of single
+    // positions: 1.00 / 1.00 with four sums a tile, 1.01 / 1.02 with two)
+    constexpr uint32_t SCOL = 0, OCOL = 256, SUMS = VP == 64 ? 4 : 1;
     if (warp == 0 && lane == 0) {
         for (uint32_t i = 0; i < n; i++) {
             if (i && !mbar_wait(bar(KFREE), (i - 1u) & 1u)) { bad_s = 1; break; }
@@ -229,10 +230,11 @@ __global__ void __launch_bounds__(192, 1) k_attn_tc(const AttnTcArgs ta) {
 #pragma unroll
                 for (uint32_t ks = 0; ks < kTile / 16; ks++) {
                     const uint32_t off = (ks >> 2) * VP * 128u + (ks & 3u) * 32u;
-                    tc_mma_ts(tmem + OCOL + (ks >> 2) * HCOL, tmem + PCOL + (p == 0 ? 64u : 0u) + ks * 8u, tc_desc(vsm + (p == 1 ? VP * 256u : 0u) + off), id_o, p > 0 || (HCOL ? ks & 3u : ks) > 0);
+                    const uint32_t w = SCOL + (i & 1u) * kTile + (ks >> 1) * 32u + (ks & 1u) * 8u + (p == 0 ? 16u : 0u);
+                    tc_mma_ts(tmem + OCOL + (SUMS > 1 ? (ks >> 1) * VP : 0u), tmem + w, tc_desc(vsm + (p == 1 ? VP * 256u : 0u) + off), id_o, p > 0 || (SUMS > 1 ? ks & 1u : ks) > 0);
                 }
             tc_commit(bar(VFREE)); tc_commit(bar(OREADY));
-            if (i + 2u < n) ok = scores(i + 2u);          // its buffer's scores have been read: the weights of tile i are there
+            if (i + 2u < n) ok = mbar_wait(bar(OREADY), i & 1u) && scores(i + 2u);          // they overwrite the weights that the products before read (tile i + 1's scores are there meanwhile)
         }
         if (!ok) bad_s = 3;
     } else if (warp >= 2) {
@@ -255,8 +257,9 @@ __global__ void __launch_bounds__(192, 1) k_attn_tc(const AttnTcArgs ta) {
                 tc_ld32(tmem + lane_base + OCOL + c, w);
 #pragma unroll
                 for (int j = 0; j < 32; j++) o[c + j] = fmaf(__uint_as_float(w[j]), f, o[c + j] * corr);
-                if (HCOL) {
-                    tc_ld32(tmem + lane_base + OCOL + HCOL + c, w);
+#pragma unroll
+                for (uint32_t q = 1; q < SUMS; q++) {
+                    tc_ld32(tmem + lane_base + OCOL + q * VP + c, w);
 #pragma unroll
                     for (int j = 0; j < 32; j++) o[c + j] = fmaf(__uint_as_float(w[j]), f, o[c + j]);
                 }
@@ -313,8 +316,8 @@ __global__ void __launch_bounds__(192, 1) k_attn_tc(const AttnTcArgs ta) {
                 sum += (s4[0] + s4[1]) + (s4[2] + s4[3]);
 #pragma unroll
                 for (uint32_t j = 0; j < 16; j++) split2(p[2 * j] * kWeightScale, p[2 * j + 1] * kWeightScale, wh[j], wl[j]);
-                tc_st16(tmem + lane_base + PCOL + c / 2u, wh);
-                tc_st16(tmem + lane_base + PCOL + 64u + c / 2u, wl);
+                tc_st16(s_at + c, wh);
+                tc_st16(s_at + c + 16u, wl);
             }
             l = fmaf(l, corr, sum);
             m = mn;
