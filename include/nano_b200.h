@@ -83,6 +83,8 @@ enum nb200_field {
     NB200_F_ACT_SCALE = 21
 };
 
+/* After a create that returned 0 it is empty or says which prompts or portions run on the kernels that need no workspace (the workspaces take at
+ * most an eighth of the device memory that is free after everything else has been allocated). */
 const char *nb200_last_error(void);
 int nb200_device_count(void);
 

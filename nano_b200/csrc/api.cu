@@ -63,6 +63,7 @@ int nb200_device_count(void) {
 
 int nb200_engine_create(nb200_engine **out, const uint8_t *image, uint64_t image_bytes, uint32_t max_seq_len, int device, uint32_t flags) {
     if (!out || !image || image_bytes < 8) return fail(NB200_EINVAL, "bad arguments");
+    nb::g_err.clear();
     if (!nb_family_nano_create) return fail(NB200_EINVAL, "the model-file family (engine.cu) is not part of this build of the library");
     return nb_family_nano_create(out, image, image_bytes, max_seq_len, device, flags);
 }
@@ -70,6 +71,7 @@ int nb200_engine_create(nb200_engine **out, const uint8_t *image, uint64_t image
 int nb200_engine_create_dir(nb200_engine **out, const char *model_dir, uint32_t max_tokens, int device, uint32_t flags) {
     if (!out || !model_dir || max_tokens == 0) return fail(NB200_EINVAL, "bad arguments");
     *out = nullptr;
+    nb::g_err.clear();
     nb::ModelDir dir;
     std::string err;
     if (nb::modeldir_open(model_dir, &dir, &err)) return fail(NB200_EINVAL, "%s", err.c_str());

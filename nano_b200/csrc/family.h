@@ -40,6 +40,14 @@ inline cudaError_t smem_at_least(const void *kernel, int bytes) {
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, fa.maxDynamicSharedSizeBytes > bytes ? fa.maxDynamicSharedSizeBytes : bytes);
 }
 
+// Memory that makes an engine faster and nothing else: at most an eighth of what is free once all the rest has been allocated, so that the next model a program
+// opens finds the other seven.  What does not get it runs through the kernels that need none.
+inline size_t optional_room() {
+    size_t left = 0, total = 0;
+    if (cudaMemGetInfo(&left, &total) != cudaSuccess) { cudaGetLastError(); return 0; }
+    return left / 8u;
+}
+
 struct EngineOps {
     void (*destroy)(nb200_engine *);
     int (*get_config)(const nb200_engine *, nb200_config *);

@@ -352,7 +352,6 @@ int load_latent_attn(Loader &ld, const nb::Json *m, const std::string &p, Layer 
     for (uint64_t h = 0; h < H; h++)          // [H*dim, R] -> per head [R, dim]: absorbed query = q_h W_uk,h
         for (uint64_t dd = 0; dd < D; dd++)
             for (uint64_t k = 0; k < R; k++) t[(h * R + k) * D + dd] = uk[(h * D + dd) * R + k];
-    if (latent_up(ld.e, *L) && ld.stacked({p + "uk", p + "uv"}, {H * D, H * VD}, R, &L->ukv)) { L->ukv = Weight{}; cudaGetLastError(); }      // (no room: portions stay absorbed)
     return ld.put_w(t, (uint32_t)(H * R), (uint32_t)D, &L->ukT);
 }
 
@@ -693,7 +692,6 @@ int load_latent_attn_direct(Loader &ld, const nb::Json *m, const std::string &p,
     for (uint64_t h = 0; h < H; h++)          // [H*dim, R] -> per head [R, dim]: absorbed query = q_h W_uk,h
         for (uint64_t dd = 0; dd < D; dd++)
             for (uint64_t k = 0; k < R; k++) t[(h * R + k) * D + dd] = uk[(h * D + dd) * R + k];
-    if (latent_up(ld.e, *L) && ld.stacked({p + "uk", p + "uv"}, {H * D, H * VD}, R, &L->ukv)) { L->ukv = Weight{}; cudaGetLastError(); }      // (no room: portions stay absorbed)
     return ld.put_w(t, (uint32_t)(H * R), (uint32_t)D, &L->ukT);
 }
 
@@ -2199,6 +2197,59 @@ const nb::EngineOps kLayeredOps = {lm_destroy, lm_get_config, lm_forward, lm_rea
                                    lm_seq_open, lm_seq_close, lm_step, lm_read_residual, lm_step_timed};
 
 
+// What long portions need beside the engine: rounded rows of every product (rows: numbers), images of keys and values for as many keys as a sequence can hold
+// (up to 1 GB), for latents that can be multiplied out the up-projections as one matrix, the keys and values and the latents in parts.  Allocated last; where the
+// memory does not reach for all keys, longer contexts (or all) go through the kernels that need none of it, and nb200_last_error says so.
+int portion_memory(LayeredEngine *e, Loader &ld, size_t rows) {
+    constexpr size_t kMost = (size_t)1 << 30;
+    const size_t all = nb::optional_room(), keys = (size_t)e->n_pages * kPage;
+    size_t room = all;
+    if (rows * 6u > room || tc_setup(&e->tc, rows, (uint32_t)e->num_sms)) {
+        tc_free(&e->tc); cudaGetLastError();
+        fail(NB200_ENOMEM, "portions run on the kernels that need no workspace: %zu bytes asked, %zu allowed", rows * 6u, all);
+        return 0;
+    }
+    room -= rows * 6u;
+    size_t image = 0, kv = 0, planes = 0, ukv = 0;          // bytes for a key; weights
+    uint32_t heads = 0;
+    bool grouped = false;
+    for (const Layer &L : e->layers) {
+        const bool up = L.type == MIX_LATENT_ATTN && latent_up(e, L);
+        if (!up && L.type != MIX_ATTN_DELTA && L.type != MIX_GQA) continue;
+        const uint32_t G = up ? L.H : L.G;
+        image = std::max(image, nb::attn_tc_bytes(128, G, L.dim, L.vdim) / 128u); heads = std::max(heads, G);
+        if (!up) { grouped = true; continue; }
+        const size_t row = (size_t)L.H * (L.dim + L.vdim);
+        kv = std::max(kv, row * 4u); planes = std::max(planes, (size_t)tc_split_width(L.R) * 2u); ukv += row * L.R * 2u;
+    }
+    if (!image) return 0;
+    if (ukv >= room) kv = planes = ukv = 0;
+    room -= ukv;
+    const size_t most = kMost / std::max(image, kv), fit = std::min(most, room / (image + kv + planes + heads / 16u + 1u)), n = fit >= keys ? keys : fit / 128u * 128u;
+    if (n < keys && most >= keys) fail(NB200_ENOMEM, "contexts of more than %zu positions run on the kernels that need no workspace: %zu bytes are allowed for it", n, all);
+    if (!n || nb::attn_tc_setup(&e->ta, image * ((n + 127u) / 128u * 128u), (n + 127u) / 128u * heads, e->tc.err_dev)) { nb::attn_tc_free(&e->ta); cudaGetLastError(); return 0; }
+    if (!kv) return 0;
+    const size_t mark = e->allocs.size();
+    const uint64_t weights = e->weight_bytes;
+    int r = dmalloc(e, (void **)&e->b_kv, n * kv);
+    if (!r) r = tc_split_setup(&e->tc, n * planes / 2u);
+    for (size_t i = 0; i < e->layers.size() && !r; i++) {
+        Layer &L = e->layers[i];
+        const std::string p = "l" + std::to_string(i) + ".mix.";
+        if (L.type == MIX_LATENT_ATTN && latent_up(e, L)) r = ld.stacked({p + "uk", p + "uv"}, {(uint64_t)L.H * L.dim, (uint64_t)L.H * L.vdim}, L.R, &L.ukv);
+    }
+    e->weight_bytes = weights;          // (a second form of weights that are counted already)
+    if (!r) { e->kv_floats = n * kv / 4u; return 0; }
+    for (size_t i = mark; i < e->allocs.size(); i++) cudaFree(e->allocs[i]);
+    e->allocs.resize(mark);
+    for (Layer &L : e->layers) L.ukv = Weight{};
+    e->b_kv = nullptr;
+    tc_split_free(&e->tc);
+    if (!grouped) nb::attn_tc_free(&e->ta);
+    cudaGetLastError();
+    return 0;
+}
+
 int create(LayeredEngine *e, const nb::ModelDir *dir, uint32_t max_tokens) {
     const nb::Json &cfg = dir->config;
     const nb::Json *layers = cfg.get("layers");
@@ -2625,25 +2676,7 @@ int create(LayeredEngine *e, const nb::ModelDir *dir, uint32_t max_tokens) {
     if (!e->f32) {      // the widest rows any product reads (a routed product: one row per token and choice)
         size_t w = std::max<size_t>(E, mTop * E);
         for (uint32_t v : {2 * mC, mZ, mQR, mQ, mHR, mOV, sP, sQK, sXC, sA, sRO, sDBC, sF, sF2, sXC2, sY, dV, dSp, dGt, mMO, mFF, mFF2, mSFF, mSFF2}) w = std::max<size_t>(w, v);
-        // images of every key a sequence can hold, up to 1 GB (longer contexts of many heads go through the fp32 kernels)
-        size_t bytes = 0, tiles = 0;
-        const uint32_t keys = e->n_pages * kPage;
-        for (const Layer &L : e->layers)
-            if (L.type == MIX_ATTN_DELTA || L.type == MIX_GQA) { bytes = std::max(bytes, nb::attn_tc_bytes(keys, L.G, L.dim, L.vdim)); tiles = std::max(tiles, nb::attn_tc_tiles(keys, L.G)); }
-        size_t kv = 0, planes = 0;
-        for (const Layer &L : e->layers)
-            if (L.ukv.p) {
-                const size_t row = (size_t)L.H * (L.dim + L.vdim), n = std::min<size_t>(keys, ((size_t)1 << 28) / row);
-                kv = std::max(kv, n * row); planes = std::max(planes, n * tc_split_width(L.R));
-                bytes = std::max(bytes, nb::attn_tc_bytes((uint32_t)n, L.H, L.dim, L.vdim)); tiles = std::max(tiles, nb::attn_tc_tiles((uint32_t)n, L.H));
-            }
-        // All of this makes long portions faster and nothing else: allocated last, and where the memory does not reach, they go through the kernels that need none of it
-        if (tc_setup(&e->tc, std::max<size_t>(T, kWantBatch) * ((w + 7u) & ~(size_t)7u), (uint32_t)e->num_sms)) tc_free(&e->tc);
-        else {
-            if (bytes && nb::attn_tc_setup(&e->ta, std::min<size_t>(bytes, (size_t)1 << 30), tiles, e->tc.err_dev)) nb::attn_tc_free(&e->ta);
-            if (kv && e->ta.images && cudaMalloc(&e->b_kv, kv * 4) == cudaSuccess) { e->allocs.push_back(e->b_kv); if (!tc_split_setup(&e->tc, planes)) e->kv_floats = kv; }
-        }
-        cudaGetLastError();
+        if ((r = portion_memory(e, ld, std::max<size_t>(T, kWantBatch) * ((w + 7u) & ~(size_t)7u)))) return r;
     }
     CK(cudaDeviceSynchronize());
     return 0;

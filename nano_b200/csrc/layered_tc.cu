@@ -313,10 +313,13 @@ int tc_setup(TcState *t, size_t elems, uint32_t sms) {
 }
 void tc_free(TcState *t) {
     for (auto &p : t->rows) { if (p) cudaFree(p); p = nullptr; }
-    if (t->planes) cudaFree(t->planes);
-    t->planes = nullptr;
+    tc_split_free(t);
     if (t->err_host) cudaFreeHost(t->err_host);
-    t->err_host = t->err_dev = nullptr; t->encode = nullptr; t->elems = t->plane_elems = 0;
+    t->err_host = t->err_dev = nullptr; t->encode = nullptr; t->elems = 0;
+}
+void tc_split_free(TcState *t) {
+    if (t->planes) cudaFree(t->planes);
+    t->planes = nullptr; t->plane_elems = 0;
 }
 int tc_check(TcState *t) {
     if (!t->err_host || !*static_cast<volatile uint32_t *>(t->err_host)) return 0;

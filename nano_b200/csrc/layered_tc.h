@@ -30,6 +30,7 @@ int tc_gemm(TcState *t, GemmArgs a, uint32_t groups, uint32_t maxM, uint32_t row
 // goes in as three bfloat16 parts (W is bfloat16 anyway).  Room for keys * tc_split_width(K) numbers is asked from setup.
 inline uint32_t tc_split_width(uint32_t K) { return 3u * ((K + 63u) & ~63u); }
 int tc_split_setup(TcState *t, size_t elems);
+void tc_split_free(TcState *t);
 bool tc_split_fits(const TcState *t, uint32_t N, uint32_t K, uint32_t rows, const void *W, const float *cache, uint32_t ld);
 int tc_gemm_split(TcState *t, const float *cache, const uint32_t *table, uint32_t ld, uint32_t first, uint32_t rows, const void *W, uint32_t N, uint32_t K, float *C, uint32_t ldc, cudaStream_t stream, bool pdl);
 

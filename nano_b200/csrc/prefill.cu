@@ -434,19 +434,21 @@ int create(PrefillState *s, const PrefillModel &m) {
     NB_CK(cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &got));
     if (got != cudaDriverEntryPointSuccess || !fn) return fail(NB200_ECUDA, "the driver has no cuTensorMapEncodeTiled");
     s->encode = reinterpret_cast<decltype(s->encode)>(fn);
+    const uint32_t C = std::min(kChunk, (m.max_seq + 127u) & ~127u), wide = std::max(std::max(m.E, m.q_dim), m.F), wp = std::max(m.q_dim + 2 * m.kv_dim, 2 * m.F);
+    const size_t act = (size_t)C * (q80 ? wide : ((wide + 63u) & ~63u) * 6u), scales = q80 ? (size_t)(wide / m.gs) * kChunk : 0u, tiles = attn_tc_tiles(m.max_seq, m.KV);
+    size_t parts = 0;          // F32: the largest matrix
+    if (!q80) for (const auto *list : {&m.qkv, &m.wo, &m.w13, &m.w2}) for (const PrefillMat &a : *list) parts = std::max(parts, (size_t)a.rows * ((a.n + 63u) & ~63u) * 6u);
+    // images of keys and values for max_seq positions, up to 1 GB and to what is allowed (longer prompts run position by position)
+    const size_t rest = parts + (size_t)C * (m.E + wp + 2 * m.q_dim) * 4u + act + scales * 4u + tiles * 8u, room = optional_room();
+    if (rest >= room) return fail(NB200_ENOMEM, "prompts run position by position: portions need a workspace of %zu bytes, %zu are allowed", rest, room);
+    const size_t images = std::min(std::min(attn_tc_bytes(m.max_seq, m.KV, m.hd, m.hd), (size_t)1 << 30), room - rest);
     int r;
-    if (!q80) {      // the largest matrix
-        size_t most = 0;
-        for (const auto *list : {&m.qkv, &m.wo, &m.w13, &m.w2}) for (const PrefillMat &a : *list) most = std::max(most, (size_t)a.rows * ((a.n + 63u) & ~63u) * 6u);
-        PM(s->parts, most);
-    }
+    if (parts) PM(s->parts, parts);
     for (uint32_t l = 0; l < m.L; l++) {
         if ((r = add_product(s, &s->qkv, m.qkv[l]))) return r;
         if (l + 1u < m.L && ((r = add_product(s, &s->wo, m.wo[l])) || (r = add_product(s, &s->w13, m.w13[l])) || (r = add_product(s, &s->w2, m.w2[l])))) return r;
     }
-    const uint32_t C = std::min(kChunk, (m.max_seq + 127u) & ~127u), wide = std::max(std::max(m.E, m.q_dim), m.F);
-    PM(s->x, (size_t)C * m.E * 4); PM(s->p, (size_t)C * std::max(m.q_dim + 2 * m.kv_dim, 2 * m.F) * 4); PM(s->q, (size_t)C * m.q_dim * 4); PM(s->o, (size_t)C * m.q_dim * 4);
-    const size_t act = (size_t)C * (q80 ? wide : ((wide + 63u) & ~63u) * 6u), scales = q80 ? (size_t)(wide / m.gs) * kChunk : 0u;
+    PM(s->x, (size_t)C * m.E * 4); PM(s->p, (size_t)C * wp * 4); PM(s->q, (size_t)C * m.q_dim * 4); PM(s->o, (size_t)C * m.q_dim * 4);
     PM(s->act, act); PM(s->scales, scales * 4);
     NB_CK(cudaMemset(s->act, 0, act));
     if (q80) NB_CK(cudaMemset(s->scales, 0, scales * 4));
@@ -459,7 +461,7 @@ int create(PrefillState *s, const PrefillModel &m) {
     NB_CK(cudaHostAlloc(&s->err_host, 64, cudaHostAllocMapped));
     *s->err_host = 0;
     NB_CK(cudaHostGetDevicePointer(&s->err_dev, s->err_host, 0));
-    if ((r = attn_tc_setup(&s->attn, std::min<size_t>(attn_tc_bytes(m.max_seq, m.KV, m.hd, m.hd), (size_t)1 << 30), attn_tc_tiles(m.max_seq, m.KV), s->err_dev))) return r;
+    if ((r = attn_tc_setup(&s->attn, images, tiles, s->err_dev))) return r;
     if (q80 ? ((r = optin<true, 64>()) || (r = optin<true, 128>())) : (r = optin<false, 64>())) return r;
     NB_CK(cudaDeviceSynchronize());
     return 0;
