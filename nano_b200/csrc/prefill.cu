@@ -12,8 +12,9 @@
 //   k_prompt_gemm      C[t][n] (+)= sum over groups: tcgen05.mma on 128 weight rows x TN positions, the accumulator of a GROUP in tensor memory (two
 //                      buffers), added to fp32 registers by the threads that own the rows while the next group multiplies.
 //                      Q80: kind::i8, int32 exact, times weight scale x activation scale.  F32: kind::f16 on three bfloat16 parts of both
-//                      operands, which are all of their 24 bits, all nine products, over 16 of the depth; the tensor cores cut what they add, so they
-//                      add nine times only, the small products first, and what they leave is added up with its rounding error carried along.
+//                      operands, which are all of their 24 bits; of the nine products of parts the three that are left out (small x
+//                      smallest, smallest x smallest) are 2^-26 of the whole at most.  The tensor cores cut what they add, so they
+//                      add over 16 of the depth only, the small products first, and what they leave is added up with its rounding error carried along.
 //   k_prompt_rope      head norm (Qwen3), rotary positions, K and V rows into the cache
 //   attention          attn_tc.cu
 #include "prefill.h"
@@ -222,8 +223,8 @@ __global__ void __launch_bounds__(192, Q80 && TN == 64 ? 2 : 1) k_prompt_gemm(co
                 for (uint32_t k = 0; k < 4u; k++) {
                     if (!(ok = open())) break;
 #pragma unroll
-                    for (uint32_t p = 0; p < 9; p++) {          // the smallest products first, large x large last
-                        constexpr uint32_t wp[9] = {2, 1, 2, 0, 2, 1, 0, 1, 0}, xp[9] = {2, 2, 1, 2, 0, 1, 1, 0, 0};
+                    for (uint32_t p = 0; p < 6; p++) {          // the smallest products first, large x large last
+                        constexpr uint32_t wp[6] = {0, 2, 1, 0, 1, 0}, xp[6] = {2, 0, 1, 1, 0, 0};
                         tc_mma_ss(tmem + (gi & 1u) * TN, tc_desc(base + wp[p] * WB) + 2u * k, tc_desc(xb + xp[p] * XB) + 2u * k, idesc, p > 0);
                     }
                     close();

@@ -1,5 +1,6 @@
 """Prompts of model files in portions (csrc/prefill.cu): the K and V rows and the next logits against the same positions one call at a time, at the
-edges of the kernels' tiles (64 and 128 positions, 1024 to a portion, rows of weights that no tile of 128 divides) and for every group size.
+edges of the kernels' tiles (64 and 128 positions, 1024 to a portion, rows of weights that no tile of 128 divides, depths that no stage of 128 divides) and
+for every group size.
 
 Bounds.  The rows of layer 0 come from the same activation codes (Q80) or exact products (F32): 32-bit sums in another order,
 2e-6 of a row's norm.  Deeper Q80 rows and the logits: a change in the last place turns a code here and there, which settles at 1 to
@@ -24,7 +25,11 @@ def rows(eng, spec, layer, pos):
 
 
 CASES = [("toy-nano", mf.QUANT_F32, 128), ("toy-qwen3", mf.QUANT_F32, 128), ("toy-nano", mf.QUANT_Q80, 32), ("toy-qwen3", mf.QUANT_Q80, 64), ("toy-nano", mf.QUANT_Q80, 128), ("toy-nano", mf.QUANT_Q80, 256),
-         ("mini-qwen3", mf.QUANT_Q80, 128), ("mini-nano", mf.QUANT_F32, 128), ("toy-nano-odd", mf.QUANT_F32, 128)]
+         ("mini-qwen3", mf.QUANT_Q80, 128), ("mini-nano", mf.QUANT_F32, 128), ("toy-nano-odd", mf.QUANT_F32, 128),
+         ("mini-qwen3", mf.QUANT_F32, 128), ("long-qwen3", mf.QUANT_Q80, 128)]
+# prompts of m tokens are portions of m - 1: around 64, 128 and 256; past 1024; and, 48 tiles of weight rows and more, where tiles of 128 positions leave no SM
+# without a block (from 385 positions for W1|W3, 513 for Q|K|V), the last of them with 1, 2, 64 or all of its positions
+LENGTHS = {"toy-qwen3": (34, 64, 1025, 1154), "long-qwen3": (386, 387, 449, 513, 642)}
 
 
 def check(spec, quant, gs, lengths, room=1200):
@@ -61,7 +66,7 @@ def check_file(path, spec, quant, lengths, room):
 
 @pytest.mark.parametrize("name,quant,gs", CASES)
 def test_portions_against_single_positions(name, quant, gs):
-    check(dataclasses.replace(mf.PRESETS[name], name=name + "-prompts", block_size=2048), quant, gs, (33, 65, 129, 130, 257) if name != "toy-qwen3" else (34, 64, 1025, 1154))
+    check(dataclasses.replace(mf.PRESETS[name], name=name + "-prompts", block_size=2048), quant, gs, LENGTHS.get(name, (33, 65, 129, 130, 257)))
 
 
 @pytest.mark.parametrize("width,ff,gs", [(1088, 2240, 32), (1088, 2240, 64), (544, 1120, 32), (320, 4160, 64)])
