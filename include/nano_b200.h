@@ -104,7 +104,8 @@ void nb200_engine_destroy(nb200_engine *e);
  * From then on all ranks issue the SAME sequence of forward / next_greedy / decode_greedy calls with the
  * same arguments (in lock-step; a rank that waits ~4 s for a missing peer fails with NB200_ECUDA).  Every
  * rank returns the same token ids; nb200_read_logits fills only this rank's slice
- * [rank*V/tp_size, (rank+1)*V/tp_size) of the vector.  Results are bit-identical to tp_size == 1.
+ * [rank*V/tp_size, (rank+1)*V/tp_size) of the vector.  Results are bit-identical to tp_size == 1 (but for nb200_decode_greedy with a
+ * prompt that one GPU runs in portions, see there).
  * Fast mode only; needs n_kv_head, n_embd/2, n_hidden and vocab divisible by tp_size, head_dim <= 128. */
 int nb200_engine_create_tp(nb200_engine **out, const uint8_t *image, uint64_t image_bytes,
                            uint32_t max_seq_len, int device, uint32_t flags, uint32_t tp_rank, uint32_t tp_size);
@@ -164,7 +165,7 @@ int nb200_next_sampled(nb200_engine *e, const uint32_t *ids, uint32_t pos, float
 
 /* Device-resident greedy loop: ids[0..n_prompt) is the prompt; positions 0..n_total-2 are run and
  * ids[n_prompt..n_total) are filled with greedy tokens (prompt positions are teacher-forced exactly like
- * llm_session_step; prompts of eight positions and more of F32 and Q80 files run in portions, whose fp32 sums come in another order
+ * llm_session_step; prompts of nine tokens and more -- ten when n_total == n_prompt -- of F32 and Q80 files run in portions, whose fp32 sums come in another order
  * than those of one call per position: K / V rows and logits agree as two execution paths do).  device_ms (optional) receives the CUDA-event time of the decode segment
  * (positions >= n_prompt-1); prefill_ms the prompt segment. */
 int nb200_decode_greedy(nb200_engine *e, uint32_t *ids, uint32_t n_prompt, uint32_t n_total,

@@ -1,9 +1,11 @@
 // attn_tc.cu -- softmax attention of long portions on the fifth-generation tensor cores: fp32 queries, keys and values, products of 32-bit precision.
 //
-// An fp32 number x is the sum of two f16 numbers to 2^-24 of it, h = f16(x) and l = f16(x - h), as long as it lies within 2^-17 of the largest number
-// of its tile (a tile is brought to just under 2^15 by a power of two); a smaller one is off by 2^-40 of that largest.  So
-// a b = ha hb + ha lb + la hb to about 2^-23, the size of one fp32 rounding, and three f16 products with fp32 accumulators take the place of
-// a pass of FMAs.  The tensor cores may cut what they add instead of rounding it, so sums are kept short: the two small products go first, and a
+// An fp32 number x is the sum of two f16 numbers to 2^-23 of it, h = f16(x) and l = f16(x - h) (23 of its 24 bits: a quarter of all numbers are off by the last
+// one), as long as it lies within 2^-17 of the largest number of its tile (a tile is brought to just under 2^15 by a power of two); a smaller one is
+// off by 2^-40 of that largest.  a b = ha hb + ha lb + la hb, three f16 products with fp32 accumulators, leaves out la lb, 2^-22 at most and 2^-25 as a root mean
+// square: each the size of one fp32 rounding, where a pass of FMAs makes one per term.  A tile in which one number is more than 2^17 times another holds
+// the small ones in fewer bits than fp32 does; an infinity or a NaN in a tile of values makes every row of the tile NaN (as in the FMA kernel, whose tiles are 64 keys).
+// The tensor cores cut what they add instead of rounding it, so sums are kept short: the two small products go first, and a
 // tile's weighted values join the running sum by ordinary fp32 arithmetic.
 // (mma.sync with three bfloat16 parts was built first: 550 us for 976 queries x 16 heads on 1512 keys on average, against 600 for the FMA kernel; the
 // old tensor path of this chip does some 600 multiply-adds per cycle and SM.)
@@ -13,10 +15,10 @@
 //   k_attn_tc       a block owns 128 rows (query token, query head) of one key/value head.  Warp 0 fetches, warp 1 issues tcgen05.mma, a thread of warps
 //                   2..5 owns one row: scores come out of tensor memory with a lane per row, so a row's maximum and sum need no other
 //                   thread; its weights go back into tensor memory as the A operand of the second product.  Scores are double buffered and a
-//                   tile's values are added while the next tile's scores are made, so the tensor cores work under the exponentials,
-//                   which bound the kernel.
+//                   tile's values are added while the next tile's scores are made, so the tensor cores (busy for 11 % of the time) work under the softmax
+//                   of four warps, one per scheduler, which bounds the kernel: its chain of loads, exponentials and splits issues in 26 % of the cycles.
 // 1024 queries x 16 heads over 4 key/value heads of 128 on 1536 keys on average: 102 us, 606 by the FMA kernel (k_gqa_attn), with softcap 130 and 640; error
-// against float64 0.4e-6 .. 1.1e-6 of a row's norm where the FMA kernel has 0.75e-6 .. 1.6e-6.
+// against float64 on normal numbers 0.4e-6 .. 1.1e-6 of a row's norm where the FMA kernel has 0.75e-6 .. 1.6e-6.
 #include "attn_tc.h"
 
 #include <cuda_fp16.h>
@@ -34,7 +36,7 @@ constexpr float kWeightScale = 16384.0f;                 // weights (0..1) befor
 // a power of two that brings `big` to [2^14, 2^15)
 __device__ __forceinline__ float tile_scale(float big) {
     const int e = (int)(__float_as_uint(big) >> 23) - 127;
-    if (!(big > 0.0f) || e > 127) return 1.0f;           // nothing but zeros; infinities and NaN stay what they are
+    if (!(big > 0.0f) || e > 127) return 1.0f;           // nothing but zeros; with an infinity a tile is not brought anywhere
     return __uint_as_float((uint32_t)(127 + max(-113, min(100, 14 - e))) << 23);
 }
 __device__ __forceinline__ uint32_t pack2(__half a, __half b) { return (uint32_t)__half_as_ushort(a) | ((uint32_t)__half_as_ushort(b) << 16); }

@@ -5,10 +5,10 @@
 //                 gathered into expert order where a row list says so: a dense matrix that bulk copies can read
 //   k_gemm_tc     C^T = W A^T in tiles of 128 weight rows x TN tokens: tcgen05.mma (one issuing thread), operands by cp.async.bulk.tensor into a ring of
 //                 128-byte-swizzled stages, fp32 accumulators in tensor memory.  A tensor-memory lane is an output COLUMN of C, so a
-//                 warp's stores of one token are 128 contiguous bytes and need no transposition.  Bound by the operand traffic from L2 (a 128 x 128 tile
-//                 reads 32 KB for 128 cycles of products): 1024 x 12288 x 2048 in 59 us (870 TFLOP/s, 54 % of the measured 1609) where
-//                 the mma.sync tiles it replaces took 542; 1024 x 2048 x 2048 in 18.7 us (145).  Two blocks per SM hide one's
-//                 epilogue behind the other's products.
+//                 warp's stores of one token are 128 contiguous bytes and need no transposition.  1024 x 12288 x 2048 takes
+//                 59 us (870 TFLOP/s, 52 % of the measured 1664) where the mma.sync tiles it replaces took 542; 1024 x 2048 x 2048 18.7 us (145).  Tensor pipe and
+//                 L2 are each busy for 39 % of the large one and 17 % of the small one, whose single block per SM has three stages on the way: it waits
+//                 for memory.  Two blocks per SM hide one's epilogue behind the other's products.
 //
 // Every wait is bounded: one that runs out records a code in a host-visible word, the kernel drains and leaves, and the step fails.
 #include "layered_tc.h"
