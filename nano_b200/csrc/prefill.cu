@@ -7,8 +7,8 @@
 //   k_prompt_embed     token rows
 //   k_prompt_prep      a position's activation: RMS norm with gain, plain, or SwiGLU of interleaved pairs; then Q80 codes + group scales, or
 //                      (F32) three bfloat16 parts
-//   k_weight_parts     F32: a matrix in three bfloat16 parts, into one workspace for all of them (its bytes pass through memory two and a half times
-//                      more for that; a copy that stays would hold half again as much as the file)
+//   k_weight_parts     F32: a matrix in three bfloat16 parts, into one workspace for all of them (its bytes pass through memory four times
+//                      for that; a copy that stays would hold half again as much as the file)
 //   k_prompt_gemm      C[t][n] (+)= sum over groups: tcgen05.mma on 128 weight rows x TN positions, the accumulator of a GROUP in tensor memory (two
 //                      buffers), added to fp32 registers by the threads that own the rows while the next group multiplies.
 //                      Q80: kind::i8, int32 exact, times weight scale x activation scale.  F32: kind::f16 on three bfloat16 parts of both
