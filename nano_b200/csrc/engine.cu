@@ -525,7 +525,7 @@ int setup_stream(nb200_engine *e) {
     for (;; stage_bytes -= 1024u) {
         kv_rows = (stage_bytes / (2u * d.hd * 4u)) & ~3u;
         if (kv_rows < 4) return 0;
-        const uint32_t attn_b = al(st_attn_smem_floats(d.kv_mul, d.hd, nsplit_max, (uint32_t)kStSegTiles * kv_rows) * 4u);
+        const uint32_t attn_b = al(st_attn_smem_floats(d.kv_mul, d.hd) * 4u);
         region0 = g.off_attn + attn_b;
         nst = (uint32_t)max_optin > static_smem + region0 ? ((uint32_t)max_optin - static_smem - region0) / stage_bytes : 0u;
         if (nst > nst_cap) nst = nst_cap;
@@ -616,7 +616,6 @@ int setup_stream(nb200_engine *e) {
     g.n_steps = 1; g.nsplit_max = nsplit_max;
     uint32_t ct = 32768u / (d.hd * 8u); ct &= ~7u; if (ct < 32) ct = 32;      // measured: ~32 KB of K+V per (kv head, split) item
     g.chunk_target = env_u32("NB200_ATTN_CHUNK", ct);
-    g.ablate = env_u32("NB200_ABLATE", 0);
     if (g.chunk_target < 8) g.chunk_target = 8;
     g.d = d;
     e->st_kern = (const void *)k; e->st_smem = smem; e->st_grid = NC; e->use_stream = true; e->launches_per_token = 1;

@@ -34,22 +34,24 @@ cudaError_t stream_build_launch(const uint8_t *mainp, const uint8_t *auxp, uint3
     return cudaGetLastError();
 }
 
-template <int QUANT, int LPG>
+template <int QUANT, int LPG, int HDC>
 static StreamKern pick_stream_kvm(uint32_t kvm) {
     switch (kvm) {
-        case 1: return k_decode_stream<QUANT, LPG, 1>;
-        case 2: return k_decode_stream<QUANT, LPG, 2>;
-        case 4: return k_decode_stream<QUANT, LPG, 4>;
+        case 1: return k_decode_stream<QUANT, LPG, 1, HDC>;
+        case 2: return k_decode_stream<QUANT, LPG, 2, HDC>;
+        case 4: return k_decode_stream<QUANT, LPG, 4, HDC>;
         default: return nullptr;
     }
 }
+template <int QUANT, int LPG>
+static StreamKern pick_stream_hd(const Dims &d) { return d.hd <= 64 ? pick_stream_kvm<QUANT, LPG, 64>(d.kv_mul) : pick_stream_kvm<QUANT, LPG, 128>(d.kv_mul); }
 
 StreamKern pick_stream(const Dims &d) {
     if (d.hd > 128 || (d.arch == 3u && (d.hd & (d.hd - 1)) != 0)) return nullptr;     // in-register half-split RoPE needs hd = 4 * 2^k
-    if (d.quant == 0x00u) return pick_stream_kvm<0x00, 8>(d.kv_mul);
-    if (d.quant == 0x42u) return pick_stream_kvm<0x42, 8>(d.kv_mul);
-    if (d.gs == 128) return pick_stream_kvm<0x80, 8>(d.kv_mul);
-    if (d.gs == 64) return pick_stream_kvm<0x80, 4>(d.kv_mul);
+    if (d.quant == 0x00u) return pick_stream_hd<0x00, 8>(d);
+    if (d.quant == 0x42u) return pick_stream_hd<0x42, 8>(d);
+    if (d.gs == 128) return pick_stream_hd<0x80, 8>(d);
+    if (d.gs == 64) return pick_stream_hd<0x80, 4>(d);
     return nullptr;
 }
 

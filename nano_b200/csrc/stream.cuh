@@ -21,9 +21,15 @@
 // One true grid barrier per token (release/acquire, at the classifier) orders the plain stores -- KV-cache rows, logits,
 // ids, repetition-penalty flags -- against the next token's reads (TMA reads of the cache included).
 //
+// What bounds it at batch 1 is a chain: 5 exchanges a layer, and between two of them what every SM does with what arrived (norm and quantise, barrier, row dots,
+// epilogue; attention in the CTAs that have an item).  A phase issues little work over 15 warps (4 a scheduler), so its time goes with the number of dependent
+// steps and of instructions that every warp issues, not with bytes: no per-lane trip counts, one epilogue per block of rows, polls that ask for everything again instead of one
+// word after the other, little state kept across phases.  Attention item without barriers between scores, softmax and values; one copy of each loop (197 KB of code before,
+// 110 now).  Measured per token in the device loop, before -> now: Nano-168M Q80 at 16..40 positions 603 -> 366 us, Qwen3-0.6B Q80 at 260 961 -> 591, two layers of
+// Qwen3-4B's width at 1500 143 -> 107, four of Nano's in F32 117 -> 88.
+//
 // Arithmetic (fast mode only; the bit-exact mode never runs this kernel): exact integer group dots; the fp32 combine of a
-// quantised row (infer.c:668-674, tensor.c:425-430) in the reference's order on shared tiles and as one partial per lane
-// + a warp tree on warp-owned tiles; tree reductions for rmsnorm / attention, expf and the division by sqrt(head_dim) as
+// quantised row (infer.c:668-674, tensor.c:425-430) as one partial per lane + a warp tree; tree reductions for rmsnorm / attention, expf and the division by sqrt(head_dim) as
 // the reference.  Reference: llm_forward infer/infer.c:971-1018, transformer_block_forward :713-966.
 #pragma once
 #include "kernels.cuh"
@@ -86,9 +92,13 @@ __device__ __forceinline__ unsigned long long xw_ld1(const unsigned long long *p
 __device__ __forceinline__ void xw_st(unsigned long long *p, float v, uint32_t epoch) {
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(((unsigned long long)epoch << 32) | __float_as_uint(v)) : "memory");
 }
-constexpr uint32_t kXwAny = 0xffffffffu;        // timing experiments only (NB200_ABLATE & 16): accept any epoch
-__device__ __forceinline__ bool xw_ok(unsigned long long w, uint32_t need) { return (uint32_t)(w >> 32) == need || need == kXwAny; }
+__device__ __forceinline__ bool xw_ok(unsigned long long w, uint32_t need) { return (uint32_t)(w >> 32) == need; }
 __device__ __forceinline__ float xw_val(unsigned long long w) { return __uint_as_float((uint32_t)w); }
+// now and then inside a polling loop: start the clock, or give up after ~2 s
+static __device__ __noinline__ void st_still_waiting(long long &t0, uint32_t *err, uint32_t code) {
+    if (t0 == 0) t0 = clock64();
+    else if (clock64() - t0 > 4000000000ll) st_give_up(err, code);
+}
 // 4 consecutive words (32-byte aligned) -> float4 once all of them carry `need`
 static __device__ __noinline__ float4 xw_poll4_slow(const unsigned long long *p, uint32_t need, uint32_t *err) {
     unsigned long long a, b, c, d;
@@ -109,22 +119,6 @@ __device__ __forceinline__ float4 xw_poll4(const unsigned long long *p, uint32_t
     if (xw_ok(a, need) && xw_ok(b, need) && xw_ok(c, need) && xw_ok(d, need)) return make_float4(xw_val(a), xw_val(b), xw_val(c), xw_val(d));
     return xw_poll4_slow(p, need, err);
 }
-static __device__ __noinline__ float xw_poll1(const unsigned long long *p, uint32_t need, uint32_t *err) {
-    unsigned long long a = xw_ld1(p);
-    if (!xw_ok(a, need)) {
-        const long long t0 = clock64();
-        do {
-            a = xw_ld1(p);
-            if (clock64() - t0 > 4000000000ll) st_give_up(err, 0x51u);
-        } while (!xw_ok(a, need));
-    }
-    return xw_val(a);
-}
-// one element into every replica of a vector, the stores spread over the `ts` lanes of a team (tl = lane within the team)
-__device__ __forceinline__ void xw_publish(unsigned long long *base, uint32_t rs, uint32_t idx, float v, uint32_t epoch, uint32_t tl, uint32_t ts) {
-    for (uint32_t r = tl; r < (uint32_t)kStRep; r += ts) xw_st(base + (size_t)r * rs + idx, v, epoch);
-}
-
 // ---------------------------------------------------------------- schedule helpers shared by producer and consumers
 // split of the attention range over CTAs: as few (kv head, split) items as keep an item under ~chunk_target rows
 __device__ __forceinline__ void st_attn_plan(uint32_t range, uint32_t nsplit_max, uint32_t chunk_target, uint32_t &nsplit, uint32_t &chunk) {
@@ -136,6 +130,9 @@ __device__ __forceinline__ void st_attn_plan(uint32_t range, uint32_t nsplit_max
     chunk = c;
     nsplit = (range + c - 1) / c;
 }
+
+struct StPlan { uint32_t nsplit, kvh, sp, t0, t1; };          // this CTA's attention item of the token (kvh >= KV: none)
+struct StSmem { float red[2][16]; float best_v[kConsWarps]; uint32_t best_i[kConsWarps]; float pen; uint32_t target, ti, tj; StPlan plan; };
 
 struct StRing {
     uint64_t *full, *empty;
@@ -150,15 +147,14 @@ __device__ __forceinline__ void mbar_arrive_n(uint64_t *bar, uint32_t n) {
 }
 struct StCursor { uint32_t s, par; };     // stage and parity of the next tile (producer: empty parity; consumer: full parity)
 __device__ __forceinline__ void st_advance(StCursor &c, uint32_t nstages) { if (++c.s == nstages) { c.s = 0; c.par ^= 1u; } }
-struct StOwn { uint32_t row0[5], rows[5]; };      // the rows this CTA owns of every phase kind (shared memory; computed once)
-// How the 32 lanes of a warp share the rows of a tile, per phase kind (computed once per launch, kept in shared memory:
-// run-time integer divisions cost ~150 cycles each and sat on every phase's critical path).
-// Q80: a row of G groups is owned by a team of gteam * lg2 lanes (lg2 lanes split the 16-byte chunks of one group);
-// rw = rows per warp pass.  F32 / Q4K: one warp per row.
-struct StGeo {
-    uint8_t lg2[5], gteam[5], ts[5], rw[5], mode[5];      // mode: 0 single rows, 1 pair (w1, w3) on adjacent teams, 2 pair done by one team
-    uint8_t team[5][32], tl[5][32];                       // per lane: team index within the warp, lane index within the team
-    uint8_t gl[5][32], ul[5][32];                         // per lane: group within the team pass, lane within the group
+__device__ __forceinline__ void st_skip(StCursor &c, uint32_t n, uint32_t nstages) { c.s += n; while (c.s >= nstages) { c.s -= nstages; c.par ^= 1u; } }
+// What a consumer needs of a phase kind, gathered once per launch in shared memory: two 16-byte loads at a phase's start.  (Kept in registers across the
+// layer, these spilled, and one reload of a spilled register from local memory takes 1000 to 2700 cycles here: most of L1 is shared memory, and the polls keep L2 busy.)
+struct __align__(16) StPhase {
+    uint32_t n, row_stride, aux_stride, tile_rows;
+    uint32_t rows, tiles, row0, mode;         // the rows and tiles this CTA owns; mode: owned | rb << 8 | tb << 16, shared tiles: rb = rows of a warp's pass, tb = blocks of rb rows in a full tile (mod 15)
+    const unsigned long long *src; const float *gain;      // the replica this CTA reads (null gain: no norm before this product)
+    uint32_t need, out, epi; float rn;        // epochs read and published, counted from the layer's first; rn = 1 / n
 };
 
 // ---------------------------------------------------------------- producer (warp 15, lane 0)
@@ -176,7 +172,7 @@ __device__ __forceinline__ void st_issue_kind(const StreamArgs &g, const StRing 
     }
 }
 
-static __device__ void st_producer(const StreamArgs &g, const StRing &r, const StOwn &own, uint32_t cta, volatile uint32_t *progress,
+static __device__ void st_producer(const StreamArgs &g, const StRing &r, const StPhase *own, uint32_t cta, volatile uint32_t *progress,
                                    uint32_t pos0, uint32_t causal, uint32_t advance) {
     const Dims &d = g.d;
     StCursor c{0u, 1u};                       // parity 1 passes at once on a stage's first use
@@ -190,7 +186,7 @@ static __device__ void st_producer(const StreamArgs &g, const StRing &r, const S
         st_attn_plan(range, g.nsplit_max, g.chunk_target, nsplit, chunk);
         for (uint32_t l = 0; l < d.L; l++) {
             const uint8_t *lb = base + (uint64_t)l * g.layer_stride;
-            st_issue_kind(g, r, c, issued, g.kind[SK_QKV], lb, own.rows[SK_QKV]);
+            st_issue_kind(g, r, c, issued, g.kind[SK_QKV], lb, own[SK_QKV].rows);
             if (cta < d.KV * nsplit) {
                 const uint32_t kvh = cta / nsplit, sp = cta % nsplit;
                 const uint32_t t0 = min(range, sp * chunk), t1 = min(range, t0 + chunk);
@@ -216,51 +212,38 @@ static __device__ void st_producer(const StreamArgs &g, const StRing &r, const S
                     st_advance(c, r.nstages);
                 }
             }
-            st_issue_kind(g, r, c, issued, g.kind[SK_O], lb, own.rows[SK_O]);
-            st_issue_kind(g, r, c, issued, g.kind[SK_W13], lb, own.rows[SK_W13]);
-            st_issue_kind(g, r, c, issued, g.kind[SK_W2], lb, own.rows[SK_W2]);
+            st_issue_kind(g, r, c, issued, g.kind[SK_O], lb, own[SK_O].rows);
+            st_issue_kind(g, r, c, issued, g.kind[SK_W13], lb, own[SK_W13].rows);
+            st_issue_kind(g, r, c, issued, g.kind[SK_W2], lb, own[SK_W2].rows);
         }
-        st_issue_kind(g, r, c, issued, g.kind[SK_CLS], base + g.cls_off, own.rows[SK_CLS]);
+        st_issue_kind(g, r, c, issued, g.kind[SK_CLS], base + g.cls_off, own[SK_CLS].rows);
     }
 }
 
 // ---------------------------------------------------------------- activation prologue (consumer threads)
 // Source vector (exchange words of epoch `need`, or the embedding row in shared memory) -> (rmsnorm) -> activation
-// operand of the matvec in shared memory, straight from registers:
-//   Q80 (tensor.c:21-46): one quantisation group per lane team, 4 elements per lane; F32: normalised floats;
+// operand of the matvec in shared memory:
+//   Q80 (tensor.c:21-46): one quantisation group per 16 or 32 lanes, 4 elements per lane; F32: floats;
 //   Q4K (tensor.c:144-242): one 256-element block per warp, 8 elements per lane.
-// act layouts as in kernels.cuh (act_region_bytes).  KMAX warp slots per warp stay in registers between the
-// sum-of-squares pass and the quantise pass (host checks n <= st_prep_max_n).
-// fine-grained stamps inside a phase: compiled in only with -DNB200_FINE_TRACE (each costs ~200 cycles on the stamped path: a
-// divergent clock read + generic store in front of the next warp-synchronous instruction -- they distort what they measure)
-#ifdef NB200_FINE_TRACE
-#define ST_DBG(k) do { if (dbg && threadIdx.x == 0) dbg[k] = clock64(); } while (0)
-#else
-#define ST_DBG(k) do { } while (0)
-#endif
+// act layouts as in kernels.cuh (act_region_bytes).
 template <int QUANT, int LPG>
 __device__ __forceinline__ void st_prep(const StreamArgs &g, const unsigned long long *xsrc, const float *ssrc, uint32_t need, const float *__restrict__ gain,
-                                        uint32_t n, unsigned char *act, float *red, unsigned long long *dbg) {
+                                        uint32_t n, float rn, unsigned char *act, float *red) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    ST_DBG(0);
-    if (gain) {      // the gain is applied after the sum of squares: start pulling its lines into L1 while the source is awaited
-        for (uint32_t i = threadIdx.x * 32u; i < n; i += kConsThreads * 32u) asm volatile("prefetch.global.L1 [%0];" ::"l"(gain + i));
-    }
+    auto sq = [](float4 v, float ss) -> float { return fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, ss)))); };
     auto nrm = [&](float4 v, float4 gn, float inv) -> float4 {      // infer.c:611: weight * (ss * x)
         return make_float4(__fmul_rn(gn.x, __fmul_rn(inv, v.x)), __fmul_rn(gn.y, __fmul_rn(inv, v.y)),
                            __fmul_rn(gn.z, __fmul_rn(inv, v.z)), __fmul_rn(gn.w, __fmul_rn(inv, v.w)));
     };
-    auto sq = [](float4 v, float ss) -> float { return fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, ss)))); };
     auto inverse = [&](float ss) -> float {                         // infer.c:601-609, tree sum in a fixed order
         ss = warp_sum(ss);
         if (lane == 0) red[warp] = ss;
         cbar();
-        float tot = 0.0f;
-#pragma unroll
-        for (int w = 0; w < kConsWarps; w++) tot += red[w];
-        tot = __fdiv_rn(tot, (float)n);
-        tot = __fadd_rn(tot, 1e-5f);
-        return __fdiv_rn(1.0f, __fsqrt_rn(tot));
+        const float4 *r4 = reinterpret_cast<const float4 *>(red);   // red[15] stays 0
+        const float4 a = r4[0], b = r4[1], c = r4[2], e = r4[3];
+        const float tot = (((a.x + a.y) + (a.z + a.w)) + ((b.x + b.y) + (b.z + b.w))) + (((c.x + c.y) + (c.z + c.w)) + ((e.x + e.y) + (e.z + e.w)));
+        const float q = tot * rn;                                   // tot / n, rounded: the product by the rounded reciprocal with its remainder added back
+        return __frcp_rn(__fsqrt_rn(__fadd_rn(fmaf(fmaf(-q, (float)n, tot), rn, q), 1e-5f)));
     };
     if constexpr (QUANT == 0x42) {
         uint32_t *xe = reinterpret_cast<uint32_t *>(act);
@@ -281,10 +264,8 @@ __device__ __forceinline__ void st_prep(const StreamArgs &g, const unsigned long
                 }
             }
         }
-        ST_DBG(1);
         float inv = 1.0f;
         if (gain) inv = inverse(ss);
-        ST_DBG(2);
 #pragma unroll
         for (int j = 0; j < kStKmaxQ4K; j++) {
             const uint32_t b = warp + kConsWarps * j;
@@ -303,369 +284,277 @@ __device__ __forceinline__ void st_prep(const StreamArgs &g, const unsigned long
             }
         }
     } else {
-        // Q80: a group (gs elements) is held by LG = gs/4 lanes, 4 elements (one float4) per lane, GW = 32/LG groups per warp slot
-        // (measured: one group per warp with 4 elements per lane has the shorter dependent chain; 8 per lane was ~600 cycles slower).
-        // F32: no grouping semantics, 128-element slots.
-        constexpr uint32_t gs = (QUANT == 0x80) ? LPG * 16u : 128u;
-        constexpr uint32_t LG = gs / 4u;                                 // lanes per group (16 or 32)
-        constexpr uint32_t GW = 32u / LG;                                // groups per warp slot
+        constexpr uint32_t gs = (QUANT == 0x80) ? LPG * 16u : 128u;      // Q80: elements of a group; F32: no grouping
+        constexpr uint32_t LG = gs / 4u;                                 // lanes per group
         static_assert(LG == 16 || LG == 32, "stream kernel: Q80 group size 64 or 128");
-        const uint32_t G = (n + gs - 1u) / gs;                           // F32: n % 4 == 0 only, the last slot may be partial
-        const uint32_t sub = lane / LG, li = lane % LG;
-        float4 v[kStKmax];
-        if (ssrc) {
-#pragma unroll
-            for (int j = 0; j < kStKmax; j++) {
-                const uint32_t i = ((warp + kConsWarps * j) * GW + sub) * gs + li * 4u;
-                v[j] = (i < n) ? *reinterpret_cast<const float4 *>(ssrc + i) : make_float4(0, 0, 0, 0);
-            }
-        } else {
-            // every load of the thread is in flight before the first epoch is looked at
-            unsigned long long w[kStKmax][4];
-#pragma unroll
-            for (int j = 0; j < kStKmax; j++) {
-                const uint32_t i = ((warp + kConsWarps * j) * GW + sub) * gs + li * 4u;
-                if (i < n) { xw_ld2(xsrc + i, w[j][0], w[j][1]); xw_ld2(xsrc + i + 2, w[j][2], w[j][3]); }
-            }
-#pragma unroll
-            for (int j = 0; j < kStKmax; j++) {
-                const uint32_t i = ((warp + kConsWarps * j) * GW + sub) * gs + li * 4u;
-                v[j] = make_float4(0, 0, 0, 0);
-                if (i < n) {
-                    if (xw_ok(w[j][0], need) && xw_ok(w[j][1], need) && xw_ok(w[j][2], need) && xw_ok(w[j][3], need))
-                        v[j] = make_float4(xw_val(w[j][0]), xw_val(w[j][1]), xw_val(w[j][2]), xw_val(w[j][3]));
-                    else v[j] = xw_poll4_slow(xsrc + i, need, g.err);
+        auto put = [&](float4 v, uint32_t i, bool on) {
+            if constexpr (QUANT == 0x00) {
+                if (on) *reinterpret_cast<float4 *>(act + (size_t)i * 4u) = v;
+            } else {
+                // tensor.c:21-46.  amax over the group with one REDUX (the values are non-negative: uint order == float order);
+                // the exact scale amax/127 is off the codes' critical path; codes come from q = v * (127/amax) rounded by adding 1.5 * 2^23 (the integer is
+                // then in the low bits), and any q within 1e-4 of a .5 boundary goes through the exact division + round().  (q and the quotient by sc are at most 4.2e-7 |q| apart:
+                // two ulp of the approximate division, half an ulp each for the product, for sc and for the exact division.  A window of 1e-3 sent a warp's 128 values
+                // there one time in four, so that of the warps of a row one nearly always went.)
+                float amax = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
+                const uint32_t gmask = (LG == 32u) ? 0xffffffffu : ((lane & 16) ? 0xffff0000u : 0xffffu);
+                amax = __uint_as_float(__reduce_max_sync(gmask, __float_as_uint(amax)));
+                const float sc = __fdiv_rn(amax, 127.0f), rinv = __fdividef(127.0f, amax);
+                const float q0 = v.x * rinv, q1 = v.y * rinv, q2 = v.z * rinv, q3 = v.w * rinv, magic = 12582912.0f;
+                const float r0 = q0 + magic, r1 = q1 + magic, r2 = q2 + magic, r3 = q3 + magic;
+                uint32_t c0 = __float_as_uint(r0), c1 = __float_as_uint(r1), c2 = __float_as_uint(r2), c3 = __float_as_uint(r3);
+                const float off = fmaxf(fmaxf(fabsf(q0 - (r0 - magic)), fabsf(q1 - (r1 - magic))), fmaxf(fabsf(q2 - (r2 - magic)), fabsf(q3 - (r3 - magic))));
+                if (sc == 0.0f) c0 = c1 = c2 = c3 = 0u;
+                else if (off > 0.4999f) { c0 = q80_code_slow(v.x, sc); c1 = q80_code_slow(v.y, sc); c2 = q80_code_slow(v.z, sc); c3 = q80_code_slow(v.w, sc); }
+                if (on) {
+                    *reinterpret_cast<uint32_t *>(act + i) = __byte_perm(__byte_perm(c0, c1, 0x0040), __byte_perm(c2, c3, 0x0040), 0x5410);
+                    if ((lane & (LG - 1u)) == 0) reinterpret_cast<float *>(act + ((n + 15u) & ~15u))[i / gs] = sc;
                 }
             }
-        }
-        float ss = 0.0f;
-#pragma unroll
-        for (int j = 0; j < kStKmax; j++) ss = sq(v[j], ss);
-        ST_DBG(1);
-        float inv = 1.0f;
-        if (gain && !(g.ablate & 8u)) inv = inverse(ss);
-        ST_DBG(2);
-#pragma unroll
-        for (int j = 0; j < kStKmax; j++) {
-            const uint32_t g0 = (warp + kConsWarps * j) * GW;
-            if (g0 < G) {                                            // warp-uniform
-                const uint32_t gi = g0 + sub, i = gi * gs + li * 4u;
-                const bool on = i < n;
-                float4 a = v[j];
-                if (gain && on) a = nrm(a, __ldg(reinterpret_cast<const float4 *>(gain + i)), inv);
-                if constexpr (QUANT == 0x00) {
-                    if (on) *reinterpret_cast<float4 *>(act + (size_t)i * 4u) = a;
-                } else {
-                    int8_t *codes = reinterpret_cast<int8_t *>(act);
-                    float *scales = reinterpret_cast<float *>(act + ((n + 15u) & ~15u));
-                    // tensor.c:21-46.  amax over the group with one REDUX (the values are non-negative: uint order == float order);
-                    // the exact scale amax/127 is off the codes' critical path; codes come from q = v * (127/amax) rounded with the
-                    // magic-number add, and any q within 1e-3 of a .5 boundary goes through the exact division + round().
-                    const float av[4] = {a.x, a.y, a.z, a.w};
-                    float amax = fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(a.z), fabsf(a.w)));
-                    const uint32_t gmask = (LG == 32u) ? 0xffffffffu : (0xffffu << (16u * sub));
-                    amax = __uint_as_float(__reduce_max_sync(gmask, __float_as_uint(amax)));
-                    const float sc = __fdiv_rn(amax, 127.0f);
-                    const float rinv = __fdividef(127.0f, amax);
-                    if (on) {
-                        uint32_t pk = 0;
-                        if (sc != 0.0f && !(g.ablate & 1u)) {
-                            int cq[4]; bool tie = false;
-#pragma unroll
-                            for (int u = 0; u < 4; u++) {
-                                const float q = av[u] * rinv, aq = fabsf(q);
-                                const float rr = aq + 12582912.0f;                 // 1.5 * 2^23: the integer nearest to aq sits in the mantissa
-                                const float cf = rr - 12582912.0f;
-                                const int c = __float_as_int(rr) - 0x4b400000;
-                                tie = tie || fabsf(aq - cf) > 0.499f;
-                                cq[u] = q < 0.0f ? -c : c;
+        };
+        // Two slots of 128 elements per warp and turn: all their loads are in flight before the first epoch is looked at.  With a gain the
+        // source is walked twice (sum of squares, then the operand); one turn (n <= 3840) keeps it in registers, longer ones read it again.  One copy of the
+        // loop serves both walks and a third of the slots that the longest row needs: the kernel's instructions do not fit the caches near the SM, and what is
+        // unrolled but skipped is fetched all the same (six slots unrolled: 197 KB of code, now about half).
+        constexpr uint32_t turn = 2u * kConsWarps * 128u;
+        float ss = 0.0f, inv = 1.0f;
+        float4 v0 = make_float4(0, 0, 0, 0), v1 = v0, g0 = v0, g1 = v0;
+#pragma unroll 1
+        for (uint32_t walk = gain ? 0u : 1u; walk < 2u; walk++) {
+#pragma unroll 1
+            for (uint32_t s = warp * 128u; s < n; s += turn) {
+                const uint32_t i0 = s + lane * 4u, i1 = i0 + kConsWarps * 128u;
+                const bool on0 = i0 < n, on1 = i1 < n;
+                if (walk == 0u || !gain || n > turn) {
+                    if (gain) {
+                        if (on0) g0 = __ldg(reinterpret_cast<const float4 *>(gain + i0));
+                        if (on1) g1 = __ldg(reinterpret_cast<const float4 *>(gain + i1));
+                    }
+                    if (ssrc) {
+                        v0 = v1 = make_float4(0, 0, 0, 0);
+                        if (on0) v0 = *reinterpret_cast<const float4 *>(ssrc + i0);
+                        if (on1) v1 = *reinterpret_cast<const float4 *>(ssrc + i1);
+                    } else {
+                        // both slots are asked for again until both are there: one after the other, the second would cost another trip to L2
+                        long long t0 = 0;
+#pragma unroll 1
+                        for (uint32_t it = 1;; it++) {
+                            unsigned long long w0, w1, w2, w3, z0, z1, z2, z3;
+                            w0 = w1 = w2 = w3 = z0 = z1 = z2 = z3 = (unsigned long long)need << 32;
+                            if (on0) { xw_ld2(xsrc + i0, w0, w1); xw_ld2(xsrc + i0 + 2, w2, w3); }
+                            if (on1) { xw_ld2(xsrc + i1, z0, z1); xw_ld2(xsrc + i1 + 2, z2, z3); }
+                            if (xw_ok(w0, need) && xw_ok(w1, need) && xw_ok(w2, need) && xw_ok(w3, need) && xw_ok(z0, need) && xw_ok(z1, need) && xw_ok(z2, need) && xw_ok(z3, need)) {
+                                v0 = make_float4(xw_val(w0), xw_val(w1), xw_val(w2), xw_val(w3));
+                                v1 = make_float4(xw_val(z0), xw_val(z1), xw_val(z2), xw_val(z3));
+                                break;
                             }
-                            if (tie) {                                           // rare: some q within 1e-3 of a tie -> the exact division + round()
-#pragma unroll
-                                for (int u = 0; u < 4; u++) cq[u] = q80_code_slow(av[u], sc);
-                            }
-                            pk = ((uint32_t)cq[0] & 0xffu) | (((uint32_t)cq[1] & 0xffu) << 8) | (((uint32_t)cq[2] & 0xffu) << 16) | (((uint32_t)cq[3] & 0xffu) << 24);
+                            if ((it & 255u) == 0) st_still_waiting(t0, g.err, 0x50u);          // the clock is read rarely: the loop stays loads and compares
                         }
-                        *reinterpret_cast<uint32_t *>(codes + i) = pk;
-                        if (li == 0) scales[gi] = sc;
+                        __syncwarp();
                     }
                 }
+                if (walk == 0u) { ss = sq(v1, sq(v0, ss)); continue; }
+                put(gain ? nrm(v0, g0, inv) : v0, i0, on0);
+                if (s + kConsWarps * 128u < n) put(gain ? nrm(v1, g1, inv) : v1, i1, on1);         // warp-uniform
             }
+            if (walk == 0u) inv = inverse(ss);
         }
     }
-    ST_DBG(3);
     cbar();
-    ST_DBG(4);
 }
 
 // ---------------------------------------------------------------- row dots on a shared-memory tile
-// Q80, matmul_quant infer.c:654-679.  A row of G = n/gs groups is owned by a team of gteam * LG2 lanes: LG2 lanes share
-// the 16-byte chunks of one group (chunk order rotated by the group index: the lanes of a quarter-warp hit different
-// banks), an xor-shuffle over those LG2 lanes leaves the exact integer group sum in each of them, and the fp32 terms are
-// summed in group order (the reference's left-to-right sum) by every lane of the team, so the row value ends up in all of
-// the team's lanes.  Rows longer than gteam groups take several passes (LG2 = 1 then).
-template <int LPG>
-__device__ __forceinline__ float st_row_q80_lpg(const unsigned char *wrow, const float *srow, uint32_t n, const unsigned char *act,
-                                                uint32_t lg2, uint32_t gteam, uint32_t gl, uint32_t u, uint32_t team_base, unsigned long long *dbg = nullptr) {
-    constexpr uint32_t gs = LPG * 16;
-    ST_DBG(10);
-    const float *xs = reinterpret_cast<const float *>(act + ((n + 15u) & ~15u));
-    const uint32_t G = n / gs;
-    float val = 0.0f;
-    for (uint32_t g0 = 0; g0 < G; g0 += gteam) {               // warp-uniform
-        const uint32_t gi = g0 + gl;
-        const uint32_t gc = gi < G ? gi : G - 1u;
-        const unsigned char *wp = wrow + (size_t)gc * gs, *xp = act + (size_t)gc * gs;
-        int a0 = 0, a1 = 0, a2 = 0, a3 = 0;
-        for (uint32_t c = u; c < (uint32_t)LPG; c += lg2) {
-            const uint32_t off = ((c + gl * lg2) % LPG) * 16u;
-            const int4 w = *reinterpret_cast<const int4 *>(wp + off), xq = *reinterpret_cast<const int4 *>(xp + off);
-            a0 = __dp4a(w.x, xq.x, a0); a1 = __dp4a(w.y, xq.y, a1); a2 = __dp4a(w.z, xq.z, a2); a3 = __dp4a(w.w, xq.w, a3);
-        }
-        int isum = (a0 + a1) + (a2 + a3);
-        for (uint32_t o = 1; o < lg2; o <<= 1) isum += __shfl_xor_sync(0xffffffffu, isum, o);
-        ST_DBG(11);
-        const float term = __fmul_rn(__fmul_rn((float)isum, srow[gc]), xs[gc]);
-        ST_DBG(12);
-        const uint32_t cnt = min(gteam, G - g0);
-        for (uint32_t j0 = 0; j0 < cnt; j0 += 8u) {           // the shuffles of a batch are issued before the ordered adds
-            float t8[8];
+// A warp takes RB rows, its lanes split the row in 16-byte chunks (512 bytes per step, conflict-free).  Nothing crosses lanes inside the loop: every lane
+// keeps one fp32 partial per row, the steps are independent of each other.  (Fast mode: the fp32 summation order differs from matmul_quant
+// infer.c:654-679; the bit-exact mode never runs this kernel.)  Row r of the block is rr + r; past the tile's last row the last one is read again.
+template <int QUANT, int LPG, int RB>
+__device__ __forceinline__ void st_partials(const unsigned char *tile, uint32_t row_stride, const unsigned char *aux, uint32_t aux_stride,
+                                            uint32_t rr, uint32_t tr, uint32_t n, const unsigned char *act, float (&acc)[RB]) {
+    const int lane = threadIdx.x & 31;
+    const unsigned char *w[RB], *ws[RB];
 #pragma unroll
-            for (int j = 0; j < 8; j++) t8[j] = __shfl_sync(0xffffffffu, term, team_base + ((j0 + j) * lg2 & 31u));
-#pragma unroll
-            for (int j = 0; j < 8; j++) if (j0 + j < cnt) val = __fadd_rn(val, t8[j]);
-        }
-        ST_DBG(13);
+    for (int r = 0; r < RB; r++) {
+        const uint32_t row = min(rr + (uint32_t)r, tr - 1u);
+        w[r] = tile + row * row_stride; ws[r] = aux + row * aux_stride; acc[r] = 0.0f;
     }
-    return val;
-}
-// Throughput form for warp-owned tiles: a whole warp owns RB rows, lanes split K in 16-byte chunks (512 bytes per step,
-// conflict-free).  Nothing crosses lanes inside the loop: every lane keeps one fp32 partial per row
-// (exact integer sum of its 16 codes x the two group scales), the steps are independent of each other so the loads of
-// several steps are in flight at once, and one xor-butterfly per row at the end leaves the value in every lane.
-// (Fast mode: the fp32 summation order differs from matmul_quant infer.c:654-679; the bit-exact mode never runs this kernel.)
-template <int LPG, int RB>
-__device__ __forceinline__ void st_rows_q80_warp(const unsigned char *wrow, uint32_t row_stride, const unsigned char *srow, uint32_t aux_stride,
-                                                 uint32_t n, const unsigned char *act, float (&val)[RB]) {
-    constexpr uint32_t gs = LPG * 16;
-    const int lane = threadIdx.x & 31;
-    const float *xs = reinterpret_cast<const float *>(act + ((n + 15u) & ~15u));
-    float acc[RB];
+    if constexpr (QUANT == 0x80) {
+        constexpr uint32_t gs = LPG * 16;
+        const float *xs = reinterpret_cast<const float *>(act + ((n + 15u) & ~15u));
+        // Uniform trips of two steps; a lane past the row's end reads its last chunk with scale 0 (a trip count of each lane's own made three serial paths of a 768-wide row: 650
+        // cycles a row).  The dot starts from the bits of 1.5 * 2^23, so that its float is the sum's low bits (|sum| <= 16 * 127 * 127 < 2^22).
+        for (uint32_t k0 = 0; k0 < n; k0 += 1024u) {
 #pragma unroll
-    for (int r2 = 0; r2 < RB; r2++) acc[r2] = 0.0f;
-    auto step = [&](uint32_t k) {
-        const int4 xq = *reinterpret_cast<const int4 *>(act + k);
-        const uint32_t gi = k / gs;
-        const float xsc = xs[gi];
+            for (uint32_t h = 0; h < 2u; h++) {
+                const uint32_t k = k0 + h * 512u + lane * 16u, kc = min(k, n - 16u), gi = kc / gs;
+                const int4 xq = *reinterpret_cast<const int4 *>(act + kc);
+                const float xsc = k < n ? xs[gi] : 0.0f;
 #pragma unroll
-        for (int r2 = 0; r2 < RB; r2++) {
-            const int4 w = *reinterpret_cast<const int4 *>(wrow + (size_t)r2 * row_stride + k);
-            const float ws = reinterpret_cast<const float *>(srow + (size_t)r2 * aux_stride)[gi];
-            const int s0 = __dp4a(w.y, xq.y, __dp4a(w.x, xq.x, 0)), s1 = __dp4a(w.w, xq.w, __dp4a(w.z, xq.z, 0));
-            acc[r2] = fmaf((float)(s0 + s1), ws * xsc, acc[r2]);
+                for (int r = 0; r < RB; r++) {
+                    const int4 q = *reinterpret_cast<const int4 *>(w[r] + kc);
+                    const float wsc = reinterpret_cast<const float *>(ws[r])[gi];
+                    const int s0 = __dp4a(q.y, xq.y, __dp4a(q.x, xq.x, 0x4b400000)), s1 = __dp4a(q.w, xq.w, __dp4a(q.z, xq.z, 0));
+                    acc[r] = fmaf(__int_as_float(s0 + s1) - 12582912.0f, wsc * xsc, acc[r]);
+                }
+            }
         }
-    };
-    uint32_t k = lane * 16u;
-    const uint32_t full = n & ~511u;
-#pragma unroll 2
-    for (; k < full; k += 512u) step(k);
-    if (k < n) step(k);
+    } else if constexpr (QUANT == 0x00) {          // matmul infer.c:637-651
+        const float *x = reinterpret_cast<const float *>(act);
+        for (uint32_t k0 = 0; k0 < n; k0 += 256u) {
 #pragma unroll
-    for (int r2 = 0; r2 < RB; r2++) val[r2] = warp_sum(acc[r2]);
-}
-// F32: matmul infer.c:637-651, fast mode (one warp per row: lane-split FMA + tree)
-__device__ __forceinline__ float st_row_f32(const unsigned char *wrow, uint32_t n, const unsigned char *act) {
-    const int lane = threadIdx.x & 31;
-    const float *x = reinterpret_cast<const float *>(act);
-    float acc = 0.0f;
-#pragma unroll 2
-    for (uint32_t k = lane * 4u; k < n; k += 128u) {
-        const float4 w = *reinterpret_cast<const float4 *>(wrow + (size_t)k * 4u), xv = *reinterpret_cast<const float4 *>(x + k);
-        acc = fmaf(w.x, xv.x, acc); acc = fmaf(w.y, xv.y, acc); acc = fmaf(w.z, xv.z, acc); acc = fmaf(w.w, xv.w, acc);
-    }
-    return warp_sum(acc);
-}
-// Q4K: matmul_q4k / dot_two_blocks_q4k tensor.c:359-471 (one warp per row; one lane = one 32-element group per step; side: 20-byte records)
-__device__ __forceinline__ float st_row_q4k(const unsigned char *wrow, const unsigned char *side, uint32_t n, const unsigned char *act) {
-    const int lane = threadIdx.x & 31;
-    const uint32_t *xe = reinterpret_cast<const uint32_t *>(act);
-    const uint32_t *xo = reinterpret_cast<const uint32_t *>(act + n / 2);
-    const float4 *gp = reinterpret_cast<const float4 *>(act + n);
-    const uint32_t rowbytes = n / 2u;
-    float val = 0.0f;
-    for (uint32_t k0 = 0; k0 < rowbytes; k0 += 512u) {
-        const uint32_t k = k0 + lane * 16u;
-        const bool on = k < rowbytes;
-        const uint32_t grp = k / 16u, blk = grp >> 3, gi = grp & 7u, j = gi & 3u;
-        float term = 0.0f;
-        if (on) {
-            const int4 w = *reinterpret_cast<const int4 *>(wrow + k);
-            const uint32_t *rec = reinterpret_cast<const uint32_t *>(side + (size_t)blk * 20u);
-            const float ssc = __uint_as_float(rec[0]), sbi = __uint_as_float(rec[1]);
-            const uint32_t bs = (rec[2] >> (8 * j)) & 0xff, bb = (rec[3] >> (8 * j)) & 0xff, bh = (rec[4] >> (8 * j)) & 0xff;
-            const uint32_t s6 = (gi < 4) ? (bs & 0x3f) : ((((bs >> 6) << 4) | (bh & 0x0f)) & 0x3f);
-            const uint32_t b6 = (gi < 4) ? (bb & 0x3f) : ((((bb >> 6) << 4) | (bh >> 4)) & 0x3f);
-            const float sp = __fmul_rn((float)s6, ssc), bp = __fmul_rn((float)b6, sbi);
+            for (uint32_t h = 0; h < 2u; h++) {
+                const uint32_t k = k0 + h * 128u + lane * 4u, kc = min(k, n - 4u);
+                float4 xv = *reinterpret_cast<const float4 *>(x + kc);
+                if (k >= n) xv = make_float4(0, 0, 0, 0);
+#pragma unroll
+                for (int r = 0; r < RB; r++) {
+                    const float4 q = *reinterpret_cast<const float4 *>(w[r] + (size_t)kc * 4u);
+                    acc[r] = fmaf(q.x, xv.x, acc[r]); acc[r] = fmaf(q.y, xv.y, acc[r]); acc[r] = fmaf(q.z, xv.z, acc[r]); acc[r] = fmaf(q.w, xv.w, acc[r]);
+                }
+            }
+        }
+    } else {
+        // matmul_q4k / dot_two_blocks_q4k tensor.c:359-471: one lane = one 32-element group per step; side: 20-byte records
+        const uint32_t *xe = reinterpret_cast<const uint32_t *>(act);
+        const uint32_t *xo = reinterpret_cast<const uint32_t *>(act + n / 2);
+        const float4 *gp = reinterpret_cast<const float4 *>(act + n);
+        for (uint32_t k = lane * 16u; k < n / 2u; k += 512u) {
+            const uint32_t grp = k / 16u, blk = grp >> 3, gi = grp & 7u, j = gi & 3u;
             const int4 e4 = *reinterpret_cast<const int4 *>(xe + grp * 4), o4 = *reinterpret_cast<const int4 *>(xo + grp * 4);
             const float4 q = gp[grp];
-            const int wv[4] = {w.x, w.y, w.z, w.w}, ev[4] = {e4.x, e4.y, e4.z, e4.w}, ov[4] = {o4.x, o4.y, o4.z, o4.w};
-            int spq = 0, spp = 0;
 #pragma unroll
-            for (int t = 0; t < 4; t++) {
-                const int lo = wv[t] & 0x0f0f0f0f, hi = (wv[t] >> 4) & 0x0f0f0f0f;
-                spq = __dp4a(lo, ev[t], spq); spq = __dp4a(hi, ov[t], spq);
-                spp = __dp4a(lo, 0x01010101, spp); spp = __dp4a(hi, 0x01010101, spp);
+            for (int r = 0; r < RB; r++) {
+                const int4 wq = *reinterpret_cast<const int4 *>(w[r] + k);
+                const uint32_t *rec = reinterpret_cast<const uint32_t *>(ws[r] + (size_t)blk * 20u);
+                const float ssc = __uint_as_float(rec[0]), sbi = __uint_as_float(rec[1]);
+                const uint32_t bs = (rec[2] >> (8 * j)) & 0xff, bb = (rec[3] >> (8 * j)) & 0xff, bh = (rec[4] >> (8 * j)) & 0xff;
+                const uint32_t s6 = (gi < 4) ? (bs & 0x3f) : ((((bs >> 6) << 4) | (bh & 0x0f)) & 0x3f);
+                const uint32_t b6 = (gi < 4) ? (bb & 0x3f) : ((((bb >> 6) << 4) | (bh >> 4)) & 0x3f);
+                const float sp = __fmul_rn((float)s6, ssc), bp = __fmul_rn((float)b6, sbi);
+                const int wv[4] = {wq.x, wq.y, wq.z, wq.w}, ev[4] = {e4.x, e4.y, e4.z, e4.w}, ov[4] = {o4.x, o4.y, o4.z, o4.w};
+                int spq = 0, spp = 0;
+#pragma unroll
+                for (int t = 0; t < 4; t++) {
+                    const int lo = wv[t] & 0x0f0f0f0f, hi = (wv[t] >> 4) & 0x0f0f0f0f;
+                    spq = __dp4a(lo, ev[t], spq); spq = __dp4a(hi, ov[t], spq);
+                    spp = __dp4a(lo, 0x01010101, spp); spp = __dp4a(hi, 0x01010101, spp);
+                }
+                float term = __fmul_rn(__fmul_rn(sp, q.x), (float)spq);                       // tensor.c:425-428, left to right
+                term = __fsub_rn(term, __fmul_rn(__fmul_rn(sp, q.y), (float)spp));
+                term = __fsub_rn(term, __fmul_rn(__fmul_rn(q.x, bp), q.z));
+                term = __fadd_rn(term, __fmul_rn(__fmul_rn(32.0f, bp), q.y));
+                acc[r] = __fadd_rn(acc[r], term);             // lane-local partial (fast mode: the order of the fp32 sum differs from tensor.c:425-471)
             }
-            term = __fmul_rn(__fmul_rn(sp, q.x), (float)spq);                       // tensor.c:425-428, left to right
-            term = __fsub_rn(term, __fmul_rn(__fmul_rn(sp, q.y), (float)spp));
-            term = __fsub_rn(term, __fmul_rn(__fmul_rn(q.x, bp), q.z));
-            term = __fadd_rn(term, __fmul_rn(__fmul_rn(32.0f, bp), q.y));
         }
-        val = __fadd_rn(val, term);             // lane-local partial (fast mode: the order of the fp32 sum differs from tensor.c:425-471)
     }
-    return warp_sum(val);
+}
+// Row totals: lane l ends with the total of row rr + (l >> shift), the same number in all of that row's lanes, so that a row's epilogue and its stores into
+// the replicas run once for the whole block (RB rows x 8 replicas = 8, 16 or 32 lanes).  The first steps trade rows for lanes: 6 shuffles for 4 rows, not 20.
+template <int QUANT, int LPG, int RB>
+__device__ __forceinline__ float st_rows(const unsigned char *tile, uint32_t row_stride, const unsigned char *aux, uint32_t aux_stride,
+                                         uint32_t rr, uint32_t tr, uint32_t n, const unsigned char *act) {
+    const int lane = threadIdx.x & 31;
+    float acc[RB];
+    st_partials<QUANT, LPG, RB>(tile, row_stride, aux, aux_stride, rr, tr, n, act, acc);
+    float v;
+    if constexpr (RB == 4) {
+        const bool hi = lane & 16, od = lane & 8;
+        const float k0 = hi ? acc[2] : acc[0], k1 = hi ? acc[3] : acc[1], s0 = hi ? acc[0] : acc[2], s1 = hi ? acc[1] : acc[3];
+        const float a = k0 + __shfl_xor_sync(0xffffffffu, s0, 16), b = k1 + __shfl_xor_sync(0xffffffffu, s1, 16);
+        v = od ? b : a;
+        v += __shfl_xor_sync(0xffffffffu, od ? a : b, 8);
+    } else if constexpr (RB == 2) {
+        const bool hi = lane & 16;
+        v = hi ? acc[1] : acc[0];
+        v += __shfl_xor_sync(0xffffffffu, hi ? acc[0] : acc[1], 16);
+        v += __shfl_xor_sync(0xffffffffu, v, 8);
+    } else {
+        v = acc[0];
+        v += __shfl_xor_sync(0xffffffffu, v, 16);
+        v += __shfl_xor_sync(0xffffffffu, v, 8);
+    }
+    v += __shfl_xor_sync(0xffffffffu, v, 4);
+    v += __shfl_xor_sync(0xffffffffu, v, 2);
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    return v;
 }
 
 // ---------------------------------------------------------------- one matvec phase: tiles from the ring -> epilogue
 // The epilogue is selected at run time so that the kernel holds ONE copy of the row loops.
 // Every finished element is published at once (st.relaxed {value, epoch}); nothing else marks the end of a phase.
 // Two ways to share the tiles of a phase among the 15 consumer warps:
-//   shared tiles (few rows per CTA: latency matters): every warp works on every tile, rows spread over lane teams;
+//   shared tiles (few rows per CTA: latency matters): every warp takes `rb` rows of every tile, the fewest that cover a tile in one pass;
 //   owned tiles  (many rows per CTA: throughput matters): tile j belongs to warp j % 15, which walks its rows alone
-//                with full-warp K-split dots while the other warps do the same on their tiles.
+//                while the other warps do the same on their tiles.
 template <int QUANT, int LPG>
-__device__ __forceinline__ void st_consume(const StreamArgs &g, const StRing &r, StCursor &c, uint32_t &tcount, const StKind &k, uint32_t epi, uint32_t layer,
-                                           uint32_t row0, uint32_t rows, uint32_t epoch, const unsigned char *act, uint32_t pos, float pen,
-                                           float *xown, MatvecSmem &ms, const StGeo &geo, uint32_t kid, unsigned long long *dbg) {
+__device__ __forceinline__ void st_consume(const StreamArgs &g, const StRing &r, StCursor &c, uint32_t &tcount, const StPhase &ph, uint32_t layer,
+                                           uint32_t epoch, const unsigned char *act, uint32_t pos, float *xown, StSmem &ms) {
     const Dims &d = g.d;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint4 pa = *reinterpret_cast<const uint4 *>(&ph), pb = *(reinterpret_cast<const uint4 *>(&ph) + 1);
+    const uint32_t n = pa.x, row_stride = pa.y, aux_stride = pa.z, tile_rows = pa.w, rows = pb.x, nt = pb.y, row0 = pb.z, epi = ph.epi;
+    const bool owned = pb.w & 1u;
+    const uint32_t rb = owned ? (QUANT == 0x42 ? 2u : 4u) : (pb.w >> 8) & 255u, step = owned ? rb : rb * kConsWarps, tb = pb.w >> 16;
     float bestv = -FLT_MAX; uint32_t besti = 0xffffffffu;
-    // epilogue of one finished row (value in all `ts` lanes of its team; `ri` = index among the rows this CTA owns)
-    auto emit = [&](uint32_t row, uint32_t ri, float v, float v3, bool pub, uint32_t tl, uint32_t ts) {
-        if (epi == EPI_SWIGLU) {
-            // rows (2i, 2i+1) = (w1 row i, w3 row i); infer.c:937-944
-            if (pub) {
-                const float sg = __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-v)));
-                xw_publish(g.xv[2], g.rs[2], row >> 1, __fmul_rn(__fmul_rn(v, sg), v3), epoch, tl, ts);
-            }
-        } else if (epi == EPI_RESID) {
-            const float xn = __fadd_rn(xown[ri], v);                    // infer.c:906, :963
-            __syncwarp();
-            if (pub) {
-                if (tl == 0) xown[ri] = xn;
-                xw_publish(g.xv[0], g.rs[0], row, xn, epoch, tl, ts);
-            }
-        } else if (epi == EPI_QKV) {
-            if (pub && tl == 0) {
-                xw_st(g.xq + row, v, epoch);
-                if (row >= d.q_dim + d.kv_dim) {                         // V rows also go to the cache for later positions
-                    const uint32_t cc = row - d.q_dim - d.kv_dim, h = cc / d.hd, i = cc % d.hd;
-                    g.vc[(size_t)layer * d.KV * d.max_seq * d.hd + ((size_t)h * d.max_seq + pos) * d.hd + i] = v;
-                }
-            }
-        } else if (pub) {
-            // classifier: infer.c:1156-1167 penalty (division, any sign), then first-max argmax :1026-1037 (rows ascend per lane)
-            if (pen != 1.0f && __ldcg(g.seen + row)) v = __fdiv_rn(v, pen);
-            if (tl == 0) g.logits[row] = v;
-            if (v > bestv) { bestv = v; besti = row; }
+    const uint32_t jstep = owned ? (uint32_t)kConsWarps : 1u;
+    uint32_t turn = (uint32_t)warp;                         // shared tiles: which block of rows of the tile is this warp's first
+    StCursor cc = c;
+    if (owned) st_skip(cc, (uint32_t)warp, r.nstages);
+#pragma unroll 1
+    for (uint32_t j = owned ? (uint32_t)warp : 0u; j < nt; j += jstep) {
+        const uint32_t done = j * tile_rows, tr = min(tile_rows, rows - done);
+        if (owned && r.tile_id[cc.s] != tcount + j) {
+            const long long t0 = clock64();
+            while (r.tile_id[cc.s] != tcount + j) { __nanosleep(20); if (clock64() - t0 > 4000000000ll) st_give_up(g.err, 0x28u); }
         }
-    };
-    if (k.owned) {
-        // ---- owned tiles ----
-        StCursor cc = c;
-        uint32_t j = 0;
-        for (uint32_t done = 0; done < rows; done += k.tile_rows, j++) {
-            if (j % kConsWarps == (uint32_t)warp) {
-                const uint32_t tr = min(k.tile_rows, rows - done), want = tcount + j;
-                if (r.tile_id[cc.s] != want) {
-                    const long long t0 = clock64();
-                    while (r.tile_id[cc.s] != want) { __nanosleep(20); if (clock64() - t0 > 4000000000ll) st_give_up(g.err, 0x28u); }
+        mbar_wait(&r.full[cc.s], cc.par, g.err, 0x20u + epi);
+        const unsigned char *tile = r.buf + (size_t)cc.s * r.stage_bytes;
+        const unsigned char *aux = tile + tr * row_stride;
+#pragma unroll 1
+        for (uint32_t rr = owned ? 0u : rb * turn; rr < tr; rr += step) {
+            const uint32_t cnt = min(rb, tr - rr);
+            uint32_t sh = 5u;                                   // lanes of a row: 2^sh
+            float v;
+            if (QUANT != 0x42 && cnt > 2u) { v = st_rows<QUANT, LPG, (QUANT == 0x42 ? 2 : 4)>(tile, row_stride, aux, aux_stride, rr, tr, n, act); sh = 3u; }
+            else if (cnt == 2u) { v = st_rows<QUANT, LPG, 2>(tile, row_stride, aux, aux_stride, rr, tr, n, act); sh = 4u; }
+            else v = st_rows<QUANT, LPG, 1>(tile, row_stride, aux, aux_stride, rr, tr, n, act);
+            // ---- epilogue: lane = (row u of the block, replica) ----
+            const uint32_t u = (uint32_t)lane >> sh, rep = lane & 7u, ri = done + rr + u, row = row0 + ri;
+            const bool on = u < cnt && (lane & ((1u << sh) - 1u)) < (uint32_t)kStRep;
+            if (epi == EPI_SWIGLU) {
+                // rows (2i, 2i+1) = (w1 row i, w3 row i); infer.c:937-944
+                const float v3 = __shfl_down_sync(0xffffffffu, v, 1u << (sh & 31u));
+                if (on && !(u & 1u)) {
+                    const float sg = __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-v)));
+                    xw_st(g.xv[2] + rep * g.rs[2] + (row >> 1), __fmul_rn(__fmul_rn(v, sg), v3), epoch);
                 }
-                mbar_wait(&r.full[cc.s], cc.par, g.err, 0x29u);
-                const unsigned char *tile = r.buf + (size_t)cc.s * r.stage_bytes;
-                const unsigned char *aux = tile + (size_t)tr * k.row_stride;
-                // rows in blocks of 4 / 2 / 1 (SwiGLU tiles hold whole (w1, w3) pairs: an even row count)
-                auto out = [&](uint32_t rr, const float *v, uint32_t cnt) {
-                    if (epi == EPI_SWIGLU) { for (uint32_t u = 0; u + 1u < cnt; u += 2u) emit(row0 + done + rr + u, done + rr + u, v[u], v[u + 1u], true, (uint32_t)lane, 32u); }
-                    else { for (uint32_t u = 0; u < cnt; u++) emit(row0 + done + rr + u, done + rr + u, v[u], 0.0f, true, (uint32_t)lane, 32u); }
-                };
-                uint32_t rr = 0;
-                if constexpr (QUANT == 0x80) {
-                    for (; rr + 4u <= tr; rr += 4u) {
-                        float v[4];
-                        st_rows_q80_warp<LPG, 4>(tile + (size_t)rr * k.row_stride, k.row_stride, aux + (size_t)rr * k.aux_stride, k.aux_stride, k.n, act, v);
-                        out(rr, v, 4u);
-                    }
-                    if (rr + 2u <= tr) {
-                        float v[2];
-                        st_rows_q80_warp<LPG, 2>(tile + (size_t)rr * k.row_stride, k.row_stride, aux + (size_t)rr * k.aux_stride, k.aux_stride, k.n, act, v);
-                        out(rr, v, 2u); rr += 2u;
-                    }
-                    if (rr < tr) {
-                        float v[1];
-                        st_rows_q80_warp<LPG, 1>(tile + (size_t)rr * k.row_stride, k.row_stride, aux + (size_t)rr * k.aux_stride, k.aux_stride, k.n, act, v);
-                        out(rr, v, 1u);
-                    }
-                } else {
-                    for (; rr < tr; rr += 2u) {
-                        const bool two = rr + 1u < tr;
-                        const uint32_t r1 = two ? rr + 1u : rr;
-                        float v[2];
-                        if constexpr (QUANT == 0x42) {
-                            v[0] = st_row_q4k(tile + (size_t)rr * k.row_stride, aux + (size_t)rr * k.aux_stride, k.n, act);
-                            v[1] = two ? st_row_q4k(tile + (size_t)r1 * k.row_stride, aux + (size_t)r1 * k.aux_stride, k.n, act) : 0.0f;
-                        } else {
-                            v[0] = st_row_f32(tile + (size_t)rr * k.row_stride, k.n, act);
-                            v[1] = two ? st_row_f32(tile + (size_t)r1 * k.row_stride, k.n, act) : 0.0f;
-                        }
-                        out(rr, v, two ? 2u : 1u);
-                    }
-                }
+            } else if (epi == EPI_RESID) {
+                float xn = 0.0f;
+                if (on) { xn = __fadd_rn(xown[ri], v); xw_st(g.xv[0] + rep * g.rs[0] + row, xn, epoch); }      // infer.c:906, :963
                 __syncwarp();
-                if (lane == 0) mbar_arrive_n(&r.empty[cc.s], kConsWarps);      // the only consumer of this stage
+                if (on && rep == 0) xown[ri] = xn;
+            } else if (epi == EPI_QKV) {
+                if (on && rep == 0) {
+                    xw_st(g.xq + row, v, epoch);
+                    if (row >= d.q_dim + d.kv_dim) {                         // V rows also go to the cache for later positions
+                        const uint32_t vc = row - d.q_dim - d.kv_dim, h = vc / d.hd, i = vc % d.hd;
+                        g.vc[(size_t)layer * d.KV * d.max_seq * d.hd + ((size_t)h * d.max_seq + pos) * d.hd + i] = v;
+                    }
+                }
+            } else if (on && rep == 0) {
+                // classifier: infer.c:1156-1167 penalty (division, any sign), then first-max argmax :1026-1037 (rows ascend per lane)
+                const float pen = ms.pen;
+                if (pen != 1.0f && __ldcg(g.seen + row)) v = __fdiv_rn(v, pen);
+                g.logits[row] = v;
+                if (v > bestv) { bestv = v; besti = row; }
             }
-            st_advance(cc, r.nstages);
         }
-        c = cc; tcount += j;
-    } else {
-        // ---- shared tiles: lanes per row team and rows per warp pass from the table computed at kernel start ----
-        const uint32_t TS = geo.ts[kid], RW = geo.rw[kid], mode = geo.mode[kid], lg2 = geo.lg2[kid], gteam = geo.gteam[kid];
-        const uint32_t team = geo.team[kid][lane], tl = geo.tl[kid][lane], team_base = team * TS, gl = geo.gl[kid][lane], ul = geo.ul[kid][lane];
-        const bool lane_on = (uint32_t)lane < RW * TS;
-        for (uint32_t done = 0; done < rows; done += k.tile_rows) {
-            const uint32_t tr = min(k.tile_rows, rows - done);
-            ST_DBG(5);
-            mbar_wait(&r.full[c.s], c.par, g.err, 0x20u + epi);
-            ST_DBG(6);
-            const unsigned char *tile = r.buf + (size_t)c.s * r.stage_bytes;
-            const unsigned char *aux = tile + (size_t)tr * k.row_stride;
-            // rows of a warp pass: mode 0 one row per team; mode 1 the teams 2t, 2t+1 do the two rows of a pair; mode 2 a team does both
-            const uint32_t step_rows = (mode == 2u) ? 2u * RW : RW;
-            for (uint32_t rb = warp * step_rows; rb < tr; rb += kConsWarps * step_rows) {       // warp-uniform trip count
-                const uint32_t rr = rb + (mode == 2u ? 2u * team : team);
-                const bool valid = lane_on && rr < tr;
-                const uint32_t rc = (rr < tr) ? rr : tr - 1u;
-                auto one = [&](uint32_t r2) -> float {
-                    const unsigned char *wrow = tile + (size_t)r2 * k.row_stride, *ax = aux + (size_t)r2 * k.aux_stride;
-                    if constexpr (QUANT == 0x80) return st_row_q80_lpg<LPG>(wrow, reinterpret_cast<const float *>(ax), k.n, act, lg2, gteam, gl, ul, team_base, dbg);
-                    else if constexpr (QUANT == 0x42) return st_row_q4k(wrow, ax, k.n, act);
-                    else return st_row_f32(wrow, k.n, act);
-                };
-                float v = (g.ablate & 2u) ? 0.0f : one(rc), v3 = 0.0f;
-                bool pub = valid;                                                 // does this team publish the element?
-                if (mode == 2u && !(g.ablate & 2u)) v3 = one(min(rc + 1u, tr - 1u));
-                else if (mode == 1u) { v3 = __shfl_sync(0xffffffffu, v, (lane + TS) & 31u); pub = valid && !(team & 1u); }
-                ST_DBG(7);
-                emit(row0 + done + rc, done + rc, v, v3, pub, tl, TS);
-            }
-            ST_DBG(8);
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&r.empty[c.s]);
-            st_advance(c, r.nstages);
-            tcount++;
-        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive_n(&r.empty[cc.s], owned ? (uint32_t)kConsWarps : 1u);      // an owned tile has this one consumer
+        if (!owned) { turn += kConsWarps - tb; if (turn >= (uint32_t)kConsWarps) turn -= kConsWarps; }      // long rows: few to a tile, the next tile's go to the next warps
+        st_skip(cc, jstep, r.nstages);
     }
-    ST_DBG(9);
+    st_skip(c, nt, r.nstages);
+    tcount += nt;
     if (epi == EPI_CLS) {
 #pragma unroll
         for (uint32_t o = 1u; o < 32u; o <<= 1) {                          // first max over the lanes of the warp
@@ -677,276 +566,256 @@ __device__ __forceinline__ void st_consume(const StreamArgs &g, const StRing &r,
 }
 
 // ---------------------------------------------------------------- attention item (infer.c:814-879) on K/V tiles from the ring
-// One CTA = one (kv head, split).  The item's rows are processed in segments of up to kStSegTiles ring tiles that are
-// resident at the same time; per segment three passes with no cross-lane traffic in their inner loops:
-//   scores : four lanes per cache row, all KVM query heads of the kv head (K row and q read in 16-byte chunks whose order
-//            is rotated by the row index: conflict-free although rows are a multiple of 128 bytes apart)
-//   softmax: warp m owns query head m: running max / sum over the segments (online softmax), p = exp(s - max) in place
-//   P.V    : one thread per (head, pair of output dims), rows in order
+// One CTA = one (kv head, split).  The item's rows are processed in segments of up to kStSegTiles ring tiles that are resident at the same time.  A cache
+// row belongs to LPR lanes of a warp, each with NC of its 16-byte chunks for all KVM query heads: a score is log2(LPR) shuffles, and the weighted value row stays
+// in the lanes that have the weight, so there is no barrier and no shared memory between scores, softmax and values.  Every row slot keeps a running maximum, sum and
+// accumulators of its own (KVM * NC = 4 or 8 float4).  LPR is the least that fits them: what bounds an item of this size is the instructions that its
+// 15 warps issue (4 warps a scheduler), and those go with the number of passes.
+// The slots are merged within the warp, the warps through shared memory, under the item's second and last barrier.
 // q (and the position's k) are normalised + RoPE'd in registers (norm_rope_apply) by one warp each; the position's own K / V
-// rows (this step's QKV outputs) are written into their slots of the resident tile, so the passes treat all rows alike.
-// A range held by one item is normalised and published at once; otherwise every item publishes its partial and the item
-// of split 0 merges them in split order.
-template <int KVM>
-static __device__ void st_attention(const StreamArgs &g, const StRing &r, StCursor &c, uint32_t &tcount, uint32_t layer, uint32_t cta, uint32_t pos, uint32_t range,
-                                    uint32_t nsplit, uint32_t chunk, uint32_t e_in, uint32_t e_out, float *sm, unsigned long long *dbg) {
+// rows (this step's QKV outputs) are read from where those warps put them, not from the tile.
+// A range held by one item is normalised and published at once; otherwise every item publishes its partial and the items of the kv head share the merge:
+// a warp per 32 elements of a head, in split order.
+template <int KVM, int HDC>
+static __device__ void st_attention(const StreamArgs &g, const StRing &r, StCursor &c, uint32_t &tcount, uint32_t layer, uint32_t cta, uint32_t pos, const StPlan &plan,
+                                    uint32_t e_in, uint32_t e_out, float *sm) {
+    constexpr uint32_t LPR = KVM * HDC / 32 < HDC / 16 ? HDC / 16 : KVM * HDC / 32, NC = HDC / 4 / LPR, RP = 32 / LPR;          // lanes of a row, chunks of a lane, rows of a warp's pass
     const Dims &d = g.d;
-    if (cta >= d.KV * nsplit) return;
-    ST_DBG(0);
-    const uint32_t hd = d.hd, hd4 = hd / 4u, hd2 = hd / 2u;
-    const uint32_t kvh = cta / nsplit, sp = cta % nsplit;
-    const uint32_t t0 = min(range, sp * chunk), t1 = min(range, t0 + chunk);
-    const size_t kvl = (size_t)d.KV * d.max_seq * hd;
-    float *kbase = g.kc + layer * kvl + (size_t)kvh * d.max_seq * hd;
-    const float *qn = g.qnorm ? g.qnorm + (size_t)layer * hd : nullptr, *kn = g.knorm ? g.knorm + (size_t)layer * hd : nullptr;
-    const float *cr = g.rope_cos + (size_t)pos * (hd / 2), *ci = g.rope_sin + (size_t)pos * (hd / 2);
-    uint32_t lpr = 1; while (lpr * 4 < hd) lpr <<= 1;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t li = lane % lpr, col = li * 4;
-    const bool colon = col < hd;
-    const float dv = sqrtf((float)hd);
-    const bool owns = pos >= t0 && pos < t1;
+    const uint32_t nsplit = plan.nsplit, kvh = plan.kvh, sp = plan.sp, t0 = plan.t0, t1 = plan.t1;
+    if (kvh >= d.KV) return;
+    const uint32_t hd = d.hd;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t kvr = g.kv_tile_rows, seg_max = (uint32_t)kStSegTiles * kvr;
 
     // shared-memory carve-up (floats)
     float *q_s = sm;                                   // [KVM][hd]   normalised + RoPE'd query heads
-    float *S = q_s + KVM * hd;                         // [KVM][seg_max] scores, then probabilities
-    float *st_scale = S + KVM * seg_max;               // [KVM] e^{m_old - m_new} of the current segment
-    float *krow = st_scale + ((KVM + 3) & ~3);         // [hd] the position's k (post-RoPE), [hd] the position's v (16-byte aligned)
-    float *outp = krow + 2 * hd;                       // [KVM][hd + 2]: acc, M, L
+    float *krow = q_s + KVM * hd;                      // [hd] the position's k (post-RoPE), [hd] the position's v
+    float *part_s = krow + 2 * hd;                     // [15][KVM][hd] the warps' weighted sums
+    float *pm = part_s + kConsWarps * KVM * hd;        // [KVM][16] their maxima
+    float *pl = pm + KVM * 16;                         // [KVM][16] their sums of weights
 
     // ---- this step's q / k / v: warp m < KVM prepares query head m, warp KVM the k row, warp KVM + 1 the v row ----
-    if (warp < KVM + 2) {
-        const RopeTab rt = rope_tab_load(cr, ci, d, col, colon);
-        float4 gn = make_float4(0, 0, 0, 0), v4 = make_float4(0, 0, 0, 0);
-        if (warp < KVM) {
-            if (d.arch == 3u && colon) gn = __ldg(reinterpret_cast<const float4 *>(qn + col));
-            if (colon) v4 = xw_poll4(g.xq + ((size_t)kvh * KVM + warp) * hd + col, e_in, g.err);
-            v4 = norm_rope_apply(v4, gn, rt, d, lpr, col, colon);
-            if (colon && (uint32_t)lane < lpr) *reinterpret_cast<float4 *>(q_s + warp * hd + col) = v4;
-        } else if (owns) {
-            if (warp == KVM) {
-                if (d.arch == 3u && colon) gn = __ldg(reinterpret_cast<const float4 *>(kn + col));
-                if (colon) v4 = xw_poll4(g.xq + d.q_dim + (size_t)kvh * hd + col, e_in, g.err);
-                v4 = norm_rope_apply(v4, gn, rt, d, lpr, col, colon);
-                if (colon && (uint32_t)lane < lpr) {
-                    *reinterpret_cast<float4 *>(krow + col) = v4;
-                    *reinterpret_cast<float4 *>(kbase + (size_t)pos * hd + col) = v4;             // K rows are cached post-RoPE
-                }
-            } else {
-                if (colon) v4 = xw_poll4(g.xq + d.q_dim + d.kv_dim + (size_t)kvh * hd + col, e_in, g.err);
-                if (colon && (uint32_t)lane < lpr) *reinterpret_cast<float4 *>(krow + hd + col) = v4;
-            }
+    if (warp < KVM + ((pos >= t0 && pos < t1) ? 2u : 0u)) {
+        uint32_t lpr = 1; while (lpr * 4 < hd) lpr <<= 1;
+        const uint32_t col = (lane & (lpr - 1u)) * 4;
+        const bool colon = col < hd;
+        const float *gains = warp < KVM ? g.qnorm : g.knorm;
+        RopeTab rt; rt.c = rt.sn = make_float4(0, 0, 0, 0);
+        float4 gn = make_float4(0, 0, 0, 0), v4 = gn;
+        if (warp <= KVM) {
+            rt = rope_tab_load(g.rope_cos + (size_t)pos * (hd / 2), g.rope_sin + (size_t)pos * (hd / 2), d, col, colon);
+            if (d.arch == 3u && colon) gn = __ldg(reinterpret_cast<const float4 *>(gains + (size_t)layer * hd + col));
+        }
+        const uint32_t at = warp < KVM ? (kvh * KVM + warp) * hd : d.q_dim + (warp == KVM ? 0u : d.kv_dim) + kvh * hd;
+        if (colon) v4 = xw_poll4(g.xq + at + col, e_in, g.err);
+        __syncwarp();
+        if (warp <= KVM) v4 = norm_rope_apply(v4, gn, rt, d, lpr, col, colon);
+        if (colon && lane < lpr) {
+            *reinterpret_cast<float4 *>(q_s + warp * hd + col) = v4;               // krow follows q_s: row KVM is k, row KVM + 1 is v
+            if (warp == KVM)                                                       // K rows are cached post-RoPE
+                *reinterpret_cast<float4 *>(g.kc + ((size_t)(layer * d.KV + kvh) * d.max_seq + pos) * hd + col) = v4;
         }
     }
-    // running state: warp m < KVM keeps (max, sum) of head m; thread j (and j + 480) keeps the accumulators of (head, dim pair) j
-    float m_run = -FLT_MAX, l_run = 0.0f;
-    float2 acc[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
+    const uint32_t slot = lane / LPR, part = lane % LPR;
+    const uint32_t rot = LPR == 4u ? (slot & 1u) : 0u;          // four lanes a row: neighbouring rows of a load read chunk groups of different banks
+    uint32_t col[NC];
+#pragma unroll
+    for (uint32_t i = 0; i < NC; i++) col[i] = (part + LPR * ((i + rot) & (NC - 1u))) * 4u;
+    float m_run[KVM], l_run[KVM]; float4 acc[KVM][NC];
+#pragma unroll
+    for (int m = 0; m < KVM; m++) {
+        m_run[m] = -FLT_MAX; l_run[m] = 0.0f;
+#pragma unroll
+        for (uint32_t i = 0; i < NC; i++) acc[m][i] = make_float4(0, 0, 0, 0);
+    }
+    const float dv = sqrtf((float)hd), rdv = 1.0f / dv;
     cbar();
-    ST_DBG(1);
 
+#pragma unroll 1
     for (uint32_t s0 = t0; s0 < t1; s0 += seg_max) {
         const uint32_t rows_seg = min(seg_max, t1 - s0), nt = (rows_seg + kvr - 1u) / kvr;
-        uint32_t stg[kStSegTiles];
+        // stage of tile i of the segment (at most one turn of the ring away); lane i waits for tile i
+        uint32_t my_s = c.s + lane, my_par = c.par;
+        if (my_s >= r.nstages) { my_s -= r.nstages; my_par ^= 1u; }
+        if (lane < nt) mbar_wait(&r.full[my_s], my_par, g.err, 0x30u);
+        __syncwarp();
+#pragma unroll 1
+        for (uint32_t base = RP * warp; base < rows_seg; base += RP * kConsWarps) {          // warp-uniform
+            const bool on = base + slot < rows_seg;
+            const uint32_t idx = on ? base + slot : base;
+            const uint32_t ti = __umulhi(idx, g.kv_tile_magic);
+            uint32_t st = c.s + ti;
+            if (st >= r.nstages) st -= r.nstages;
+            const float *kr = reinterpret_cast<const float *>(r.buf + (size_t)st * r.stage_bytes) + (idx - ti * kvr) * hd, *vr = kr + kvr * hd;
+            if (s0 + idx == pos) { kr = krow; vr = krow + hd; }
+            float s[KVM];
 #pragma unroll
-        for (int i = 0; i < kStSegTiles; i++) {
-            stg[i] = 0;
-            if ((uint32_t)i < nt) { mbar_wait(&r.full[c.s], c.par, g.err, 0x30u); stg[i] = c.s; st_advance(c, r.nstages); tcount++; }
-        }
-        auto tile_k = [&](uint32_t ti) -> float * {
-            uint32_t sidx = stg[0];
+            for (int m = 0; m < KVM; m++) s[m] = 0.0f;
 #pragma unroll
-            for (int i = 1; i < kStSegTiles; i++) if (ti == (uint32_t)i) sidx = stg[i];
-            return reinterpret_cast<float *>(r.buf + (size_t)sidx * r.stage_bytes);
-        };
-        ST_DBG(2);
-        if (owns && pos >= s0 && pos < s0 + rows_seg) {     // CTA-uniform: this step's k / v into their slots of the resident tile
-            const uint32_t pr = pos - s0, ti = __umulhi(pr, g.kv_tile_magic), rr = pr - ti * kvr;
-            float *kt = tile_k(ti);
-            for (uint32_t i = threadIdx.x; i < hd; i += kConsThreads) {
-                kt[(size_t)rr * hd + i] = krow[i];
-                kt[(size_t)kvr * hd + (size_t)rr * hd + i] = krow[hd + i];
-            }
-            cbar();
-        }
-        ST_DBG(3);
-        // ---- scores: task = (row, quarter of the dims), 4 adjacent lanes per row.  The K chunks of the row are loaded once and used for
-        //      all KVM query heads (q chunks are broadcast reads); chunk order rotated by the row index: conflict-free although rows are
-        //      a multiple of 128 bytes apart.  One round covers 120 rows. ----
-        if (!(g.ablate & 4u)) {
-            const uint32_t part = threadIdx.x & 3u;
-            for (uint32_t idx = threadIdx.x >> 2; idx < ((rows_seg + 7u) & ~7u); idx += kConsThreads / 4u) {       // warp-uniform trip count (8 rows per warp)
-                const bool on = idx < rows_seg;
-                const uint32_t ic = on ? idx : 0u;
-                const uint32_t ti = __umulhi(ic, g.kv_tile_magic), rr = ic - ti * kvr;
-                const float *kr = tile_k(ti) + (size_t)rr * hd;
-                const uint32_t rot = (hd4 & 3u) ? 0u : (4u * (ic & 7u)) % hd4;       // rotation keeps the 4 lanes' chunk sets disjoint only if hd % 16 == 0
-                float a[KVM];
-#pragma unroll
-                for (int m = 0; m < KVM; m++) a[m] = 0.0f;
-#pragma unroll 4
-                for (uint32_t cc = part; cc < hd4; cc += 4u) {
-                    uint32_t ch = cc + rot; if (ch >= hd4) ch -= hd4;
-                    const float4 k4 = *reinterpret_cast<const float4 *>(kr + ch * 4u);
+            for (uint32_t i = 0; i < NC; i++)
+                if (col[i] < hd) {
+                    const float4 k4 = *reinterpret_cast<const float4 *>(kr + col[i]);
 #pragma unroll
                     for (int m = 0; m < KVM; m++) {
-                        const float4 q4 = *reinterpret_cast<const float4 *>(q_s + m * hd + ch * 4u);
-                        a[m] = fmaf(k4.x, q4.x, fmaf(k4.y, q4.y, fmaf(k4.z, q4.z, fmaf(k4.w, q4.w, a[m]))));
+                        const float4 q = *reinterpret_cast<const float4 *>(q_s + m * hd + col[i]);
+                        s[m] = fmaf(k4.x, q.x, fmaf(k4.y, q.y, fmaf(k4.z, q.z, fmaf(k4.w, q.w, s[m]))));
                     }
                 }
+#pragma unroll
+            for (uint32_t o = 1; o < LPR; o <<= 1)
+#pragma unroll
+                for (int m = 0; m < KVM; m++) s[m] += __shfl_xor_sync(0xffffffffu, s[m], o);
+            bool up = false;
+#pragma unroll
+            for (int m = 0; m < KVM; m++) {          // infer.c:858: s / sqrt(head dim), as the product by the reciprocal with the remainder added back
+                const float y = s[m] * rdv, e = fmaf(-y, dv, s[m]);
+                s[m] = on ? (fabsf(y) < 3.0e38f ? fmaf(e, rdv, y) : y) : -INFINITY;
+                up = up || s[m] > m_run[m];
+            }
+            if (__any_sync(0xffffffffu, up)) {       // some slot has a new maximum (the first rows, then rarely)
 #pragma unroll
                 for (int m = 0; m < KVM; m++) {
-                    a[m] += __shfl_xor_sync(0xffffffffu, a[m], 1);
-                    a[m] += __shfl_xor_sync(0xffffffffu, a[m], 2);
-                    if (on && part == 0) S[m * seg_max + idx] = __fdiv_rn(a[m], dv);         // infer.c:858
+                    const float mn = fmaxf(m_run[m], s[m]), sc = expf(m_run[m] - mn);
+                    m_run[m] = mn; l_run[m] *= sc;
+#pragma unroll
+                    for (uint32_t i = 0; i < NC; i++) { acc[m][i].x *= sc; acc[m][i].y *= sc; acc[m][i].z *= sc; acc[m][i].w *= sc; }
                 }
             }
-        }
-        cbar();
-        ST_DBG(4);
-        // ---- online softmax over the segment: warp m owns head m ----
-        if (warp < KVM && !(g.ablate & 4u)) {
-            float *Sm = S + warp * seg_max;
-            float mx = -FLT_MAX;
-            for (uint32_t i = lane; i < rows_seg; i += 32) mx = fmaxf(mx, Sm[i]);
-            ST_DBG(12);
-            mx = warp_max(mx);
-            ST_DBG(13);
-            const float mn = fmaxf(m_run, mx);
-            const float sc_old = expf(m_run - mn);
-            ST_DBG(14);
-            float ls = 0.0f;
-            for (uint32_t i = lane; i < rows_seg; i += 32) { const float pr = expf(Sm[i] - mn); Sm[i] = pr; ls += pr; }
-            ST_DBG(15);
-            ls = warp_sum(ls);
-            l_run = fmaf(l_run, sc_old, ls);
-            m_run = mn;
-            if (lane == 0) st_scale[warp] = sc_old;
-        }
-        cbar();
-        ST_DBG(5);
-        // ---- P.V: thread j owns (head, dim pair) j; rows in order, four at a time (probabilities as one float4) ----
 #pragma unroll
-        for (int u = 0; u < 2; u++) {
-            const uint32_t j = threadIdx.x + u * kConsThreads;
-            if (j < KVM * hd2 && !(g.ablate & 4u)) {
-                const uint32_t m = j / hd2, dd = (j - m * hd2) * 2u;
-                const float *Sm = S + m * seg_max;
-                const float sc = st_scale[m];
-                float2 a0 = make_float2(acc[u].x * sc, acc[u].y * sc), a1 = make_float2(0, 0), a2 = a1, a3 = a1;
-                for (uint32_t ti = 0; ti < nt; ti++) {
-                    const float *vt = tile_k(ti) + (size_t)kvr * hd + dd;
-                    const uint32_t nr = min(kvr, rows_seg - ti * kvr);
-                    const float *sp2 = Sm + ti * kvr;                   // kvr % 4 == 0: 16-byte aligned
-                    uint32_t rr = 0;
-                    for (; rr + 4u <= nr; rr += 4u) {
-                        const float4 p4 = *reinterpret_cast<const float4 *>(sp2 + rr);
-                        const float2 v0 = *reinterpret_cast<const float2 *>(vt + (size_t)rr * hd), v1 = *reinterpret_cast<const float2 *>(vt + (size_t)(rr + 1u) * hd);
-                        const float2 v2 = *reinterpret_cast<const float2 *>(vt + (size_t)(rr + 2u) * hd), v3 = *reinterpret_cast<const float2 *>(vt + (size_t)(rr + 3u) * hd);
-                        a0.x = fmaf(p4.x, v0.x, a0.x); a0.y = fmaf(p4.x, v0.y, a0.y); a1.x = fmaf(p4.y, v1.x, a1.x); a1.y = fmaf(p4.y, v1.y, a1.y);
-                        a2.x = fmaf(p4.z, v2.x, a2.x); a2.y = fmaf(p4.z, v2.y, a2.y); a3.x = fmaf(p4.w, v3.x, a3.x); a3.y = fmaf(p4.w, v3.y, a3.y);
-                    }
-                    for (; rr < nr; rr++) {
-                        const float pr = sp2[rr]; const float2 v0 = *reinterpret_cast<const float2 *>(vt + (size_t)rr * hd);
-                        a0.x = fmaf(pr, v0.x, a0.x); a0.y = fmaf(pr, v0.y, a0.y);
+            for (int m = 0; m < KVM; m++) { s[m] = expf(s[m] - m_run[m]); l_run[m] += s[m]; }
+#pragma unroll
+            for (uint32_t i = 0; i < NC; i++)
+                if (col[i] < hd) {
+                    const float4 v4 = *reinterpret_cast<const float4 *>(vr + col[i]);
+#pragma unroll
+                    for (int m = 0; m < KVM; m++) {
+                        acc[m][i].x = fmaf(s[m], v4.x, acc[m][i].x); acc[m][i].y = fmaf(s[m], v4.y, acc[m][i].y);
+                        acc[m][i].z = fmaf(s[m], v4.z, acc[m][i].z); acc[m][i].w = fmaf(s[m], v4.w, acc[m][i].w);
                     }
                 }
-                acc[u] = make_float2((a0.x + a1.x) + (a2.x + a3.x), (a0.y + a1.y) + (a2.y + a3.y));
-            }
         }
-        cbar();
-        ST_DBG(6);
-        if (lane == 0) {
-#pragma unroll
-            for (int i = 0; i < kStSegTiles; i++) if ((uint32_t)i < nt) mbar_arrive(&r.empty[stg[i]]);
-        }
-    }
-    ST_DBG(7);
-    // ---- the item's partial: per head [acc[hd], M, L] ----
-#pragma unroll
-    for (int u = 0; u < 2; u++) {
-        const uint32_t j = threadIdx.x + u * kConsThreads;
-        if (j < KVM * hd2) { const uint32_t m = j / hd2, dd = (j - m * hd2) * 2u; outp[m * (hd + 2) + dd] = acc[u].x; outp[m * (hd + 2) + dd + 1u] = acc[u].y; }
-    }
-    if (warp < KVM && lane == 0) { outp[warp * (hd + 2) + hd] = m_run; outp[warp * (hd + 2) + hd + 1] = l_run; }
-    const uint32_t pw = KVM * (hd + 2);                               // words of one partial
-    cbar();
-    ST_DBG(8);
-    if (nsplit == 1) {          // the whole range in one item: normalise and publish
-        for (uint32_t el = threadIdx.x; el < KVM * hd; el += kConsThreads) {
-            const uint32_t m = el / hd, i = el - m * hd;
-            const float ov = __fdiv_rn(outp[m * (hd + 2) + i], outp[m * (hd + 2) + hd + 1]);
-#pragma unroll
-            for (uint32_t rep = 0; rep < (uint32_t)kStRep; rep++) xw_st(g.xv[1] + (size_t)rep * g.rs[1] + ((size_t)kvh * KVM + m) * hd + i, ov, e_out);
-        }
-        return;
-    }
-    unsigned long long *part = g.xws + ((size_t)kvh * g.nsplit_max) * pw;
-    if (sp != 0) {              // publish the partial; split 0 of the kv head merges
-        for (uint32_t idx = threadIdx.x; idx < pw; idx += kConsThreads) xw_st(part + (size_t)sp * pw + idx, outp[idx], e_out);
-        return;
-    }
-    ST_DBG(9);
-    // ---- merge (split 0): own partial from shared memory, the others polled from the exchange words ----
-    uint32_t region = st_attn_work_floats(KVM, hd, seg_max);
-    if (g.nsplit_max * KVM * hd > region) region = g.nsplit_max * KVM * hd;
-    float *wsc = sm + region;                            // [KVM][nsplit_max] weights e^{m_s - M}; before that: the maxima
-    float *stat = wsc + KVM * g.nsplit_max;              // [KVM] L, then [KVM][nsplit_max] partial sums
-    float own[4];                                        // this thread's slice of the own partial (pw <= 4 * 480 for hd <= 128, KVM <= 8)
-#pragma unroll
-    for (int u = 0; u < 4; u++) { const uint32_t idx = threadIdx.x + u * kConsThreads; own[u] = idx < pw ? outp[idx] : 0.0f; }
-    cbar();                                              // outp / ws are about to be overwritten by the staging area
-    float *macc = sm;                                    // [KVM][nsplit][hd]
-    float *pl = stat + KVM;                              // [KVM][nsplit_max]
-    auto place = [&](uint32_t s2, uint32_t idx, float v) {
-        const uint32_t m = idx / (hd + 2), i = idx % (hd + 2);
-        if (i < hd) macc[(m * nsplit + s2) * hd + i] = v;
-        else if (i == hd) wsc[m * g.nsplit_max + s2] = v;
-        else pl[m * g.nsplit_max + s2] = v;
-    };
-#pragma unroll
-    for (int u = 0; u < 4; u++) { const uint32_t idx = threadIdx.x + u * kConsThreads; if (idx < pw) place(0, idx, own[u]); }
-    for (uint32_t e0 = pw + threadIdx.x; e0 < nsplit * pw; e0 += 8u * kConsThreads) {       // eight loads in flight per thread before any epoch is checked
-        unsigned long long w8[8];
-#pragma unroll
-        for (int u = 0; u < 8; u++) { const uint32_t e = e0 + u * kConsThreads; if (e < nsplit * pw) w8[u] = xw_ld1(part + e); }
-#pragma unroll
-        for (int u = 0; u < 8; u++) {
-            const uint32_t e = e0 + u * kConsThreads;
-            if (e < nsplit * pw) place(e / pw, e % pw, xw_ok(w8[u], e_out) ? xw_val(w8[u]) : xw_poll1(part + e, e_out, g.err));
-        }
-    }
-    cbar();
-    ST_DBG(10);
-    if (warp < KVM) {
-        float pm[2], pls[2];                             // nsplit_max <= 64: two slots per lane
-#pragma unroll
-        for (int q2 = 0; q2 < 2; q2++) {
-            const uint32_t s2 = lane + 32 * q2;
-            pm[q2] = (s2 < nsplit) ? wsc[warp * g.nsplit_max + s2] : -FLT_MAX;
-            pls[q2] = (s2 < nsplit) ? pl[warp * g.nsplit_max + s2] : 0.0f;
-        }
-        const float M = warp_max(fmaxf(pm[0], pm[1]));
-        float L = 0.0f;
         __syncwarp();
+        if (lane < nt) mbar_arrive(&r.empty[my_s]);          // this warp is done with the segment's tiles
+        st_skip(c, nt, r.nstages);
+        tcount += nt;
+    }
+    // ---- the row slots of a warp (trading elements for lanes: the lane ends with KVM * HDC / 32 of them), then the warps that had rows ----
+    const uint32_t nact = min((uint32_t)kConsWarps, (min(seg_max, t1 - t0) + RP - 1u) / RP);          // (t0 < t1: every split of the plan holds rows)
+    if (warp < nact) {
+        constexpr uint32_t NV = KVM * NC * 4;
+        float f[NV];
 #pragma unroll
-        for (int q2 = 0; q2 < 2; q2++) {
-            const uint32_t s2 = lane + 32 * q2;
-            if (s2 < nsplit) { const float w = expf(pm[q2] - M); wsc[warp * g.nsplit_max + s2] = w; L += pls[q2] * w; }
+        for (int m = 0; m < KVM; m++) {
+            float mn = m_run[m];
+#pragma unroll
+            for (uint32_t o = LPR; o < 32; o <<= 1) mn = fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+            const float sc = expf(m_run[m] - mn);
+            float l = l_run[m] * sc;
+#pragma unroll
+            for (uint32_t o = LPR; o < 32; o <<= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+            if (lane == 0) { pm[m * 16 + warp] = mn; pl[m * 16 + warp] = l; }
+#pragma unroll
+            for (uint32_t i = 0; i < NC; i++) {
+                const float4 e = acc[m][i], w = acc[m][(i + NC - 1u) & (NC - 1u)];          // rotated lanes hold chunk i one place earlier
+                f[(m * NC + i) * 4] = sc * (rot ? w.x : e.x); f[(m * NC + i) * 4 + 1] = sc * (rot ? w.y : e.y);
+                f[(m * NC + i) * 4 + 2] = sc * (rot ? w.z : e.z); f[(m * NC + i) * 4 + 3] = sc * (rot ? w.w : e.w);
+            }
         }
-        L = warp_sum(L);
-        if (lane == 0) stat[warp] = L;
+        uint32_t f0 = 0;
+#pragma unroll
+        for (uint32_t o = 16, n = NV / 2; o >= LPR; o >>= 1, n >>= 1) {
+            const bool hi = lane & o;
+#pragma unroll
+            for (uint32_t j = 0; j < n; j++) {
+                const float keep = hi ? f[j + n] : f[j], give = hi ? f[j] : f[j + n];
+                f[j] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+            }
+            f0 += hi ? n : 0u;
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < NV / RP; j += 2) {
+            const uint32_t e = f0 + j, at = (part + LPR * (e / 4u % NC)) * 4u + (e & 3u);
+            if (at < hd) *reinterpret_cast<float2 *>(part_s + (warp * KVM + e / (NC * 4u)) * hd + at) = make_float2(f[j], f[j + 1]);
+        }
     }
     cbar();
-    for (uint32_t el = threadIdx.x; el < KVM * hd; el += kConsThreads) {
-        const uint32_t m = el / hd, i = el - m * hd;
-        float o = 0.0f;
-        for (uint32_t s2 = 0; s2 < nsplit; s2++) o = fmaf(macc[(m * nsplit + s2) * hd + i], wsc[m * g.nsplit_max + s2], o);
-        const float ov = __fdiv_rn(o, stat[m]);
+    const uint32_t pw = KVM * (hd + 2u);                               // words of one partial
+    unsigned long long *part_x = g.xws + (size_t)kvh * g.nsplit_max * pw;
+    const uint32_t slabs = (hd + 31u) / 32u, units = KVM * slabs;
+    auto publish = [&](uint32_t m, uint32_t i, float v) {
+        unsigned long long *dst = g.xv[1] + (kvh * KVM + m) * hd + i;
+        const uint32_t rs = g.rs[1];
 #pragma unroll
-        for (uint32_t rep = 0; rep < (uint32_t)kStRep; rep++) xw_st(g.xv[1] + (size_t)rep * g.rs[1] + ((size_t)kvh * KVM + m) * hd + i, ov, e_out);
+        for (uint32_t rep = 0; rep < (uint32_t)kStRep; rep++) xw_st(dst + rep * rs, v, e_out);
+    };
+#pragma unroll 1
+    for (uint32_t u = warp; u < units; u += kConsWarps) {
+        const uint32_t m = u / slabs, i = (u - m * slabs) * 32u + lane, src = lane & 15u;
+        const float pmv = src < nact ? pm[m * 16 + src] : -FLT_MAX, plv = src < nact ? pl[m * 16 + src] : 0.0f;
+        float M = pmv;
+#pragma unroll
+        for (int o = 1; o < 16; o <<= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+        const float w = src < nact ? expf(pmv - M) : 0.0f;
+        float L = w * plv, o = 0.0f;
+#pragma unroll
+        for (int b = 1; b < 16; b <<= 1) L += __shfl_xor_sync(0xffffffffu, L, b);
+        const float *ps = part_s + m * hd + i;
+#pragma unroll 4
+        for (uint32_t q = 0; q < nact; q++) {
+            const float wq = __shfl_sync(0xffffffffu, w, q);
+            if (i < hd) o = fmaf(wq, ps[q * KVM * hd], o);
+        }
+        if (nsplit == 1) { if (i < hd) publish(m, i, __fdiv_rn(o, L)); continue; }
+        unsigned long long *dst = part_x + (size_t)sp * pw + m * (hd + 2u);
+        if (i < hd) xw_st(dst + i, o, e_out);
+        if (i == 0) { xw_st(dst + hd, M, e_out); xw_st(dst + hd + 1u, L, e_out); }
     }
-    ST_DBG(11);
+    if (nsplit == 1) return;
+    // ---- merge: 32 elements of a head per warp, dealt out over the items of the kv head ----
+#pragma unroll 1
+    for (uint32_t u = sp + nsplit * warp; u < units; u += nsplit * kConsWarps) {
+        const uint32_t m = u / slabs, i = (u - m * slabs) * 32u + lane;
+        const unsigned long long *src = part_x + m * (hd + 2u), *el = src + (i < hd ? i : 0u);
+        // Eight splits' elements and (with the first eight) all statistics are asked for together, again until all are there: nothing is polled one by one.
+        // nsplit_max <= 64: two splits' statistics per lane.
+        const unsigned long long there = (unsigned long long)e_out << 32;
+        unsigned long long w8[8], a0, a1, b0, b1;
+        auto ask = [&](uint32_t s2, bool stats) {
+            long long t0 = 0;
+#pragma unroll 1
+            for (uint32_t it = 1;; it++) {
+                bool ok = true;
+                if (stats) {
+                    a0 = a1 = b0 = b1 = there;
+                    if (lane < nsplit) xw_ld2(src + (size_t)lane * pw + hd, a0, a1);
+                    if (lane + 32u < nsplit) xw_ld2(src + (size_t)(lane + 32u) * pw + hd, b0, b1);
+                }
+#pragma unroll
+                for (uint32_t q = 0; q < 8u; q++) w8[q] = s2 + q < nsplit ? xw_ld1(el + (size_t)(s2 + q) * pw) : there;
+#pragma unroll
+                for (uint32_t q = 0; q < 8u; q++) ok = ok && xw_ok(w8[q], e_out);
+                if (stats) ok = ok && xw_ok(a0, e_out) && xw_ok(a1, e_out) && xw_ok(b0, e_out) && xw_ok(b1, e_out);
+                if (__all_sync(0xffffffffu, ok)) return;
+                if ((it & 255u) == 0) st_still_waiting(t0, g.err, 0x51u);
+            }
+        };
+        ask(0, true);
+        const float m0 = lane < nsplit ? xw_val(a0) : -FLT_MAX, m1 = lane + 32u < nsplit ? xw_val(b0) : -FLT_MAX;
+        const float M = warp_max(fmaxf(m0, m1));
+        const float w0 = lane < nsplit ? expf(m0 - M) : 0.0f, w1 = lane + 32u < nsplit ? expf(m1 - M) : 0.0f;
+        const float L = warp_sum(fmaf(lane < nsplit ? xw_val(a1) : 0.0f, w0, (lane + 32u < nsplit ? xw_val(b1) : 0.0f) * w1));
+        float o = 0.0f;
+#pragma unroll 1
+        for (uint32_t s2 = 0; s2 < nsplit; s2 += 8u) {
+            if (s2) ask(s2, false);
+#pragma unroll
+            for (uint32_t q = 0; q < 8u; q++) {
+                const float wq = __shfl_sync(0xffffffffu, s2 < 32u ? w0 : w1, (s2 + q) & 31u);
+                if (s2 + q < nsplit) o = fmaf(xw_val(w8[q]), wq, o);
+            }
+        }
+        if (i < hd) publish(m, i, __fdiv_rn(o, L));
+    }
 }
 
 // ---------------------------------------------------------------- grid barrier, once per token (consumer warps; the producer keeps streaming)
@@ -967,7 +836,7 @@ __device__ __forceinline__ void st_grid_barrier(const StreamArgs &g, unsigned in
 }
 
 // ---------------------------------------------------------------- the kernel
-template <int QUANT, int LPG, int KVM>
+template <int QUANT, int LPG, int KVM, int HDC>
 __global__ void __launch_bounds__(kThreads, 1) k_decode_stream(const __grid_constant__ StreamArgs gparam) {
     extern __shared__ __align__(128) unsigned char ssm[];
     // The argument block is read from shared memory: kernel parameters live in the constant bank, whose cache shares the
@@ -978,115 +847,90 @@ __global__ void __launch_bounds__(kThreads, 1) k_decode_stream(const __grid_cons
     const StreamArgs &g = sg;
     __shared__ uint64_t full_bar[kStMaxStages], empty_bar[kStMaxStages];
     __shared__ volatile uint32_t stage_tile[kStMaxStages];
-    __shared__ MatvecSmem ms;
-    __shared__ StOwn own;
-    __shared__ StGeo geo;
+    __shared__ __align__(16) StSmem ms;
+    __shared__ StPhase phase[5];
     __shared__ float xown[kStOwnMax];
     __shared__ volatile uint32_t s_progress;
-    __shared__ unsigned int s_target;
     const Dims &d = g.d;
     const uint32_t cta = blockIdx.x, ncta = gridDim.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 
-    StRing ring{full_bar, empty_bar, stage_tile, ssm + g.off_ring, g.nstages, g.stage_bytes};
+    const StRing ring{full_bar, empty_bar, stage_tile, ssm + g.off_ring, g.nstages, g.stage_bytes};
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < g.nstages; s++) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], kConsWarps); stage_tile[s] = 0xffffffffu; }
-        s_progress = 0; s_target = 0;
+        s_progress = 0; ms.target = 0; ms.ti = ms.tj = 0; ms.pen = __ldcg(&g.st->penalty);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (threadIdx.x < 5) {          // the rows this CTA owns of every kind (64-bit divisions: once, not once per phase)
-        const StKind &k = g.kind[threadIdx.x];
+    if (threadIdx.x < 5) {          // (64-bit divisions: once, not once per phase)
+        const uint32_t kid = threadIdx.x;
+        const StKind &k = g.kind[kid];
         const uint32_t u0 = (uint32_t)(((uint64_t)cta * k.units) / ncta), u1 = (uint32_t)(((uint64_t)(cta + 1) * k.units) / ncta);
-        own.row0[threadIdx.x] = u0 * k.unit_rows; own.rows[threadIdx.x] = (u1 - u0) * k.unit_rows;
-        // how a warp shares the rows of this kind: the candidate with the cheapest (passes x estimated chain latency)
-        const uint32_t kid = threadIdx.x, rows = (u1 - u0) * k.unit_rows;
-        uint32_t b_lg2 = 1, b_gt = 32, b_ts = 32, b_rw = 1, b_mode = (kid == SK_W13) ? 2u : 0u;
-        if (QUANT == 0x80) {
-            const uint32_t G = k.n / (LPG * 16u);
-            uint32_t best = 0xffffffffu;
-            for (uint32_t cand = LPG; cand >= 1u; cand >>= 1) {
-                if (G * cand > 32u && cand > 1u) continue;
-                const uint32_t gt = G < 32u / cand ? G : 32u / cand, t = gt * cand, rw = 32u / t;
-                const uint32_t md = (kid == SK_W13) ? ((rw >= 2u && !(rw & 1u)) ? 1u : 2u) : 0u;
-                const uint32_t per_pass = kConsWarps * (md == 2u ? 2u * rw : rw);
-                const uint32_t tr = rows < k.tile_rows ? rows : k.tile_rows, ntl = tr ? (rows + k.tile_rows - 1u) / k.tile_rows : 0u;
-                const uint32_t passes = ntl * ((tr + per_pass - 1u) / (per_pass ? per_pass : 1u));
-                uint32_t lat = 300u + ((G + gt - 1u) / gt) * (80u * (LPG / cand) + 35u * (31u - __clz(cand)) + 120u + 5u * gt);
-                if (md == 2u) lat *= 2u;
-                const uint32_t cost = passes * lat;
-                if (cost < best) { best = cost; b_lg2 = cand; b_gt = gt; b_ts = t; b_rw = rw; b_mode = md; }
-            }
-        }
-        geo.lg2[kid] = (uint8_t)b_lg2; geo.gteam[kid] = (uint8_t)b_gt; geo.ts[kid] = (uint8_t)b_ts; geo.rw[kid] = (uint8_t)b_rw; geo.mode[kid] = (uint8_t)b_mode;
+        const uint32_t rows = (u1 - u0) * k.unit_rows, xi = kid == SK_O ? 1u : kid == SK_W2 ? 2u : 0u;
+        uint32_t rb = k.unit_rows;
+        while (rb < (QUANT == 0x42 ? 2u : 4u) && rb * kConsWarps < min(rows, k.tile_rows)) rb *= 2u;
+        StPhase &ph = phase[kid];
+        ph.n = k.n; ph.row_stride = k.row_stride; ph.aux_stride = k.aux_stride; ph.tile_rows = k.tile_rows;
+        ph.rows = rows; ph.tiles = (rows + k.tile_rows - 1u) / k.tile_rows; ph.row0 = u0 * k.unit_rows;
+        ph.mode = (k.owned ? 1u : 0u) | rb << 8 | (((k.tile_rows + rb - 1u) / rb) % kConsWarps) << 16;
+        ph.src = g.xv[xi] + (size_t)(cta % (uint32_t)kStRep) * g.rs[xi];
+        ph.gain = kid == SK_QKV ? g.g_attn : kid == SK_W13 ? g.g_ffn : kid == SK_CLS ? g.g_final : nullptr;
+        // layer l publishes e0 + 5l + {1: q/k/v, 2: attention output, 3: x after O, 4: SwiGLU output, 5: x after W2}; x before a layer carries the epoch e0 + 5l
+        ph.need = kid == SK_O ? 2u : kid == SK_W13 ? 3u : kid == SK_W2 ? 4u : 0u;
+        ph.out = kid == SK_QKV ? 1u : ph.need + 1u;
+        ph.epi = kid == SK_QKV ? EPI_QKV : kid == SK_W13 ? EPI_SWIGLU : kid == SK_CLS ? EPI_CLS : EPI_RESID;
+        ph.rn = 1.0f / (float)k.n;
     }
-    __syncthreads();
-    if (threadIdx.x < 160) {
-        const uint32_t kid = threadIdx.x >> 5, ln = threadIdx.x & 31u, ts = geo.ts[kid], rw = geo.rw[kid], lg2 = geo.lg2[kid];
-        const uint32_t tm = ln / ts, tl = ln % ts;
-        geo.team[kid][ln] = (uint8_t)(tm < rw ? tm : rw - 1u); geo.tl[kid][ln] = (uint8_t)tl;
-        geo.gl[kid][ln] = (uint8_t)(tl / lg2); geo.ul[kid][ln] = (uint8_t)(tl % lg2);
-    }
+    if (threadIdx.x < 32) reinterpret_cast<float *>(ms.red)[threadIdx.x] = 0.0f;
     __syncthreads();
 
     // step state (identical in every CTA; advanced locally)
     uint32_t pos = __ldcg(&g.st->pos);
-    const uint32_t causal = __ldcg(&g.st->is_causal), n_prompt = __ldcg(&g.st->n_prompt), advance = __ldcg(&g.st->advance);
-    const float pen = __ldcg(&g.st->penalty);
     uint32_t tok = __ldcg(&g.st->use_token) ? __ldcg(&g.st->token) : __ldcg(g.ids + pos);
 
     if (warp == kConsWarps) {
-        if (lane == 0) st_producer(g, ring, own, cta, &s_progress, pos, causal, advance);
+        if (lane == 0) st_producer(g, ring, phase, cta, &s_progress, pos, __ldcg(&g.st->is_causal), __ldcg(&g.st->advance));
         return;
     }
 
-    unsigned char *act = ssm + g.off_act, *act_other = ssm + g.off_act2;
-    float *x_s = reinterpret_cast<float *>(ssm + g.off_xs);
-    float *attn_ws = reinterpret_cast<float *>(ssm + g.off_attn);
-    const uint32_t rep = cta % (uint32_t)kStRep;                       // the replica this CTA reads
-    const unsigned long long *rx = g.xv[0] + (size_t)rep * g.rs[0], *rxba = g.xv[1] + (size_t)rep * g.rs[1], *rhb = g.xv[2] + (size_t)rep * g.rs[2];
     StCursor cur{0u, 0u};
     uint32_t tcount = 0;                                                // tiles consumed so far (the producer counts the same way)
-    uint32_t ti = 0, tj = 0;
+    uint32_t half = 0, el = g.epoch_base;                               // epochs: see StPhase
     // stamps (trace != nullptr: CTA 0 / thread 0, last step): [0..] after every phase; [1024..] inside layer L/2
-#define ST_TRACE() do { if (g.trace && cta == 0 && threadIdx.x == 0 && step + 1 == g.n_steps && ti < 1000) g.trace[ti++] = clock64(); } while (0)
-#define ST_STAMP() do { if (g.trace && cta == 0 && threadIdx.x == 0 && step + 1 == g.n_steps && l == d.L / 2 && tj < 60) g.trace[1024 + tj++] = clock64(); } while (0)
+#define ST_TRACE() do { if (g.trace && cta == 0 && threadIdx.x == 0 && step + 1 == g.n_steps && ms.ti < 1000) g.trace[ms.ti++] = clock64(); } while (0)
+#define ST_STAMP() do { if (g.trace && cta == 0 && threadIdx.x == 0 && step + 1 == g.n_steps && l == d.L / 2 && ms.tj < 60) g.trace[1024 + ms.tj++] = clock64(); } while (0)
 
+#pragma unroll 1
     for (uint32_t step = 0; step < g.n_steps; step++) {
         ST_TRACE();
-        const uint32_t range = causal ? pos + 1u : d.max_seq;
-        uint32_t nsplit, chunk;
-        st_attn_plan(range, g.nsplit_max, g.chunk_target, nsplit, chunk);
+        float *x_s = reinterpret_cast<float *>(ssm + g.off_xs);
+        if (threadIdx.x == 0) {
+            const uint32_t range = __ldcg(&g.st->is_causal) ? pos + 1u : d.max_seq;
+            uint32_t nsplit, chunk;
+            st_attn_plan(range, g.nsplit_max, g.chunk_target, nsplit, chunk);
+            const uint32_t kvh = cta / nsplit, sp = cta - kvh * nsplit, t0 = min(range, sp * chunk);
+            ms.plan = StPlan{nsplit, kvh, sp, t0, min(range, t0 + chunk)};
+        }
         // embedding row (infer.c:987-988) into shared memory; the rows this CTA owns in the residual phases start from it
         embed_row<kConsThreads>(g.emb_w, g.emb_aux, x_s, tok, d);
         cbar();
-        for (uint32_t i = threadIdx.x; i < own.rows[SK_O]; i += kConsThreads) xown[i] = x_s[own.row0[SK_O] + i];
-        // epochs of this token's exchanges: layer l publishes e0 + 5l + {1: q/k/v, 2: attention output, 3: x after O, 4: SwiGLU output, 5: x after W2}
-        const uint32_t e0 = g.epoch_base + step * 5u * d.L;
+        for (uint32_t i = threadIdx.x; i < phase[SK_O].rows; i += kConsThreads) xown[i] = x_s[phase[SK_O].row0 + i];
 
         // ---- layers 0..L-1: QKV | attention | O | W1,W3 | W2 ; pseudo-layer L: the classifier.  One call site per function. ----
 #pragma unroll 1
         for (uint32_t l = 0; l <= d.L; l++) {
             ST_STAMP();
-            const uint32_t el = e0 + 5u * l;
 #pragma unroll 1
-            for (uint32_t ph = 0; ph < 4; ph++) {
+            for (uint32_t p4 = 0; p4 < 4; p4++) {
                 const bool cls = (l == d.L);
-                const uint32_t kid = cls ? (uint32_t)SK_CLS : ph;
-                const StKind &k = g.kind[kid];
-                const unsigned long long *xsrc = rx; const float *ssrc = nullptr; const float *gain = nullptr;
-                uint32_t epi, need = el, eout = 0;                        // x after the previous layer's W2 carries epoch e0 + 5(l-1) + 5 = el
-                if (cls) { gain = g.g_final; epi = EPI_CLS; }
-                else if (ph == SK_QKV) { if (l == 0) { xsrc = nullptr; ssrc = x_s; } gain = g.g_attn + (size_t)l * d.E; epi = EPI_QKV; eout = el + 1u; }
-                else if (ph == SK_O) { xsrc = rxba; need = el + 2u; epi = EPI_RESID; eout = el + 3u; }
-                else if (ph == SK_W13) { need = el + 3u; gain = g.g_ffn + (size_t)l * d.E; epi = EPI_SWIGLU; eout = el + 4u; }
-                else { xsrc = rhb; need = el + 4u; epi = EPI_RESID; eout = el + 5u; }
-                unsigned long long *dbg = (g.trace && cta == 0 && step + 1 == g.n_steps && l == d.L / 2) ? g.trace + 1100 + 16 * ph : nullptr;
-                if (g.ablate & 16u) need = kXwAny;
-                if (own.rows[kid]) {          // CTA-uniform: a CTA without rows of this kind neither reads the source nor publishes
-                    { unsigned char *t = act; act = act_other; act_other = t; }      // consecutive phases alternate between the two operands
-                    st_prep<QUANT, LPG>(g, xsrc, ssrc, need, gain, k.n, act, ms.red, dbg);
+                const StPhase &ph = phase[cls ? (uint32_t)SK_CLS : p4];
+                if (ph.rows) {                // CTA-uniform: a CTA without rows of this kind neither reads the source nor publishes
+                    half ^= 1u;               // consecutive phases alternate between the two operands
+                    unsigned char *act = ssm + (half ? g.off_act2 : g.off_act);
+                    const float *gain = ph.gain;
+                    if (gain && !cls) gain += (size_t)l * d.E;
+                    st_prep<QUANT, LPG>(g, ph.src, l == 0 && p4 == SK_QKV && !cls ? x_s : nullptr, el + ph.need, gain, ph.n, ph.rn, act, ms.red[half]);
                     ST_STAMP();
-                    st_consume<QUANT, LPG>(g, ring, cur, tcount, k, epi, l, own.row0[kid], own.rows[kid], eout, act, pos, pen, xown, ms, geo, kid, dbg);
+                    st_consume<QUANT, LPG>(g, ring, cur, tcount, ph, l, el + ph.out, act, pos, xown, ms);
                 } else {
                     ST_STAMP();
                     if (cls && lane == 0) { ms.best_v[warp] = -FLT_MAX; ms.best_i[warp] = 0xffffffffu; }
@@ -1094,12 +938,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_decode_stream(const __grid_cons
                 ST_STAMP();
                 ST_TRACE();
                 if (cls) break;
-                if (ph == SK_QKV) {
-                    st_attention<KVM>(g, ring, cur, tcount, l, cta, pos, range, nsplit, chunk, (g.ablate & 16u) ? kXwAny : el + 1u, el + 2u, attn_ws, dbg ? g.trace + 1100 + 64 : nullptr);
+                if (p4 == SK_QKV) {
+                    st_attention<KVM, HDC>(g, ring, cur, tcount, l, cta, pos, ms.plan, el + 1u, el + 2u, reinterpret_cast<float *>(ssm + g.off_attn));
                     ST_STAMP();
                     ST_TRACE();
                 }
             }
+            if (l < d.L) el += 5u;
         }
         cbar();
         if (threadIdx.x == 0) {
@@ -1108,7 +953,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_decode_stream(const __grid_cons
                 if (ms.best_i[w] != 0xffffffffu && (bi == 0xffffffffu || ms.best_v[w] > bv || (ms.best_v[w] == bv && ms.best_i[w] < bi))) { bv = ms.best_v[w]; bi = ms.best_i[w]; }
             g.cls_val[cta] = bv; g.cls_idx[cta] = bi;
         }
-        st_grid_barrier(g, s_target, &s_progress, ncta);
+        st_grid_barrier(g, ms.target, &s_progress, ncta);
         ST_TRACE();
         // ---- every CTA picks the token from the per-CTA partials (no second barrier) and advances its copy of the state ----
         {
@@ -1130,8 +975,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_decode_stream(const __grid_cons
                 if (ms.best_i[w] != 0xffffffffu && (bi == 0xffffffffu || ms.best_v[w] > bv || (ms.best_v[w] == bv && ms.best_i[w] < bi))) { bv = ms.best_v[w]; bi = ms.best_i[w]; }
             if (bi == 0xffffffffu) bi = 0;       // all-NaN row: the reference's argmax returns index 0
             uint32_t nxt = bi;
-            if (advance) {
-                const bool forced = (pos + 1 < n_prompt);            // infer.c:1250 is_prefilling
+            if (__ldcg(&g.st->advance)) {
+                const bool forced = (pos + 1 < __ldcg(&g.st->n_prompt));            // infer.c:1250 is_prefilling
                 if (forced) nxt = __ldcg(g.ids + pos + 1);
                 if (cta == 0 && threadIdx.x == 0) {
                     g.seen[tok] = 1;                                 // ids[0..pos] are "seen" for step pos+1

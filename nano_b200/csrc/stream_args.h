@@ -45,32 +45,20 @@ struct StreamArgs {
     unsigned int *bar;                                // grid barrier counter (zeroed by the host before every launch)
     uint32_t *err;                                    // set to a nonzero code before a spin gives up (and traps)
     uint32_t n_steps, nsplit_max, chunk_target;
-    uint32_t ablate;                                  // timing experiments only (NB200_ABLATE, results are wrong): 1 no quantise math, 2 no row dots, 4 no attention math,
-                                                      // 8 no sum of squares, 16 no waiting for epochs, 32 no publishing to replicas 1..7
     unsigned long long *trace;                        // optional: CTA 0 / thread 0 clock64() after every barrier of the LAST step
     Dims d;
 };
 
-// activation prologue: warp slots held in registers between the sum-of-squares pass and the quantise pass; the host
-// checks n <= st_prep_max_n before choosing the streaming kernel
-constexpr int kStKmax = 6, kStKmaxQ4K = 2;           // warp slots of 128 (Q80 / F32) or 256 (Q4K) elements
+// the longest row whose activation operand the prologue prepares (Q4K: warp slots of 256 elements stay in registers between the sum of squares and the
+// quantise pass); the host checks it before choosing the streaming kernel
+constexpr int kStKmax = 6, kStKmaxQ4K = 2;
 __host__ __device__ inline uint32_t st_prep_max_n(uint32_t quant, uint32_t gs) {
     (void)gs;
     return quant == 0x42u ? (uint32_t)kConsWarps * kStKmaxQ4K * 256u : (uint32_t)kConsWarps * kStKmax * 128u;
 }
 
-// attention workspace of one CTA (floats): q [KVM][hd] | scores of a segment [KVM][seg rows] | per-head scale [KVM] |
-// the position's k, v [2][hd] | the item's partial [KVM][hd + 2]; the merge of a multi-split head stages the partials of
-// all splits in the same region, followed by the merge weights / partial sums [2][KVM][nsplit_max] and totals [KVM]
+// attention workspace of one CTA (floats): q [KVM][hd] | the position's k, v [2][hd] | the warps' weighted sums [15][KVM][hd] | their maxima and sums of weights [2][KVM][16]
 constexpr int kStSegTiles = 8;                    // ring tiles of K/V that an attention segment keeps resident
-__host__ __device__ inline uint32_t st_attn_work_floats(uint32_t kvm, uint32_t hd, uint32_t seg_rows) {
-    return kvm * hd + kvm * seg_rows + ((kvm + 3u) & ~3u) + 2u * hd + kvm * (hd + 2u) + 16u;
-}
-__host__ __device__ inline uint32_t st_attn_smem_floats(uint32_t kvm, uint32_t hd, uint32_t nsplit_max, uint32_t seg_rows) {
-    uint32_t ws = st_attn_work_floats(kvm, hd, seg_rows);
-    const uint32_t merge = nsplit_max * kvm * hd;
-    if (merge > ws) ws = merge;
-    return ws + 2u * kvm * nsplit_max + 2u * kvm + 16u;
-}
+__host__ __device__ inline uint32_t st_attn_smem_floats(uint32_t kvm, uint32_t hd) { return (1u + kConsWarps) * kvm * hd + 2u * hd + 2u * kvm * 16u; }
 
 }  // namespace nb

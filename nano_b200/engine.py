@@ -68,7 +68,7 @@ def lib(layered_ok: bool = False):
     (built in seconds) when the full one has not been built."""
     global _lib
     if _lib is None:
-        path = os.environ.get("NB200_ENGINE_SO", _build.ENGINE_SO)     # developer hook: the fine-trace build (tools/gpu_trace.py)
+        path = os.environ.get("NB200_ENGINE_SO", _build.ENGINE_SO)     # developer hook: another build of the library
         if not os.path.exists(path) and layered_ok and os.path.exists(_build.LAYERED_SO):
             path = _build.LAYERED_SO
         if not os.path.exists(path):

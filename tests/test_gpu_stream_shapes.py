@@ -1,0 +1,55 @@
+"""The streaming decode kernel over the shapes its instances and row blocks are chosen by, against the oracle: query heads per kv head x head sizes
+(lanes of a cache row), attention items of one pass, of several segments and merged over several CTAs, rows shorter and longer than a warp's step."""
+import numpy as np
+import pytest
+
+from nano_b200 import engine as E, modelfile as mf
+from oracle import bindings as ob
+
+pytestmark = pytest.mark.gpu
+
+#          arch           heads kv  head  width  hidden
+SHAPES = [(mf.ARCH_NANO, 2, 2, 12, 24, 20), (mf.ARCH_NANO, 4, 4, 48, 192, 36), (mf.ARCH_NANO, 4, 2, 100, 400, 64), (mf.ARCH_QWEN3, 3, 3, 128, 96, 260),
+          (mf.ARCH_QWEN3, 4, 2, 64, 1028, 300), (mf.ARCH_QWEN3, 4, 2, 128, 64, 516), (mf.ARCH_QWEN3, 4, 1, 32, 128, 128), (mf.ARCH_QWEN3, 8, 2, 128, 64, 2052)]
+#        rows of an attention item, ring stage in KB: default; 8 rows (many items); several segments per item
+PLANS = [(0, 16), (8, 16), (512, 5)]
+
+
+def run(spec, quant, gs, chunk, stage, monkeypatch, n):
+    monkeypatch.setenv("NB200_STREAM", "1")
+    monkeypatch.setenv("NB200_STAGE_KB", str(stage))
+    if chunk:
+        monkeypatch.setenv("NB200_ATTN_CHUNK", str(chunk))
+    path = mf.cached_model(spec, quant, gs)
+    eng = E.Engine(path, n)
+    assert eng.path.startswith("streaming"), eng.path
+    o = ob.NanoOracle(path, n)
+    toks = mf.teacher_tokens(n, spec.vocab)
+    a, b = np.zeros((2, n, spec.vocab))
+    for pos in range(n):
+        a[pos], b[pos] = eng.forward(toks[pos], pos), o.forward(toks[pos], pos)
+    eng.close()
+    o.close()
+    return a, b
+
+
+@pytest.mark.parametrize("chunk,stage", PLANS)
+@pytest.mark.parametrize("arch,H,KV,hd,E_,F", SHAPES)
+def test_f32_shapes(arch, H, KV, hd, E_, F, chunk, stage, monkeypatch):
+    spec = mf.ModelSpec("shape-%d-%d-%d-%d-%d-%d" % (arch, H, KV, hd, E_, F), arch, 128, 97, 2, E_, H, KV, F, hd)
+    if chunk == 512 and (stage * 1024 // (8 * hd)) * 8 >= 75:
+        pytest.skip("one segment holds the whole context of so small a head")
+    a, b = run(spec, mf.QUANT_F32, 128, chunk, stage, monkeypatch, 75)
+    # both sides hold 24 bits in every sum: rows of up to 2052 products and 75 weighted rows, through two layers, differ by their order
+    # only, about sqrt(2052) * 2^-24 = 3e-6 of a row's size a layer at most
+    assert np.linalg.norm(a - b) <= 1e-5 * np.linalg.norm(b)
+
+
+# widths of one quantisation group, of an odd number of them, of more than one 1024-byte step of a warp, and of more than one turn of the prologue's warps
+@pytest.mark.parametrize("E_,F,gs", [(64, 64, 64), (192, 320, 64), (640, 1152, 128), (128, 4224, 128), (3968, 128, 128)])
+def test_q80_rows(E_, F, gs, monkeypatch):
+    spec = mf.ModelSpec("rows-%d-%d-%d" % (E_, F, gs), mf.ARCH_QWEN3, 128, 131, 1, E_, 4, 2, F, 64 if E_ != 3968 else 128)
+    a, b = run(spec, mf.QUANT_Q80, gs, 0, 16, monkeypatch, 20)
+    # sums in another order turn an activation code here and there, by one of 127 steps of its group: 2^-8 of a row's size at most, where not so it is 1e-6
+    assert np.linalg.norm(a - b) <= 4e-3 * np.linalg.norm(b)
+    assert np.median(np.linalg.norm(a - b, axis=1) / np.linalg.norm(b, axis=1)) <= 2e-3
