@@ -96,7 +96,8 @@ struct nb200_engine : nb::EngineBase {
     float calib_ms[2] = {0.0f, 0.0f};      // ms per token of {streaming, multi-kernel} measured by calibrate_paths (0 = not calibrated)
     bool use_stream = false; const void *st_kern = nullptr; StreamArgs sa{}; uint32_t st_smem = 0, st_grid = 0;
     uint32_t *st_err_host = nullptr, *st_err_dev = nullptr;      // mapped pinned word: the code a device-side spin recorded before trapping
-    uint32_t st_epoch = 0;                                       // exchange epochs handed out so far (stream.cuh)
+    uint32_t st_epoch = 0, st_bar = 0;                           // exchange epochs handed out so far, what the grid barrier's counter stands at (stream.cuh)
+    float *logits_host = nullptr; bool logits_on_host = false;   // pinned copy of the logits that one-token calls of the streaming kernel write; whether it holds the last step's
     void *samp_ws = nullptr; size_t samp_cub = 0; uint32_t *samp_host = nullptr;       // device-side sampler workspace (sample.cu), pinned result
     uint64_t stream_bytes = 0;
     unsigned int *bar = nullptr;
@@ -378,19 +379,23 @@ int run_classifier(nb200_engine *e) {
 
 int run_token(nb200_engine *e) {
     int r;
+    e->logits_on_host = false;
     if ((r = run_embed(e))) return r;
     for (uint32_t l = 0; l < e->d.L; l++) if ((r = run_layer(e, l))) return r;
     return run_classifier(e);
 }
 
-// n_steps tokens in ONE cooperative launch of the streaming kernel
-int launch_stream(nb200_engine *e, uint32_t n_steps) {
+// n_steps tokens in ONE cooperative launch of the streaming kernel.  st: the state of its first step (null: what the launch before left on the device);
+// with_logits: the (last) step's logits also go to the pinned copy
+int launch_stream(nb200_engine *e, uint32_t n_steps, const DevState *st = nullptr, bool with_logits = false) {
+    e->logits_on_host = false;
     if (n_steps == 0) return 0;
     StreamArgs g = e->sa;
     g.n_steps = n_steps; g.trace = e->trace_dev;
-    g.epoch_base = e->st_epoch;
-    e->st_epoch += n_steps * 5u * e->d.L;
-    CK(cudaMemsetAsync(e->bar, 0, sizeof(unsigned int), e->stream));
+    g.epoch_base = e->st_epoch; g.bar_base = e->st_bar;
+    e->st_epoch += n_steps * 5u * e->d.L; e->st_bar += n_steps * e->st_grid;
+    if (st) { g.st0 = *st; g.with_state = 1; g.next_host = e->tok_host; }
+    if (with_logits) g.logits_host = e->logits_host;
     void *params[] = {&g};
     CK(cudaLaunchCooperativeKernel(e->st_kern, dim3(e->st_grid), dim3(kThreads), params, e->st_smem, e->stream));
     e->launches++;
@@ -400,6 +405,7 @@ int launch_stream(nb200_engine *e, uint32_t n_steps) {
 int launch_token(nb200_engine *e) {
     if (e->tp_size > 1 && !e->tp_attached) return fail(NB200_EINVAL, "tensor-parallel engine: attach the peer ranks first (nb200_tp_attach_*)");
     if (e->use_stream) return launch_stream(e, 1);
+    e->logits_on_host = false;
     if (e->graph) {
         CK(cudaGraphLaunch(e->graph, e->stream));
         e->launches += e->launches_per_token;
@@ -594,6 +600,7 @@ int setup_stream(nb200_engine *e) {
     CK(cudaHostAlloc(&e->st_err_host, 64, cudaHostAllocMapped));
     memset(e->st_err_host, 0, 64);
     CK(cudaHostGetDevicePointer((void **)&e->st_err_dev, e->st_err_host, 0));
+    if (cudaHostAlloc(&e->logits_host, (size_t)d.V * 4, cudaHostAllocMapped) != cudaSuccess) { e->logits_host = nullptr; cudaGetLastError(); }      // without it logits are copied
 
     g.stream = stream; g.nstages = nst; g.stage_bytes = stage_bytes; g.kv_tile_rows = kv_rows;
     g.kv_tile_magic = (uint32_t)((0x100000000ull + kv_rows - 1) / kv_rows);
@@ -640,6 +647,7 @@ static void nano_destroy(nb200_engine *e) {
     if (e->st_host) cudaFreeHost(e->st_host);
     if (e->samp_host) cudaFreeHost(e->samp_host);
     if (e->tok_host) cudaFreeHost(e->tok_host);
+    if (e->logits_host) cudaFreeHost(e->logits_host);
     if (e->stream) cudaStreamDestroy(e->stream);
     delete e;
 }
@@ -1154,19 +1162,31 @@ static int push_state(nb200_engine *e, uint32_t pos, uint32_t causal, uint32_t n
     return 0;
 }
 
+// one token whose state comes from the host.  On the streaming kernel the state travels with the launch, the chosen token and (for forward) the logits come back through
+// pinned memory that the kernel writes while it works: a copy in front of the kernel, one behind it and the waits between cost 45 us of a 134 us
+// call (four F32 layers of Nano's width), and 100 of 690 for the 608 KB of Qwen3's logits.
+static int run_one(nb200_engine *e, uint32_t pos, uint32_t causal, float penalty, uint32_t token, bool with_logits) {
+    if (!e->use_stream) { const int r = push_state(e, pos, causal, 0, 0, penalty, token, 1); return r ? r : launch_token(e); }
+    DevState st;
+    memset(&st, 0, sizeof st);
+    st.pos = pos; st.is_causal = causal; st.penalty = penalty; st.token = token; st.use_token = 1;
+    return launch_stream(e, 1, &st, with_logits);
+}
+
 static int nano_forward(nb200_engine *e, uint32_t token, uint32_t pos, uint32_t is_causal) {
     if (!e) return fail(NB200_EINVAL, "null engine");
     if (pos >= e->d.max_seq || token >= e->d.V) return fail(NB200_EINVAL, "token/pos out of range");
     CK(cudaSetDevice(e->device));
     int r;
-    if ((r = push_state(e, pos, is_causal ? 1u : 0u, 0, 0, 1.0f, token, 1))) return r;
-    if ((r = launch_token(e))) return r;
+    if ((r = run_one(e, pos, is_causal ? 1u : 0u, 1.0f, token, true))) return r;
     CK(cudaStreamSynchronize(e->stream));
+    e->logits_on_host = e->use_stream && e->logits_host;
     return tp_check(e);
 }
 
 static int nano_read_logits(nb200_engine *e, float *host_logits) {
     if (!e || !host_logits) return fail(NB200_EINVAL, "null argument");
+    if (e->logits_on_host) { memcpy(host_logits, e->logits_host, (size_t)e->d.V * 4); return 0; }
     CK(cudaSetDevice(e->device));
     CK(cudaMemcpyAsync(host_logits, e->logits, (size_t)e->d.V * 4, cudaMemcpyDeviceToHost, e->stream));
     CK(cudaStreamSynchronize(e->stream));
@@ -1196,10 +1216,9 @@ static int nano_next_greedy(nb200_engine *e, const uint32_t *ids, uint32_t pos, 
     if (pos >= e->d.max_seq || ids[pos] >= e->d.V) return fail(NB200_EINVAL, "token/pos out of range");
     CK(cudaSetDevice(e->device));
     int r;
-    if ((r = push_state(e, pos, 1, 0, 0, is_prefilling ? 1.0f : penalty, ids[pos], 1))) return r;
     if (!is_prefilling && penalty != 1.0f) { if ((r = sync_seen(e, ids, pos))) return r; }
-    if ((r = launch_token(e))) return r;
-    CK(cudaMemcpyAsync(e->tok_host, &e->st->next_token, 4, cudaMemcpyDeviceToHost, e->stream));
+    if ((r = run_one(e, pos, 1, is_prefilling ? 1.0f : penalty, ids[pos], false))) return r;
+    if (!e->use_stream) CK(cudaMemcpyAsync(e->tok_host, &e->st->next_token, 4, cudaMemcpyDeviceToHost, e->stream));
     CK(cudaStreamSynchronize(e->stream));
     *next = is_prefilling ? ids[pos + 1] : *e->tok_host;
     return tp_check(e);

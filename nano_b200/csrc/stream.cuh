@@ -95,9 +95,10 @@ __device__ __forceinline__ void xw_st(unsigned long long *p, float v, uint32_t e
 __device__ __forceinline__ bool xw_ok(unsigned long long w, uint32_t need) { return (uint32_t)(w >> 32) == need; }
 __device__ __forceinline__ float xw_val(unsigned long long w) { return __uint_as_float((uint32_t)w); }
 // now and then inside a polling loop: start the clock, or give up after ~2 s
-static __device__ __noinline__ void st_still_waiting(long long &t0, uint32_t *err, uint32_t code) {
-    if (t0 == 0) t0 = clock64();
-    else if (clock64() - t0 > 4000000000ll) st_give_up(err, code);
+static __device__ __noinline__ long long st_still_waiting(long long t0, uint32_t *err, uint32_t code) {
+    const long long now = clock64();
+    if (t0 && now - t0 > 4000000000ll) st_give_up(err, code);
+    return t0 ? t0 : now;
 }
 // 4 consecutive words (32-byte aligned) -> float4 once all of them carry `need`
 static __device__ __noinline__ float4 xw_poll4_slow(const unsigned long long *p, uint32_t need, uint32_t *err) {
@@ -132,7 +133,7 @@ __device__ __forceinline__ void st_attn_plan(uint32_t range, uint32_t nsplit_max
 }
 
 struct StPlan { uint32_t nsplit, kvh, sp, t0, t1; };          // this CTA's attention item of the token (kvh >= KV: none)
-struct StSmem { float red[2][16]; float best_v[kConsWarps]; uint32_t best_i[kConsWarps]; float pen; uint32_t target, ti, tj; StPlan plan; };
+struct StSmem { float red[2][16]; float best_v[kConsWarps]; uint32_t best_i[kConsWarps]; DevState st; uint32_t target, ti, tj; StPlan plan; };
 
 struct StRing {
     uint64_t *full, *empty;
@@ -348,7 +349,7 @@ __device__ __forceinline__ void st_prep(const StreamArgs &g, const unsigned long
                                 v1 = make_float4(xw_val(z0), xw_val(z1), xw_val(z2), xw_val(z3));
                                 break;
                             }
-                            if ((it & 255u) == 0) st_still_waiting(t0, g.err, 0x50u);          // the clock is read rarely: the loop stays loads and compares
+                            if ((it & 255u) == 0) t0 = st_still_waiting(t0, g.err, 0x50u);          // the clock is read rarely: the loop stays loads and compares
                         }
                         __syncwarp();
                     }
@@ -494,7 +495,7 @@ __device__ __forceinline__ void st_consume(const StreamArgs &g, const StRing &r,
     const uint32_t n = pa.x, row_stride = pa.y, aux_stride = pa.z, tile_rows = pa.w, rows = pb.x, nt = pb.y, row0 = pb.z, epi = ph.epi;
     const bool owned = pb.w & 1u;
     const uint32_t rb = owned ? (QUANT == 0x42 ? 2u : 4u) : (pb.w >> 8) & 255u, step = owned ? rb : rb * kConsWarps, tb = pb.w >> 16;
-    float bestv = -FLT_MAX; uint32_t besti = 0xffffffffu;
+    float bestv = -FLT_MAX, kept = 0.0f; uint32_t besti = 0xffffffffu;
     const uint32_t jstep = owned ? (uint32_t)kConsWarps : 1u;
     uint32_t turn = (uint32_t)warp;                         // shared tiles: which block of rows of the tile is this warp's first
     StCursor cc = c;
@@ -540,12 +541,23 @@ __device__ __forceinline__ void st_consume(const StreamArgs &g, const StRing &r,
                         g.vc[(size_t)layer * d.KV * d.max_seq * d.hd + ((size_t)h * d.max_seq + pos) * d.hd + i] = v;
                     }
                 }
-            } else if (on && rep == 0) {
-                // classifier: infer.c:1156-1167 penalty (division, any sign), then first-max argmax :1026-1037 (rows ascend per lane)
-                const float pen = ms.pen;
-                if (pen != 1.0f && __ldcg(g.seen + row)) v = __fdiv_rn(v, pen);
-                g.logits[row] = v;
-                if (v > bestv) { bestv = v; besti = row; }
+            } else {
+                // classifier: up to 32 rows of an owned tile are gathered, lane by lane, so that they leave in one store (to the host as well, across PCIe, when a call returns logits)
+                const uint32_t q = (uint32_t)lane - (owned ? rr & 31u : 0u);
+                const float got = __shfl_sync(0xffffffffu, v, (q << (sh & 31u)) & 31u);
+                if (q < cnt) kept = got;
+                if (!owned || ((rr + step) & 31u) == 0u || rr + step >= tr) {
+                    const uint32_t crow = row0 + done + (owned ? rr & ~31u : rr) + lane;
+                    if ((uint32_t)lane < (owned ? (rr & 31u) + cnt : cnt)) {
+                        // infer.c:1156-1167 penalty (division, any sign), then first-max argmax :1026-1037 (rows ascend per lane)
+                        float w = kept;
+                        const float pen = ms.st.penalty;
+                        if (pen != 1.0f && __ldcg(g.seen + crow)) w = __fdiv_rn(w, pen);
+                        g.logits[crow] = w;
+                        if (g.logits_host) g.logits_host[crow] = w;
+                        if (w > bestv) { bestv = w; besti = crow; }
+                    }
+                }
             }
         }
         __syncwarp();
@@ -796,7 +808,7 @@ static __device__ void st_attention(const StreamArgs &g, const StRing &r, StCurs
                 for (uint32_t q = 0; q < 8u; q++) ok = ok && xw_ok(w8[q], e_out);
                 if (stats) ok = ok && xw_ok(a0, e_out) && xw_ok(a1, e_out) && xw_ok(b0, e_out) && xw_ok(b1, e_out);
                 if (__all_sync(0xffffffffu, ok)) return;
-                if ((it & 255u) == 0) st_still_waiting(t0, g.err, 0x51u);
+                if ((it & 255u) == 0) t0 = st_still_waiting(t0, g.err, 0x51u);
             }
         };
         ask(0, true);
@@ -825,9 +837,9 @@ __device__ __forceinline__ void st_grid_barrier(const StreamArgs &g, unsigned in
         const unsigned int target = target_smem + ncta;
         target_smem = target;
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(g.bar) : "memory");       // release: this CTA's plain stores of the token
-        if (ld_acquire_u32(g.bar) < target) {
+        if ((int32_t)(ld_acquire_u32(g.bar) - target) < 0) {
             const long long t0 = clock64();
-            while (ld_acquire_u32(g.bar) < target) { if (clock64() - t0 > 4000000000ll) st_give_up(g.err, 0x40u); }
+            while ((int32_t)(ld_acquire_u32(g.bar) - target) < 0) { if (clock64() - t0 > 4000000000ll) st_give_up(g.err, 0x40u); }
         }
         asm volatile("fence.proxy.async.global;" ::: "memory");      // the token's plain K/V stores are TMA-read by later tokens
         *progress = *progress + 1u;
@@ -858,7 +870,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_decode_stream(const __grid_cons
     const StRing ring{full_bar, empty_bar, stage_tile, ssm + g.off_ring, g.nstages, g.stage_bytes};
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < g.nstages; s++) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], kConsWarps); stage_tile[s] = 0xffffffffu; }
-        s_progress = 0; ms.target = 0; ms.ti = ms.tj = 0; ms.pen = __ldcg(&g.st->penalty);
+        s_progress = 0; ms.target = g.bar_base; ms.ti = ms.tj = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (threadIdx.x < 5) {          // (64-bit divisions: once, not once per phase)
@@ -881,14 +893,16 @@ __global__ void __launch_bounds__(kThreads, 1) k_decode_stream(const __grid_cons
         ph.rn = 1.0f / (float)k.n;
     }
     if (threadIdx.x < 32) reinterpret_cast<float *>(ms.red)[threadIdx.x] = 0.0f;
+    if (threadIdx.x < sizeof(DevState) / 4)        // the call's state: with the launch, or left on the device by the launch before
+        reinterpret_cast<uint32_t *>(&ms.st)[threadIdx.x] = g.with_state ? reinterpret_cast<const uint32_t *>(&g.st0)[threadIdx.x] : __ldcg(reinterpret_cast<const uint32_t *>(g.st) + threadIdx.x);
     __syncthreads();
 
     // step state (identical in every CTA; advanced locally)
-    uint32_t pos = __ldcg(&g.st->pos);
-    uint32_t tok = __ldcg(&g.st->use_token) ? __ldcg(&g.st->token) : __ldcg(g.ids + pos);
+    uint32_t pos = ms.st.pos;
+    uint32_t tok = ms.st.use_token ? ms.st.token : __ldcg(g.ids + pos);
 
     if (warp == kConsWarps) {
-        if (lane == 0) st_producer(g, ring, phase, cta, &s_progress, pos, __ldcg(&g.st->is_causal), __ldcg(&g.st->advance));
+        if (lane == 0) st_producer(g, ring, phase, cta, &s_progress, pos, ms.st.is_causal, ms.st.advance);
         return;
     }
 
@@ -904,7 +918,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_decode_stream(const __grid_cons
         ST_TRACE();
         float *x_s = reinterpret_cast<float *>(ssm + g.off_xs);
         if (threadIdx.x == 0) {
-            const uint32_t range = __ldcg(&g.st->is_causal) ? pos + 1u : d.max_seq;
+            const uint32_t range = ms.st.is_causal ? pos + 1u : d.max_seq;
             uint32_t nsplit, chunk;
             st_attn_plan(range, g.nsplit_max, g.chunk_target, nsplit, chunk);
             const uint32_t kvh = cta / nsplit, sp = cta - kvh * nsplit, t0 = min(range, sp * chunk);
@@ -975,8 +989,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_decode_stream(const __grid_cons
                 if (ms.best_i[w] != 0xffffffffu && (bi == 0xffffffffu || ms.best_v[w] > bv || (ms.best_v[w] == bv && ms.best_i[w] < bi))) { bv = ms.best_v[w]; bi = ms.best_i[w]; }
             if (bi == 0xffffffffu) bi = 0;       // all-NaN row: the reference's argmax returns index 0
             uint32_t nxt = bi;
-            if (__ldcg(&g.st->advance)) {
-                const bool forced = (pos + 1 < __ldcg(&g.st->n_prompt));            // infer.c:1250 is_prefilling
+            if (ms.st.advance) {
+                const bool forced = (pos + 1 < ms.st.n_prompt);            // infer.c:1250 is_prefilling
                 if (forced) nxt = __ldcg(g.ids + pos + 1);
                 if (cta == 0 && threadIdx.x == 0) {
                     g.seen[tok] = 1;                                 // ids[0..pos] are "seen" for step pos+1
@@ -987,6 +1001,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_decode_stream(const __grid_cons
                 tok = nxt; pos = pos + 1;
             } else if (cta == 0 && threadIdx.x == 0) {
                 g.st->next_token = bi;
+                if (g.next_host) *g.next_host = bi;
             }
             cbar();
         }

@@ -42,7 +42,10 @@ struct StreamArgs {
     uint32_t epoch_base;                              // epochs handed out before this launch (host-maintained, monotonic)
     float *cls_val; uint32_t *cls_idx;                // per-CTA argmax partials
     DevState *st; uint32_t *ids; uint8_t *seen;
-    unsigned int *bar;                                // grid barrier counter (zeroed by the host before every launch)
+    unsigned int *bar;                                // grid barrier counter; every CTA of every token adds one, never reset
+    uint32_t bar_base;                                // what it stands at when this launch begins (host-maintained, modulo 2^32)
+    DevState st0; uint32_t with_state;                // 1: the step's state is st0, not *st (a call of one token needs no copy in front of it)
+    float *logits_host; uint32_t *next_host;          // pinned host copies of the logits and of the chosen token, or null
     uint32_t *err;                                    // set to a nonzero code before a spin gives up (and traps)
     uint32_t n_steps, nsplit_max, chunk_target;
     unsigned long long *trace;                        // optional: CTA 0 / thread 0 clock64() after every barrier of the LAST step

@@ -7,6 +7,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import sys
 from typing import Optional, Tuple
 
 import numpy as np
@@ -139,6 +140,32 @@ def _p(a: np.ndarray, t):
     return a.ctypes.data_as(t)
 
 
+class RowPool:
+    """Float arrays of n values whose memory is used again once nothing refers to it: a fresh array of Qwen3's 608 KB of logits costs 42 us of page faults, more
+    than twice what filling it takes.  take() gives a view of a kept buffer that nobody else holds (views, and whatever is built on them, refer to their
+    buffer), or of a new one.  At most 32 MB are kept; arrays below 64 KB come from the allocator, which has them without faults."""
+
+    def __init__(self, n: int):
+        self.n, self.kept = n, []
+
+    def take(self) -> np.ndarray:
+        if 4 * self.n < 1 << 16:
+            return np.empty(self.n, np.float32)
+        for _ in range(4):          # the one given out longest ago is first; no long search while a caller keeps many
+            try:
+                buf = self.kept.pop(0)          # out of the list while it is looked at: no other thread can take it
+            except IndexError:
+                break
+            out = buf[:] if sys.getrefcount(buf) == 2 else None          # 2: this name and the argument
+            self.kept.append(buf)
+            if out is not None:
+                return out
+        buf = np.empty(self.n, np.float32)
+        if (len(self.kept) + 1) * 4 * self.n <= 32 << 20:
+            self.kept.append(buf)
+        return buf[:]
+
+
 class Engine:
     """One model resident in the HBM of one B200."""
 
@@ -171,6 +198,8 @@ class Engine:
         for n, _t in Config._fields_[:-1]:
             setattr(self, n, int(getattr(cfg, n)))
         self.vocab = self.vocab_size
+        if not hasattr(self, "_rows"):
+            self._rows = RowPool(self.vocab)
         self.path = {4: "streaming kernel (persistent grid, per-CTA TMA ring over weights and KV, L2 grid barriers)",
                      1: "multi-kernel CUDA graph with PDL", 0: "multi-kernel direct launches"}[int(cfg.reserved[0])]
         # creation-time calibration of the two fast paths (large one-GPU Q80 engines): us per token of each, None when not measured
@@ -189,7 +218,7 @@ class Engine:
     def step(self, seq: int, tokens, want=()) -> np.ndarray:
         """Runs the next tokens of `seq`; returns the logits [len(want), vocab] at the places `want` (indices into tokens)."""
         t = np.ascontiguousarray(tokens, np.uint32); w = np.ascontiguousarray(sorted(want), np.uint32)
-        out = np.empty((w.size, self.vocab), np.float32)
+        out = self._rows.take().reshape(1, -1) if w.size == 1 else np.empty((w.size, self.vocab), np.float32)
         _check(lib().nb200_step(self.h, int(seq), _p(t, u32p), t.size, _p(w, u32p) if w.size else None, w.size,
                                 _p(out, f32p) if w.size else None))
         return out
@@ -263,7 +292,7 @@ class Engine:
         _check(lib().nb200_forward(self.h, int(token), int(pos), int(causal)))
 
     def logits(self) -> np.ndarray:
-        out = np.empty(self.vocab, dtype=np.float32)
+        out = self._rows.take()
         _check(lib().nb200_read_logits(self.h, _p(out, f32p)))
         return out
 

@@ -53,3 +53,28 @@ def test_q80_rows(E_, F, gs, monkeypatch):
     # sums in another order turn an activation code here and there, by one of 127 steps of its group: 2^-8 of a row's size at most, where not so it is 1e-6
     assert np.linalg.norm(a - b) <= 4e-3 * np.linalg.norm(b)
     assert np.median(np.linalg.norm(a - b, axis=1) / np.linalg.norm(b, axis=1)) <= 2e-3
+
+
+def test_logits_are_those_of_the_last_step(monkeypatch):
+    """forward leaves its logits in pinned host memory; whatever runs afterwards must not be answered from there."""
+    monkeypatch.setenv("NB200_STREAM", "1")
+    spec = mf.PRESETS["toy-qwen3"]
+    eng = E.Engine(mf.cached_model(spec, mf.QUANT_Q80, 64), 64)
+
+    def device():
+        return eng.read(E.F_LOGITS, spec.vocab)
+    a = eng.forward(5, 0)
+    assert np.array_equal(a, device())
+    b = eng.forward(7, 1)
+    assert np.array_equal(b, device()) and not np.array_equal(a, b)
+    eng.next_greedy(np.array([5, 7, 9, 0], np.uint32), 2, 0)
+    c = eng.logits()
+    assert np.array_equal(c, device()) and not np.array_equal(b, c)
+    assert np.array_equal(eng.forward(9, 2), c)
+    ids = np.zeros(40, np.uint32)
+    ids[:3] = [5, 7, 9]
+    eng.decode_greedy(ids, 3, 20)
+    d = eng.logits()
+    assert np.array_equal(d, device()) and not np.array_equal(c, d)
+    assert eng.next_greedy(ids, 19, 0) == int(np.argmax(eng.logits()))
+    eng.close()
