@@ -67,6 +67,7 @@
 #include "layered_mixers3.cuh"
 #include "layered_mixers4.cuh"
 #include "layered_mixers5.cuh"
+#include "layered_one.cuh"
 #include "layered_tc.h"
 #include "modeldir.h"
 #include "sample_host.h"
@@ -893,6 +894,36 @@ uint32_t gemv_blocks(const LayeredEngine *e, uint32_t N, uint32_t groups) {
 
 uint32_t ew_grid(size_t n) { return (uint32_t)std::min<size_t>((n + 255) / 256, 148 * 16); }
 
+// does the product of one row per group run on k_gemv_one: 16-byte loads of weights and activations, a row that fits its shared memory
+bool one_fits(const GemmArgs &a, bool f32) {
+    const uint32_t vn = f32 ? 4u : 8u;
+    auto at16 = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
+    return a.K && a.K % vn == 0 && a.K <= kOneMaxK && a.ldw % vn == 0 && a.w_gstride % vn == 0 && at16(a.W) && at16(a.A) && a.lda % 4u == 0 && a.a_gcols % 4u == 0 &&
+           (!a.a_norm_w || at16(a.a_norm_w)) && (a.a_parts <= 1 || (a.a_parts <= 32u && (a.K / a.a_parts) % 4u == 0)) && a.cv_K <= 32u && a.cr[0].K <= 32u && a.cr[1].K <= 32u;
+}
+// blocks of a group, and how many warps share a row (2^one_split): as many as still leave each of them 4 steps of a row and all blocks one turn, resident at
+// once.  A link of a chain from HBM, us, by one_split 0 / 1 / 2 / 3: 1024 x 4096 columns 5.4 / 4.5 / 4.4 / 7.1, 512 x 8192 8.8 / 6.4 / 5.4 / 5.4, 2048 x 6144 10.1 / 8.0 / 9.6,
+// 2048 x 2048 4.0 / 3.9 / 5.4; rows of 4 steps and less are slower when shared (1024 x 1024 2.9 / 2.9 / 3.1).
+template <typename WT>
+uint32_t one_blocks(const LayeredEngine *e, GemmArgs *a, uint32_t groups) {
+    const uint32_t most = std::max(1u, (uint32_t)e->num_sms * 4u / groups), steps = (a->K + one_step<WT>() - 1u) / one_step<WT>();
+    uint32_t s = 0;
+    while (s < 3u && steps >> (s + 1u) >= 4u && (((uint64_t)a->N << (s + 1u)) + kOneWarps - 1u) / kOneWarps <= most) s++;
+    a->one_split = s;
+    return (uint32_t)std::min<uint64_t>((((uint64_t)a->N << s) + kOneWarps - 1u) / kOneWarps, most);
+}
+
+template <int EXT>
+int gemv_launch(LayeredEngine *e, GemmArgs a, uint32_t groups, uint32_t live, bool one, bool f32) {
+    if (one) {
+        const dim3 grid(f32 ? one_blocks<float>(e, &a, live) : one_blocks<__nv_bfloat16>(e, &a, live), groups), block(kOneThreads);
+        return f32 ? launch<GemmArgs>(e, k_gemv_one<float, EXT>, grid, block, one_smem<float>(a.K), a) : launch<GemmArgs>(e, k_gemv_one<__nv_bfloat16, EXT>, grid, block, one_smem<__nv_bfloat16>(a.K), a);
+    }
+    const dim3 grid(gemv_blocks(e, a.N, live), groups), block(256);
+    if (EXT == 0) return f32 ? launch<GemmArgs>(e, k_gemv<float>, grid, block, 0, a) : launch<GemmArgs>(e, k_gemv<__nv_bfloat16>, grid, block, 0, a);
+    return f32 ? launch<GemmArgs>(e, k_gemv_ext<float, EXT>, grid, block, 0, a) : launch<GemmArgs>(e, k_gemv_ext<__nv_bfloat16, EXT>, grid, block, 0, a);
+}
+
 // one matrix product; maxM = the most rows any group can have.  wf32: the weights are fp32 whatever the engine's mode (router).
 // active: how many of the groups can have rows at all (routed products: tokens x top); the matrix-vector grid is sized for those
 int gemm(LayeredEngine *e, GemmArgs a, uint32_t groups, uint32_t maxM, bool wf32 = false, uint32_t active = 0) {
@@ -900,19 +931,15 @@ int gemm(LayeredEngine *e, GemmArgs a, uint32_t groups, uint32_t maxM, bool wf32
     const bool f32 = e->f32 || wf32;
     if (maxM <= kGemvMaxM) {
         a.round_a = f32 ? 0u : 1u;
-        const uint32_t gx = gemv_blocks(e, a.N, active ? std::min(active, groups) : groups);
-        if (a.g_act && active) groups = std::min(active, groups);          // only the groups with rows are launched
-        if (a.epi == EPI_CONV_RANGES)
-            return f32 ? launch<GemmArgs>(e, k_gemv_ext<float, 1>, dim3(gx, groups), dim3(256), 0, a) : launch<GemmArgs>(e, k_gemv_ext<__nv_bfloat16, 1>, dim3(gx, groups), dim3(256), 0, a);
-        if (a.res_x && a.a_parts <= 1)
-            return f32 ? launch<GemmArgs>(e, k_gemv_ext<float, 5>, dim3(gx, groups), dim3(256), 0, a) : launch<GemmArgs>(e, k_gemv_ext<__nv_bfloat16, 5>, dim3(gx, groups), dim3(256), 0, a);
-        if (a.a_parts > 1)
-            return f32 ? launch<GemmArgs>(e, k_gemv_ext<float, 4>, dim3(gx, groups), dim3(256), 0, a) : launch<GemmArgs>(e, k_gemv_ext<__nv_bfloat16, 4>, dim3(gx, groups), dim3(256), 0, a);
-        if (a.glu)
-            return f32 ? launch<GemmArgs>(e, k_gemv_ext<float, 3>, dim3(gx, groups), dim3(256), 0, a) : launch<GemmArgs>(e, k_gemv_ext<__nv_bfloat16, 3>, dim3(gx, groups), dim3(256), 0, a);
-        if (a.a_poly)
-            return f32 ? launch<GemmArgs>(e, k_gemv_ext<float, 2>, dim3(gx, groups), dim3(256), 0, a) : launch<GemmArgs>(e, k_gemv_ext<__nv_bfloat16, 2>, dim3(gx, groups), dim3(256), 0, a);
-        return f32 ? launch<GemmArgs>(e, k_gemv<float>, dim3(gx, groups), dim3(256), 0, a) : launch<GemmArgs>(e, k_gemv<__nv_bfloat16>, dim3(gx, groups), dim3(256), 0, a);
+        const uint32_t live = active ? std::min(active, groups) : groups;
+        if (a.g_act && active) groups = live;          // only the groups with rows are launched
+        const bool one = maxM == 1 && one_fits(a, f32);
+        if (a.epi == EPI_CONV_RANGES) return gemv_launch<1>(e, a, groups, live, one, f32);
+        if (a.res_x && a.a_parts <= 1) return gemv_launch<5>(e, a, groups, live, one, f32);
+        if (a.a_parts > 1) return gemv_launch<4>(e, a, groups, live, one, f32);
+        if (a.glu) return gemv_launch<3>(e, a, groups, live, one, f32);
+        if (a.a_poly) return gemv_launch<2>(e, a, groups, live, one, f32);
+        return gemv_launch<0>(e, a, groups, live, one, f32);
     }
     if (a.glu) return fail(NB200_EINVAL, "the gated-pair product is a matrix-vector instance (portions of at most %u tokens)", kGemvMaxM);
     const uint32_t rows = a.g_off && active ? active : a.M;
@@ -984,7 +1011,10 @@ int mix_rglru(LayeredEngine *e, const Layer &L, const Run &run, const Ctx &cx) {
         if ((r = gemm(e, yx, 1, T))) return r;
         GatesScanArgs gs{e->b_u, L.gates.p, L.gates_b, e->b_yx, 2 * C, L.lam, st + run.st_S, e->b_sy, T, C, bs, kRglruDecay, e->f32 ? 0u : 1u};
         const dim3 grid((C + 7u) / 8u), block(256);
-        if ((r = e->f32 ? launch<GatesScanArgs>(e, k_rglru_gates_scan<float>, grid, block, 0, gs) : launch<GatesScanArgs>(e, k_rglru_gates_scan<__nv_bfloat16>, grid, block, 0, gs))) return r;
+        const uint32_t vn = e->f32 ? 4u : 8u;
+        if (T == 1 && bs % vn == 0 && bs <= 64u * vn && (reinterpret_cast<uintptr_t>(L.gates.p) & 15u) == 0) {
+            if ((r = e->f32 ? launch<GatesScanArgs>(e, k_rglru_gates_one<float>, grid, block, 0, gs) : launch<GatesScanArgs>(e, k_rglru_gates_one<__nv_bfloat16>, grid, block, 0, gs))) return r;
+        } else if ((r = e->f32 ? launch<GatesScanArgs>(e, k_rglru_gates_scan<float>, grid, block, 0, gs) : launch<GatesScanArgs>(e, k_rglru_gates_scan<__nv_bfloat16>, grid, block, 0, gs))) return r;
     } else {
         if ((r = gemm(e, plain(e->hm, E, L.yx, e->b_yx, 2 * C, T, L.yx_b, EPI_GELU_SPLIT, C), 1, T))) return r;
         ConvArgs ca{e->b_yx + C, 2 * C, L.conv, L.conv_b, st + run.st_conv, e->b_u, T, C, L.taps};
@@ -1030,7 +1060,10 @@ int mix_latent_attn(LayeredEngine *e, const Layer &L, const Run &run, const Ctx 
             GemvLatentArgs ga{plain(e->b_z, QR + R, L.uq, e->b_q, H * L.dim, T), na, T};
             ga.g.a_norm_w = L.dq_norm; ga.g.a_eps = e->eps; ga.g.round_a = e->f32 ? 0u : 1u;
             const dim3 grid(gemv_blocks(e, ga.g.N, 1)), block(256);
-            if ((r = e->f32 ? launch<GemvLatentArgs>(e, k_gemv_latent<float>, grid, block, 0, ga) : launch<GemvLatentArgs>(e, k_gemv_latent<__nv_bfloat16>, grid, block, 0, ga))) return r;
+            if (T == 1 && one_fits(ga.g, e->f32)) {
+                const dim3 grid1((e->f32 ? one_blocks<float>(e, &ga.g, 1) : one_blocks<__nv_bfloat16>(e, &ga.g, 1)) + 1u), block1(kOneThreads);
+                if ((r = e->f32 ? launch<GemvLatentArgs>(e, k_gemv_one_latent<float>, grid1, block1, one_smem<float>(QR), ga) : launch<GemvLatentArgs>(e, k_gemv_one_latent<__nv_bfloat16>, grid1, block1, one_smem<__nv_bfloat16>(QR), ga))) return r;
+            } else if ((r = e->f32 ? launch<GemvLatentArgs>(e, k_gemv_latent<float>, grid, block, 0, ga) : launch<GemvLatentArgs>(e, k_gemv_latent<__nv_bfloat16>, grid, block, 0, ga))) return r;
         } else {
             if ((r = launch<LatentNormArgs>(e, k_latent_norm, dim3(T), dim3(128), 0, na))) return r;
             if ((r = gemm(e, plain(e->b_cq, QR, L.uq, e->b_q, H * L.dim, T), 1, T))) return r;
@@ -1047,7 +1080,10 @@ int mix_latent_attn(LayeredEngine *e, const Layer &L, const Run &run, const Ctx 
             GemvLatentRopeArgs ga{g, ra};
             ga.g.round_a = e->f32 ? 0u : 1u;
             const dim3 grid(gemv_blocks(e, g.N, H), H), block(256);
-            if ((r = e->f32 ? launch<GemvLatentRopeArgs>(e, k_gemv_latent_rope<float>, grid, block, 0, ga) : launch<GemvLatentRopeArgs>(e, k_gemv_latent_rope<__nv_bfloat16>, grid, block, 0, ga))) return r;
+            if (T == 1 && one_fits(ga.g, e->f32)) {
+                const dim3 grid1(e->f32 ? one_blocks<float>(e, &ga.g, H) : one_blocks<__nv_bfloat16>(e, &ga.g, H), H + 1u), block1(kOneThreads);
+                if ((r = e->f32 ? launch<GemvLatentRopeArgs>(e, k_gemv_one_latent_rope<float>, grid1, block1, one_smem<float>(g.K), ga) : launch<GemvLatentRopeArgs>(e, k_gemv_one_latent_rope<__nv_bfloat16>, grid1, block1, one_smem<__nv_bfloat16>(g.K), ga))) return r;
+            } else if ((r = e->f32 ? launch<GemvLatentRopeArgs>(e, k_gemv_latent_rope<float>, grid, block, 0, ga) : launch<GemvLatentRopeArgs>(e, k_gemv_latent_rope<__nv_bfloat16>, grid, block, 0, ga))) return r;
         } else if ((r = launch<LatentRopeArgs>(e, k_latent_rope, dim3(T), dim3(128), 0, ra)) || (!up && (r = gemm(e, g, H, T)))) return r;
     }
     if (up) {
@@ -1738,7 +1774,10 @@ int run_layers(LayeredEngine *e, uint32_t slot, uint32_t T, uint32_t pos0, const
         if (run.add_embed) { k_add<<<ew_grid((size_t)T * E), 256, 0, e->stream>>>(e->x, e->x0, (size_t)T * E); CK(cudaGetLastError()); e->launches++; }
         {
             NormShiftArgs a{e->x, L.norm1, L.has_mlp ? L.norm2 : nullptr, L.shift, st + run.st_prev, e->hm, L.has_mlp ? e->h2 : nullptr, T, E, e->eps};
-            if ((r = launch<NormShiftArgs>(e, k_norm_shift, dim3(T > 1 ? T - 1 : 1), dim3(256), 0, a))) return r;
+            auto at16 = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
+            if (T == 1 && E % 4u == 0 && E <= 16u * kOneThreads && at16(a.mu) && at16(a.state) && at16(a.hm) && at16(a.h2) && at16(a.x)) {
+                if ((r = launch<NormShiftArgs>(e, k_norm_shift_one, dim3(1), dim3(kOneThreads), 0, a))) return r;
+            } else if ((r = launch<NormShiftArgs>(e, k_norm_shift, dim3(T > 1 ? T - 1 : 1), dim3(256), 0, a))) return r;
             if (L.has_mlp && e->branch_streams) CK(cudaEventRecord(e->ev_fork, e->stream));
         }
         if ((r = mix(e, L, run, cx))) return r;

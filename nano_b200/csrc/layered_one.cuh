@@ -1,0 +1,371 @@
+// layered_one.cuh -- the matrix-vector products of a single token (the captured decode step), in the argument block of layered_common.cuh.
+//
+// What bounds a step is the chain of its launches, and of a link the latency of what it does after the kernel before it has finished (an empty link of this
+// chain takes 0.5 us, one load and store 1.0).  So everything that does not depend on that kernel happens before the wait: a warp's first weight row is in
+// registers by then, constants of the epilogue too.  After it the block brings the activation row into shared memory ONCE, normed and rounded there, with a
+// single trip to L2, and the epilogue's operands travel at the same time; what is left is the row's dot from registers and shared memory.
+// k_gemv, which serves up to four rows and any alignment, reads the row in every warp, converts it there, and its epilogue starts a trip of its own.
+// A chain of 1024 x 1024 products from HBM, us a link: k_gemv 4.5, weights in registers 2.9, this 2.1.
+#pragma once
+#include "layered_kernels.cuh"
+#include "layered_mixers3.cuh"
+
+namespace nb {
+namespace lm {
+
+constexpr uint32_t kOneThreads = 256, kOneWarps = kOneThreads / 32;
+constexpr uint32_t kOneMaxK = 11264;          // the row in shared memory (fp32) and the static part stay below 48 KB
+template <typename WT> constexpr __host__ __device__ uint32_t one_step() { return 512u / sizeof(WT); }          // columns a warp covers with one 16-byte load a lane
+template <typename WT> inline uint32_t one_smem(uint32_t K) { return (K + one_step<WT>() - 1u) / one_step<WT>() * one_step<WT>() * 4u; }
+
+// a load that stays in front of the wait (the compiler may move an ordinary read-only load behind it, to where its value is used)
+__device__ __forceinline__ uint4 load_now(const void *p) {
+    uint4 v;
+    asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ float load_now_f(const float *p) {
+    float v;
+    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+    return v;
+}
+// where 4-column chunk c of the activation row lies in shared memory: a lane of the dot reads the 8 columns of its 16 bytes of bf16 weights as two loads,
+// each of them over 32 neighbouring chunks
+template <typename WT> __device__ __forceinline__ uint32_t one_place(uint32_t c) {
+    return sizeof(WT) == 2 ? (c & ~63u) + ((c & 1u) << 5) + ((c & 63u) >> 1) : c;
+}
+template <typename WT> __device__ __forceinline__ void one_fma(const uint4 &w, const float4 *x, uint32_t step, uint32_t lane, float &a0, float &a1) {
+    if (sizeof(WT) == 2) {
+        const float4 p = x[step * 64u + lane], q = x[step * 64u + 32u + lane];
+        a0 = fmaf(__uint_as_float(w.x << 16), p.x, a0); a1 = fmaf(__uint_as_float(w.x & 0xffff0000u), p.y, a1);
+        a0 = fmaf(__uint_as_float(w.y << 16), p.z, a0); a1 = fmaf(__uint_as_float(w.y & 0xffff0000u), p.w, a1);
+        a0 = fmaf(__uint_as_float(w.z << 16), q.x, a0); a1 = fmaf(__uint_as_float(w.z & 0xffff0000u), q.y, a1);
+        a0 = fmaf(__uint_as_float(w.w << 16), q.z, a0); a1 = fmaf(__uint_as_float(w.w & 0xffff0000u), q.w, a1);
+    } else {
+        const float4 p = x[step * 32u + lane];
+        a0 = fmaf(__uint_as_float(w.x), p.x, a0); a1 = fmaf(__uint_as_float(w.y), p.y, a1);
+        a0 = fmaf(__uint_as_float(w.z), p.z, a0); a1 = fmaf(__uint_as_float(w.w), p.w, a1);
+    }
+}
+__device__ __forceinline__ float4 round4(float4 v) { return make_float4(round_bf16(v.x), round_bf16(v.y), round_bf16(v.z), round_bf16(v.w)); }
+__device__ __forceinline__ float sum_sq4(float4 v, float s) { return fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, s)))); }
+
+// The activation row, as the product uses it, into shared memory (chunks past K zero).  Ends with a barrier.
+template <typename WT, int EXT>
+__device__ __forceinline__ void one_stage(const GemmArgs &a, const float *row, float4 *x, float *red) {
+    const uint32_t K4 = a.K / 4u, P4 = (a.K + one_step<WT>() - 1u) / one_step<WT>() * one_step<WT>() / 4u;
+    const float4 *src = reinterpret_cast<const float4 *>(row), *nw = reinterpret_cast<const float4 *>(a.a_norm_w);
+    const bool poly = EXT == 2 && a.a_poly, raw = nw || poly;
+    float s2 = 0.0f, s4 = 0.0f, s6 = 0.0f;
+#pragma unroll 4
+    for (uint32_t c = threadIdx.x; c < P4; c += kOneThreads) {
+        float4 v = make_float4(0, 0, 0, 0);
+        if (c < K4) v = src[c];
+        if (EXT != 4) s2 = sum_sq4(v, s2);
+        if (EXT == 2) {
+            const float q[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int j = 0; j < 4; j++) { const float v2 = q[j] * q[j], v3 = v2 * q[j]; s4 = fmaf(v2, v2, s4); s6 = fmaf(v3, v3, s6); }
+        }
+        x[one_place<WT>(c)] = !raw && a.round_a ? round4(v) : v;
+    }
+    if (raw) {
+        float sc = 1.0f;
+        PolyRow pc{0.0f, 0.0f, 0.0f, 0.0f};
+        __shared__ float gsc[EXT == 4 ? 32 : 1];
+        const uint32_t plen = EXT == 4 ? a.K / a.a_parts : 1u;
+        if (EXT == 4) {          // a warp per part: the part's root mean square
+            __syncthreads();
+            const uint32_t lane = threadIdx.x & 31u;
+            for (uint32_t p = threadIdx.x >> 5; p < a.a_parts; p += kOneWarps) {
+                float s = 0.0f;
+                for (uint32_t c = p * plen / 4u + lane; c < (p + 1u) * plen / 4u; c += 32u) s = sum_sq4(x[one_place<WT>(c)], s);
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+                if (lane == 0) gsc[p] = 1.0f / sqrtf(s / (float)plen + a.a_eps);
+            }
+            __syncthreads();
+        } else {
+            s2 = block_sum(s2, red);
+            if (EXT == 2 && poly) {
+                s4 = block_sum(s4, red); s6 = block_sum(s6, red);
+                pc.r1 = a.a_poly[0] / sqrtf(s2 / (float)a.K + a.a_eps); pc.r2 = a.a_poly[1] / sqrtf(s4 / (float)a.K + a.a_eps);
+                pc.r3 = a.a_poly[2] / sqrtf(s6 / (float)a.K + a.a_eps); pc.e = a.a_poly[3];
+            } else sc = 1.0f / sqrtf(s2 / (float)a.K + a.a_eps);
+        }
+        for (uint32_t c = threadIdx.x; c < K4; c += kOneThreads) {          // a thread's own chunks
+            float4 v = x[one_place<WT>(c)];
+            if (nw) {
+                const float si = EXT == 4 ? gsc[c * 4u / plen] : sc;
+                const float4 g = __ldg(nw + c);
+                v.x = v.x * si * g.x; v.y = v.y * si * g.y; v.z = v.z * si * g.z; v.w = v.w * si * g.w;
+            }
+            if (EXT == 2 && poly) { v.x = poly_of(v.x, pc); v.y = poly_of(v.y, pc); v.z = poly_of(v.z, pc); v.w = poly_of(v.w, pc); }
+            x[one_place<WT>(c)] = a.round_a ? round4(v) : v;
+        }
+    }
+    __syncthreads();
+}
+
+// what a column's epilogue reads from memory, asked for long before it is needed (tap, tail: lane j holds those of tap j)
+struct OneEpi { float bias, mul, tap, tail, x, pw, pb, nw, nb; };
+
+// Block bx of nbx, place gy in the list of groups; a group has one row.  The instances (EXT) are k_gemv's.
+template <typename WT, int EXT>
+__device__ __forceinline__ void gemv_one(const GemmArgs &a, uint32_t bx, uint32_t nbx, uint32_t gy) {
+    constexpr uint32_t VN = WVec<WT>::N, STEP = one_step<WT>(), NW = EXT == 3 ? 2u : 1u, PRE = EXT == 3 ? 4u : 8u;
+    extern __shared__ float4 one_x[];
+    __shared__ float red[32];
+    __shared__ float part_s[2][NW][kOneWarps];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, steps = (a.K + STEP - 1u) / STEP;
+    // a row is shared by 2^a.one_split warps, each with its share of the steps; a block has kOneWarps / that many rows at a time
+    const uint32_t split = a.one_split, part = warp & ((1u << split) - 1u), rpb = kOneWarps >> split, share = (steps + (1u << split) - 1u) >> split;
+    const uint32_t s_lo = min(steps, part * share), s_hi = min(steps, s_lo + share), nrows = nbx * rpb;
+    const WT *W = static_cast<const WT *>(a.W);
+    const bool fixed = !a.g_off;
+    const uint32_t n0 = bx * rpb + (warp >> split);
+    uint32_t n = n0;
+    uint4 w[NW][PRE];
+    auto fetch = [&](uint32_t row, uint32_t s0) {
+#pragma unroll
+        for (uint32_t h = 0; h < NW; h++)
+#pragma unroll
+            for (uint32_t i = 0; i < PRE; i++) {
+                const uint32_t k = (s0 + i) * STEP + lane * VN;
+                w[h][i] = make_uint4(0, 0, 0, 0);
+                if (row < a.N && k < a.K) w[h][i] = load_now(W + (size_t)(h * a.N + row) * a.ldw + k);
+            }
+    };
+    if (fixed) {
+        W += (uint64_t)gy * a.w_gstride;
+        fetch(n, s_lo);
+        if (share > PRE || n + nrows < a.N) prefetch_weight_rows(W, sizeof(WT), a.ldw, a.K, a.N, n, nrows, 2u);          // the rest of the first row, the second
+        if (a.a_norm_w) for (uint32_t k = threadIdx.x * 32u; k < a.K; k += kOneThreads * 32u) asm volatile("prefetch.global.L1 [%0];" ::"l"(a.a_norm_w + k));
+    }
+    // arguments that are read after the wait: a launch's arguments lie in memory that no cache near the SM holds yet
+    uint32_t group = gy, r0 = 0;
+    const float *bias = a.bias, *row = a.A;
+    float *C = a.C;
+    auto place = [&]() {          // of the group
+        if (bias) bias += (size_t)group * a.b_gstride;
+        if (a.a_gmod > 1u) row += (size_t)(group % a.a_gmod) * a.a_gcols;
+        C += (size_t)group * a.c_gcols;
+    };
+    OneEpi e{};
+    if (fixed) {
+        place();
+        if (bias && n < a.N) e.bias = load_now_f(bias + n);
+    }
+    pdl_wait();
+    if (!fixed) {
+        group = a.g_act ? a.g_act[gy] : gy;
+        if (group == 0xffffffffu) return;
+        r0 = a.g_off[group];
+        if (a.g_off[group + 1u] == r0) return;
+        W += (uint64_t)group * a.w_gstride;
+        fetch(n, s_lo);
+        place();
+        if (bias && n < a.N) e.bias = __ldg(bias + n);
+        C += (size_t)r0 * a.ldc;
+        row += (size_t)(a.a_rows ? a.a_rows[r0] : r0) * a.lda;
+    } else if (a.a_rows) row += (size_t)a.a_rows[0] * a.lda;
+    const uint32_t c0 = group * a.c_gcols;
+    // the convolution that column n is a channel of, if any
+    auto conv_of = [&](uint32_t col, GemmArgs::ConvRange &r) -> bool {
+        if (EXT == 0 && a.epi == EPI_GELU_CONV && col >= a.split) { r = GemmArgs::ConvRange{a.split, a.N, a.cv_taps, a.cv_bias, a.cv_state, a.cv_out, a.cv_K, 0u}; return true; }
+        if (EXT == 1 && a.epi == EPI_CONV_RANGES) {
+            if (col >= a.cr[0].n0 && col < a.cr[0].n1) { r = a.cr[0]; return true; }
+            if (col >= a.cr[1].n0 && col < a.cr[1].n1) { r = a.cr[1]; return true; }
+        }
+        return false;
+    };
+    auto early = [&](uint32_t col) {
+        if (col >= a.N) return;
+        if (col != n0 && bias) e.bias = __ldg(bias + col);
+        if (a.mul) e.mul = a.mul[(size_t)r0 * a.ldm + c0 + col];
+        GemmArgs::ConvRange r;
+        if ((EXT == 0 || EXT == 1) && conv_of(col, r)) {
+            const uint32_t c = col - r.n0, C = r.n1 - r.n0;
+            if (lane < r.K) e.tap = __ldg(r.taps + (size_t)c * r.K + lane);
+            if (lane + 1u < r.K) e.tail = r.state[(size_t)lane * C + c];
+            e.pb = r.bias ? __ldg(r.bias + c) : 0.0f;
+        }
+        if ((EXT == 4 || EXT == 5) && a.res_x) {
+            e.x = a.res_x[(size_t)r0 * a.N + col]; e.pw = __ldg(a.res_pw + col); e.pb = __ldg(a.res_pb + col);
+            if (a.res_out) { e.nw = __ldg(a.res_nw + col); e.nb = __ldg(a.res_nb + col); }
+        }
+    };
+    if (!part) early(n);
+    const float scale = EXT == 3 && a.row_scale ? a.row_scale[r0] : 1.0f;
+    one_stage<WT, EXT>(a, row, one_x, red);
+
+    for (uint32_t base = bx * rpb, turn = 0; base < a.N; base += nrows, n += nrows, turn ^= 1u) {          // the same turns for all of the block's warps
+        float acc[NW][2];
+#pragma unroll
+        for (uint32_t h = 0; h < NW; h++) acc[h][0] = acc[h][1] = 0.0f;
+        for (uint32_t s0 = s_lo;;) {
+#pragma unroll
+            for (uint32_t i = 0; i < PRE; i++)
+                if (s0 + i < s_hi) {
+#pragma unroll
+                    for (uint32_t h = 0; h < NW; h++) one_fma<WT>(w[h][i], one_x, s0 + i, lane, acc[h][0], acc[h][1]);
+                }
+            s0 += PRE;
+            if (s0 >= s_hi) break;
+            fetch(n, s0);
+        }
+        const OneEpi now = e;
+        if (n + nrows < a.N) { fetch(n + nrows, s_lo); if (!part) early(n + nrows); }          // on their way during the sum and the epilogue
+        float v = acc[0][0] + acc[0][1], up = NW == 2 ? acc[NW - 1u][0] + acc[NW - 1u][1] : 0.0f;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (NW == 2) up += __shfl_xor_sync(0xffffffffu, up, o);
+        }
+        if (split) {
+            if (lane == 0) { part_s[turn][0][warp] = v; if (NW == 2) part_s[turn][NW - 1u][warp] = up; }
+            __syncthreads();
+            if (part) continue;
+            for (uint32_t p = 1; p < 1u << split; p++) { v += part_s[turn][0][warp + p]; if (NW == 2) up += part_s[turn][NW - 1u][warp + p]; }
+        }
+        if (n >= a.N) continue;
+        float *dst = C + n;
+        GemmArgs::ConvRange r;
+        if ((EXT == 0 || EXT == 1) && conv_of(n, r)) {          // one new input: lane j holds input j of the window, the last one is new
+            const float in = lane + 1u == r.K ? (EXT == 0 ? v + now.bias : v) : now.tail;
+            float s = now.pb;
+            for (uint32_t j = 0; j < r.K; j++) s = fmaf(__shfl_sync(0xffffffffu, now.tap, j), __shfl_sync(0xffffffffu, in, j), s);
+            const float next = __shfl_down_sync(0xffffffffu, in, 1);
+            const uint32_t c = n - r.n0, C = r.n1 - r.n0;
+            if (lane + 1u < r.K) r.state[(size_t)lane * C + c] = next;
+            if (r.act) s = s / (1.0f + expf(-s));
+            if (lane == 0) r.out[(size_t)r0 * C + c] = s;
+            continue;
+        }
+        if (lane != 0) continue;
+        if (EXT == 3) {          // the gated pair
+            const float g = v * scale, u = up * scale;
+            store_c(a, dst, (a.glu == 3u ? clamped_glu(g, u, a.glu_limit) : (a.glu == 2u ? g / (1.0f + expf(-g)) : gelu_tanh(g)) * u));
+            continue;
+        }
+        v = epilogue(v + now.bias, a, nullptr, n);
+        if ((EXT == 4 || EXT == 5) && a.res_x) {
+            const size_t at = (size_t)r0 * a.N + n;
+            const float xv = now.x + fmaf(tanhf(a.res_pa * v), now.pw, now.pb);
+            a.res_x[at] = xv;
+            if (a.res_keep) a.res_keep[at] = xv;
+            if (a.res_out) a.res_out[at] = fmaf(tanhf(a.res_na * xv), now.nw, now.nb);
+        } else store_c(a, dst, a.mul ? v * now.mul : v);
+    }
+}
+
+template <typename WT, int EXT>
+__global__ void __launch_bounds__(kOneThreads, 4) k_gemv_one(const GemmArgs a) {
+    pdl_launch_next();
+    gemv_one<WT, EXT>(a, blockIdx.x, gridDim.x, blockIdx.y);
+}
+// the products that also norm (and turn) the token's latent into the cache: one more block does that beside them
+template <typename WT>
+__global__ void __launch_bounds__(kOneThreads, 4) k_gemv_one_latent(const GemvLatentArgs a) {
+    pdl_launch_next();
+    if (blockIdx.x + 1u == gridDim.x) {
+        __shared__ float red[32];
+        pdl_wait();
+        latent_kv_row(a.n, 0, red);
+        return;
+    }
+    gemv_one<WT, 0>(a.g, blockIdx.x, gridDim.x - 1u, 0u);
+}
+template <typename WT>
+__global__ void __launch_bounds__(kOneThreads, 4) k_gemv_one_latent_rope(const GemvLatentRopeArgs a) {
+    pdl_launch_next();
+    if (blockIdx.y + 1u == gridDim.y) {
+        __shared__ float red[32];
+        pdl_wait();
+        if (blockIdx.x == 0) latent_rope_row(a.n, 0, red);
+        return;
+    }
+    gemv_one<WT, 0>(a.g, blockIdx.x, gridDim.x, blockIdx.y);
+}
+
+// k_rglru_gates_scan for one token: a warp per channel, both gate rows and the channel's constants in registers before the wait (blocks of at most
+// 2 steps of columns, a multiple of a 16-byte load)
+template <typename WT>
+__global__ void __launch_bounds__(kOneThreads) k_rglru_gates_one(const GatesScanArgs a) {
+    constexpr uint32_t VN = WVec<WT>::N, STEP = one_step<WT>();
+    pdl_launch_next();
+    const uint32_t lane = threadIdx.x & 31u, c = blockIdx.x * kOneWarps + (threadIdx.x >> 5);
+    if (c >= a.C) return;
+    const WT *wr = static_cast<const WT *>(a.W) + (size_t)c * a.bs, *wi = static_cast<const WT *>(a.W) + (size_t)(a.C + c) * a.bs;
+    float r[2][VN], g[2][VN];
+#pragma unroll
+    for (uint32_t i = 0; i < 2u; i++) {
+        const uint32_t k = i * STEP + lane * VN;
+        if (k < a.bs) { WVec<WT>::load(wr + k, r[i]); WVec<WT>::load(wi + k, g[i]); }
+        else
+#pragma unroll
+            for (uint32_t j = 0; j < VN; j++) r[i][j] = g[i][j] = 0.0f;
+    }
+    const float sp = softplusf_(__ldg(a.lam + c)), br = __ldg(a.bias + c), bi = __ldg(a.bias + a.C + c);
+    pdl_wait();
+    const float *u = a.u + (size_t)(c / a.bs) * a.bs;
+    const float S0 = a.S[c], uc = a.u[c], y = a.y[c];
+    float sr = 0.0f, si = 0.0f;
+#pragma unroll
+    for (uint32_t i = 0; i < 2u; i++) {
+        const uint32_t k = i * STEP + lane * VN;
+        if (k < a.bs) {
+#pragma unroll
+            for (uint32_t j = 0; j < VN; j += 4u) {
+                float4 x = *reinterpret_cast<const float4 *>(u + k + j);
+                if (a.round_a) x = round4(x);
+                sr = fmaf(r[i][j], x.x, sr); sr = fmaf(r[i][j + 1], x.y, sr); sr = fmaf(r[i][j + 2], x.z, sr); sr = fmaf(r[i][j + 3], x.w, sr);
+                si = fmaf(g[i][j], x.x, si); si = fmaf(g[i][j + 1], x.y, si); si = fmaf(g[i][j + 2], x.z, si); si = fmaf(g[i][j + 3], x.w, si);
+            }
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) { sr += __shfl_xor_sync(0xffffffffu, sr, o); si += __shfl_xor_sync(0xffffffffu, si, o); }
+    if (lane) return;
+    const float gr = sigmoidf_(sr + br), gi = sigmoidf_(si + bi), av = expf(-a.c_decay * gr * sp);
+    const float S = av * S0 + sqrtf(1.0f - av * av) * (gi * uc);
+    a.out[c] = S * y;
+    a.S[c] = S;
+}
+
+// k_norm_shift for one token of at most 4096 columns (a multiple of 4): the row in registers, one trip to memory and one sum
+__global__ void __launch_bounds__(kOneThreads) k_norm_shift_one(const NormShiftArgs a) {
+    pdl_launch_next();
+    __shared__ float red[32];
+    const uint32_t E4 = a.E / 4u;
+    const float4 *x4 = reinterpret_cast<const float4 *>(a.x), *mu4 = reinterpret_cast<const float4 *>(a.mu);
+    float4 *st4 = reinterpret_cast<float4 *>(a.state);
+    float4 x[4], p[4], mu[4];
+#pragma unroll
+    for (uint32_t i = 0; i < 4u; i++) { const uint32_t c = threadIdx.x + i * kOneThreads; mu[i] = make_float4(0, 0, 0, 0); if (mu4 && c < E4) mu[i] = __ldg(mu4 + c); }
+    const float g1 = __ldg(a.g1), g2 = a.g2 ? __ldg(a.g2) : 0.0f;
+    pdl_wait();
+    float s = 0.0f;
+#pragma unroll
+    for (uint32_t i = 0; i < 4u; i++) {
+        const uint32_t c = threadIdx.x + i * kOneThreads;
+        x[i] = p[i] = make_float4(0, 0, 0, 0);
+        if (c < E4) { x[i] = x4[c]; p[i] = st4[c]; }
+    }
+#pragma unroll
+    for (uint32_t i = 0; i < 4u; i++) s = sum_sq4(x[i], s);
+    s = block_sum(s, red);
+    const float rinv = 1.0f / sqrtf(s / (float)a.E + a.eps);
+#pragma unroll
+    for (uint32_t i = 0; i < 4u; i++) {
+        const uint32_t c = threadIdx.x + i * kOneThreads;
+        if (c >= E4) break;
+        const float4 u = make_float4(x[i].x * rinv, x[i].y * rinv, x[i].z * rinv, x[i].w * rinv), n1 = make_float4(u.x * g1, u.y * g1, u.z * g1, u.w * g1);
+        reinterpret_cast<float4 *>(a.hm)[c] = !mu4 ? n1 : make_float4(fmaf(p[i].x - n1.x, mu[i].x, n1.x), fmaf(p[i].y - n1.y, mu[i].y, n1.y), fmaf(p[i].z - n1.z, mu[i].z, n1.z), fmaf(p[i].w - n1.w, mu[i].w, n1.w));
+        if (a.h2) reinterpret_cast<float4 *>(a.h2)[c] = make_float4(u.x * g2, u.y * g2, u.z * g2, u.w * g2);
+        st4[c] = n1;
+    }
+}
+
+}  // namespace lm
+}  // namespace nb
