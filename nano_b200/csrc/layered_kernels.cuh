@@ -457,8 +457,10 @@ __device__ __forceinline__ float block_sum(float v, float *red) {
     __syncthreads();
     if ((threadIdx.x & 31u) == 0) red[threadIdx.x >> 5] = v;
     __syncthreads();
-    float s = 0.0f;
-    for (uint32_t w = 0; w < (blockDim.x >> 5); w++) s += red[w];
+    // the warps' sums over the lanes: a loop over up to 32 of them is a chain of as many additions
+    float s = (threadIdx.x & 31u) < (blockDim.x >> 5) ? red[threadIdx.x & 31u] : 0.0f;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     return s;
 }
 
@@ -470,6 +472,21 @@ __global__ void k_embed(const uint32_t *__restrict__ tokens, const uint32_t *__r
     pdl_enter();
     const uint32_t t = blockIdx.x;
     const WT *src = embed + (size_t)tokens[t + (pos_ptr ? *pos_ptr : 0u)] * E;
+    constexpr uint32_t VN = WVec<WT>::N;
+    if (E % VN == 0 && ((reinterpret_cast<uintptr_t>(embed) | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(x0)) & 15u) == 0) {
+#pragma unroll 2
+        for (uint32_t i = threadIdx.x * VN; i < E; i += blockDim.x * VN) {
+            float v[VN];
+            WVec<WT>::load(src + i, v);
+#pragma unroll
+            for (uint32_t j = 0; j < VN; j += 4u) {
+                const float4 f = make_float4(v[j] * scale, v[j + 1] * scale, v[j + 2] * scale, v[j + 3] * scale);
+                *reinterpret_cast<float4 *>(x + (size_t)t * E + i + j) = f;
+                if (x0) *reinterpret_cast<float4 *>(x0 + (size_t)t * E + i + j) = f;
+            }
+        }
+        return;
+    }
     for (uint32_t i = threadIdx.x; i < E; i += blockDim.x) {
         const float v = wval(src + i) * scale;
         x[(size_t)t * E + i] = v;
@@ -1185,17 +1202,46 @@ __global__ void k_combine(const CombineArgs a) {
 
 // scalar-gain RMS norm of the rows whose logits are asked for: out[i] = x[want[i]] / rms * g
 // (vec 1: the gain is a vector stored around zero, out = x / rms * (1 + g[i]); vec 2: a plain vector, out = x / rms * g[i])
+// Rows of at most 8192 columns (a multiple of 4) stay in registers between the sum and the result, their gains are asked for before the wait: the row of
+// 2048 that ends every step took 10 us as two walks of single loads, now 3.
 __global__ void __launch_bounds__(256) k_final_norm(const float *__restrict__ x, const uint32_t *__restrict__ want, const float *__restrict__ g,
                                                     float *__restrict__ out, uint32_t E, float eps, uint32_t vec) {
-    pdl_enter();
+    pdl_launch_next();
     __shared__ float red[32];
+    auto at16 = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
+    const bool regs = E % 4u == 0 && E <= 8192u && at16(x) && at16(out) && (!vec || at16(g));
+    const float gs = vec ? 0.0f : __ldg(g);
+    if (regs && vec) for (uint32_t i = threadIdx.x * 32u; i < E; i += 8192u) asm volatile("prefetch.global.L1 [%0];" ::"l"(g + i));
+    pdl_wait();
     const float *xt = x + (size_t)want[blockIdx.x] * E;
+    float *o = out + (size_t)blockIdx.x * E;
     float s = 0.0f;
+    if (regs) {
+        float4 v[8];
+#pragma unroll
+        for (uint32_t k = 0; k < 8u; k++) {
+            const uint32_t i = (threadIdx.x + k * 256u) * 4u;
+            v[k] = make_float4(0, 0, 0, 0);
+            if (i < E) v[k] = *reinterpret_cast<const float4 *>(xt + i);
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < 8u; k++) s = fmaf(v[k].x, v[k].x, fmaf(v[k].y, v[k].y, fmaf(v[k].z, v[k].z, fmaf(v[k].w, v[k].w, s))));
+        s = block_sum(s, red);
+        const float rinv = 1.0f / sqrtf(s / (float)E + eps);
+#pragma unroll
+        for (uint32_t k = 0; k < 8u; k++) {
+            const uint32_t i = (threadIdx.x + k * 256u) * 4u;
+            if (i >= E) break;
+            float4 w = make_float4(gs, gs, gs, gs);
+            if (vec) { w = __ldg(reinterpret_cast<const float4 *>(g + i)); if (vec != 2u) { w.x += 1.0f; w.y += 1.0f; w.z += 1.0f; w.w += 1.0f; } }
+            *reinterpret_cast<float4 *>(o + i) = make_float4(v[k].x * rinv * w.x, v[k].y * rinv * w.y, v[k].z * rinv * w.z, v[k].w * rinv * w.w);
+        }
+        return;
+    }
     for (uint32_t i = threadIdx.x; i < E; i += blockDim.x) s = fmaf(xt[i], xt[i], s);
     s = block_sum(s, red);
-    const float rinv = 1.0f / sqrtf(s / (float)E + eps) * 1.0f;
-    const float gv = vec ? 0.0f : *g;
-    for (uint32_t i = threadIdx.x; i < E; i += blockDim.x) out[(size_t)blockIdx.x * E + i] = xt[i] * rinv * (vec ? (vec == 2u ? g[i] : 1.0f + g[i]) : gv);
+    const float rinv = 1.0f / sqrtf(s / (float)E + eps);
+    for (uint32_t i = threadIdx.x; i < E; i += blockDim.x) o[i] = xt[i] * rinv * (vec ? (vec == 2u ? g[i] : 1.0f + g[i]) : gs);
 }
 
 // greedy choice with the repetition penalty of the generation hosts: logits of ids seen before are divided (positive) or multiplied

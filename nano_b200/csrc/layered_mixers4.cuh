@@ -31,14 +31,27 @@ __device__ __forceinline__ float2 block_sum2(float2 v, float2 *red) {
     __syncthreads();
     if ((threadIdx.x & 31u) == 0) red[threadIdx.x >> 5] = v;
     __syncthreads();
-    float2 s = make_float2(0.0f, 0.0f);
-    for (uint32_t w = 0; w < (blockDim.x >> 5); w++) { s.x += red[w].x; s.y += red[w].y; }
+    float2 s = (threadIdx.x & 31u) < (blockDim.x >> 5) ? red[threadIdx.x & 31u] : make_float2(0.0f, 0.0f);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) { s.x += __shfl_xor_sync(0xffffffffu, s.x, o); s.y += __shfl_xor_sync(0xffffffffu, s.y, o); }
     return s;
 }
 template <int NV>
 __global__ void __launch_bounds__(1024) k_post_norm(const PostNormArgs a) {
-    pdl_enter();
+    pdl_launch_next();
     __shared__ float2 red[32];
+    // the gains are nobody's result: short portions have them in registers before the wait
+    constexpr bool kGains = NV > 0 && NV <= 2;
+    float w[kGains ? NV : 1], w1[kGains ? NV : 1], w2[kGains ? NV : 1];
+    if constexpr (kGains) {
+#pragma unroll
+        for (int k = 0; k < NV; k++) {
+            const uint32_t i = threadIdx.x + k * blockDim.x;
+            const bool ok = i < a.E;
+            w[k] = ok ? __ldg(a.w + i) : 0.0f; w1[k] = ok && a.d2 ? __ldg(a.w1 + i) : 0.0f; w2[k] = ok && a.d2 ? __ldg(a.w2 + i) : 0.0f;
+        }
+    }
+    pdl_wait();
     const size_t row = (size_t)blockIdx.x * a.E;
     const float *d = a.d + row, *d2 = a.d2 ? a.d2 + row : nullptr;
     float *x = a.x + row;
@@ -64,7 +77,8 @@ __global__ void __launch_bounds__(1024) k_post_norm(const PostNormArgs a) {
 #pragma unroll
             for (int k = 0; k < NV; k++) {
                 const uint32_t i = threadIdx.x + k * blockDim.x;
-                y[k] = i < a.E ? a.mix * (y[k] * ra * a.w1[i] + z[k] * rb * a.w2[i]) : 0.0f;
+                if constexpr (kGains) y[k] = i < a.E ? a.mix * (y[k] * ra * w1[k] + z[k] * rb * w2[k]) : 0.0f;
+                else y[k] = i < a.E ? a.mix * (y[k] * ra * a.w1[i] + z[k] * rb * a.w2[i]) : 0.0f;
                 s.x = fmaf(y[k], y[k], s.x);
             }
         } else {
@@ -78,7 +92,9 @@ __global__ void __launch_bounds__(1024) k_post_norm(const PostNormArgs a) {
         for (int k = 0; k < NV; k++) {
             const uint32_t i = threadIdx.x + k * blockDim.x;
             if (i >= a.E) continue;
-            const float v = xv[k] + y[k] * rinv * a.w[i];
+            float wi;
+            if constexpr (kGains) wi = w[k]; else wi = a.w[i];
+            const float v = xv[k] + y[k] * rinv * wi;
             x[i] = v;
             if (a.keep) a.keep[row + i] = v;
         }

@@ -26,8 +26,17 @@ template <int VW> __device__ __forceinline__ void stg_vec(float *p, const float 
 }
 template <int NV, int VW>
 __global__ void __launch_bounds__(1024) k_post_ln(const PostLnArgs a) {
-    pdl_enter();
+    pdl_launch_next();
     __shared__ float red[32];
+    float gain[NV > 0 ? NV : 1][VW];          // nobody's result: in registers before the wait
+    if constexpr (NV > 0) {
+#pragma unroll
+        for (int k = 0; k < NV; k++) {
+            const uint32_t i = (threadIdx.x + k * blockDim.x) * VW;
+            if (i < a.E) lds_vec<VW>(a.w + i, gain[k]);
+        }
+    }
+    pdl_wait();
     const uint32_t t = blockIdx.x;
     const size_t row = (size_t)t * a.E;
     float *x = a.x + row;
@@ -48,9 +57,12 @@ __global__ void __launch_bounds__(1024) k_post_ln(const PostLnArgs a) {
 #pragma unroll
         for (int e = 0; e < VW; e++) u[e] = fmaf(a.alpha, xv[e], u[e]);
     };
-    auto store = [&](uint32_t i, const float (&u)[VW], float rinv) {
+    auto store = [&](uint32_t i, const float (&u)[VW], float rinv, int k) {
         float w[VW];
-        lds_vec<VW>(a.w + i, w);
+        if constexpr (NV > 0) {
+#pragma unroll
+            for (int e = 0; e < VW; e++) w[e] = gain[k][e];
+        } else lds_vec<VW>(a.w + i, w);
 #pragma unroll
         for (int e = 0; e < VW; e++) w[e] *= u[e] * rinv;
         stg_vec<VW>(x + i, w);
@@ -79,9 +91,9 @@ __global__ void __launch_bounds__(1024) k_post_ln(const PostLnArgs a) {
     const float rinv = 1.0f / sqrtf(s / (float)a.E + a.eps);
     if constexpr (NV > 0) {
 #pragma unroll
-        for (int k = 0; k < NV; k++) { const uint32_t i = (threadIdx.x + k * blockDim.x) * VW; if (i < a.E) store(i, u[k], rinv); }
+        for (int k = 0; k < NV; k++) { const uint32_t i = (threadIdx.x + k * blockDim.x) * VW; if (i < a.E) store(i, u[k], rinv, k); }
     } else
-        for (uint32_t i = threadIdx.x * VW; i < a.E; i += blockDim.x * VW) { lds_vec<VW>(x + i, u[0]); store(i, u[0], rinv); }
+        for (uint32_t i = threadIdx.x * VW; i < a.E; i += blockDim.x * VW) { lds_vec<VW>(x + i, u[0]); store(i, u[0], rinv, 0); }
 }
 
 // ------------------------------------------------------------------------------------------------
