@@ -888,6 +888,28 @@ int launch(LayeredEngine *e, void (*k)(const A), dim3 grid, dim3 block, size_t s
     return 0;
 }
 
+// a kernel with the cluster size as a second argument
+int launch_split(LayeredEngine *e, void (*k)(const GemmArgs, const uint32_t), dim3 grid, dim3 block, const GemmArgs &args, uint32_t cluster) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.stream = e->cur;
+    cudaLaunchAttribute attr[2];
+    cfg.attrs = attr;
+    if (e->use_pdl) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = cluster; attr[cfg.numAttrs].val.clusterDim.y = 1; attr[cfg.numAttrs++].val.clusterDim.z = 1;
+    CK(cudaLaunchKernelEx(&cfg, k, args, cluster));
+    e->launches++;
+    return 0;
+}
+// does a product of the 32-bit mode run on k_gemm_f32_async: rows of both operands in whole 16-byte pieces
+bool gemm_f32_fits(const GemmArgs &a) {
+    auto at16 = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
+    return a.K % 4u == 0 && a.lda % 4u == 0 && a.ldw % 4u == 0 && a.a_gcols % 4u == 0 && a.w_gstride % 4u == 0 && at16(a.A) && at16(a.W);
+}
+
 uint32_t gemv_blocks(const LayeredEngine *e, uint32_t N, uint32_t groups) {
     return std::min((N + 7u) / 8u, std::max(1u, (uint32_t)e->num_sms * 8u / groups));
 }
@@ -948,6 +970,12 @@ int gemm(LayeredEngine *e, GemmArgs a, uint32_t groups, uint32_t maxM, bool wf32
         return tc_gemm(&e->tc, a, groups, maxM, rows, a.g_off ? std::max(1u, (active + groups - 1u) / groups) : maxM, e->cur == e->side ? 1u : e->cur == e->side2 ? 2u : 0u, e->cur, e->use_pdl);
     }
     const dim3 grid((a.N + 63u) / 64u, (maxM + 63u) / 64u, groups);
+    if (f32 && gemm_f32_fits(a)) {      // blocks of a cluster share a tile's depth while all of them still find a place at once (two to an SM), 64 columns each at least
+        const uint32_t tiles = grid.x * ((a.g_off && active ? std::max(1u, (active + groups - 1u) / groups) : maxM) + 63u) / 64u * groups;
+        uint32_t split = 1;
+        while (split < 8u && tiles * split * 2u <= 2u * (uint32_t)e->num_sms && a.K >= split * 2u * 64u) split *= 2u;
+        return launch_split(e, k_gemm_f32_async, dim3(grid.x * split, grid.y, groups), dim3(kF32Threads), a, split);
+    }
     return f32 ? launch<GemmArgs>(e, k_gemm_f32<float>, grid, dim3(256), 0, a) : launch<GemmArgs>(e, k_gemm_bf16, grid, dim3(128), 0, a);
 }
 

@@ -2,7 +2,7 @@
 // mixer plus an optional feed-forward, over an fp32 residual stream.  Every mechanism is a kernel (or a GEMM epilogue) of its own
 // with its constants as arguments, so a new design combines them by configuration:
 //
-//   matrix products      k_gemm_f32 (fp32 FMA tiles, the true-32-bit mode), k_gemm_bf16 (mma.sync m16n8k16, bf16 operands, fp32
+//   matrix products      k_gemm_f32_async (fp32 FMA tiles, the true-32-bit mode; k_gemm_f32 for rows that are not whole 16-byte pieces), k_gemm_bf16 (mma.sync m16n8k16, bf16 operands, fp32
 //                        accumulators: prefill of odd sizes; layered_tc.cu has the tcgen05 product of all others), k_gemv (a warp per output row, weights streamed once: decode and portions of <= 4 tokens).
 //                        One argument block serves plain, grouped (block-diagonal gates, per-head absorb / value up-projection) and
 //                        routed (rows gathered per expert, group sizes read on the device) products; bias / gelu_tanh / sigmoid /
@@ -91,6 +91,97 @@ __global__ void __launch_bounds__(256) k_gemm_f32(const GemmArgs a) {
             if (n < a.N) store_c(a, a.C + (size_t)(gv.r0 + r) * a.ldc + gv.c0 + n, gated(a, epilogue(acc[i][j], a, gv.bias, n), gv.r0 + r, gv.c0 + n));
         }
     }
+}
+
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ float ld_cluster(const float *p, uint32_t rank) {      // *p of block `rank` of this cluster
+    uint32_t at = (uint32_t)__cvta_generic_to_shared(p), there; float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(at), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(there) : "memory");
+    return v;
+}
+// fp32 tile product for rows of whole 16-byte pieces (gemm_f32_fits): 64 x 64 tile, 128 threads with an 8 x 4 micro-tile, 16-deep k steps that travel
+// three ahead (cp.async).  A thread reads four k of a row at once, rows 20 floats apart (8 neighbouring rows hit 8 bank groups), so nothing is transposed: 12 shared-memory
+// loads per 128 FMA.  Portions of this mode are short: where the tiles alone would leave SMs idle, a cluster shares a tile's depth, and its blocks add up
+// their parts of the tile from each other's shared memory, a share of the rows each, in the order of the depth.
+// The 203-token portion of two Famudra w1024 layers took 1569 us with k_gemm_f32 for all products (one stage, scalar loads, 64 blocks; 1177 of it theirs), now 714 (489).
+constexpr uint32_t kF32Threads = 128, kF32Pitch = 20, kF32Stages = 3;
+__global__ void __launch_bounds__(kF32Threads, 4) k_gemm_f32_async(const GemmArgs a, const uint32_t split) {
+    pdl_enter();
+    const GroupView gv = group_view(a, blockIdx.z);
+    const uint32_t rank = blockIdx.x % split, m0 = blockIdx.y * 64u, n0 = blockIdx.x / split * 64u;
+    if (m0 >= gv.rows) return;          // the same for a whole cluster
+    __shared__ __align__(16) float st[kF32Stages][128][kF32Pitch];          // rows 0..63 of A, 64..127 of W; then a 64 x 64 part of the tile
+    const uint32_t tid = threadIdx.x, tx = tid & 15u, ty = tid >> 4, c = (tid & 3u) * 4u;
+    const uint32_t nk = (a.K + 15u) / 16u, per = (nk + split - 1u) / split, k_lo = min(nk, rank * per), k_hi = min(nk, k_lo + per);
+    const float *src[4];
+#pragma unroll
+    for (uint32_t h = 0; h < 4u; h++) {          // this thread's rows of a stage: two of A, two of W (null: past the end, zeros)
+        const uint32_t r = (h & 1u) * 32u + (tid >> 2);
+        if (h < 2u) src[h] = m0 + r < gv.rows ? a.A + (size_t)(a.a_rows ? a.a_rows[gv.r0 + m0 + r] : gv.r0 + m0 + r) * a.lda + gv.a0 + c : nullptr;
+        else src[h] = n0 + r < a.N ? static_cast<const float *>(a.W) + gv.w0 + (size_t)(n0 + r) * a.ldw + c : nullptr;
+    }
+    auto fetch = [&](uint32_t k) {
+        if (k < k_hi) {
+#pragma unroll
+            for (uint32_t h = 0; h < 4u; h++) {
+                const bool ok = src[h] && k * 16u + c < a.K;
+                const uint32_t d = (uint32_t)__cvta_generic_to_shared(&st[k % kF32Stages][(h >> 1) * 64u + (h & 1u) * 32u + (tid >> 2)][c]), n = ok ? 16u : 0u;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(ok ? src[h] + k * 16u : a.A), "r"(n) : "memory");
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    float acc[8][4] = {};
+    for (uint32_t k = k_lo; k < k_lo + kF32Stages - 1u; k++) fetch(k);
+    for (uint32_t k = k_lo; k < k_hi; k++) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kF32Stages - 2) : "memory");
+        __syncthreads();          // this stage has landed for every thread, and the one before it is done with
+        fetch(k + kF32Stages - 1u);
+        const float (*s)[kF32Pitch] = st[k % kF32Stages];
+#pragma unroll
+        for (uint32_t q = 0; q < 16u; q += 4u) {
+            float4 b[4];
+#pragma unroll
+            for (uint32_t j = 0; j < 4u; j++) b[j] = *reinterpret_cast<const float4 *>(&s[64u + tx + 16u * j][q]);
+#pragma unroll
+            for (uint32_t i = 0; i < 8u; i++) {
+                const float4 v = *reinterpret_cast<const float4 *>(&s[ty * 8u + i][q]);
+#pragma unroll
+                for (uint32_t j = 0; j < 4u; j++) acc[i][j] = fmaf(v.w, b[j].w, fmaf(v.z, b[j].z, fmaf(v.y, b[j].y, fmaf(v.x, b[j].x, acc[i][j]))));
+            }
+        }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    auto out = [&](uint32_t r, uint32_t n, float v) {
+        if (r < gv.rows && n < a.N) store_c(a, a.C + (size_t)(gv.r0 + r) * a.ldc + gv.c0 + n, gated(a, epilogue(v, a, gv.bias, n), gv.r0 + r, gv.c0 + n));
+    };
+    if (split == 1u) {
+#pragma unroll
+        for (uint32_t i = 0; i < 8u; i++)
+#pragma unroll
+            for (uint32_t j = 0; j < 4u; j++) out(m0 + ty * 8u + i, n0 + tx + 16u * j, acc[i][j]);
+        return;
+    }
+    __syncthreads();
+    float *part = &st[0][0][0];
+#pragma unroll
+    for (uint32_t i = 0; i < 8u; i++)
+#pragma unroll
+        for (uint32_t j = 0; j < 4u; j++) part[(ty * 8u + i) * 64u + tx + 16u * j] = acc[i][j];
+    __syncwarp();
+    cluster_arrive();
+    cluster_wait();
+    const uint32_t share = 4096u / split;
+    for (uint32_t i = rank * share + tid; i < (rank + 1u) * share; i += kF32Threads) {
+        float v = 0.0f;
+        for (uint32_t q = 0; q < split; q++) v += ld_cluster(part + i, q);
+        out(m0 + i / 64u, n0 + i % 64u, v);
+    }
+    __syncwarp();
+    cluster_arrive();          // no block leaves while another reads its part
+    cluster_wait();
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -1072,8 +1163,6 @@ __global__ void __launch_bounds__(256) k_route(const RouteArgs a) {
 // k_route + k_route_place; the global counters are not touched.  act (optional): the experts that have rows, 0xffffffff up to T top places.
 constexpr uint32_t kRouteBlocks = 8, kRouteThreads = 512;
 inline size_t route_small_smem(uint32_t NL) { return ((size_t)2 * kGemvMaxM * NL + (size_t)kGemvMaxM * (NL > kRouteThreads / 32u ? NL : kRouteThreads / 32u)) * 4; }
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void st_cluster(float *p, uint32_t rank, float v) {      // *p of block `rank` of this cluster
     uint32_t at = (uint32_t)__cvta_generic_to_shared(p), there;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(at), "r"(rank));
