@@ -1592,6 +1592,8 @@ int ff_glu_dense(LayeredEngine *e, const Layer &L, uint32_t T) {
 // routing of a short portion: a cluster of blocks shares the router's rows
 int route_small(LayeredEngine *e, const RouteArgs &ra) {
     const uint32_t NL = ra.NE + ra.extra, nb = NL >= 8u ? kRouteBlocks : NL >= 4u ? 4u : NL >= 2u ? 2u : 1u;
+    if (ra.T == 1 && NL <= 32u && ra.top <= 32u && ra.E % 4u == 0 && ((reinterpret_cast<uintptr_t>(ra.router) | reinterpret_cast<uintptr_t>(ra.h)) & 15u) == 0)
+        return launch<RouteArgs>(e, k_route_one, dim3(nb), dim3(kRouteOneThreads), 0, ra, nb);
     return launch<RouteArgs>(e, k_route_small, dim3(nb), dim3(kRouteThreads), route_small_smem(NL), ra, nb);
 }
 

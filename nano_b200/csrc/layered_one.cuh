@@ -110,7 +110,7 @@ __device__ __forceinline__ void one_stage(const GemmArgs &a, const float *row, f
 // what a column's epilogue reads from memory, asked for long before it is needed (tap, tail: lane j holds those of tap j)
 struct OneEpi { float bias, mul, tap, tail, x, pw, pb, nw, nb; };
 
-// Block bx of nbx, place gy in the list of groups; a group has one row.  The instances (EXT) are k_gemv's.
+// Block bx of nbx, place gy in the list of groups; a group has one row, or several of the same token.  The instances (EXT) are k_gemv's.
 template <typename WT, int EXT>
 __device__ __forceinline__ void gemv_one(const GemmArgs &a, uint32_t bx, uint32_t nbx, uint32_t gy) {
     constexpr uint32_t VN = WVec<WT>::N, STEP = one_step<WT>(), NW = EXT == 3 ? 2u : 1u, PRE = EXT == 3 ? 4u : 8u;
@@ -133,7 +133,7 @@ __device__ __forceinline__ void gemv_one(const GemmArgs &a, uint32_t bx, uint32_
             for (uint32_t i = 0; i < PRE; i++) {
                 const uint32_t k = (s0 + i) * STEP + lane * VN;
                 w[h][i] = make_uint4(0, 0, 0, 0);
-                if (row < a.N && k < a.K) w[h][i] = load_now(W + (size_t)(h * a.N + row) * a.ldw + k);
+                if (row < a.N && s0 + i < s_hi && k < a.K) w[h][i] = load_now(W + (size_t)(h * a.N + row) * a.ldw + k);
             }
     };
     if (fixed) {
@@ -143,7 +143,7 @@ __device__ __forceinline__ void gemv_one(const GemmArgs &a, uint32_t bx, uint32_
         if (a.a_norm_w) for (uint32_t k = threadIdx.x * 32u; k < a.K; k += kOneThreads * 32u) asm volatile("prefetch.global.L1 [%0];" ::"l"(a.a_norm_w + k));
     }
     // arguments that are read after the wait: a launch's arguments lie in memory that no cache near the SM holds yet
-    uint32_t group = gy, r0 = 0;
+    uint32_t group = gy, r0 = 0, rows = 1;          // (several rows of one expert hold the same token: choices that tie at -infinity)
     const float *bias = a.bias, *row = a.A;
     float *C = a.C;
     auto place = [&]() {          // of the group
@@ -160,10 +160,11 @@ __device__ __forceinline__ void gemv_one(const GemmArgs &a, uint32_t bx, uint32_
     if (!fixed) {
         group = a.g_act ? a.g_act[gy] : gy;
         if (group == 0xffffffffu) return;
-        r0 = a.g_off[group];
-        if (a.g_off[group + 1u] == r0) return;
         W += (uint64_t)group * a.w_gstride;
         fetch(n, s_lo);
+        r0 = a.g_off[group];
+        rows = a.g_off[group + 1u] - r0;
+        if (rows == 0) return;
         place();
         if (bias && n < a.N) e.bias = __ldg(bias + n);
         C += (size_t)r0 * a.ldc;
@@ -244,8 +245,10 @@ __device__ __forceinline__ void gemv_one(const GemmArgs &a, uint32_t bx, uint32_
         }
         if (lane != 0) continue;
         if (EXT == 3) {          // the gated pair
-            const float g = v * scale, u = up * scale;
-            store_c(a, dst, (a.glu == 3u ? clamped_glu(g, u, a.glu_limit) : (a.glu == 2u ? g / (1.0f + expf(-g)) : gelu_tanh(g)) * u));
+            for (uint32_t i = 0; i < rows; i++) {
+                const float f = i && a.row_scale ? a.row_scale[r0 + i] : scale, g = v * f, u = up * f;
+                store_c(a, dst + (size_t)i * a.ldc, (a.glu == 3u ? clamped_glu(g, u, a.glu_limit) : (a.glu == 2u ? g / (1.0f + expf(-g)) : gelu_tanh(g)) * u));
+            }
             continue;
         }
         v = epilogue(v + now.bias, a, nullptr, n);
@@ -255,7 +258,7 @@ __device__ __forceinline__ void gemv_one(const GemmArgs &a, uint32_t bx, uint32_
             a.res_x[at] = xv;
             if (a.res_keep) a.res_keep[at] = xv;
             if (a.res_out) a.res_out[at] = fmaf(tanhf(a.res_na * xv), now.nw, now.nb);
-        } else store_c(a, dst, a.mul ? v * now.mul : v);
+        } else for (uint32_t i = 0; i < rows; i++) store_c(a, dst + (size_t)i * a.ldc, a.mul ? v * now.mul : v);
     }
 }
 
@@ -364,6 +367,127 @@ __global__ void __launch_bounds__(kOneThreads) k_norm_shift_one(const NormShiftA
         reinterpret_cast<float4 *>(a.hm)[c] = !mu4 ? n1 : make_float4(fmaf(p[i].x - n1.x, mu[i].x, n1.x), fmaf(p[i].y - n1.y, mu[i].y, n1.y), fmaf(p[i].z - n1.z, mu[i].z, n1.z), fmaf(p[i].w - n1.w, mu[i].w, n1.w));
         if (a.h2) reinterpret_cast<float4 *>(a.h2)[c] = make_float4(u.x * g2, u.y * g2, u.z * g2, u.w * g2);
         st4[c] = n1;
+    }
+}
+
+// k_route_small for one token and at most 32 rows of the router: the same choice, weights and places (RouteArgs, route_pick), in registers.  A cluster of blocks
+// shares the logits, with the router's rows in registers before the wait; the first block's first warp then holds an expert per lane, and everything it leaves is written
+// once, by the lane that has it.  (k_route_small keeps the choice in memory and reads it back: 27 us of the chain of a step with eight routed layers, now 6.)
+constexpr uint32_t kRouteOneThreads = 256;
+__global__ void __launch_bounds__(kRouteOneThreads) k_route_one(const RouteArgs a) {
+    pdl_launch_next();
+    cluster_arrive();                          // waited for before the first access to another block's shared memory
+    __shared__ float z_s[32], zp[kRouteOneThreads / 32];
+    constexpr uint32_t NW = kRouteOneThreads / 32, PRE = 8;
+    const uint32_t NL = a.NE + a.extra, rank = blockIdx.x, nb = gridDim.x, nloc = (NL - rank + nb - 1u) / nb, ns = NW / nloc;      // this block's rows: rank, rank + nb, ...
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u, per = ((a.E + ns - 1u) / ns + 3u) & ~3u;
+    const uint32_t k0 = min(a.E, warp % ns * per), k1 = warp < nloc * ns ? min(a.E, k0 + per) : k0;
+    const float *w = a.router + (size_t)(rank + min(warp / ns, nloc - 1u) * nb) * a.E;
+    uint4 wv[PRE];
+#pragma unroll
+    for (uint32_t i = 0; i < PRE; i++) { const uint32_t k = k0 + i * 128u + lane * 4u; wv[i] = make_uint4(0, 0, 0, 0); if (k < k1) wv[i] = load_now(w + k); }
+    pdl_wait();
+    float acc = 0.0f;
+    float4 h[PRE];
+#pragma unroll
+    for (uint32_t i = 0; i < PRE; i++) { const uint32_t k = k0 + i * 128u + lane * 4u; h[i] = make_float4(0, 0, 0, 0); if (k < k1) h[i] = *reinterpret_cast<const float4 *>(a.h + k); }
+#pragma unroll
+    for (uint32_t i = 0; i < PRE; i++)
+        acc = fmaf(h[i].w, __uint_as_float(wv[i].w), fmaf(h[i].z, __uint_as_float(wv[i].z), fmaf(h[i].y, __uint_as_float(wv[i].y), fmaf(h[i].x, __uint_as_float(wv[i].x), acc))));
+    for (uint32_t k = k0 + PRE * 128u + lane * 4u; k < k1; k += 128u) {
+        const float4 v = __ldg(reinterpret_cast<const float4 *>(w + k)), x = *reinterpret_cast<const float4 *>(a.h + k);
+        acc = fmaf(x.w, v.w, fmaf(x.z, v.z, fmaf(x.y, v.y, fmaf(x.x, v.x, acc))));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (lane == 0) zp[warp] = acc;
+    __syncthreads();
+    cluster_wait();                            // every block of the cluster runs
+    if (tid < nloc) {
+        const uint32_t e = rank + tid * nb;
+        float v = 0.0f;
+        for (uint32_t sl = 0; sl < ns; sl++) v += zp[tid * ns + sl];
+        st_cluster(z_s + e, 0u, a.mode == 3u && e < a.NE ? sigmoidf_(v) : v);
+    }
+    __syncwarp();
+    cluster_arrive();
+    cluster_wait();
+    if (rank || warp) return;
+    const bool expert = lane < a.NE;
+    float z = lane < NL ? z_s[lane] : -INFINITY;
+    if (lane >= a.NE && lane < NL) a.extra_out[lane - a.NE] = z;
+    // the largest of `v` over the lanes below n (ties: the lower lane)
+    auto argmax = [&](float v, uint32_t n, float *value) {
+        float best = lane < n ? v : -INFINITY; uint32_t bi = lane < n ? lane : 0xffffffffu;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float ov = __shfl_xor_sync(0xffffffffu, best, o); const uint32_t oi = __shfl_xor_sync(0xffffffffu, bi, o);
+            if (oi != 0xffffffffu && (bi == 0xffffffffu || ov > best || (ov == best && oi < bi))) { best = ov; bi = oi; }
+        }
+        *value = best;
+        return bi;
+    };
+    float zmax = expert ? z : -INFINITY, zden = 0.0f;
+    if (a.mode == 2u) {                        // softmax over ALL experts
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) zmax = fmaxf(zmax, __shfl_xor_sync(0xffffffffu, zmax, o));
+        zden = expert ? expf(z - zmax) : 0.0f;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) zden += __shfl_xor_sync(0xffffffffu, zden, o);
+    }
+    if (a.mode == 3u && a.keep < a.groups) {   // lane g: group g's score; then the experts of the groups that are not kept leave the choice
+        const uint32_t size = a.NE / a.groups, g0 = min(lane, a.groups - 1u) * size;
+        float b1 = -INFINITY, b2 = -INFINITY, v;
+        for (uint32_t i = 0; i < size; i++) { const float x = __shfl_sync(0xffffffffu, z, g0 + i); b2 = fmaxf(b2, fminf(b1, x)); b1 = fmaxf(b1, x); }
+        float zg = size > 1u ? b1 + b2 : b1;
+        for (uint32_t j = 0; j < a.keep; j++) {
+            const uint32_t g = argmax(zg, a.groups, &v);
+            if (lane == g) zg = -INFINITY;
+        }
+        // a kept group's score is -infinity by now (one that was so from the start stays in the choice as well)
+        const uint32_t open = __ballot_sync(0xffffffffu, lane < a.groups && zg == -INFINITY);
+        if (expert && !(open >> (lane / size) & 1u)) z = -INFINITY;
+    }
+    uint32_t mine = 0xffffffffu;               // lane j: choice j and its weight
+    float wt = 0.0f;
+    for (uint32_t j = 0; j < a.top; j++) {
+        float best;
+        const uint32_t bi = argmax(z, a.NE, &best);
+        if (lane == j) { mine = bi; wt = best; }
+        if (lane == bi) z = -INFINITY;
+    }
+    const bool chose = lane < a.top;
+    if (a.mode == 1u) wt = sigmoidf_(wt);
+    else if (a.mode == 3u) wt *= a.wscale;
+    else {
+        const float first = __shfl_sync(0xffffffffu, wt, 0);
+        wt = a.mode == 2u ? expf(wt - zmax) / zden : expf(wt - first);
+        float s = 0.0f;
+        for (uint32_t j = 0; j < a.top; j++) s += __shfl_sync(0xffffffffu, wt, j);
+        wt /= a.mode == 2u ? s + 1e-20f : s;
+    }
+    // rows sorted by expert; choices of the same expert (-infinities only) follow in their order
+    uint32_t before = 0, place = 0, below = 0, all = 0;
+    bool first_of = chose;
+    for (uint32_t j = 0; j < a.top; j++) {
+        const uint32_t other = __shfl_sync(0xffffffffu, mine, j);
+        if (other < mine || (other == mine && j < lane)) before++;
+        if (other == mine && j < lane) first_of = false;
+        if (other < lane) below++;
+        if (other < 32u) all++;
+    }
+    const uint32_t heads = __ballot_sync(0xffffffffu, first_of);
+    for (uint32_t j = 0; j < a.top; j++) {
+        const uint32_t other = __shfl_sync(0xffffffffu, mine, j);
+        if ((heads >> j & 1u) && other < mine) place++;
+    }
+    if (lane <= a.NE) a.off[lane] = below;     // rows of experts below
+    if (a.NE == 32u && lane == 0) a.off[32] = all;
+    if (chose) {
+        a.idx[lane] = mine; a.wt[lane] = wt; a.slot[lane] = before; a.rows[before] = 0u;
+        if (a.wrow) a.wrow[before] = wt;
+        if (a.act && first_of) a.act[place] = mine;
+        if (a.act && lane >= (uint32_t)__popc(heads)) a.act[lane] = 0xffffffffu;
     }
 }
 

@@ -1,0 +1,96 @@
+"""Products of a single token (csrc/layered_one.cuh) where their depth meets the edges of a warp's step, of the steps it holds before the wait, of rows that several warps
+share and of the longest row in shared memory; the 32-bit tiles (k_gemm_f32_async) at the edges of tiles, steps and shared depths.
+
+Bounds, root mean squares over all rows against the float64 restatements: in 32 bits a sum of up to 11272 products is off by about sqrt(11272) 2^-24 = 6e-6 of itself, a
+few of them on the way; with bfloat16 operands as in the portions' tests, ten roundings of up to 2^-9 on the longest way."""
+import numpy as np
+import pytest
+
+from nano_b200 import engine as E, modeldir as md
+import famudra_oracle as A
+import fidatar_oracle as F
+import kadesun_oracle as K
+
+pytestmark = pytest.mark.gpu
+BOUND = {True: 2e-5, False: 2e-2}
+
+
+def model(design, width, ff, vocab):
+    if design == "kadesun":
+        cfg = md.kadesun_config(vocab, width, [("delta", {"heads": 2, "kv_heads": 1, "dim": 24, "vdim": 40, "conv": 3}, ff),
+                                               ("parallel", {"left": {"heads": 4, "kv_heads": 2, "dim": 16, "vdim": 24, "scale": 0.25, "softcap": 20.0, "rot": {"dims": 8, "base": 100.0}},
+                                                             "right": {"heads": 2, "kv_heads": 2, "dim": 16, "vdim": 16, "conv": 4}}, ff)])
+        return cfg, md.kadesun_random(cfg, 3, decay_rank=8, gate_rank=16), K
+    if design == "famudra":          # every expert is chosen by every token: no close call of the router
+        mlp = {"experts": 2, "top": 2, "ff": ff, "shared_ff": width}
+        cfg = md.famudra_config(vocab, width, [("latent_attention", {"heads": 4, "dim": 16, "vdim": 8, "kv_rank": 20, "q_rank": 24, "scale": 0.25}, mlp),
+                                               ("rglru", {"width": width, "blocks": 2, "conv": 4}, mlp)])
+        return cfg, md.famudra_random(cfg, 3), A
+    moe = {"kind": "moe", "router": {"experts": 3, "top": 3, "groups": {"count": 1, "keep": 1}, "scale": 0.7}, "expert": {"ff": ff}}
+    cfg = md.fidatar_config(vocab, width, [("attention", {"heads": 4, "kv_heads": 2, "dim": 16, "vdim": 24, "scale": 0.25}, moe),
+                                           ("mlstm", {"heads": 2, "dim": 24, "vdim": 40, "gate_cap": 8.0}, {"kind": "dense", "ff": ff})], alpha=2.0, scale=2.0)
+    return cfg, md.fidatar_random(cfg, 3), F
+
+
+def off(got, want):
+    return np.linalg.norm(got - want) / np.linalg.norm(want)
+
+
+def one_by_one(eng, toks):
+    s = eng.seq_open()
+    out = np.concatenate([eng.step(s, toks[i:i + 1], [0]) for i in range(toks.size)])
+    eng.seq_close(s)
+    return out
+
+
+@pytest.mark.parametrize("f32", [True, False])
+@pytest.mark.parametrize("design,width,ff", [("kadesun", 248, 264), ("kadesun", 256, 2048), ("famudra", 264, 2056), ("famudra", 1024, 512), ("fidatar", 520, 4104), ("fidatar", 128, 11264), ("kadesun", 128, 11272)])
+def test_one_token_depths(tmp_path, design, width, ff, f32):
+    cfg, w, O = model(design, width, ff, 131)
+    eng = E.Engine(md.write_model_dir(str(tmp_path / "m"), cfg, w), 64, flags=E.FLAG_F32 if f32 else 0)
+    toks = np.random.default_rng(1).integers(0, 131, size=9).astype(np.uint32)
+    assert off(one_by_one(eng, toks), O.forward(cfg, w, toks)) < BOUND[f32]
+    eng.close()
+
+
+# choices of a token over the router's sizes: one lane to 32, as many choices as experts, groups of one and of many
+@pytest.mark.parametrize("experts,top,count,keep", [(1, 1, 1, 1), (3, 2, 3, 2), (8, 8, 2, 2), (12, 3, 4, 2), (32, 5, 4, 2), (32, 32, 1, 1), (33, 3, 3, 2)])
+def test_one_token_routes(tmp_path, experts, top, count, keep):
+    moe = {"kind": "moe", "router": {"experts": experts, "top": top, "groups": {"count": count, "keep": keep}, "scale": 0.7}, "expert": {"ff": 24}}
+    cfg = md.fidatar_config(97, 64, [("mlstm", {"heads": 2, "dim": 24, "vdim": 40, "gate_cap": 8.0}, moe)], alpha=2.0, scale=2.0)
+    w = md.fidatar_random(cfg, 5)
+    eng = E.Engine(md.write_model_dir(str(tmp_path / "m"), cfg, w), 64, flags=E.FLAG_F32)
+    toks = np.random.default_rng(2).integers(0, 97, size=24).astype(np.uint32)
+    got, want = one_by_one(eng, toks), F.forward(cfg, w, toks)
+    r = np.linalg.norm(got - want, axis=1) / np.linalg.norm(want, axis=1)
+    assert np.median(r) < BOUND[True] and (r < BOUND[True]).mean() >= 0.95          # (a choice closer than 2^-24 may fall either way)
+    eng.close()
+
+
+@pytest.mark.parametrize("design,width,ff", [("famudra", 64, 20), ("kadesun", 132, 516), ("fidatar", 516, 1028), ("famudra", 1024, 256)])
+def test_f32_tiles(tmp_path, design, width, ff):
+    cfg, w, O = model(design, width, ff, 131)
+    eng = E.Engine(md.write_model_dir(str(tmp_path / "m"), cfg, w), 512, flags=E.FLAG_F32)
+    toks = np.random.default_rng(1).integers(0, 131, size=130).astype(np.uint32)
+    ref = O.forward(cfg, w, toks)
+    for n in (5, 63, 64, 65, 130):
+        s = eng.seq_open()
+        got = eng.step(s, toks[:n], range(n))
+        eng.seq_close(s)
+        assert off(got, ref[:n]) < BOUND[True], n
+    eng.close()
+
+
+@pytest.mark.parametrize("dim,vdim", [(8, 4), (32, 17), (40, 64), (128, 33), (132, 20)])
+def test_delta_scan_sizes(tmp_path, dim, vdim):
+    cfg = md.kadesun_config(97, 64, [("delta", {"heads": 3, "kv_heads": 1, "dim": dim, "vdim": vdim, "conv": 4}, 48)])
+    w = md.kadesun_random(cfg, 7, decay_rank=8, gate_rank=16)
+    eng = E.Engine(md.write_model_dir(str(tmp_path / "m"), cfg, w), 256, flags=E.FLAG_F32)
+    toks = np.random.default_rng(3).integers(0, 97, size=101).astype(np.uint32)
+    ref = K.forward(cfg, w, toks)
+    for cut in (5, 8, 9, 50):          # two portions: the state that one leaves is the other's
+        s = eng.seq_open()
+        got = np.concatenate([eng.step(s, toks[:cut], range(cut)), eng.step(s, toks[cut:], range(toks.size - cut))])
+        eng.seq_close(s)
+        assert off(got, ref) < 5 * BOUND[True], cut          # 101 tokens of a recurrence on top of the products
+    eng.close()
