@@ -5,7 +5,7 @@
 // differs, as it does between the decode paths.  What a prompt leaves behind is its K and V rows, so the last layer stops there.
 //
 //   k_prompt_embed     token rows
-//   k_prompt_prep      a position's activation: RMS norm with gain, plain, or SwiGLU of interleaved pairs; then Q80 codes + group scales, or
+//   k_prompt_rows      a position's activation: RMS norm with gain, plain, or SwiGLU of interleaved pairs; then Q80 codes + group scales, or
 //                      (F32) three bfloat16 parts
 //   k_weight_parts     F32: a matrix in three bfloat16 parts, into one workspace for all of them (its bytes pass through memory four times
 //                      for that; a copy that stays would hold half again as much as the file)
@@ -16,7 +16,7 @@
 //                      smallest, smallest x smallest) are 2^-26 of the whole at most.  The tensor cores cut what they add, so they
 //                      add over 16 of the depth only, the small products first, and what they leave is added up with its rounding error carried along.
 //   k_prompt_rope      head norm (Qwen3), rotary positions, K and V rows into the cache
-//   attention          attn_tc.cu
+//   attention          attn_tc.cu; k_prompt_attn for few positions
 #include "prefill.h"
 
 #include <cuda_bf16.h>
@@ -33,6 +33,8 @@ namespace nb {
 namespace {
 
 constexpr uint32_t kChunk = 1024, kRows = 128;
+constexpr uint64_t kPromptAttnWork = 50 * 50;          // positions x keys up to which k_prompt_attn is ahead: Nano-168M (16 heads of 48) 16 positions 1.02 ms against 1.33 on the
+                                                       // tensor cores, 40 1.27 / 1.47; Qwen3-0.6B (16 of 128) 33 1.59 / 1.92, 65 2.29 / 2.09
 enum { PREP_NORM = 0, PREP_PLAIN = 1, PREP_SWIGLU = 2 };
 
 __device__ __forceinline__ void dep_enter() { asm volatile("griddepcontrol.launch_dependents;\ngriddepcontrol.wait;" ::: "memory"); }
@@ -69,7 +71,7 @@ __device__ __forceinline__ float prep_value(const PromptPrepArgs &a, const float
     return __fmul_rn(__fmul_rn(v.x, __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-v.x)))), v.y);
 }
 constexpr uint32_t kPrepThreads = 512;
-template <bool Q80>
+// groups of 256: every other size runs on k_prompt_rows
 __global__ void __launch_bounds__(kPrepThreads) k_prompt_prep(const PromptPrepArgs a) {
     dep_enter();
     __shared__ float red[32];
@@ -82,24 +84,105 @@ __global__ void __launch_bounds__(kPrepThreads) k_prompt_prep(const PromptPrepAr
         acc = block_sum<kPrepThreads>(acc, red);
         inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(acc, (float)a.n), 1e-5f)));
     }
-    if (Q80) {
-        const uint32_t G = a.n / a.gs, epl = a.gs / 32u;      // gs in {32, 64, 128, 256}
-        for (uint32_t g = warp; g < G; g += kPrepThreads / 32u) {
-            float v[8], amax = 0.0f;
+    const uint32_t G = a.n / a.gs, epl = a.gs / 32u;
+    for (uint32_t g = warp; g < G; g += kPrepThreads / 32u) {
+        float v[8], amax = 0.0f;
 #pragma unroll
-            for (uint32_t j = 0; j < 8; j++) if (j < epl) { v[j] = prep_value(a, s, inv, g * a.gs + j * 32u + lane); amax = fmaxf(amax, fabsf(v[j])); }
-            amax = warp_max(amax);
-            const float sc = __fdiv_rn(amax, 127.0f), rinv = __frcp_rn(sc);
+        for (uint32_t j = 0; j < 8; j++) if (j < epl) { v[j] = prep_value(a, s, inv, g * a.gs + j * 32u + lane); amax = fmaxf(amax, fabsf(v[j])); }
+        amax = warp_max(amax);
+        const float sc = __fdiv_rn(amax, 127.0f), rinv = __frcp_rn(sc);
 #pragma unroll
-            for (uint32_t j = 0; j < 8; j++) if (j < epl) a.codes[(size_t)t * a.n + g * a.gs + j * 32u + lane] = (int8_t)((sc == 0.0f) ? 0 : q80_code(v[j], sc, rinv));
-            if (lane == 0) a.scales[(size_t)g * a.lds + t] = sc;
+        for (uint32_t j = 0; j < 8; j++) if (j < epl) a.codes[(size_t)t * a.n + g * a.gs + j * 32u + lane] = (int8_t)((sc == 0.0f) ? 0 : q80_code(v[j], sc, rinv));
+        if (lane == 0) a.scales[(size_t)g * a.lds + t] = sc;
+    }
+}
+// The same for groups of 32, 64 and 128 (8, 16 and 32 lanes) and for F32: a thread holds runs of 4 neighbours, 4 of them in registers, gains are there before the
+// wait, codes and parts leave in 4- and 8-byte pieces.  A row is one trip to memory, one sum and one store; a prompt of 250 positions spent 5.1 us in each of its 109
+// walks of single values, now 4.3 (16 positions: 3.6, now 2.7).
+constexpr uint32_t kRowThreads = 256, kRowRuns = 4, kRowTurn = kRowThreads * 4u * kRowRuns;
+template <bool Q80>
+__global__ void __launch_bounds__(kRowThreads) k_prompt_rows(const PromptPrepArgs a) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    __shared__ float red[32];
+    const uint32_t t = blockIdx.x, lane = threadIdx.x & 31u;
+    const float *s = a.src + (size_t)t * a.ld;
+    const bool norm = a.mode == PREP_NORM;
+    float4 v[kRowRuns], g[kRowRuns];
+    auto at = [&](uint32_t base, uint32_t j) { return base + (threadIdx.x + j * kRowThreads) * 4u; };
+    auto gains = [&](uint32_t base) {
+#pragma unroll
+        for (uint32_t j = 0; j < kRowRuns; j++) { const uint32_t i = at(base, j); g[j] = norm && i < a.n ? __ldg(reinterpret_cast<const float4 *>(a.gain + i)) : make_float4(1, 1, 1, 1); }
+    };
+    auto load = [&](uint32_t base) {
+#pragma unroll
+        for (uint32_t j = 0; j < kRowRuns; j++) {
+            const uint32_t i = at(base, j);
+            v[j] = make_float4(0, 0, 0, 0);
+            if (i >= a.n) continue;
+            if (a.mode == PREP_SWIGLU) {
+                const float4 p = *reinterpret_cast<const float4 *>(s + 2u * i), q = *reinterpret_cast<const float4 *>(s + 2u * i + 4u);
+                auto glu = [](float x, float y) { return __fmul_rn(__fmul_rn(x, __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-x)))), y); };
+                v[j] = make_float4(glu(p.x, p.y), glu(p.z, p.w), glu(q.x, q.y), glu(q.z, q.w));
+            } else v[j] = *reinterpret_cast<const float4 *>(s + i);
         }
-    } else {
-        __nv_bfloat16 *to = a.parts + (size_t)t * 3u * a.np;
-        for (uint32_t i = threadIdx.x; i < a.np; i += kPrepThreads) {
-            __nv_bfloat16 p[3];
-            split3(i < a.n ? prep_value(a, s, inv, i) : 0.0f, p);
-            to[i] = p[0]; to[a.np + i] = p[1]; to[2u * a.np + i] = p[2];
+    };
+    gains(0);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    load(0);
+    float inv = 1.0f;
+    if (norm) {
+        float acc = 0.0f;
+        for (uint32_t base = 0;;) {
+#pragma unroll
+            for (uint32_t j = 0; j < kRowRuns; j++) acc = fmaf(v[j].x, v[j].x, fmaf(v[j].y, v[j].y, fmaf(v[j].z, v[j].z, fmaf(v[j].w, v[j].w, acc))));
+            base += kRowTurn;
+            if (base >= a.n) break;
+            load(base);
+        }
+        acc = block_sum<kRowThreads>(acc, red);
+        inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(acc, (float)a.n), 1e-5f)));
+    }
+    const uint32_t LG = Q80 ? a.gs / 4u : 1u, end = Q80 ? a.n : a.np;
+    for (uint32_t base = 0; base < end; base += kRowTurn) {
+        if (base || (norm && a.n > kRowTurn)) { gains(base); load(base); }
+#pragma unroll
+        for (uint32_t j = 0; j < kRowRuns; j++) {
+            const uint32_t i = at(base, j);
+            if (i - lane * 4u >= end) continue;          // the same for the whole warp
+            float4 x = v[j];
+            if (norm) x = make_float4(__fmul_rn(g[j].x, __fmul_rn(inv, x.x)), __fmul_rn(g[j].y, __fmul_rn(inv, x.y)), __fmul_rn(g[j].z, __fmul_rn(inv, x.z)), __fmul_rn(g[j].w, __fmul_rn(inv, x.w)));
+            if (Q80) {
+                float amax = fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w)));
+                for (uint32_t o = 1; o < LG; o <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+                // rounded by adding 1.5 * 2^23; what lies within 1e-4 of a .5 boundary takes the exact division (the product is at most 2.3e-5 from the quotient)
+                const float sc = __fdiv_rn(amax, 127.0f), rinv = __frcp_rn(sc), magic = 12582912.0f;
+                const float q[4] = {x.x * rinv, x.y * rinv, x.z * rinv, x.w * rinv}, xv[4] = {x.x, x.y, x.z, x.w};
+                uint32_t pk = 0;
+                if (sc != 0.0f)
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        const float r = q[e] + magic;
+                        const uint32_t c = fabsf(q[e] - (r - magic)) > 0.4999f ? (uint32_t)q80_code_slow(xv[e], sc) : __float_as_uint(r);
+                        pk |= (c & 0xffu) << (8 * e);
+                    }
+                if (i < a.n) {
+                    *reinterpret_cast<uint32_t *>(a.codes + (size_t)t * a.n + i) = pk;
+                    if ((lane & (LG - 1u)) == 0) a.scales[(size_t)(i / a.gs) * a.lds + t] = sc;
+                }
+            } else if (i < a.np) {
+                __nv_bfloat16 *to = a.parts + (size_t)t * 3u * a.np + i;
+                const float xv[4] = {x.x, x.y, x.z, x.w};
+                __align__(8) __nv_bfloat16 o[3][4];
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    __nv_bfloat16 p[3];
+                    split3(xv[e], p);
+#pragma unroll
+                    for (int k = 0; k < 3; k++) o[k][e] = p[k];
+                }
+#pragma unroll
+                for (int k = 0; k < 3; k++) *reinterpret_cast<uint2 *>(to + (size_t)k * a.np) = *reinterpret_cast<const uint2 *>(o[k]);
+            }
         }
     }
 }
@@ -369,6 +452,67 @@ __global__ void __launch_bounds__(256) k_prompt_rope(const PromptRopeArgs a) {
     }
 }
 
+// A head per warp and four of its values per lane, table and gains before the wait: heads of 4, 8, .. 128 values with a norm, of any multiple of 4 without.  (k_prompt_rope
+// walks its heads through shared memory, four for every warp: 9.5 us for 250 positions of 32 heads, now 3.4.)
+__global__ void __launch_bounds__(256) k_prompt_rope_warp(const PromptRopeArgs a) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const uint32_t t = blockIdx.x, pos = a.pos0 + t, hd = a.d.hd, lane = threadIdx.x & 31u, h = blockIdx.y * 8u + (threadIdx.x >> 5);
+    if (h >= a.H + 2u * a.KV) return;
+    uint32_t lpr = 1;
+    while (lpr * 4u < hd) lpr <<= 1;
+    const uint32_t col = (lane & (lpr - 1u)) * 4u;
+    const bool on = col < hd, isq = h < a.H, isk = !isq && h < a.H + a.KV;
+    const uint32_t g = isq ? 0u : (h - a.H) % a.KV;
+    const RopeTab rt = rope_tab_load(a.cos_ + (size_t)pos * (hd / 2u), a.sin_ + (size_t)pos * (hd / 2u), a.d, col, on);
+    float4 gn = make_float4(0, 0, 0, 0), v = gn;
+    if (a.d.arch == 3u && on && (isq || isk)) gn = __ldg(reinterpret_cast<const float4 *>((isq ? a.qn : a.kn) + col));
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (on) v = *reinterpret_cast<const float4 *>(a.p + (size_t)t * a.ld + (size_t)h * hd + col);
+    if (isq || isk) v = norm_rope_apply(v, gn, rt, a.d, lpr, col, on);
+    if (on && lane < lpr) {
+        float *dst = isq ? a.q + (size_t)t * a.H * hd + (size_t)h * hd : (isk ? a.kc : a.vc) + ((size_t)g * a.d.max_seq + pos) * hd;
+        *reinterpret_cast<float4 *>(dst + col) = v;
+    }
+}
+
+// Attention of a short portion in fp32: a warp per query and head, lane = key for the scores, = columns for the values, 32 keys a turn.  The tensor-core kernels
+// take 18 us for as little as 16 positions of Nano's 16 heads (images of keys and values, then one wave of tiles); this one 6, growing with positions x keys.
+struct PromptAttnArgs { const float *q, *kc, *vc; float *out; uint32_t H, KV, hd, max_seq, pos0; float scale; };
+__global__ void __launch_bounds__(256) k_prompt_attn(const PromptAttnArgs a) {
+    dep_enter();
+    __shared__ __align__(16) float q_s[8][128];
+    const uint32_t t = blockIdx.x, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, h = blockIdx.y * 8u + warp, hd = a.hd, nkeys = a.pos0 + t + 1u;
+    if (h >= a.H) return;
+    const uint32_t g = h / (a.H / a.KV);
+    const float *K = a.kc + (size_t)g * a.max_seq * hd, *V = a.vc + (size_t)g * a.max_seq * hd, *q = a.q + ((size_t)t * a.H + h) * hd;
+    if (lane * 4u < hd) *reinterpret_cast<float4 *>(&q_s[warp][lane * 4u]) = *reinterpret_cast<const float4 *>(q + lane * 4u);
+    __syncwarp();
+    float m = -INFINITY, l = 0.0f;
+    float4 o = make_float4(0, 0, 0, 0);
+    for (uint32_t k0 = 0; k0 < nkeys; k0 += 32u) {
+        const uint32_t n = min(32u, nkeys - k0);
+        float s0 = 0.0f, s1 = 0.0f, s2 = 0.0f, s3 = 0.0f;
+        const float4 *kr = reinterpret_cast<const float4 *>(K + (size_t)(k0 + min(lane, n - 1u)) * hd);
+#pragma unroll 8
+        for (uint32_t c = 0; c < hd / 4u; c++) {
+            const float4 k = kr[c], x = *reinterpret_cast<const float4 *>(&q_s[warp][c * 4u]);
+            s0 = fmaf(k.x, x.x, s0); s1 = fmaf(k.y, x.y, s1); s2 = fmaf(k.z, x.z, s2); s3 = fmaf(k.w, x.w, s3);
+        }
+        const float s = lane < n ? ((s0 + s1) + (s2 + s3)) * a.scale : -INFINITY, mn = fmaxf(m, warp_max(s)), keep = expf(m - mn), p = lane < n ? expf(s - mn) : 0.0f;
+        l = fmaf(l, keep, warp_sum(p));
+        m = mn;
+        o.x *= keep; o.y *= keep; o.z *= keep; o.w *= keep;
+        const float *vr = V + (size_t)k0 * hd + lane * 4u;
+#pragma unroll 8
+        for (uint32_t j = 0; j < 32u; j++) {
+            const float w = __shfl_sync(0xffffffffu, p, j);
+            if (j < n && lane * 4u < hd) { const float4 v = *reinterpret_cast<const float4 *>(vr + (size_t)j * hd); o.x = fmaf(w, v.x, o.x); o.y = fmaf(w, v.y, o.y); o.z = fmaf(w, v.z, o.z); o.w = fmaf(w, v.w, o.w); }
+        }
+    }
+    const float inv = 1.0f / l;
+    if (lane * 4u < hd) *reinterpret_cast<float4 *>(a.out + ((size_t)t * a.H + h) * hd + lane * 4u) = make_float4(o.x * inv, o.y * inv, o.z * inv, o.w * inv);
+}
+
 template <typename A>
 int launch(void (*k)(const A), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, bool pdl, const A &args, uint32_t cluster_z = 1) {
     cudaLaunchConfig_t cfg{};
@@ -469,7 +613,9 @@ int create(PrefillState *s, const PrefillModel &m) {
 }
 int prep(PrefillState *s, const float *src, uint32_t ld, const float *gain, uint32_t n, uint32_t mode, uint32_t T, cudaStream_t stream) {
     const PromptPrepArgs a{src, ld, gain, n, s->m.gs, mode, reinterpret_cast<int8_t *>(s->act), s->scales, kChunk, reinterpret_cast<__nv_bfloat16 *>(s->act), (n + 63u) & ~63u};
-    return launch<PromptPrepArgs>(s->m.quant == 0x80u ? k_prompt_prep<true> : k_prompt_prep<false>, dim3(T), dim3(kPrepThreads), 0, stream, s->pdl, a);
+    const bool q80 = s->m.quant == 0x80u;
+    if (q80 && s->m.gs > 128u) return launch<PromptPrepArgs>(k_prompt_prep, dim3(T), dim3(kPrepThreads), 0, stream, s->pdl, a);
+    return launch<PromptPrepArgs>(q80 ? k_prompt_rows<true> : k_prompt_rows<false>, dim3(T), dim3(kRowThreads), 0, stream, s->pdl, a);
 }
 int product(PrefillState *s, const Product &w, float *C, uint32_t ldc, bool add, uint32_t T, cudaStream_t stream) {
     // 64 positions per tile where tiles of 128 leave SMs without a block (1024 rows of the O product: 8 blocks for 128 positions), and in F32, whose
@@ -529,6 +675,7 @@ int prefill_run(PrefillState *s, const uint32_t *ids, uint32_t n, cudaStream_t s
     const size_t kvl = (size_t)m.KV * m.max_seq * m.hd;
     Dims d{};
     d.arch = m.arch; d.hd = m.hd; d.max_seq = m.max_seq;
+    const bool by_warp = m.arch != 3u || (m.hd & (m.hd - 1u)) == 0;          // the norm's exchange of halves between lanes wants 4 x 2^k values
     int r;
     for (uint32_t p0 = 0; p0 < n; p0 += kChunk) {
         const uint32_t T = std::min(kChunk, n - p0);
@@ -537,17 +684,20 @@ int prefill_run(PrefillState *s, const uint32_t *ids, uint32_t n, cudaStream_t s
         for (uint32_t l = 0; l < m.L; l++) {
             const PromptRopeArgs ra{s->p, W, m.H, m.KV, p0, s->q, m.kc + l * kvl, m.vc + l * kvl, m.qnorm ? m.qnorm + (size_t)l * m.hd : nullptr, m.knorm ? m.knorm + (size_t)l * m.hd : nullptr, m.rope_cos, m.rope_sin, d};
             if ((r = prep(s, s->x, m.E, m.norm_attn + (size_t)l * m.E, m.E, PREP_NORM, T, stream)) || (r = product(s, s->qkv[l], s->p, W, false, T, stream)) ||
-                (r = launch<PromptRopeArgs>(k_prompt_rope, dim3(T), dim3(256), 0, stream, pdl, ra))) return r;
+                (r = by_warp ? launch<PromptRopeArgs>(k_prompt_rope_warp, dim3(T, (m.H + 2u * m.KV + 7u) / 8u), dim3(256), 0, stream, pdl, ra)
+                             : launch<PromptRopeArgs>(k_prompt_rope, dim3(T), dim3(256), 0, stream, pdl, ra))) return r;
             *launches += 3u + extra;
             if (l + 1u == m.L) break;          // nothing reads what the last layer would make of these positions
             TcAttn a{};
             a.q = s->q; a.ldq = m.q_dim; a.q_head = m.hd; a.k = m.kc + l * kvl; a.v = m.vc + l * kvl; a.ldk = a.ldv = m.hd; a.k_head = a.v_head = (uint64_t)m.max_seq * m.hd;
             a.out = s->o; a.T = T; a.H = m.H; a.G = m.KV; a.D = a.VD = m.hd; a.pos0 = p0; a.scale = (float)(1.0 / sqrt((double)m.hd));
-            if (!attn_tc_fits(&s->attn, a)) return fail(NB200_EINVAL, "a prompt of %u positions does not fit the attention's buffers", n);
-            if ((r = attn_tc_launch(&s->attn, a, stream, pdl)) || (r = prep(s, s->o, m.q_dim, nullptr, m.q_dim, PREP_PLAIN, T, stream)) || (r = product(s, s->wo[l], s->x, m.E, true, T, stream)) ||
+            const bool few = (uint64_t)T * (p0 + T) <= kPromptAttnWork;
+            const PromptAttnArgs pa{s->q, m.kc + l * kvl, m.vc + l * kvl, s->o, m.H, m.KV, m.hd, m.max_seq, p0, a.scale};
+            if (!few && !attn_tc_fits(&s->attn, a)) return fail(NB200_EINVAL, "a prompt of %u positions does not fit the attention's buffers", n);
+            if ((r = few ? launch<PromptAttnArgs>(k_prompt_attn, dim3(T, (m.H + 7u) / 8u), dim3(256), 0, stream, pdl, pa) : attn_tc_launch(&s->attn, a, stream, pdl)) || (r = prep(s, s->o, m.q_dim, nullptr, m.q_dim, PREP_PLAIN, T, stream)) || (r = product(s, s->wo[l], s->x, m.E, true, T, stream)) ||
                 (r = prep(s, s->x, m.E, m.norm_ffn + (size_t)l * m.E, m.E, PREP_NORM, T, stream)) || (r = product(s, s->w13[l], s->p, 2 * m.F, false, T, stream)) ||
                 (r = prep(s, s->p, 2 * m.F, nullptr, m.F, PREP_SWIGLU, T, stream)) || (r = product(s, s->w2[l], s->x, m.E, true, T, stream))) return r;
-            *launches += 8u + 3u * extra;
+            *launches += (few ? 7u : 8u) + 3u * extra;
         }
     }
     return 0;
