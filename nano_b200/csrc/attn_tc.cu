@@ -12,11 +12,12 @@
 //
 //   k_attn_images   a tile of 128 keys of one head: its scale, then keys and transposed values in two planes each, in the byte order of
 //                   the swizzled shared-memory operand: the attention kernel fetches a tile with two bulk copies
-//   k_attn_tc       a block owns 128 rows (query token, query head) of one key/value head.  Warp 0 fetches, warp 1 issues tcgen05.mma, a thread of warps
-//                   2..5 owns one row: scores come out of tensor memory with a lane per row, so a row's maximum and sum need no other
-//                   thread; its weights go back into tensor memory as the A operand of the second product.  Scores are double buffered and a
+//   k_attn_tc       a block owns 128 rows (query token, query head) of one key/value head.  Warp 0 fetches, warp 1 issues tcgen05.mma, two threads of warps
+//                   2..9 own one row, 64 keys of a tile and half of the values each: scores come out of tensor memory with a lane per row, and what the two tell each other is
+//                   the tile's maximum; its weights go back into tensor memory as the A operand of the second product.  Scores are double buffered and a
 //                   tile's values are added while the next tile's scores are made, so the tensor cores (busy for 11 % of the time) work under the softmax
-//                   of four warps, one per scheduler, which bounds the kernel: its chain of loads, exponentials and splits issues in 26 % of the cycles.
+//                   of eight warps, two per scheduler, which bounds the kernel: with a thread per row, one warp per scheduler, its chain of loads, exponentials and splits
+//                   issued in 26 % of the cycles.
 // 1024 queries x 16 heads over 4 key/value heads of 128 on 1536 keys on average: 102 us, 606 by the FMA kernel (k_gqa_attn), with softcap 130 and 640; error
 // against float64 on normal numbers 0.4e-6 .. 1.1e-6 of a row's norm where the FMA kernel has 0.75e-6 .. 1.6e-6.
 #include "attn_tc.h"
@@ -133,15 +134,16 @@ __global__ void __launch_bounds__(kImageThreads) k_attn_images(const ImageArgs i
 
 struct AttnTcArgs { TcAttn a; const unsigned char *images; const float *scales; uint32_t tile0, tiles; uint32_t *err; };
 
+constexpr uint32_t kAttnThreads = 320;
 template <int DP, int VP> constexpr size_t attn_smem() { return (size_t)(DP + DP + VP) * 512u + 1024u; }          // queries, keys, values
 
 template <int DP, int VP>
-__global__ void __launch_bounds__(192, 1) k_attn_tc(const AttnTcArgs ta) {
+__global__ void __launch_bounds__(kAttnThreads, 1) k_attn_tc(const AttnTcArgs ta) {
     extern __shared__ uint8_t tc_raw[];
     enum { KFULL, KFREE, VFULL, VFREE, SFULL0, SFULL1, PREADY, OREADY, NBAR };
     __shared__ __align__(8) uint64_t bars[NBAR];
     __shared__ uint32_t tmem_s, bad_s;
-    __shared__ float red[8];
+    __shared__ float red[16], top_s[2][2][kTile], sum_s[2][kTile];          // of a row's halves: the largest score of a tile (tiles alternate), the sum of weights
     const TcAttn &a = ta.a;
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
     const uint32_t qs = (smem_u32(tc_raw) + 1023u) & ~1023u, ksm = qs + DP * 512u, vsm = ksm + DP * 512u;
@@ -149,7 +151,7 @@ __global__ void __launch_bounds__(192, 1) k_attn_tc(const AttnTcArgs ta) {
     const uint32_t b0 = smem_u32(bars);
     auto bar = [&](uint32_t i) { return b0 + i * 8u; };
     if (tid == 0) {
-        for (uint32_t i = 0; i < NBAR; i++) mbar_init(bar(i), i == PREADY ? 4 : 1);
+        for (uint32_t i = 0; i < NBAR; i++) mbar_init(bar(i), i == PREADY ? 8 : 1);
         bad_s = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -171,15 +173,15 @@ __global__ void __launch_bounds__(192, 1) k_attn_tc(const AttnTcArgs ta) {
         constexpr uint32_t d8 = DP / 8;
         const uint32_t D8 = (a.D + 7u) / 8u;
         float x[8], m = 0.0f;
-        for (uint32_t i = tid; i < (last - r0 + 1u) * D8; i += 192u) {
+        for (uint32_t i = tid; i < (last - r0 + 1u) * D8; i += kAttnThreads) {
             const uint32_t rr = r0 + i / D8, c = i % D8 * 8u;
             load8(a.q + (size_t)(rr / rep) * a.ldq + (size_t)(g * rep + rr % rep) * a.q_head + c, a.D - c, x);
             m = fmaxf(m, max8(x));
         }
-        float s = tile_scale(block_max<192>(m, red));
+        float s = tile_scale(block_max<kAttnThreads>(m, red));
         qinv = 1.0f / s;
         if (a.scale < 0.0f) s = -s;          // the largest raw score is to be the largest score: the sign of a negative scale goes with the query
-        for (uint32_t i = tid; i < kTile * d8; i += 192u) {
+        for (uint32_t i = tid; i < kTile * d8; i += kAttnThreads) {
             const uint32_t r = i / d8, c = i % d8, rr = min(r0 + r, last);
             load8(a.q + (size_t)(rr / rep) * a.ldq + (size_t)(g * rep + rr % rep) * a.q_head + c * 8u, c * 8u < a.D ? a.D - c * 8u : 0u, x);
             uint4 h, l;
@@ -242,9 +244,13 @@ __global__ void __launch_bounds__(192, 1) k_attn_tc(const AttnTcArgs ta) {
     } else if (warp >= 2) {
         const uint32_t quad = warp & 3u, r = quad * 32u + lane, rr = min(r0 + r, last), t = rr / rep, h = g * rep + rr % rep;
         const uint32_t pos = a.pos0 + t, low = oldest(a, pos), low_last = oldest(a, last_pos), lane_base = (quad * 32u) << 16;
-        float m = a.sink ? a.sink[h] : -INFINITY, l = a.sink ? 1.0f : 0.0f, o[VP];
+        // a row belongs to two threads, of warps that reach the same lanes of tensor memory: each has 64 keys of a tile and half of the values.  They share the row's
+        // maximum once a tile (the barrier of their two warps, which also says whether both go on) and their sums at the end.
+        constexpr int VH = VP / 2;
+        const uint32_t half = (warp - 2u) >> 2, c_lo = half * (kTile / 2u), v_lo = half * (uint32_t)VH;
+        float m = a.sink ? a.sink[h] : -INFINITY, l = a.sink && half == 0 ? 1.0f : 0.0f, o[VH];
 #pragma unroll
-        for (int d = 0; d < VP; d++) o[d] = 0.0f;
+        for (int d = 0; d < VH; d++) o[d] = 0.0f;
         bool ok = true;
         float vinv = 0.0f;
         // the values of the tile before join the sum, which then moves to the new maximum
@@ -254,14 +260,14 @@ __global__ void __launch_bounds__(192, 1) k_attn_tc(const AttnTcArgs ta) {
             tc_fence_after();
             const float f = vinv * corr;
 #pragma unroll
-            for (int c = 0; c < VP; c += 32) {
+            for (int c = 0; c < VH; c += 32) {
                 uint32_t w[32];
-                tc_ld32(tmem + lane_base + OCOL + c, w);
+                tc_ld32(tmem + lane_base + OCOL + v_lo + c, w);
 #pragma unroll
                 for (int j = 0; j < 32; j++) o[c + j] = fmaf(__uint_as_float(w[j]), f, o[c + j] * corr);
 #pragma unroll
                 for (uint32_t q = 1; q < SUMS; q++) {
-                    tc_ld32(tmem + lane_base + OCOL + q * VP + c, w);
+                    tc_ld32(tmem + lane_base + OCOL + q * VP + v_lo + c, w);
 #pragma unroll
                     for (int j = 0; j < 32; j++) o[c + j] = fmaf(__uint_as_float(w[j]), f, o[c + j]);
                 }
@@ -271,13 +277,13 @@ __global__ void __launch_bounds__(192, 1) k_attn_tc(const AttnTcArgs ta) {
             const uint32_t key0 = (lo + i) * kTile, s_at = tmem + lane_base + SCOL + (i & 1u) * kTile;
             const float kc = qinv * scales[2u * i] * (a.softcap > 0.0f ? fabsf(a.scale) / a.softcap : fabsf(a.scale));
             const bool whole = key0 + kTile <= first_pos + 1u && key0 >= low_last;          // every row of the block sees every key of the tile
-            ok = mbar_wait_warp(bar(SFULL0 + (i & 1u)), (i >> 1) & 1u);
-            if (!ok) break;
+            ok = ok && mbar_wait_warp(bar(SFULL0 + (i & 1u)), (i >> 1) & 1u);
             tc_fence_after();
             const uint32_t j0 = low > key0 ? low - key0 : 0u, j1 = pos < key0 ? 0u : min(kTile, pos - key0 + 1u);          // the keys this row sees
             float top = -INFINITY;
+            if (ok)
 #pragma unroll 1
-            for (uint32_t c = 0; c < kTile; c += 32u) {
+            for (uint32_t c = c_lo; c < c_lo + kTile / 2u; c += 32u) {
                 uint32_t w[32];
                 tc_ld32(s_at + c, w);
                 if (whole) {
@@ -288,15 +294,17 @@ __global__ void __launch_bounds__(192, 1) k_attn_tc(const AttnTcArgs ta) {
                     for (uint32_t j = 0; j < 32; j++) top = c + j >= j0 && c + j < j1 ? fmaxf(top, __uint_as_float(w[j])) : top;
                 }
             }
-            top *= kc;
+            top_s[i & 1u][half][r] = top;
+            if (bar_any(1u + quad, 64u, !ok)) { ok = false; break; }
+            top = fmaxf(top, top_s[i & 1u][half ^ 1u][r]) * kc;
             if (a.softcap > 0.0f && top != -INFINITY) top = a.softcap * tanhf(top);
             const float mn = fmaxf(m, top), corr = mn == -INFINITY ? 1.0f : expf(m - mn);
             if (i) collect(i - 1u, corr);
-            if (!ok) break;
+            if (!ok) continue;          // both warps leave at the next barrier, or after the last tile
             vinv = scales[2u * i + 1u] / kWeightScale;
             float sum = 0.0f;
 #pragma unroll 1          // (a tile's whole code does not fit the instruction cache)
-            for (uint32_t c = 0; c < kTile; c += 32u) {
+            for (uint32_t c = c_lo; c < c_lo + kTile / 2u; c += 32u) {
                 uint32_t w[32], wh[16], wl[16];
                 tc_ld32(s_at + c, w);
                 float p[32];
@@ -329,15 +337,17 @@ __global__ void __launch_bounds__(192, 1) k_attn_tc(const AttnTcArgs ta) {
             if (lane == 0) mbar_arrive(bar(PREADY));
         }
         if (ok) collect(n - 1u, 1.0f);
+        sum_s[half][r] = l;
+        ok = !bar_any(1u + quad, 64u, !ok);
         if (!ok) bad_s = 4;
         if (ok && r0 + r <= last) {
-            float f = 1.0f / l;
+            float f = 1.0f / (sum_s[0][r] + sum_s[1][r]);
             if (a.gate) f *= 1.0f / (1.0f + expf(-a.gate[(size_t)t * a.ldg + h]));
-            float *dst = a.out + ((size_t)t * a.H + h) * a.VD;
-            const float *mul = a.mul ? a.mul + (size_t)t * a.ldm + (size_t)h * a.VD : nullptr;
+            float *dst = a.out + ((size_t)t * a.H + h) * a.VD + v_lo;
+            const float *mul = a.mul ? a.mul + (size_t)t * a.ldm + (size_t)h * a.VD + v_lo : nullptr;
 #pragma unroll
-            for (int d = 0; d < VP; d += 4)
-                if (d < (int)a.VD) {
+            for (int d = 0; d < VH; d += 4)
+                if (v_lo + d < a.VD) {
                     float4 y = make_float4(o[d] * f, o[d + 1] * f, o[d + 2] * f, o[d + 3] * f);
                     if (mul) { y.x *= mul[d]; y.y *= mul[d + 1]; y.z *= mul[d + 2]; y.w *= mul[d + 3]; }
                     *reinterpret_cast<float4 *>(dst + d) = y;
@@ -404,7 +414,7 @@ int attn_tc_launch(TcAttnState *s, const TcAttn &a, cudaStream_t stream, bool pd
     int r;
     if ((r = launch<ImageArgs>(k_attn_images, dim3(tiles, a.G, 2), dim3(kImageThreads), 0, stream, pdl, ImageArgs{a, s->images, s->scales, tile0, tiles, nkeys}))) return r;
     const AttnTcArgs ta{a, s->images, s->scales, tile0, tiles, s->err_dev};
-    const dim3 grid((a.T * (a.H / a.G) + kTile - 1u) / kTile, a.G), block(192);
+    const dim3 grid((a.T * (a.H / a.G) + kTile - 1u) / kTile, a.G), block(kAttnThreads);
     if (a.D <= 64u) return a.VD <= 64u ? launch<AttnTcArgs>(k_attn_tc<64, 64>, grid, block, attn_smem<64, 64>(), stream, pdl, ta) : launch<AttnTcArgs>(k_attn_tc<64, 128>, grid, block, attn_smem<64, 128>(), stream, pdl, ta);
     return a.VD <= 64u ? launch<AttnTcArgs>(k_attn_tc<128, 64>, grid, block, attn_smem<128, 64>(), stream, pdl, ta) : launch<AttnTcArgs>(k_attn_tc<128, 128>, grid, block, attn_smem<128, 128>(), stream, pdl, ta);
 }
