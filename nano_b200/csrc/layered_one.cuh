@@ -370,6 +370,65 @@ __global__ void __launch_bounds__(kOneThreads) k_norm_shift_one(const NormShiftA
     }
 }
 
+// k_combine of one token and k_norm_shift_one of the run that follows, in one link: the updated row stays in the registers of the block that norms it
+struct CombineNormArgs { CombineArgs c; NormShiftArgs n; };
+__global__ void __launch_bounds__(kOneThreads) k_combine_norm_one(const CombineNormArgs a) {
+    pdl_launch_next();
+    __shared__ float red[32];
+    const CombineArgs &c = a.c;
+    const NormShiftArgs &m = a.n;
+    const uint32_t E4 = m.E / 4u;
+    auto row = [&](const float *p, uint32_t i) { return reinterpret_cast<const float4 *>(p)[i]; };
+    float4 x[4], p[4], mu[4];
+#pragma unroll
+    for (uint32_t k = 0; k < 4u; k++) {          // the state is the token before's, the shift a weight
+        const uint32_t i = threadIdx.x + k * kOneThreads;
+        mu[k] = p[k] = make_float4(0, 0, 0, 0);
+        if (i < E4) { if (m.mu) mu[k] = __ldg(reinterpret_cast<const float4 *>(m.mu) + i); }
+    }
+    const float g1 = __ldg(m.g1), g2 = m.g2 ? __ldg(m.g2) : 0.0f;
+    pdl_wait();
+    uint32_t slot[4]; float wt[4];
+#pragma unroll
+    for (uint32_t j = 0; j < 4u; j++) { slot[j] = 0; wt[j] = 0.0f; if (c.eo && j < c.top) { slot[j] = c.slot[j]; wt[j] = c.wt[j]; } }
+    float4 d[4], sh[4];
+#pragma unroll
+    for (uint32_t k = 0; k < 4u; k++) {
+        const uint32_t i = threadIdx.x + k * kOneThreads;
+        x[k] = d[k] = sh[k] = make_float4(0, 0, 0, 0);
+        if (i < E4) { x[k] = row(c.x, i); d[k] = row(c.d, i); p[k] = row(m.state, i); if (c.eo && c.shared) sh[k] = row(c.shared, i); }
+    }
+    float s = 0.0f;
+#pragma unroll
+    for (uint32_t k = 0; k < 4u; k++) {
+        const uint32_t i = threadIdx.x + k * kOneThreads;
+        if (i >= E4) continue;
+        if (c.eo) {
+            float4 f = make_float4(0, 0, 0, 0);
+            auto add = [&](float w, uint32_t at) { const float4 v = row(c.eo + (size_t)at * m.E, i); f.x = fmaf(w, v.x, f.x); f.y = fmaf(w, v.y, f.y); f.z = fmaf(w, v.z, f.z); f.w = fmaf(w, v.w, f.w); };
+#pragma unroll
+            for (uint32_t j = 0; j < 4u; j++) if (j < c.top) add(wt[j], slot[j]);
+            for (uint32_t j = 4u; j < c.top; j++) add(c.wt[j], c.slot[j]);
+            d[k].x += f.x + sh[k].x; d[k].y += f.y + sh[k].y; d[k].z += f.z + sh[k].z; d[k].w += f.w + sh[k].w;
+        }
+        x[k].x += d[k].x; x[k].y += d[k].y; x[k].z += d[k].z; x[k].w += d[k].w;
+        reinterpret_cast<float4 *>(c.x)[i] = x[k];
+        if (c.keep) reinterpret_cast<float4 *>(c.keep)[i] = x[k];
+        s = sum_sq4(x[k], s);
+    }
+    s = block_sum(s, red);
+    const float rinv = 1.0f / sqrtf(s / (float)m.E + m.eps);
+#pragma unroll
+    for (uint32_t k = 0; k < 4u; k++) {
+        const uint32_t i = threadIdx.x + k * kOneThreads;
+        if (i >= E4) break;
+        const float4 u = make_float4(x[k].x * rinv, x[k].y * rinv, x[k].z * rinv, x[k].w * rinv), n1 = make_float4(u.x * g1, u.y * g1, u.z * g1, u.w * g1);
+        reinterpret_cast<float4 *>(m.hm)[i] = !m.mu ? n1 : make_float4(fmaf(p[k].x - n1.x, mu[k].x, n1.x), fmaf(p[k].y - n1.y, mu[k].y, n1.y), fmaf(p[k].z - n1.z, mu[k].z, n1.z), fmaf(p[k].w - n1.w, mu[k].w, n1.w));
+        if (m.h2) reinterpret_cast<float4 *>(m.h2)[i] = make_float4(u.x * g2, u.y * g2, u.z * g2, u.w * g2);
+        reinterpret_cast<float4 *>(m.state)[i] = n1;
+    }
+}
+
 // k_route_small for one token and at most 32 rows of the router: the same choice, weights and places (RouteArgs, route_pick), in registers.  A cluster of blocks
 // shares the logits, with the router's rows in registers before the wait; the first block's first warp then holds an expert per lane, and everything it leaves is written
 // once, by the lane that has it.  (k_route_small keeps the choice in memory and reads it back: 27 us of the chain of a step with eight routed layers, now 6.)
