@@ -1737,14 +1737,11 @@ int run_layers(LayeredEngine *e, uint32_t slot, uint32_t T, uint32_t pos0, const
     const Ctx cx{st, e->table + (size_t)slot * e->n_pages, T, pos0, pos_ptr};
     int r;
     e->cur = e->stream;
-    // parallel layers: norms and token shift of a run; a single token's row of whole 16-byte pieces has kernels of its own
+    // parallel layers: norms and token shift of a run; a single token's row that fits the registers has kernels of its own
     auto norm_args = [&](const Layer &L, const Run &run) {
         return NormShiftArgs{e->x, L.norm1, L.has_mlp ? L.norm2 : nullptr, L.shift, st + run.st_prev, e->hm, L.has_mlp ? e->h2 : nullptr, T, E, e->eps};
     };
-    auto norm_one_fits = [&](const NormShiftArgs &a) {
-        auto at16 = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
-        return T == 1 && E % 4u == 0 && E <= 16u * kOneThreads && at16(a.mu) && at16(a.state) && at16(a.hm) && at16(a.h2) && at16(a.x);
-    };
+    const bool norm_one = T == 1 && E <= 16u * kOneThreads;
     bool normed = false;
     for (size_t ri = 0; ri < e->runs.size(); ri++) {
         const Run &run = e->runs[ri];
@@ -1814,7 +1811,7 @@ int run_layers(LayeredEngine *e, uint32_t slot, uint32_t T, uint32_t pos0, const
         {
             const NormShiftArgs a = norm_args(L, run);
             if (normed) normed = false;          // by the update before
-            else if (norm_one_fits(a)) {
+            else if (norm_one) {
                 if ((r = launch<NormShiftArgs>(e, k_norm_shift_one, dim3(1), dim3(kOneThreads), 0, a))) return r;
             } else if ((r = launch<NormShiftArgs>(e, k_norm_shift, dim3(T > 1 ? T - 1 : 1), dim3(256), 0, a))) return r;
             if (L.has_mlp && e->branch_streams) CK(cudaEventRecord(e->ev_fork, e->stream));
@@ -1838,8 +1835,7 @@ int run_layers(LayeredEngine *e, uint32_t slot, uint32_t T, uint32_t pos0, const
         // a lone token: the update also norms the row for the run that follows (two links of 2.4 and 2.3 us, now one)
         const Run *nrun = ri + 1 < e->runs.size() && !e->runs[ri + 1].add_embed ? &e->runs[ri + 1] : nullptr;
         const CombineNormArgs cn{c, nrun ? norm_args(e->layers[nrun->layer], *nrun) : NormShiftArgs{}};
-        auto at16 = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
-        if (nrun && norm_one_fits(cn.n) && at16(c.d) && at16(c.eo) && at16(c.shared) && at16(c.keep)) {
+        if (nrun && norm_one) {
             if ((r = launch<CombineNormArgs>(e, k_combine_norm_one, dim3(1), dim3(kOneThreads), 0, cn))) return r;
             normed = true;
         } else if ((r = launch<CombineArgs>(e, k_combine, dim3(ew_grid((size_t)T * E)), dim3(256), 0, c))) return r;

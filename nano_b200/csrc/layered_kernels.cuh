@@ -548,10 +548,15 @@ __device__ __forceinline__ float block_sum(float v, float *red) {
     __syncthreads();
     if ((threadIdx.x & 31u) == 0) red[threadIdx.x >> 5] = v;
     __syncthreads();
-    // the warps' sums over the lanes: a loop over up to 32 of them is a chain of as many additions
-    float s = (threadIdx.x & 31u) < (blockDim.x >> 5) ? red[threadIdx.x & 31u] : 0.0f;
+    float s = 0.0f;          // in order, eight loads at a time (a loop of single loads waits for each of them)
+    const uint32_t nw = blockDim.x >> 5;
+    for (uint32_t w0 = 0; w0 < nw; w0 += 8u) {
+        float r[8];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        for (uint32_t w = 0; w < 8u; w++) r[w] = w0 + w < nw ? red[w0 + w] : 0.0f;
+#pragma unroll
+        for (uint32_t w = 0; w < 8u; w++) if (w0 + w < nw) s += r[w];
+    }
     return s;
 }
 
@@ -1291,46 +1296,32 @@ __global__ void k_combine(const CombineArgs a) {
 
 // scalar-gain RMS norm of the rows whose logits are asked for: out[i] = x[want[i]] / rms * g
 // (vec 1: the gain is a vector stored around zero, out = x / rms * (1 + g[i]); vec 2: a plain vector, out = x / rms * g[i])
-// Rows of at most 8192 columns (a multiple of 4) stay in registers between the sum and the result, their gains are asked for before the wait: the row of
+// Rows of at most 4096 columns stay in registers between the sum and the result (the same sums in the same order), their gains are asked for before the wait: the row of
 // 2048 that ends every step took 10 us as two walks of single loads, now 3.
 __global__ void __launch_bounds__(256) k_final_norm(const float *__restrict__ x, const uint32_t *__restrict__ want, const float *__restrict__ g,
                                                     float *__restrict__ out, uint32_t E, float eps, uint32_t vec) {
     pdl_launch_next();
     __shared__ float red[32];
-    auto at16 = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
-    const bool regs = E % 4u == 0 && E <= 8192u && at16(x) && at16(out) && (!vec || at16(g));
     const float gs = vec ? 0.0f : __ldg(g);
-    if (regs && vec) for (uint32_t i = threadIdx.x * 32u; i < E; i += 8192u) asm volatile("prefetch.global.L1 [%0];" ::"l"(g + i));
+    if (vec) for (uint32_t i = threadIdx.x * 32u; i < E; i += 8192u) asm volatile("prefetch.global.L1 [%0];" ::"l"(g + i));
     pdl_wait();
     const float *xt = x + (size_t)want[blockIdx.x] * E;
     float *o = out + (size_t)blockIdx.x * E;
-    float s = 0.0f;
+    float s = 0.0f, v[16];
+    const bool regs = E <= 4096u;
     if (regs) {
-        float4 v[8];
 #pragma unroll
-        for (uint32_t k = 0; k < 8u; k++) {
-            const uint32_t i = (threadIdx.x + k * 256u) * 4u;
-            v[k] = make_float4(0, 0, 0, 0);
-            if (i < E) v[k] = *reinterpret_cast<const float4 *>(xt + i);
-        }
+        for (uint32_t k = 0; k < 16u; k++) { const uint32_t i = threadIdx.x + k * 256u; v[k] = i < E ? xt[i] : 0.0f; }
 #pragma unroll
-        for (uint32_t k = 0; k < 8u; k++) s = fmaf(v[k].x, v[k].x, fmaf(v[k].y, v[k].y, fmaf(v[k].z, v[k].z, fmaf(v[k].w, v[k].w, s))));
-        s = block_sum(s, red);
-        const float rinv = 1.0f / sqrtf(s / (float)E + eps);
-#pragma unroll
-        for (uint32_t k = 0; k < 8u; k++) {
-            const uint32_t i = (threadIdx.x + k * 256u) * 4u;
-            if (i >= E) break;
-            float4 w = make_float4(gs, gs, gs, gs);
-            if (vec) { w = __ldg(reinterpret_cast<const float4 *>(g + i)); if (vec != 2u) { w.x += 1.0f; w.y += 1.0f; w.z += 1.0f; w.w += 1.0f; } }
-            *reinterpret_cast<float4 *>(o + i) = make_float4(v[k].x * rinv * w.x, v[k].y * rinv * w.y, v[k].z * rinv * w.z, v[k].w * rinv * w.w);
-        }
-        return;
-    }
-    for (uint32_t i = threadIdx.x; i < E; i += blockDim.x) s = fmaf(xt[i], xt[i], s);
+        for (uint32_t k = 0; k < 16u; k++) s = fmaf(v[k], v[k], s);
+    } else for (uint32_t i = threadIdx.x; i < E; i += blockDim.x) s = fmaf(xt[i], xt[i], s);
     s = block_sum(s, red);
     const float rinv = 1.0f / sqrtf(s / (float)E + eps);
-    for (uint32_t i = threadIdx.x; i < E; i += blockDim.x) o[i] = xt[i] * rinv * (vec ? (vec == 2u ? g[i] : 1.0f + g[i]) : gs);
+    auto put = [&](uint32_t i, float u) { o[i] = u * rinv * (vec ? (vec == 2u ? g[i] : 1.0f + g[i]) : gs); };
+    if (regs) {
+#pragma unroll
+        for (uint32_t k = 0; k < 16u; k++) { const uint32_t i = threadIdx.x + k * 256u; if (i < E) put(i, v[k]); }
+    } else for (uint32_t i = threadIdx.x; i < E; i += blockDim.x) put(i, xt[i]);
 }
 
 // greedy choice with the repetition penalty of the generation hosts: logits of ids seen before are divided (positive) or multiplied

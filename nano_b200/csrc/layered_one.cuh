@@ -34,17 +34,18 @@ __device__ __forceinline__ float load_now_f(const float *p) {
 template <typename WT> __device__ __forceinline__ uint32_t one_place(uint32_t c) {
     return sizeof(WT) == 2 ? (c & ~63u) + ((c & 1u) << 5) + ((c & 63u) >> 1) : c;
 }
-template <typename WT> __device__ __forceinline__ void one_fma(const uint4 &w, const float4 *x, uint32_t step, uint32_t lane, float &a0, float &a1) {
+// (one running sum in the order of the columns: the same bits as k_gemv where a row has one warp)
+template <typename WT> __device__ __forceinline__ void one_fma(const uint4 &w, const float4 *x, uint32_t step, uint32_t lane, float &acc) {
     if (sizeof(WT) == 2) {
         const float4 p = x[step * 64u + lane], q = x[step * 64u + 32u + lane];
-        a0 = fmaf(__uint_as_float(w.x << 16), p.x, a0); a1 = fmaf(__uint_as_float(w.x & 0xffff0000u), p.y, a1);
-        a0 = fmaf(__uint_as_float(w.y << 16), p.z, a0); a1 = fmaf(__uint_as_float(w.y & 0xffff0000u), p.w, a1);
-        a0 = fmaf(__uint_as_float(w.z << 16), q.x, a0); a1 = fmaf(__uint_as_float(w.z & 0xffff0000u), q.y, a1);
-        a0 = fmaf(__uint_as_float(w.w << 16), q.z, a0); a1 = fmaf(__uint_as_float(w.w & 0xffff0000u), q.w, a1);
+        acc = fmaf(__uint_as_float(w.x << 16), p.x, acc); acc = fmaf(__uint_as_float(w.x & 0xffff0000u), p.y, acc);
+        acc = fmaf(__uint_as_float(w.y << 16), p.z, acc); acc = fmaf(__uint_as_float(w.y & 0xffff0000u), p.w, acc);
+        acc = fmaf(__uint_as_float(w.z << 16), q.x, acc); acc = fmaf(__uint_as_float(w.z & 0xffff0000u), q.y, acc);
+        acc = fmaf(__uint_as_float(w.w << 16), q.z, acc); acc = fmaf(__uint_as_float(w.w & 0xffff0000u), q.w, acc);
     } else {
         const float4 p = x[step * 32u + lane];
-        a0 = fmaf(__uint_as_float(w.x), p.x, a0); a1 = fmaf(__uint_as_float(w.y), p.y, a1);
-        a0 = fmaf(__uint_as_float(w.z), p.z, a0); a1 = fmaf(__uint_as_float(w.w), p.w, a1);
+        acc = fmaf(__uint_as_float(w.x), p.x, acc); acc = fmaf(__uint_as_float(w.y), p.y, acc);
+        acc = fmaf(__uint_as_float(w.z), p.z, acc); acc = fmaf(__uint_as_float(w.w), p.w, acc);
     }
 }
 __device__ __forceinline__ float4 round4(float4 v) { return make_float4(round_bf16(v.x), round_bf16(v.y), round_bf16(v.z), round_bf16(v.w)); }
@@ -61,7 +62,7 @@ __device__ __forceinline__ void one_stage(const GemmArgs &a, const float *row, f
     for (uint32_t c = threadIdx.x; c < P4; c += kOneThreads) {
         float4 v = make_float4(0, 0, 0, 0);
         if (c < K4) v = src[c];
-        if (EXT != 4) s2 = sum_sq4(v, s2);
+        if (EXT == 2) s2 = sum_sq4(v, s2);
         if (EXT == 2) {
             const float q[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
@@ -86,6 +87,11 @@ __device__ __forceinline__ void one_stage(const GemmArgs &a, const float *row, f
             }
             __syncthreads();
         } else {
+            if (EXT != 2) {          // single values in k_gemv's order
+                __syncthreads();
+                const float *xf = reinterpret_cast<const float *>(x);
+                for (uint32_t k = threadIdx.x; k < a.K; k += kOneThreads) { const float v = xf[one_place<WT>(k / 4u) * 4u + (k & 3u)]; s2 = fmaf(v, v, s2); }
+            }
             s2 = block_sum(s2, red);
             if (EXT == 2 && poly) {
                 s4 = block_sum(s4, red); s6 = block_sum(s6, red);
@@ -201,15 +207,15 @@ __device__ __forceinline__ void gemv_one(const GemmArgs &a, uint32_t bx, uint32_
     one_stage<WT, EXT>(a, row, one_x, red);
 
     for (uint32_t base = bx * rpb, turn = 0; base < a.N; base += nrows, n += nrows, turn ^= 1u) {          // the same turns for all of the block's warps
-        float acc[NW][2];
+        float acc[NW];
 #pragma unroll
-        for (uint32_t h = 0; h < NW; h++) acc[h][0] = acc[h][1] = 0.0f;
+        for (uint32_t h = 0; h < NW; h++) acc[h] = 0.0f;
         for (uint32_t s0 = s_lo;;) {
 #pragma unroll
             for (uint32_t i = 0; i < PRE; i++)
                 if (s0 + i < s_hi) {
 #pragma unroll
-                    for (uint32_t h = 0; h < NW; h++) one_fma<WT>(w[h][i], one_x, s0 + i, lane, acc[h][0], acc[h][1]);
+                    for (uint32_t h = 0; h < NW; h++) one_fma<WT>(w[h][i], one_x, s0 + i, lane, acc[h]);
                 }
             s0 += PRE;
             if (s0 >= s_hi) break;
@@ -217,7 +223,7 @@ __device__ __forceinline__ void gemv_one(const GemmArgs &a, uint32_t bx, uint32_
         }
         const OneEpi now = e;
         if (n + nrows < a.N) { fetch(n + nrows, s_lo); if (!part) early(n + nrows); }          // on their way during the sum and the epilogue
-        float v = acc[0][0] + acc[0][1], up = NW == 2 ? acc[NW - 1u][0] + acc[NW - 1u][1] : 0.0f;
+        float v = acc[0], up = NW == 2 ? acc[NW - 1u] : 0.0f;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -336,38 +342,40 @@ __global__ void __launch_bounds__(kOneThreads) k_rglru_gates_one(const GatesScan
     a.S[c] = S;
 }
 
-// k_norm_shift for one token of at most 4096 columns (a multiple of 4): the row in registers, one trip to memory and one sum
-__global__ void __launch_bounds__(kOneThreads) k_norm_shift_one(const NormShiftArgs a) {
-    pdl_launch_next();
-    __shared__ float red[32];
-    const uint32_t E4 = a.E / 4u;
-    const float4 *x4 = reinterpret_cast<const float4 *>(a.x), *mu4 = reinterpret_cast<const float4 *>(a.mu);
-    float4 *st4 = reinterpret_cast<float4 *>(a.state);
-    float4 x[4], p[4], mu[4];
+// k_norm_shift for one token of at most 4096 columns: the row in registers, one trip to memory and one sum (in the same order), weights before the wait.  What the
+// combined kernel below shares with it: x[k], prev[k] are columns threadIdx.x + 256 k
+struct NormOne { float mu[16]; float g1, g2; };
+__device__ __forceinline__ void norm_one_weights(const NormShiftArgs &a, NormOne &w) {
 #pragma unroll
-    for (uint32_t i = 0; i < 4u; i++) { const uint32_t c = threadIdx.x + i * kOneThreads; mu[i] = make_float4(0, 0, 0, 0); if (mu4 && c < E4) mu[i] = __ldg(mu4 + c); }
-    const float g1 = __ldg(a.g1), g2 = a.g2 ? __ldg(a.g2) : 0.0f;
-    pdl_wait();
+    for (uint32_t k = 0; k < 16u; k++) { const uint32_t i = threadIdx.x + k * kOneThreads; w.mu[k] = a.mu && i < a.E ? __ldg(a.mu + i) : 0.0f; }
+    w.g1 = __ldg(a.g1); w.g2 = a.g2 ? __ldg(a.g2) : 0.0f;
+}
+__device__ __forceinline__ void norm_one_row(const NormShiftArgs &a, const NormOne &w, const float (&x)[16], const float (&prev)[16], float *red) {
     float s = 0.0f;
 #pragma unroll
-    for (uint32_t i = 0; i < 4u; i++) {
-        const uint32_t c = threadIdx.x + i * kOneThreads;
-        x[i] = p[i] = make_float4(0, 0, 0, 0);
-        if (c < E4) { x[i] = x4[c]; p[i] = st4[c]; }
-    }
-#pragma unroll
-    for (uint32_t i = 0; i < 4u; i++) s = sum_sq4(x[i], s);
+    for (uint32_t k = 0; k < 16u; k++) s = fmaf(x[k], x[k], s);
     s = block_sum(s, red);
     const float rinv = 1.0f / sqrtf(s / (float)a.E + a.eps);
 #pragma unroll
-    for (uint32_t i = 0; i < 4u; i++) {
-        const uint32_t c = threadIdx.x + i * kOneThreads;
-        if (c >= E4) break;
-        const float4 u = make_float4(x[i].x * rinv, x[i].y * rinv, x[i].z * rinv, x[i].w * rinv), n1 = make_float4(u.x * g1, u.y * g1, u.z * g1, u.w * g1);
-        reinterpret_cast<float4 *>(a.hm)[c] = !mu4 ? n1 : make_float4(fmaf(p[i].x - n1.x, mu[i].x, n1.x), fmaf(p[i].y - n1.y, mu[i].y, n1.y), fmaf(p[i].z - n1.z, mu[i].z, n1.z), fmaf(p[i].w - n1.w, mu[i].w, n1.w));
-        if (a.h2) reinterpret_cast<float4 *>(a.h2)[c] = make_float4(u.x * g2, u.y * g2, u.z * g2, u.w * g2);
-        st4[c] = n1;
+    for (uint32_t k = 0; k < 16u; k++) {
+        const uint32_t i = threadIdx.x + k * kOneThreads;
+        if (i >= a.E) break;
+        const float u = x[k] * rinv, n1 = u * w.g1;
+        a.hm[i] = a.mu ? n1 + (prev[k] - n1) * w.mu[k] : n1;
+        if (a.h2) a.h2[i] = u * w.g2;
+        a.state[i] = n1;
     }
+}
+__global__ void __launch_bounds__(kOneThreads) k_norm_shift_one(const NormShiftArgs a) {
+    pdl_launch_next();
+    __shared__ float red[32];
+    NormOne w;
+    norm_one_weights(a, w);
+    pdl_wait();
+    float x[16], p[16];
+#pragma unroll
+    for (uint32_t k = 0; k < 16u; k++) { const uint32_t i = threadIdx.x + k * kOneThreads; x[k] = i < a.E ? a.x[i] : 0.0f; p[k] = i < a.E ? a.state[i] : 0.0f; }
+    norm_one_row(a, w, x, p, red);
 }
 
 // k_combine of one token and k_norm_shift_one of the run that follows, in one link: the updated row stays in the registers of the block that norms it
@@ -376,63 +384,43 @@ __global__ void __launch_bounds__(kOneThreads) k_combine_norm_one(const CombineN
     pdl_launch_next();
     __shared__ float red[32];
     const CombineArgs &c = a.c;
-    const NormShiftArgs &m = a.n;
-    const uint32_t E4 = m.E / 4u;
-    auto row = [&](const float *p, uint32_t i) { return reinterpret_cast<const float4 *>(p)[i]; };
-    float4 x[4], p[4], mu[4];
-#pragma unroll
-    for (uint32_t k = 0; k < 4u; k++) {          // the state is the token before's, the shift a weight
-        const uint32_t i = threadIdx.x + k * kOneThreads;
-        mu[k] = p[k] = make_float4(0, 0, 0, 0);
-        if (i < E4) { if (m.mu) mu[k] = __ldg(reinterpret_cast<const float4 *>(m.mu) + i); }
-    }
-    const float g1 = __ldg(m.g1), g2 = m.g2 ? __ldg(m.g2) : 0.0f;
+    NormOne w;
+    norm_one_weights(a.n, w);
     pdl_wait();
     uint32_t slot[4]; float wt[4];
 #pragma unroll
     for (uint32_t j = 0; j < 4u; j++) { slot[j] = 0; wt[j] = 0.0f; if (c.eo && j < c.top) { slot[j] = c.slot[j]; wt[j] = c.wt[j]; } }
-    float4 d[4], sh[4];
+    float x[16], p[16], d[16], sh[16];
 #pragma unroll
-    for (uint32_t k = 0; k < 4u; k++) {
+    for (uint32_t k = 0; k < 16u; k++) {
         const uint32_t i = threadIdx.x + k * kOneThreads;
-        x[k] = d[k] = sh[k] = make_float4(0, 0, 0, 0);
-        if (i < E4) { x[k] = row(c.x, i); d[k] = row(c.d, i); p[k] = row(m.state, i); if (c.eo && c.shared) sh[k] = row(c.shared, i); }
+        x[k] = p[k] = d[k] = sh[k] = 0.0f;
+        if (i < c.E) { x[k] = c.x[i]; d[k] = c.d[i]; p[k] = a.n.state[i]; if (c.eo && c.shared) sh[k] = c.shared[i]; }
     }
-    float s = 0.0f;
 #pragma unroll
-    for (uint32_t k = 0; k < 4u; k++) {
+    for (uint32_t k = 0; k < 16u; k++) {
         const uint32_t i = threadIdx.x + k * kOneThreads;
-        if (i >= E4) continue;
+        if (i >= c.E) break;
+        float delta = d[k];
         if (c.eo) {
-            float4 f = make_float4(0, 0, 0, 0);
-            auto add = [&](float w, uint32_t at) { const float4 v = row(c.eo + (size_t)at * m.E, i); f.x = fmaf(w, v.x, f.x); f.y = fmaf(w, v.y, f.y); f.z = fmaf(w, v.z, f.z); f.w = fmaf(w, v.w, f.w); };
+            float f = 0.0f;
 #pragma unroll
-            for (uint32_t j = 0; j < 4u; j++) if (j < c.top) add(wt[j], slot[j]);
-            for (uint32_t j = 4u; j < c.top; j++) add(c.wt[j], c.slot[j]);
-            d[k].x += f.x + sh[k].x; d[k].y += f.y + sh[k].y; d[k].z += f.z + sh[k].z; d[k].w += f.w + sh[k].w;
+            for (uint32_t j = 0; j < 4u; j++) if (j < c.top) f = fmaf(wt[j], c.eo[(size_t)slot[j] * c.E + i], f);
+            for (uint32_t j = 4u; j < c.top; j++) f = fmaf(c.wt[j], c.eo[(size_t)c.slot[j] * c.E + i], f);
+            if (c.shared) f += sh[k];
+            delta += f;
         }
-        x[k].x += d[k].x; x[k].y += d[k].y; x[k].z += d[k].z; x[k].w += d[k].w;
-        reinterpret_cast<float4 *>(c.x)[i] = x[k];
-        if (c.keep) reinterpret_cast<float4 *>(c.keep)[i] = x[k];
-        s = sum_sq4(x[k], s);
+        x[k] += delta;
+        c.x[i] = x[k];
+        if (c.keep) c.keep[i] = x[k];
     }
-    s = block_sum(s, red);
-    const float rinv = 1.0f / sqrtf(s / (float)m.E + m.eps);
-#pragma unroll
-    for (uint32_t k = 0; k < 4u; k++) {
-        const uint32_t i = threadIdx.x + k * kOneThreads;
-        if (i >= E4) break;
-        const float4 u = make_float4(x[k].x * rinv, x[k].y * rinv, x[k].z * rinv, x[k].w * rinv), n1 = make_float4(u.x * g1, u.y * g1, u.z * g1, u.w * g1);
-        reinterpret_cast<float4 *>(m.hm)[i] = !m.mu ? n1 : make_float4(fmaf(p[k].x - n1.x, mu[k].x, n1.x), fmaf(p[k].y - n1.y, mu[k].y, n1.y), fmaf(p[k].z - n1.z, mu[k].z, n1.z), fmaf(p[k].w - n1.w, mu[k].w, n1.w));
-        if (m.h2) reinterpret_cast<float4 *>(m.h2)[i] = make_float4(u.x * g2, u.y * g2, u.z * g2, u.w * g2);
-        reinterpret_cast<float4 *>(m.state)[i] = n1;
-    }
+    norm_one_row(a.n, w, x, p, red);
 }
 
 // k_route_small for one token and at most 32 rows of the router: the same choice, weights and places (RouteArgs, route_pick), in registers.  A cluster of blocks
 // shares the logits, with the router's rows in registers before the wait; the first block's first warp then holds an expert per lane, and everything it leaves is written
 // once, by the lane that has it.  (k_route_small keeps the choice in memory and reads it back: 27 us of the chain of a step with eight routed layers, now 6.)
-constexpr uint32_t kRouteOneThreads = 256;
+constexpr uint32_t kRouteOneThreads = 512;          // as k_route_small: the same shares of a row, the same sums
 __global__ void __launch_bounds__(kRouteOneThreads) k_route_one(const RouteArgs a) {
     pdl_launch_next();
     cluster_arrive();                          // waited for before the first access to another block's shared memory
