@@ -5,7 +5,8 @@
 // registers by then, constants of the epilogue too.  After it the block brings the activation row into shared memory ONCE, normed and rounded there, with a
 // single trip to L2, and the epilogue's operands travel at the same time; what is left is the row's dot from registers and shared memory.
 // k_gemv, which serves up to four rows and any alignment, reads the row in every warp, converts it there, and its epilogue starts a trip of its own.
-// A chain of 1024 x 1024 products from HBM, us a link: k_gemv 4.5, weights in registers 2.9, this 2.1.
+// A chain of 1024 x 1024 products from HBM, us a link: k_gemv 4.5, weights in registers 2.9, this 2.1 (with two
+// running sums; one, in k_gemv's order, makes a whole step of eight routed layers bit for bit that of the general kernels: 290 us a token, 265 with two, 364 before).
 #pragma once
 #include "layered_kernels.cuh"
 #include "layered_mixers3.cuh"
@@ -419,7 +420,8 @@ __global__ void __launch_bounds__(kOneThreads) k_combine_norm_one(const CombineN
 
 // k_route_small for one token and at most 32 rows of the router: the same choice, weights and places (RouteArgs, route_pick), in registers.  A cluster of blocks
 // shares the logits, with the router's rows in registers before the wait; the first block's first warp then holds an expert per lane, and everything it leaves is written
-// once, by the lane that has it.  (k_route_small keeps the choice in memory and reads it back: 27 us of the chain of a step with eight routed layers, now 6.)
+// once, by the lane that has it.  (k_route_small keeps the choice in memory and reads it back: 27 us of the chain of a step with eight routed layers; 6 here
+// with 256 threads. 512 give each thread the share of a row that it has there, and so its sums: close calls between experts fall the same way.)
 constexpr uint32_t kRouteOneThreads = 512;          // as k_route_small: the same shares of a row, the same sums
 __global__ void __launch_bounds__(kRouteOneThreads) k_route_one(const RouteArgs a) {
     pdl_launch_next();
