@@ -243,8 +243,10 @@ __device__ __forceinline__ void st_prep(const StreamArgs &g, const unsigned long
         const float4 *r4 = reinterpret_cast<const float4 *>(red);   // red[15] stays 0
         const float4 a = r4[0], b = r4[1], c = r4[2], e = r4[3];
         const float tot = (((a.x + a.y) + (a.z + a.w)) + ((b.x + b.y) + (b.z + b.w))) + (((c.x + c.y) + (c.z + c.w)) + ((e.x + e.y) + (e.z + e.w)));
-        const float q = tot * rn;                                   // tot / n, rounded: the product by the rounded reciprocal with its remainder added back
-        return __frcp_rn(__fsqrt_rn(__fadd_rn(fmaf(fmaf(-q, (float)n, tot), rn, q), 1e-5f)));
+        // tot / n, rounded: the product by the rounded reciprocal with its remainder added back (Markstein's final step of a quotient, IBM J. Res. Dev. 34, 1990).  An
+        // infinite sum has no remainder (inf - inf): it stays, and the row norms to zeros as on every other path
+        const float q = tot * rn, mean = tot < INFINITY ? fmaf(fmaf(-q, (float)n, tot), rn, q) : tot;
+        return __frcp_rn(__fsqrt_rn(__fadd_rn(mean, 1e-5f)));
     };
     if constexpr (QUANT == 0x42) {
         uint32_t *xe = reinterpret_cast<uint32_t *>(act);

@@ -78,3 +78,35 @@ def test_logits_are_those_of_the_last_step(monkeypatch):
     assert np.array_equal(d, device()) and not np.array_equal(c, d)
     assert eng.next_greedy(ids, 19, 0) == int(np.argmax(eng.logits()))
     eng.close()
+
+
+@pytest.mark.parametrize("quant,gs", [(mf.QUANT_F32, 128), (mf.QUANT_Q80, 64), (mf.QUANT_Q80, 128), (mf.QUANT_Q4K, 128)])
+@pytest.mark.parametrize("arch", [mf.ARCH_NANO, mf.ARCH_QWEN3])
+def test_rows_whose_squares_overflow(arch, quant, gs, monkeypatch, tmp_path):
+    """The sum of squares of every third token's row is infinite in 32 bits and one over its root zero: such a row norms to zeros, as in the oracle, and gives zeros
+    for logits and for its keys and values; the tokens between have theirs within the bounds above (Q4K: as finite numbers)."""
+    monkeypatch.setenv("NB200_STREAM", "1")
+    spec = mf.ModelSpec("overflow-%d-%d-%d" % (arch, quant, gs), arch, 128, 96, 2, 256, 4, 2, 256, 64)
+    rng = np.random.default_rng(11)
+    L, W, F, Q, K = spec.n_layer, spec.n_embd, spec.n_hidden, spec.q_dim, spec.kv_dim
+    shapes = {"attn_norm": (L, W), "ffn_norm": (L, W), "final_norm": (W,), "emb": (spec.vocab, W), "wq": (L, Q, W), "wk": (L, K, W), "wv": (L, K, W), "wo": (L, W, Q), "w1": (L, F, W), "w2": (L, W, F), "w3": (L, F, W)}
+    if arch == mf.ARCH_QWEN3:
+        shapes.update(q_norm=(L, spec.hd), k_norm=(L, spec.hd))
+    w = {k: (1.0 if "norm" in k else 0.0) + rng.standard_normal(s).astype(np.float32) * np.float32(0.05) for k, s in shapes.items()}
+    w["emb"][::3] *= np.float32(2.0 ** 70)
+    path = str(tmp_path / "overflow.bin")
+    mf.write_model_from_weights(path, spec, quant, gs, w)
+    eng, o = E.Engine(path, 64), ob.NanoOracle(path, 64)
+    assert eng.path.startswith("streaming"), eng.path
+    small = np.arange(spec.vocab) % 3 != 0          # (the classifier's rows are the embedding's)
+    toks = np.array([4, 6, 7, 9, 12, 5, 8, 10, 3, 11, 13, 15, 2], np.uint32)
+    for pos, t in enumerate(toks):
+        a, b = eng.forward(int(t), pos), o.forward(int(t), pos)
+        if t % 3 == 0:
+            assert not a.any() and not b.any(), pos
+        elif quant == mf.QUANT_Q4K:
+            assert np.isfinite(a).all() and a[small].any(), pos
+        else:
+            assert np.linalg.norm((a - b)[small]) <= (1e-5 if quant == mf.QUANT_F32 else 2e-2) * np.linalg.norm(b[small]), pos
+    eng.close()
+    o.close()
