@@ -465,7 +465,9 @@ __global__ void __launch_bounds__(kRouteOneThreads) k_route_one(const RouteArgs 
     const bool expert = lane < a.NE;
     float z = lane < NL ? z_s[lane] : -INFINITY;
     if (lane >= a.NE && lane < NL) a.extra_out[lane - a.NE] = z;
-    // the largest of `v` over the lanes below n (ties: the lower lane)
+    // the largest of `v` over the lanes below n (ties: the lower lane).  A score that is no number compares with nothing, so the lanes may end with different answers:
+    // the first lane's counts, as in route_pick
+    const bool odd = __any_sync(0xffffffffu, z != z);
     auto argmax = [&](float v, uint32_t n, float *value) {
         float best = lane < n ? v : -INFINITY; uint32_t bi = lane < n ? lane : 0xffffffffu;
 #pragma unroll
@@ -473,6 +475,7 @@ __global__ void __launch_bounds__(kRouteOneThreads) k_route_one(const RouteArgs 
             const float ov = __shfl_xor_sync(0xffffffffu, best, o); const uint32_t oi = __shfl_xor_sync(0xffffffffu, bi, o);
             if (oi != 0xffffffffu && (bi == 0xffffffffu || ov > best || (ov == best && oi < bi))) { best = ov; bi = oi; }
         }
+        if (odd) { best = __shfl_sync(0xffffffffu, best, 0); bi = __shfl_sync(0xffffffffu, bi, 0); }
         *value = best;
         return bi;
     };

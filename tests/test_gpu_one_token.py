@@ -9,6 +9,7 @@ import pytest
 from nano_b200 import engine as E, modeldir as md
 import famudra_oracle as A
 import fidatar_oracle as F
+import gokinex_oracle as G
 import kadesun_oracle as K
 
 pytestmark = pytest.mark.gpu
@@ -65,6 +66,33 @@ def test_one_token_routes(tmp_path, experts, top, count, keep):
     r = np.linalg.norm(got - want, axis=1) / np.linalg.norm(want, axis=1)
     assert np.median(r) < BOUND[True] and (r < BOUND[True]).mean() >= 0.95          # (a choice closer than 2^-24 may fall either way)
     eng.close()
+
+
+# Scores that are no number or minus infinity: router rows with infinite weights over inputs that the norm makes 1.  The choice is the one of the general kernels: the
+# first lane's of a warp that looks for the largest (a NaN compares with nothing).  It is that of a finite router which chooses `chosen` only.
+@pytest.mark.parametrize("rows,top,chosen", [(["0.1", "0.2", "0.3", "nan"], 2, [2, 1]), (["0.1", "0.2", "0.3", "nan"], 3, [2, 1, 0]), (["0.1", "nan", "0.4", "0.2", "nan"], 2, [2, 0]), (["nan", "0.2", "0.3"], 2, None)])
+def test_one_token_routes_of_odd_scores(tmp_path, rows, top, chosen):
+    n, toks = len(rows), np.random.default_rng(2).integers(0, 97, size=12).astype(np.uint32)
+
+    def model(values, top):
+        cfg = md.gokinex_config(97, 64, [("mamba2", {"heads": 2, "vdim": 16, "state": 16, "groups": 1, "conv": 4, "norm_groups": 1}, {"kind": "moe", "router": {"experts": n, "top": top}, "expert": {"ff": 40}})])
+        w = md.gokinex_random(cfg, 5)
+        w["l0.norm2"][:], w["l0.norm2.b"][:] = 0.0, 1.0          # the experts and the router read a row of ones
+        r = w["l0.mlp.router"]
+        r[:] = 0.0
+        for e, v in enumerate(values):
+            r[e, 7] = float(v) if v not in ("-inf", "nan") else 0.0
+            r[e, 3], r[e, 40] = -np.inf if v in ("-inf", "nan") else 0.0, np.inf if v == "nan" else 0.0
+        return cfg, w
+    cfg, w = model(rows, top)
+    eng = E.Engine(md.write_model_dir(str(tmp_path / "m"), cfg, w), 64, flags=E.FLAG_F32)
+    got = one_by_one(eng, toks)
+    eng.close()
+    if chosen is None:
+        assert np.isnan(got).all()
+        return
+    cfg, w = model([md.bf16_round(np.float32(v)) if e in chosen else -50.0 for e, v in enumerate(rows)], len(chosen))
+    assert off(got, G.forward(cfg, w, toks)) < BOUND[True]
 
 
 @pytest.mark.parametrize("design,width,ff", [("famudra", 64, 20), ("kadesun", 132, 516), ("fidatar", 516, 1028), ("famudra", 1024, 256)])
