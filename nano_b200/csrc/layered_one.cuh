@@ -117,6 +117,32 @@ __device__ __forceinline__ void one_stage(const GemmArgs &a, const float *row, f
 // what a column's epilogue reads from memory, asked for long before it is needed (tap, tail: lane j holds those of tap j)
 struct OneEpi { float bias, mul, tap, tail, x, pw, pb, nw, nb; };
 
+// Rows of a group past its first, where they are not the same: block bx's columns of them, the row from memory.  Such rows come from choices that tie at minus infinity,
+// which no trained model makes: what counts is that the products of all others pay nothing for it, so everything is found anew here and nothing is kept from there.
+template <typename WT>
+__device__ __forceinline__ void one_more_rows(const GemmArgs &a, uint32_t bx, uint32_t nbx, uint32_t gy) {
+    constexpr uint32_t VN = WVec<WT>::N;
+    const GroupView gv = group_view(a, a.g_act ? a.g_act[gy] : gy);
+    const uint32_t lane = threadIdx.x & 31u;
+#pragma unroll 1
+    for (uint32_t i = 1; i < gv.rows; i++) {
+        const float *row = a.A + (size_t)(gv.r0 + i) * a.lda + gv.a0;
+#pragma unroll 1
+        for (uint32_t n = bx * kOneWarps + (threadIdx.x >> 5); n < a.N; n += nbx * kOneWarps) {
+            float v = 0.0f, w[VN];
+#pragma unroll 1
+            for (uint32_t k = lane * VN; k < a.K; k += 32u * VN) {
+                WVec<WT>::load(static_cast<const WT *>(a.W) + gv.w0 + (size_t)n * a.ldw + k, w);
+#pragma unroll
+                for (uint32_t j = 0; j < VN; j++) v = fmaf(w[j], a.round_a ? round_bf16(row[k + j]) : row[k + j], v);
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (lane == 0) store_c(a, a.C + (size_t)(gv.r0 + i) * a.ldc + gv.c0 + n, gated(a, epilogue(v, a, gv.bias, n), gv.r0 + i, gv.c0 + n));
+        }
+    }
+}
+
 // Block bx of nbx, place gy in the list of groups; a group has one row, or several of the same token.  The instances (EXT) are k_gemv's.
 template <typename WT, int EXT>
 __device__ __forceinline__ void gemv_one(const GemmArgs &a, uint32_t bx, uint32_t nbx, uint32_t gy) {
@@ -150,7 +176,7 @@ __device__ __forceinline__ void gemv_one(const GemmArgs &a, uint32_t bx, uint32_
         if (a.a_norm_w) for (uint32_t k = threadIdx.x * 32u; k < a.K; k += kOneThreads * 32u) asm volatile("prefetch.global.L1 [%0];" ::"l"(a.a_norm_w + k));
     }
     // arguments that are read after the wait: a launch's arguments lie in memory that no cache near the SM holds yet
-    uint32_t group = gy, r0 = 0, rows = 1;          // (several rows of one expert hold the same token: choices that tie at -infinity)
+    uint32_t group = gy, r0 = 0, rows = 1;          // (several rows of one expert: choices that tie at -infinity)
     const float *bias = a.bias, *row = a.A;
     float *C = a.C;
     auto place = [&]() {          // of the group
@@ -265,8 +291,10 @@ __device__ __forceinline__ void gemv_one(const GemmArgs &a, uint32_t bx, uint32_
             a.res_x[at] = xv;
             if (a.res_keep) a.res_keep[at] = xv;
             if (a.res_out) a.res_out[at] = fmaf(tanhf(a.res_na * xv), now.nw, now.nb);
-        } else for (uint32_t i = 0; i < rows; i++) store_c(a, dst + (size_t)i * a.ldc, a.mul ? v * now.mul : v);
+        } else for (uint32_t i = 0; i < (EXT == 0 && !a.a_rows ? 1u : rows); i++) store_c(a, dst + (size_t)i * a.ldc, a.mul ? v * now.mul : v);
     }
+    // rows that name a token are all the same; those of the second product, whose input was weighted by the choice, are not
+    if (EXT == 0 && rows > 1u && !a.a_rows) one_more_rows<WT>(a, bx, nbx, gy);
 }
 
 template <typename WT, int EXT>

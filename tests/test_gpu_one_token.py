@@ -70,7 +70,10 @@ def test_one_token_routes(tmp_path, experts, top, count, keep):
 
 # Scores that are no number or minus infinity: router rows with infinite weights over inputs that the norm makes 1.  The choice is the one of the general kernels: the
 # first lane's of a warp that looks for the largest (a NaN compares with nothing).  It is that of a finite router which chooses `chosen` only.
-@pytest.mark.parametrize("rows,top,chosen", [(["0.1", "0.2", "0.3", "nan"], 2, [2, 1]), (["0.1", "0.2", "0.3", "nan"], 3, [2, 1, 0]), (["0.1", "nan", "0.4", "0.2", "nan"], 2, [2, 0]), (["nan", "0.2", "0.3"], 2, None)])
+@pytest.mark.parametrize("rows,top,chosen", [(["0.1", "0.2", "0.3", "nan"], 2, [2, 1]), (["0.1", "0.2", "0.3", "nan"], 3, [2, 1, 0]), (["0.1", "nan", "0.4", "0.2", "nan"], 2, [2, 0]), (["nan", "0.2", "0.3"], 2, None),
+                                             # rows of one expert that differ: taken with its weight and, tied at minus infinity, once more with weight 0
+                                             (["1", "-inf", "-inf", "-inf"], 2, [0]), (["1", "-inf", "-inf", "-inf"], 4, [0]), (["-inf", "0.5", "-inf", "-inf"], 3, [1]), (["0.1", "0.2", "0.3", "nan"], 4, [2, 1, 0]),
+                                             (["0.1", "nan", "0.4", "0.2", "nan"], 4, [2, 0])])
 def test_one_token_routes_of_odd_scores(tmp_path, rows, top, chosen):
     n, toks = len(rows), np.random.default_rng(2).integers(0, 97, size=12).astype(np.uint32)
 
