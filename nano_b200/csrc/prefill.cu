@@ -487,7 +487,7 @@ __global__ void __launch_bounds__(256) k_prompt_attn(const PromptAttnArgs a) {
     const float *K = a.kc + (size_t)g * a.max_seq * hd, *V = a.vc + (size_t)g * a.max_seq * hd, *q = a.q + ((size_t)t * a.H + h) * hd;
     if (lane * 4u < hd) *reinterpret_cast<float4 *>(&q_s[warp][lane * 4u]) = *reinterpret_cast<const float4 *>(q + lane * 4u);
     __syncwarp();
-    float m = -INFINITY, l = 0.0f;
+    float m = -FLT_MAX, l = 0.0f;          // (finite, so that a turn whose keys all score minus infinity weighs nothing: -inf - -inf would be no number)
     float4 o = make_float4(0, 0, 0, 0);
     for (uint32_t k0 = 0; k0 < nkeys; k0 += 32u) {
         const uint32_t n = min(32u, nkeys - k0);

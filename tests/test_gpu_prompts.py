@@ -142,6 +142,42 @@ def test_a_wide_range_inside_a_matrix_and_a_row(tmp_path):
     check_file(path, spec, mf.QUANT_F32, (10, 65, 130), 300)
 
 
+def small_weights(spec, seed):
+    rng = np.random.default_rng(seed)
+    L, W, F, Q, K = spec.n_layer, spec.n_embd, spec.n_hidden, spec.q_dim, spec.kv_dim
+    shapes = {"attn_norm": (L, W), "ffn_norm": (L, W), "final_norm": (W,), "emb": (spec.vocab, W), "wq": (L, Q, W), "wk": (L, K, W), "wv": (L, K, W), "wo": (L, W, Q), "w1": (L, F, W), "w2": (L, W, F), "w3": (L, F, W)}
+    return {k: (1.0 if "norm" in k else 0.0) + rng.standard_normal(s).astype(np.float32) * np.float32(0.05) for k, s in shapes.items()}
+
+
+def test_keys_that_score_minus_infinity(tmp_path):
+    """Forty keys whose score with the last ten queries is below the range of 32 bits, then finite ones: such keys weigh nothing, however many come first."""
+    spec = dataclasses.replace(mf.PRESETS["toy-nano"], name="minus-infinity", block_size=512)
+    w = small_weights(spec, 3)
+    hd = spec.hd
+    for h in range(spec.q_dim // hd):          # the last pair of a head turns least: 50 positions leave its sign
+        w["wq"][0, h * hd + hd - 2:(h + 1) * hd] = 0.0
+        w["wq"][0, h * hd + hd - 1, 1] = 1e20
+    for h in range(spec.kv_dim // hd):
+        w["wk"][0, h * hd + hd - 2:(h + 1) * hd] = 0.0
+        w["wk"][0, h * hd + hd - 1, 0] = -1e20
+    w["emb"][:, :2] = 0.0
+    w["emb"][:40, 0], w["emb"][40:, 1] = 1.0, 1.0          # tokens below 40 have the keys, the others the queries
+    path = str(tmp_path / "minus-infinity.bin")
+    mf.write_model_from_weights(path, spec, mf.QUANT_F32, 128, w)
+    toks = np.concatenate([np.arange(40), np.arange(60, 70)]).astype(np.uint32)
+    eng = E.Engine(path, 100)
+    for p, t in enumerate(toks):
+        eng.forward_nolog(int(t), p)
+    want = [rows(eng, spec, 1, p) for p in range(toks.size - 1)]
+    assert np.isfinite(want).all()
+    ids = np.zeros(toks.size + 1, np.uint32)
+    ids[:-1] = toks
+    eng.decode_greedy(ids, toks.size, toks.size + 1)
+    for p in (0, 31, 32, 39, 40, 44, 48):
+        assert rel(rows(eng, spec, 1, p), want[p]) < 1e-5, p
+    eng.close()
+
+
 def test_portions_keep_no_copy_of_the_weights():
     """What prompts in portions need beside the model does not grow with its layers: an F32 file opened with them (fast mode) and without (exact mode)."""
     spec = dataclasses.replace(mf.PRESETS["mini-nano"], name="mini-nano-deep", n_layer=12, block_size=512)
