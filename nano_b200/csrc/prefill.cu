@@ -154,7 +154,8 @@ __global__ void __launch_bounds__(kRowThreads) k_prompt_rows(const PromptPrepArg
             if (Q80) {
                 float amax = fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w)));
                 for (uint32_t o = 1; o < LG; o <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-                // rounded by adding 1.5 * 2^23; what lies within 1e-4 of a .5 boundary takes the exact division (the product is at most 2.3e-5 from the quotient)
+                // rounded by adding 1.5 * 2^23; what lies within 1e-4 of a .5 boundary takes the exact division (the product is at most 2.3e-5 from the quotient), and so
+                // does what is no number or out of range (the sum's low bits say nothing then)
                 const float sc = __fdiv_rn(amax, 127.0f), rinv = __frcp_rn(sc), magic = 12582912.0f;
                 const float q[4] = {x.x * rinv, x.y * rinv, x.z * rinv, x.w * rinv}, xv[4] = {x.x, x.y, x.z, x.w};
                 uint32_t pk = 0;
@@ -162,7 +163,7 @@ __global__ void __launch_bounds__(kRowThreads) k_prompt_rows(const PromptPrepArg
 #pragma unroll
                     for (int e = 0; e < 4; e++) {
                         const float r = q[e] + magic;
-                        const uint32_t c = fabsf(q[e] - (r - magic)) > 0.4999f ? (uint32_t)q80_code_slow(xv[e], sc) : __float_as_uint(r);
+                        const uint32_t c = fabsf(q[e] - (r - magic)) <= 0.4999f ? __float_as_uint(r) : (uint32_t)q80_code_slow(xv[e], sc);
                         pk |= (c & 0xffu) << (8 * e);
                     }
                 if (i < a.n) {

@@ -178,6 +178,32 @@ def test_keys_that_score_minus_infinity(tmp_path):
     eng.close()
 
 
+@pytest.mark.parametrize("gs", [32, 64, 128, 256])
+def test_a_hidden_unit_that_is_not_a_number(gs, tmp_path):
+    """A product beyond the range of 32 bits makes one hidden unit of every prompt position minus infinity times zero.  Its activation code is 0 (what the reference's
+    conversion gives), in portions as on the path of one kernel per phase."""
+    spec = dataclasses.replace(mf.PRESETS["toy-nano"], name="no-number", block_size=512)
+    w = small_weights(spec, 4)
+    w["emb"][:, 0] = 1.0
+    w["w1"][0, 7] = 0.0
+    w["w1"][0, 7, 0] = -3e38
+    w["w2"][0, :, 7] = 3.0
+    path = str(tmp_path / "no-number.bin")
+    mf.write_model_from_weights(path, spec, mf.QUANT_Q80, gs, w)
+    toks = mf.teacher_tokens(20, spec.vocab).astype(np.uint32)
+    ref = E.Engine(path, 100, flags=E.FLAG_NO_STREAM)
+    for p, t in enumerate(toks):
+        ref.forward_nolog(int(t), p)
+    eng = E.Engine(path, 100)
+    ids = np.zeros(toks.size + 1, np.uint32)
+    ids[:-1] = toks
+    eng.decode_greedy(ids, toks.size, toks.size + 1)
+    for p in range(toks.size - 1):
+        assert rel(rows(eng, spec, 1, p), rows(ref, spec, 1, p)) < 4e-2, p
+    eng.close()
+    ref.close()
+
+
 def test_portions_keep_no_copy_of_the_weights():
     """What prompts in portions need beside the model does not grow with its layers: an F32 file opened with them (fast mode) and without (exact mode)."""
     spec = dataclasses.replace(mf.PRESETS["mini-nano"], name="mini-nano-deep", n_layer=12, block_size=512)
