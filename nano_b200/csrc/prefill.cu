@@ -33,8 +33,11 @@ namespace nb {
 namespace {
 
 constexpr uint32_t kChunk = 1024, kRows = 128;
-constexpr uint64_t kPromptAttnWork = 50 * 50;          // positions x keys up to which k_prompt_attn is ahead: Nano-168M (16 heads of 48) 16 positions 1.02 ms against 1.33 on the
-                                                       // tensor cores, 40 1.27 / 1.47; Qwen3-0.6B (16 of 128) 33 1.59 / 1.92, 65 2.29 / 2.09
+// Positions up to which a prompt's first portion has k_prompt_attn; longer ones, and what remains behind a whole portion (its walk of the keys is serial: 1 position behind 1024
+// of them 2 to 4 times as slow), have the tensor cores.  Eight layers, us, k_prompt_attn / tensor cores at 16, 33, 40, 50 and 64 positions: 16 heads of 48 323 / 402, 383 / 439,
+// 394 / 440, 419 / 449, 440 / 460; 8 of 64 310 / 389, 371 / 429, 375 / 430, 382 / 432, 407 / 445; 64 of 64 415 / 485, 480 / 510, 507 / 505, 533 / 514, 565 / 521; 16 of 128
+// 401 / 494, 476 / 533, 530 / 537, 606 / 551, 656 / 568; 32 of 128 633 / 734, 766 / 788, 814 / 803, 859 / 801; 64 of 128 522 / 618, 611 / 638, 658 / 631, 703 / 642.
+constexpr uint32_t kPromptAttnFew = 50, kPromptAttnFewWide = 36;          // heads of at most 64 values and at most 16 of them; others
 enum { PREP_NORM = 0, PREP_PLAIN = 1, PREP_SWIGLU = 2 };
 
 __device__ __forceinline__ void dep_enter() { asm volatile("griddepcontrol.launch_dependents;\ngriddepcontrol.wait;" ::: "memory"); }
@@ -692,7 +695,7 @@ int prefill_run(PrefillState *s, const uint32_t *ids, uint32_t n, cudaStream_t s
             TcAttn a{};
             a.q = s->q; a.ldq = m.q_dim; a.q_head = m.hd; a.k = m.kc + l * kvl; a.v = m.vc + l * kvl; a.ldk = a.ldv = m.hd; a.k_head = a.v_head = (uint64_t)m.max_seq * m.hd;
             a.out = s->o; a.T = T; a.H = m.H; a.G = m.KV; a.D = a.VD = m.hd; a.pos0 = p0; a.scale = (float)(1.0 / sqrt((double)m.hd));
-            const bool few = (uint64_t)T * (p0 + T) <= kPromptAttnWork;
+            const bool few = p0 == 0 && T <= (m.hd <= 64u && m.H <= 16u ? kPromptAttnFew : kPromptAttnFewWide);
             const PromptAttnArgs pa{s->q, m.kc + l * kvl, m.vc + l * kvl, s->o, m.H, m.KV, m.hd, m.max_seq, p0, a.scale};
             if (!few && !attn_tc_fits(&s->attn, a)) return fail(NB200_EINVAL, "a prompt of %u positions does not fit the attention's buffers", n);
             if ((r = few ? launch<PromptAttnArgs>(k_prompt_attn, dim3(T, (m.H + 7u) / 8u), dim3(256), 0, stream, pdl, pa) : attn_tc_launch(&s->attn, a, stream, pdl)) || (r = prep(s, s->o, m.q_dim, nullptr, m.q_dim, PREP_PLAIN, T, stream)) || (r = product(s, s->wo[l], s->x, m.E, true, T, stream)) ||

@@ -39,7 +39,7 @@ def check(spec, quant, gs, lengths, room=1200):
 def check_file(path, spec, quant, lengths, room):
     """Prompts of these lengths in portions against the same positions one call at a time."""
     eng = E.Engine(path, room)
-    toks = mf.teacher_tokens(1160, spec.vocab)
+    toks = mf.teacher_tokens(max(1160, *lengths), spec.vocab)
     n = max(lengths)
     last, want, keep = spec.n_layer - 1, {}, {}
     for p in range(n):
@@ -202,6 +202,28 @@ def test_a_hidden_unit_that_is_not_a_number(gs, tmp_path):
         assert rel(rows(eng, spec, 1, p), rows(ref, spec, 1, p)) < 4e-2, p
     eng.close()
     ref.close()
+
+
+def test_which_prompts_have_the_attention_of_one_kernel():
+    """Up to 50 positions (36 where heads are wide or many) a portion's attention is one kernel, above them two, and so it is for the 1, 2 and 3 positions behind 1024 and
+    2048 of a longer prompt, whose few queries have more than a thousand keys."""
+    spec = dataclasses.replace(mf.PRESETS["toy-qwen3"], name="toy-qwen3-behind", block_size=4096)
+    check(spec, mf.QUANT_F32, 128, (37, 38, 51, 52, 1026, 1027, 1028, 2050), 2100)
+    wide = dataclasses.replace(mf.PRESETS["mini-qwen3"], name="mini-qwen3-few")
+    check(wide, mf.QUANT_F32, 128, (37, 38, 51, 52), 100)
+
+    def launches(s, room, lengths):
+        eng, out = E.Engine(mf.cached_model(s, mf.QUANT_F32, 128), room), []
+        for m in lengths:
+            at = eng.launches
+            eng.decode_greedy(np.zeros(m + 2, np.uint32), m + 1, m + 2)
+            out.append(eng.launches - at)
+        eng.close()
+        return out
+    a, b, two, c, d, e, four, f = launches(spec, 2100, (50, 51, 1024, 1025, 1026, 1027, 2048, 2049))
+    assert a == b - 1 and two == b and c == d == e == four and f - four == four - two          # (a portion of these two layers has one attention)
+    a, b, c = launches(wide, 100, (36, 37, 51))
+    assert a == b - 3 and b == c
 
 
 def test_portions_keep_no_copy_of_the_weights():
