@@ -27,6 +27,7 @@
 
 #include "../../include/nano_b200.h"
 #include "kernels.cuh"
+#include "stream_count.h"
 #include "stream_host.h"
 #include "sample_host.h"
 #include "family.h"
@@ -96,7 +97,7 @@ struct nb200_engine : nb::EngineBase {
     float calib_ms[2] = {0.0f, 0.0f};      // ms per token of {streaming, multi-kernel} measured by calibrate_paths (0 = not calibrated)
     bool use_stream = false; const void *st_kern = nullptr; StreamArgs sa{}; uint32_t st_smem = 0, st_grid = 0;
     uint32_t *st_err_host = nullptr, *st_err_dev = nullptr;      // mapped pinned word: the code a device-side spin recorded before trapping
-    uint32_t st_epoch = 0, st_bar = 0;                           // exchange epochs handed out so far, what the grid barrier's counter stands at (stream.cuh)
+    nb::StreamCount st_count;                                    // exchange epochs and barrier arrivals used up so far (stream.cuh)
     float *logits_host = nullptr; bool logits_on_host = false;   // pinned copy of the logits that one-token calls of the streaming kernel write; whether it holds the last step's
     void *samp_ws = nullptr; size_t samp_cub = 0; uint32_t *samp_host = nullptr;       // device-side sampler workspace (sample.cu), pinned result
     uint64_t stream_bytes = 0;
@@ -392,14 +393,15 @@ int launch_stream(nb200_engine *e, uint32_t n_steps, const DevState *st = nullpt
     if (n_steps == 0) return 0;
     StreamArgs g = e->sa;
     g.n_steps = n_steps; g.trace = e->trace_dev;
-    g.epoch_base = e->st_epoch; g.bar_base = e->st_bar;
-    e->st_epoch += n_steps * 5u * e->d.L; e->st_bar += n_steps * e->st_grid;
     if (st) { g.st0 = *st; g.with_state = 1; g.next_host = e->tok_host; }
     if (with_logits) g.logits_host = e->logits_host;
-    void *params[] = {&g};
-    CK(cudaLaunchCooperativeKernel(e->st_kern, dim3(e->st_grid), dim3(kThreads), params, e->st_smem, e->stream));
-    e->launches++;
-    return 0;
+    return e->st_count.run(n_steps * 5u * e->d.L, n_steps * e->st_grid, [&](uint32_t epoch, uint32_t bar) -> int {
+        g.epoch_base = epoch; g.bar_base = bar;
+        void *params[] = {&g};
+        CK(cudaLaunchCooperativeKernel(e->st_kern, dim3(e->st_grid), dim3(kThreads), params, e->st_smem, e->stream));
+        e->launches++;
+        return 0;
+    });
 }
 
 int launch_token(nb200_engine *e) {
