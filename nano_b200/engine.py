@@ -143,20 +143,31 @@ def _p(a: np.ndarray, t):
 class RowPool:
     """Float arrays of n values whose memory is used again once nothing refers to it: a fresh array of Qwen3's 608 KB of logits costs 42 us of page faults, more
     than twice what filling it takes.  take() gives a view of a kept buffer that nobody else holds (views, and whatever is built on them, refer to their
-    buffer), or of a new one.  At most 32 MB are kept; arrays below 64 KB come from the allocator, which has them without faults."""
+    buffer), or of a new one.  At most 32 MB are kept; arrays below 64 KB come from the allocator, which has them without faults.
+    What sys.getrefcount says of a buffer that nobody holds is the interpreter's business (2 where a call's argument counts, 1 where it is lent): each pool asks it once, of
+    one that is known to be free, and keeps nothing where a view does not show in the answer."""
 
     def __init__(self, n: int):
-        self.n, self.kept = n, []
+        self.n, self.kept = n, [np.empty(1, np.float32)]
+        self.free = self._pop()[1]
+        probe = np.empty(1, np.float32)
+        self.kept, view = [probe], probe[:]
+        del probe
+        self.reuse = self._pop()[1] == self.free + 1 and view.size == 1
+
+    def _pop(self):
+        buf = self.kept.pop(0)          # out of the list while it is looked at: no other thread can take it
+        return buf, sys.getrefcount(buf)
 
     def take(self) -> np.ndarray:
-        if 4 * self.n < 1 << 16:
+        if 4 * self.n < 1 << 16 or not self.reuse:
             return np.empty(self.n, np.float32)
         for _ in range(4):          # the one given out longest ago is first; no long search while a caller keeps many
             try:
-                buf = self.kept.pop(0)          # out of the list while it is looked at: no other thread can take it
+                buf, count = self._pop()
             except IndexError:
                 break
-            out = buf[:] if sys.getrefcount(buf) == 2 else None          # 2: this name and the argument
+            out = buf[:] if count == self.free else None
             self.kept.append(buf)
             if out is not None:
                 return out
