@@ -60,6 +60,7 @@
 #include <vector>
 
 #include "attn_tc.h"
+#include "f32_split.h"
 #include "family.h"
 #include "layered_kernels.cuh"
 #include "layered_mixers.cuh"
@@ -970,10 +971,8 @@ int gemm(LayeredEngine *e, GemmArgs a, uint32_t groups, uint32_t maxM, bool wf32
         return tc_gemm(&e->tc, a, groups, maxM, rows, a.g_off ? std::max(1u, (active + groups - 1u) / groups) : maxM, e->cur == e->side ? 1u : e->cur == e->side2 ? 2u : 0u, e->cur, e->use_pdl);
     }
     const dim3 grid((a.N + 63u) / 64u, (maxM + 63u) / 64u, groups);
-    if (f32 && gemm_f32_fits(a)) {      // blocks of a cluster share a tile's depth while all of them still find a place at once (two to an SM), 64 columns each at least
-        const uint32_t tiles = grid.x * ((a.g_off && active ? std::max(1u, (active + groups - 1u) / groups) : maxM) + 63u) / 64u * groups;
-        uint32_t split = 1;
-        while (split < 8u && tiles * split * 2u <= 2u * (uint32_t)e->num_sms && a.K >= split * 2u * 64u) split *= 2u;
+    if (f32 && gemm_f32_fits(a)) {
+        const uint32_t split = nb::f32_split(grid.x, a.g_off && active ? std::max(1u, (active + groups - 1u) / groups) : maxM, groups, a.K, (uint32_t)e->num_sms);
         return launch_split(e, k_gemm_f32_async, dim3(grid.x * split, grid.y, groups), dim3(kF32Threads), a, split);
     }
     return f32 ? launch<GemmArgs>(e, k_gemm_f32<float>, grid, dim3(256), 0, a) : launch<GemmArgs>(e, k_gemm_bf16, grid, dim3(128), 0, a);
