@@ -110,3 +110,25 @@ def test_rows_whose_squares_overflow(arch, quant, gs, monkeypatch, tmp_path):
             assert np.linalg.norm((a - b)[small]) <= (1e-5 if quant == mf.QUANT_F32 else 2e-2) * np.linalg.norm(b[small]), pos
     eng.close()
     o.close()
+
+
+# classifiers of warp-owned tiles (32 rows a CTA and more): tiles of 3 rows, of one store of 32 and of more than one, vocabularies that no number of CTAs divides
+@pytest.mark.parametrize("quant,gs", [(mf.QUANT_F32, 128), (mf.QUANT_Q80, 64), (mf.QUANT_Q80, 128), (mf.QUANT_Q4K, 128)])
+@pytest.mark.parametrize("vocab", [4737, 5003, 71041, 80003])
+def test_vocabularies(vocab, quant, gs, monkeypatch):
+    monkeypatch.setenv("NB200_STREAM", "1")
+    spec = mf.ModelSpec("vocab-%d-%d" % (vocab, gs), mf.ARCH_QWEN3, 64, vocab, 1, 256, 4, 2, 256, 64)
+    path = mf.cached_model(spec, quant, gs)
+    eng, o = E.Engine(path, 8), ob.NanoOracle(path, 8)
+    assert eng.path.startswith("streaming"), eng.path
+    for pos, t in enumerate((5, vocab - 1, 3000)):
+        a, b = eng.forward(t, pos), o.forward(t, pos)
+        assert np.array_equal(a, eng.read(E.F_LOGITS, vocab))          # pinned memory and device, every row of both
+        # as above; Q4K: one layer, whose 4-bit activations re-round where a sum changes in its last place
+        assert np.linalg.norm(a - b) <= {mf.QUANT_F32: 1e-5, mf.QUANT_Q80: 1e-2, mf.QUANT_Q4K: 0.15}[quant] * np.linalg.norm(b), pos
+        assert np.abs(a - b).max() <= (0.01 if quant != mf.QUANT_Q4K else 0.5) * np.abs(b).max(), pos          # no row is lost or another's
+    ids = np.zeros(6, np.uint32)
+    ids[:3] = 5, vocab - 1, 3000
+    assert eng.next_greedy(ids, 2, 0) == int(np.argmax(a))
+    eng.close()
+    o.close()
