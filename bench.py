@@ -366,7 +366,8 @@ def measure(E, workload, steps, warmup, local, dist=None, world=1, flags=0, e2e=
             t_e2e += time.perf_counter() - t1
         t_e2e = barrier_max(dist, local, t_e2e)
         res["e2e"] = {"value": world * e2e_steps * n_dec / t_e2e, "unit": "tokens/s", "h2d_bytes_per_step": 48 * n_dec, "d2h_bytes_per_step": 4 * n_dec,
-                      "api": "nb200_next_greedy per token (pinned H2D of the 48 B step descriptor incl. token id, D2H of the next id)",
+                      "api": "nb200_next_greedy per token: 48 B of state incl. the token id in, the next id out (streaming: with the launch's arguments, and written by the kernel "
+                             "to pinned memory; multi-kernel: pinned copies)",
                       "same_ids_as_device_loop": bool(np.array_equal(ids2[:seq], timed_ids[:seq]))}
 
     # ---- roofline ----
@@ -396,7 +397,7 @@ def measure(E, workload, steps, warmup, local, dist=None, world=1, flags=0, e2e=
                 per_class[name] = {"launches": int(cnt[i]), "mean_us": dur * 1e6, "share": float(ms[i]) / tot_ms, "alg_bytes": alg[name], "gbs": alg[name] / dur / 1e9}
     traffic = None
     try:
-        traffic = json.load(open(os.path.join(ROOT, "profiles", "r2_traffic.json"))).get(workload + (":stream" if eng.path.startswith("streaming") else ":multikernel"))
+        traffic = json.load(open(os.path.join(ROOT, "profiles", "decode_traffic.json"))).get(workload + ":stream")
     except Exception:
         pass
     if eng.path.startswith("streaming"):
@@ -404,7 +405,7 @@ def measure(E, workload, steps, warmup, local, dist=None, world=1, flags=0, e2e=
         res["roofline"] = {"bound": "hbm", "kernel": f"k_decode_stream (one launch decodes {n_dec} tokens: all layers + classifier + argmax)",
                            "achieved": per_gpu_gbs, "peak": peak, "unit": "GB/s", "frac": per_gpu_gbs / peak,
                            "traffic": traffic * n_dec if traffic else None,
-                           "traffic_source": f"ncu --set full capture of one k_decode_stream launch: DRAM bytes per token x {n_dec} tokens (profiles/r2_ncu_stream.md)" if traffic else None,
+                           "traffic_source": f"ncu capture of k_decode_stream launches: DRAM bytes per token x {n_dec} tokens (profiles/decode_kernels_ncu.md)" if traffic else None,
                            "peak_source": peak_src, "alg_bytes_per_launch": bytes_tok * n_dec, "mean_launch_us": dec_ms / steps * 1e3, "share_of_step": 1.0,
                            "phase_profile_note": "per_kernel = the multi-kernel path's kernels for the same phases (graph/PDL off, CUDA events per launch), for orientation only",
                            "per_kernel": per_class}
@@ -412,7 +413,7 @@ def measure(E, workload, steps, warmup, local, dist=None, world=1, flags=0, e2e=
         dom = "w13_swiglu"
         res["roofline"] = {"bound": "hbm", "kernel": f"k_matvec<{'Q80' if quant == mf.QUANT_Q80 else 'Q4K' if quant == mf.QUANT_Q4K else 'F32'},SWIGLU> (W1|W3 + SwiGLU)",
                            "achieved": per_class[dom]["gbs"], "peak": peak, "unit": "GB/s", "frac": per_class[dom]["gbs"] / peak,
-                           "traffic": traffic, "traffic_source": "ncu --set full capture (profiles/r2_ncu_multikernel.md)" if traffic else None,
+                           "traffic": None, "traffic_source": None,
                            "peak_source": peak_src, "alg_bytes_per_launch": per_class[dom]["alg_bytes"], "mean_launch_us": per_class[dom]["mean_us"],
                            "share_of_step": per_class[dom]["share"], "per_kernel": per_class}
     if parity:
