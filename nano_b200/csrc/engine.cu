@@ -918,8 +918,8 @@ static int create_impl(nb200_engine **out, const uint8_t *img, uint64_t image_by
     {
         // Default path in fast mode on one GPU.  The streaming kernel is set up whenever the shape allows it.  F32 / Q4K models and Q80
         // models under 256 MB of weights always run it (latency-bound: one launch, no kernel boundary per phase).  For larger Q80 models
-        // neither path wins everywhere (profiles/r2_paths.md: multi-kernel ahead at 0.6B / 1.7B, streaming ahead at 4B with a long context),
-        // so the engine times both at the middle of its context and keeps the faster one (calibrate_paths).
+        // the faster path depends on shape and context, so the engine times both at the middle of its context and keeps the faster one
+        // (calibrate_paths; us a token, streaming / multi-kernel: Qwen3-0.6B at 2048 656 / 983, 1.7B at 2048 933 / 1200, 4B at 4096 1807 / 2690).
         // NB200_STREAM=1 forces the streaming kernel where the shape allows it, NB200_STREAM=0 / NB200_FLAG_NO_STREAM forbid it.
         const char *st_env = getenv("NB200_STREAM");
         const bool st_forced = st_env && atoi(st_env) == 1, st_off = (st_env && atoi(st_env) == 0) || (flags & NB200_FLAG_NO_STREAM);
@@ -1400,7 +1400,7 @@ int nb200_trace_token(nb200_engine *e, uint32_t token, uint32_t pos, unsigned lo
     if (!e || !stamps || !count) return fail(NB200_EINVAL, "null argument");
     if (!e->use_stream) return fail(NB200_EINVAL, "persistent kernel not active");
     CK(cudaSetDevice(e->device));
-    const uint32_t n = 1024 + 256;         // [0, 5L+2): per-barrier stamps; [1024, 1024+15): phase stamps of layer L/2; [1100, 1100+64): stamps inside its four matvec phases
+    const uint32_t n = 1024 + 256;         // [0, 5L+2): per-barrier stamps; [1024, 1024+60): stamps inside layer L/2, as many as it has
     if (cap < n || 5 * e->d.L + 4 > 1024) return fail(NB200_EINVAL, "need room for %u stamps", n);
     unsigned long long *buf = nullptr;
     CK(cudaMalloc(&buf, (size_t)n * 8));

@@ -140,7 +140,7 @@ struct MatvecArgs {
     int8_t *dump_codes; float *dump_scales;
     // persistent kernel: step state already in registers (saves an L2 round trip per phase)
     uint32_t state_known, pos_val; float pen_val;
-    unsigned long long *dbg;     // optional: CTA 0 / thread 0 clock64() stamps inside the phase (tools/gpu_trace.py)
+    unsigned long long *dbg;     // optional: CTA 0 / thread 0 clock64() stamps inside the phase
     Dims d;
     TpArgs tp;                   // tensor-parallel exchange (k_matvec<..., TP=true> only)
     const float *lora_add;       // RESID only: LoRA branch of the O projection, added to the matvec result BEFORE the residual (infer.c:898-908)
@@ -1147,7 +1147,7 @@ struct AttnArgs {
     uint32_t nsplit_max, chunk_cap;
     Dims d;
     TpArgs tp;               // tensor parallel: xba is pushed to every rank (k_attention_fast<KVM, true>)
-    unsigned long long *dbg; // optional %globaltimer stamps of kv head 0 (tools/gpu_attn_trace.py): [0..9] split 0, [16..21] merging CTA
+    unsigned long long *dbg; // optional %globaltimer stamps of kv head 0: [0..9] split 0, [16..21] merging CTA
 };
 __device__ __forceinline__ unsigned long long gtime() { unsigned long long t; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t)); return t; }
 #define AG_STAMP(cond, k) do { if (a.dbg && (cond) && threadIdx.x == 0) a.dbg[k] = gtime(); } while (0)

@@ -105,7 +105,7 @@ __device__ __forceinline__ float ld_cluster(const float *p, uint32_t rank) {    
 // three ahead (cp.async).  A thread reads four k of a row at once, rows 20 floats apart (8 neighbouring rows hit 8 bank groups), so nothing is transposed: 12 shared-memory
 // loads per 128 FMA.  Portions of this mode are short: where the tiles alone would leave SMs idle, a cluster shares a tile's depth, and its blocks add up
 // their parts of the tile from each other's shared memory, a share of the rows each, in the order of the depth.
-// The 203-token portion of two Famudra w1024 layers took 1569 us with k_gemm_f32 for all products (one stage, scalar loads, 64 blocks; 1177 of it theirs), now 714 (489).
+// The 203-token portion of two Famudra w1024 layers took 1569 us with k_gemm_f32 for all products (one stage, scalar loads, 64 blocks; 1177 of it theirs), 714 (489) here, 3 % less since f32_split counts whole row tiles.
 constexpr uint32_t kF32Threads = 128, kF32Pitch = 20, kF32Stages = 3;
 __global__ void __launch_bounds__(kF32Threads, 4) k_gemm_f32_async(const GemmArgs a, const uint32_t split) {
     pdl_enter();

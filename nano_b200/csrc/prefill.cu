@@ -87,15 +87,14 @@ __global__ void __launch_bounds__(kPrepThreads) k_prompt_prep(const PromptPrepAr
         acc = block_sum<kPrepThreads>(acc, red);
         inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(acc, (float)a.n), 1e-5f)));
     }
-    const uint32_t G = a.n / a.gs, epl = a.gs / 32u;
-    for (uint32_t g = warp; g < G; g += kPrepThreads / 32u) {
+    for (uint32_t g = warp; g < a.n / 256u; g += kPrepThreads / 32u) {
         float v[8], amax = 0.0f;
 #pragma unroll
-        for (uint32_t j = 0; j < 8; j++) if (j < epl) { v[j] = prep_value(a, s, inv, g * a.gs + j * 32u + lane); amax = fmaxf(amax, fabsf(v[j])); }
+        for (uint32_t j = 0; j < 8; j++) { v[j] = prep_value(a, s, inv, g * 256u + j * 32u + lane); amax = fmaxf(amax, fabsf(v[j])); }
         amax = warp_max(amax);
         const float sc = __fdiv_rn(amax, 127.0f), rinv = __frcp_rn(sc);
 #pragma unroll
-        for (uint32_t j = 0; j < 8; j++) if (j < epl) a.codes[(size_t)t * a.n + g * a.gs + j * 32u + lane] = (int8_t)((sc == 0.0f) ? 0 : q80_code(v[j], sc, rinv));
+        for (uint32_t j = 0; j < 8; j++) a.codes[(size_t)t * a.n + g * 256u + j * 32u + lane] = (int8_t)((sc == 0.0f) ? 0 : q80_code(v[j], sc, rinv));
         if (lane == 0) a.scales[(size_t)g * a.lds + t] = sc;
     }
 }

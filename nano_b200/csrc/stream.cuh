@@ -13,7 +13,7 @@
 // ONE 8-byte store, a consuming CTA polls the words it needs until they carry the epoch of the exchange it is waiting
 // for.  Value and epoch arrive together (single-copy atomic), so there is no fence, no counter and no grid barrier on
 // the per-phase path (measured on B200: release fence ~1.1-1.7 k cycles, counter barrier ~1.6 k, against ~0.3-0.6 k
-// for a store -> poll hand-off).  Vectors that every CTA reads are written to kStRep replicas (different L2 slices;
+// from one word's store to its poll; a whole exchange, which is over when the last of 148 CTAs has published and a CTA has read all of a vector, takes 1.5 to 2 k).  Vectors that every CTA reads are written to kStRep replicas (different L2 slices;
 // one hot copy read by 148 SMs at once costs ~600 cycles of slice bandwidth).
 //   Why a word is never overwritten before its readers are done: a CTA reads an entire vector before it produces
 //   anything of the next exchange, so "all of exchange k has arrived" implies every producer of exchange k has finished

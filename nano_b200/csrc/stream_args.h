@@ -52,8 +52,9 @@ struct StreamArgs {
     Dims d;
 };
 
-// the longest row whose activation operand the prologue prepares (Q4K: warp slots of 256 elements stay in registers between the sum of squares and the
-// quantise pass); the host checks it before choosing the streaming kernel
+// the longest row that the streaming kernel takes; the host checks it before choosing the kernel.  Q4K: warp slots of 256 elements stay in registers between the prologue's sum of
+// squares and its quantise pass, two of them.  Q80 and F32: the prologue walks its row in turns and has no bound of its own; rows past 11520 have never run on this
+// kernel and keep the path of one kernel per phase
 constexpr int kStKmax = 6, kStKmaxQ4K = 2;
 __host__ __device__ inline uint32_t st_prep_max_n(uint32_t quant, uint32_t gs) {
     (void)gs;
