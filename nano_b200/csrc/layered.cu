@@ -943,8 +943,8 @@ int gemv_launch(LayeredEngine *e, GemmArgs a, uint32_t groups, uint32_t live, bo
         return f32 ? launch<GemmArgs>(e, k_gemv_one<float, EXT>, grid, block, one_smem<float>(a.K), a) : launch<GemmArgs>(e, k_gemv_one<__nv_bfloat16, EXT>, grid, block, one_smem<__nv_bfloat16>(a.K), a);
     }
     const dim3 grid(gemv_blocks(e, a.N, live), groups), block(256);
-    if (EXT == 0) return f32 ? launch<GemmArgs>(e, k_gemv<float>, grid, block, 0, a) : launch<GemmArgs>(e, k_gemv<__nv_bfloat16>, grid, block, 0, a);
-    return f32 ? launch<GemmArgs>(e, k_gemv_ext<float, EXT>, grid, block, 0, a) : launch<GemmArgs>(e, k_gemv_ext<__nv_bfloat16, EXT>, grid, block, 0, a);
+    if constexpr (EXT == 0 || EXT == 6) return f32 ? launch<GemmArgs>(e, k_gemv<float>, grid, block, 0, a) : launch<GemmArgs>(e, k_gemv<__nv_bfloat16>, grid, block, 0, a);
+    else return f32 ? launch<GemmArgs>(e, k_gemv_ext<float, EXT>, grid, block, 0, a) : launch<GemmArgs>(e, k_gemv_ext<__nv_bfloat16, EXT>, grid, block, 0, a);
 }
 
 // one matrix product; maxM = the most rows any group can have.  wf32: the weights are fp32 whatever the engine's mode (router).
@@ -962,6 +962,7 @@ int gemm(LayeredEngine *e, GemmArgs a, uint32_t groups, uint32_t maxM, bool wf32
         if (a.a_parts > 1) return gemv_launch<4>(e, a, groups, live, one, f32);
         if (a.glu) return gemv_launch<3>(e, a, groups, live, one, f32);
         if (a.a_poly) return gemv_launch<2>(e, a, groups, live, one, f32);
+        if (a.own_rows) return gemv_launch<6>(e, a, groups, live, one, f32);
         return gemv_launch<0>(e, a, groups, live, one, f32);
     }
     if (a.glu) return fail(NB200_EINVAL, "the gated-pair product is a matrix-vector instance (portions of at most %u tokens)", kGemvMaxM);
@@ -1620,7 +1621,7 @@ int ff_moe_scored(LayeredEngine *e, const Layer &L, uint32_t T) {
     }
     GemmArgs dn{};
     dn.A = e->b_hb; dn.lda = L.ff; dn.W = L.down.p; dn.ldw = L.ff; dn.C = e->b_eo; dn.ldc = E; dn.M = T; dn.N = E; dn.K = L.ff; dn.a_gmod = 1;
-    dn.g_off = e->b_off; dn.g_act = small ? e->b_act : nullptr; dn.w_gstride = (uint64_t)E * L.ff;
+    dn.g_off = e->b_off; dn.g_act = small ? e->b_act : nullptr; dn.w_gstride = (uint64_t)E * L.ff; dn.own_rows = wrow != nullptr;
     if ((r = gemm(e, dn, L.NE, T, false, T * L.top))) return r;
     if (!L.has_shared) return 0;
     if (e->branch_streams) { e->cur = e->side; CK(cudaStreamWaitEvent(e->side, e->ev_fork, 0)); }

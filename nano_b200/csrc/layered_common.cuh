@@ -63,8 +63,8 @@ struct GemmArgs {
     float glu_limit;
     // EPI_SOFTCAP: cap tanh(v / cap)
     float cap;
-    // k_gemv_one only: 2^one_split warps share a row
-    uint32_t one_split;
+    // k_gemv_one only: 2^one_split warps share a row; own_rows: rows of one group may differ though they are of one token
+    uint32_t one_split; bool own_rows;
 };
 
 // Programmatic dependent launch: every kernel first lets the NEXT kernel of its stream be scheduled (its blocks then sit in their own
