@@ -125,3 +125,20 @@ def test_delta_scan_sizes(tmp_path, dim, vdim):
         eng.seq_close(s)
         assert off(got, ref) < 5 * BOUND[True], cut          # 101 tokens of a recurrence on top of the products
     eng.close()
+
+
+# chunks of 16 tokens: one short of full, full, one over, two of them; a convolution longer than the four taps that are loaded at once, and longer than a chunk
+@pytest.mark.parametrize("f32", [True, False])
+@pytest.mark.parametrize("n,dim,conv", [(15, 64, 4), (16, 128, 4), (17, 128, 1), (31, 20, 2), (33, 256, 4), (48, 128, 5), (37, 64, 21)])
+def test_delta_chunk_edges(tmp_path, n, dim, conv, f32):
+    layers = [("delta", {"heads": 2, "kv_heads": 1, "dim": dim, "vdim": 40, "conv": conv}, 48), ("delta", {"heads": 2, "kv_heads": 2, "dim": dim, "vdim": 16, "conv": conv}, None)]
+    cfg = md.kadesun_config(97, 64, layers)
+    w = md.kadesun_random(cfg, 7, decay_rank=8, gate_rank=16)
+    eng = E.Engine(md.write_model_dir(str(tmp_path / "m"), cfg, w), 256, flags=E.FLAG_F32 if f32 else 0)
+    toks = np.random.default_rng(3).integers(0, 97, size=n + 6).astype(np.uint32)
+    ref = K.forward(cfg, w, toks)
+    s = eng.seq_open()
+    got = np.concatenate([eng.step(s, toks[:n], range(n)), eng.step(s, toks[n:], range(6))])          # and the state behind it
+    eng.seq_close(s)
+    assert off(got, ref) < 5 * BOUND[f32]
+    eng.close()
