@@ -1819,7 +1819,8 @@ int run_layers(LayeredEngine *e, uint32_t slot, uint32_t T, uint32_t pos0, const
             const NormShiftArgs a = norm_args(L, run);
             if (normed) normed = false;          // by the update before
             else if (norm_one) {
-                if ((r = launch<NormShiftArgs>(e, k_norm_shift_one, dim3(1), dim3(kOneThreads), 0, a))) return r;
+                const auto k = E <= 1024u ? k_norm_shift_one<4> : E <= 2048u ? k_norm_shift_one<8> : k_norm_shift_one<16>;
+                if ((r = launch<NormShiftArgs>(e, k, dim3(1), dim3(kOneThreads), 0, a))) return r;
             } else if ((r = launch<NormShiftArgs>(e, k_norm_shift, dim3(T > 1 ? T - 1 : 1), dim3(256), 0, a))) return r;
             if (L.has_mlp && e->branch_streams) CK(cudaEventRecord(e->ev_fork, e->stream));
         }
@@ -1843,7 +1844,8 @@ int run_layers(LayeredEngine *e, uint32_t slot, uint32_t T, uint32_t pos0, const
         const Run *nrun = ri + 1 < e->runs.size() && !e->runs[ri + 1].add_embed ? &e->runs[ri + 1] : nullptr;
         const CombineNormArgs cn{c, nrun ? norm_args(e->layers[nrun->layer], *nrun) : NormShiftArgs{}};
         if (nrun && norm_one) {
-            if ((r = launch<CombineNormArgs>(e, k_combine_norm_one, dim3(1), dim3(kOneThreads), 0, cn))) return r;
+            const auto k = E <= 1024u ? k_combine_norm_one<4> : E <= 2048u ? k_combine_norm_one<8> : k_combine_norm_one<16>;
+            if ((r = launch<CombineNormArgs>(e, k, dim3(1), dim3(kOneThreads), 0, cn))) return r;
             normed = true;
         } else if ((r = launch<CombineArgs>(e, k_combine, dim3(ew_grid((size_t)T * E)), dim3(256), 0, c))) return r;
     }
@@ -1892,9 +1894,11 @@ int head_rows(LayeredEngine *e, uint32_t nw, const uint32_t *want_dev = nullptr)
         e->launches++;
         return gemm(e, plain(e->b_xn, e->E, e->head, e->logits, e->V, nw), 1, nw);
     }
-    k_final_norm<<<nw, 256, 0, e->stream>>>(e->x, want_dev ? want_dev : e->want_dev, e->final_norm, e->b_xn, e->E, e->eps, e->form == FORM_SANDWICH ? 1u : e->form == FORM_POST || e->form == FORM_POST_LN ? 2u : 0u);
-    CK(cudaGetLastError());
-    e->launches++;
+    const FinalNormArgs fa{e->x, want_dev ? want_dev : e->want_dev, e->final_norm, e->b_xn, e->E, e->eps, e->form == FORM_SANDWICH ? 1u : e->form == FORM_POST || e->form == FORM_POST_LN ? 2u : 0u};
+    const auto fk = e->E <= 1024u ? k_final_norm<4> : e->E <= 2048u ? k_final_norm<8> : e->E <= 4096u ? k_final_norm<16> : k_final_norm<0>;
+    int r;
+    e->cur = e->stream;
+    if ((r = launch<FinalNormArgs>(e, fk, dim3(nw), dim3(256), 0, fa))) return r;
     GemmArgs hd = plain(e->b_xn, e->E, e->head, e->logits, e->V, nw, nullptr, e->logit_cap > 0.0f ? EPI_SOFTCAP : EPI_NONE);
     hd.cap = e->logit_cap;
     return gemm(e, hd, 1, nw);

@@ -1296,32 +1296,37 @@ __global__ void k_combine(const CombineArgs a) {
 
 // scalar-gain RMS norm of the rows whose logits are asked for: out[i] = x[want[i]] / rms * g
 // (vec 1: the gain is a vector stored around zero, out = x / rms * (1 + g[i]); vec 2: a plain vector, out = x / rms * g[i])
-// Rows of at most 4096 columns stay in registers between the sum and the result (the same sums in the same order), their gains are asked for before the wait: the row of
-// 2048 that ends every step took 10 us as two walks of single loads, now 3.
-__global__ void __launch_bounds__(256) k_final_norm(const float *__restrict__ x, const uint32_t *__restrict__ want, const float *__restrict__ g,
-                                                    float *__restrict__ out, uint32_t E, float eps, uint32_t vec) {
+// Rows of at most 256 NK columns stay in registers between the sum and the result (the same sums in the same order; NK 0: two walks), gains before the wait.
+// As a plain launch, with one instance for rows of up to 4096, it took 3.3 us of a step of 1024 columns and 4 to 7.6 of 2048 (before that, 10 as two walks of single loads); now 1.2 to 1.9.
+struct FinalNormArgs { const float *x; const uint32_t *want; const float *g; float *out; uint32_t E; float eps; uint32_t vec; };
+template <int NK>
+__global__ void __launch_bounds__(256) k_final_norm(const FinalNormArgs a) {
     pdl_launch_next();
     __shared__ float red[32];
-    const float gs = vec ? 0.0f : __ldg(g);
-    if (vec) for (uint32_t i = threadIdx.x * 32u; i < E; i += 8192u) asm volatile("prefetch.global.L1 [%0];" ::"l"(g + i));
+    constexpr uint32_t R = NK ? NK : 1;
+    float g[R];
+    const float *gt = a.g + threadIdx.x;
+    const float base = a.vec == 1u ? 1.0f : 0.0f;          // vec 1: 1 + g
+    if (NK) {
+#pragma unroll
+        for (uint32_t k = 0; k < R; k++) g[k] = !a.vec ? __ldg(a.g) : threadIdx.x + k * 256u < a.E ? __ldg(gt + k * 256u) : 0.0f;
+    }
     pdl_wait();
-    const float *xt = x + (size_t)want[blockIdx.x] * E;
-    float *o = out + (size_t)blockIdx.x * E;
-    float s = 0.0f, v[16];
-    const bool regs = E <= 4096u;
-    if (regs) {
+    const float *xt = a.x + (size_t)a.want[blockIdx.x] * a.E + threadIdx.x;
+    float *o = a.out + (size_t)blockIdx.x * a.E + threadIdx.x;
+    float s = 0.0f, v[R];
+    if (NK) {
 #pragma unroll
-        for (uint32_t k = 0; k < 16u; k++) { const uint32_t i = threadIdx.x + k * 256u; v[k] = i < E ? xt[i] : 0.0f; }
+        for (uint32_t k = 0; k < R; k++) v[k] = threadIdx.x + k * 256u < a.E ? xt[k * 256u] : 0.0f;
 #pragma unroll
-        for (uint32_t k = 0; k < 16u; k++) s = fmaf(v[k], v[k], s);
-    } else for (uint32_t i = threadIdx.x; i < E; i += blockDim.x) s = fmaf(xt[i], xt[i], s);
+        for (uint32_t k = 0; k < R; k++) s = fmaf(v[k], v[k], s);
+    } else for (uint32_t i = 0; threadIdx.x + i < a.E; i += 256u) s = fmaf(xt[i], xt[i], s);
     s = block_sum(s, red);
-    const float rinv = 1.0f / sqrtf(s / (float)E + eps);
-    auto put = [&](uint32_t i, float u) { o[i] = u * rinv * (vec ? (vec == 2u ? g[i] : 1.0f + g[i]) : gs); };
-    if (regs) {
+    const float rinv = 1.0f / sqrtf(s / (float)a.E + a.eps);
+    if (NK) {
 #pragma unroll
-        for (uint32_t k = 0; k < 16u; k++) { const uint32_t i = threadIdx.x + k * 256u; if (i < E) put(i, v[k]); }
-    } else for (uint32_t i = threadIdx.x; i < E; i += blockDim.x) put(i, xt[i]);
+        for (uint32_t k = 0; k < R; k++) if (threadIdx.x + k * 256u < a.E) o[k * 256u] = v[k] * rinv * (base + g[k]);
+    } else for (uint32_t i = 0; threadIdx.x + i < a.E; i += 256u) o[i] = xt[i] * rinv * (base + (a.vec ? gt[i] : __ldg(a.g)));
 }
 
 // greedy choice with the repetition penalty of the generation hosts: logits of ids seen before are divided (positive) or multiplied

@@ -372,77 +372,91 @@ __global__ void __launch_bounds__(kOneThreads) k_rglru_gates_one(const GatesScan
     a.S[c] = S;
 }
 
-// k_norm_shift for one token of at most 4096 columns: the row in registers, one trip to memory and one sum (in the same order), weights before the wait.  What the
-// combined kernel below shares with it: x[k], prev[k] are columns threadIdx.x + 256 k
-struct NormOne { float mu[16]; float g1, g2; };
-__device__ __forceinline__ void norm_one_weights(const NormShiftArgs &a, NormOne &w) {
+// k_norm_shift for one token of at most 256 NK columns: the row in registers, one trip to memory and one sum (in the same order), weights before the wait.  What the
+// combined kernel below shares with it: x[k], prev[k] are columns threadIdx.x + 256 k.
+// A lone block passes its code once, and fetching it is what it waits for (some 8 cycles an instruction): so there is an instance for rows of up to 1024, 2048 and 4096, and a row's
+// columns are one pointer with constant offsets.  Update and norm of 1024 columns with one instance of 4096: 669 instructions a warp and 5.4 us a link, now 3.5; 2048: 8.7 and 4.6.
+template <int NK> struct NormOne { float mu[NK]; float g1, g2; bool on[NK]; };
+template <int NK> __device__ __forceinline__ void norm_one_weights(const NormShiftArgs &a, NormOne<NK> &w) {
+    const float *mu = a.mu + threadIdx.x;
 #pragma unroll
-    for (uint32_t k = 0; k < 16u; k++) { const uint32_t i = threadIdx.x + k * kOneThreads; w.mu[k] = a.mu && i < a.E ? __ldg(a.mu + i) : 0.0f; }
-    w.g1 = __ldg(a.g1); w.g2 = a.g2 ? __ldg(a.g2) : 0.0f;
+    for (uint32_t k = 0; k < NK; k++) { w.on[k] = threadIdx.x + k * kOneThreads < a.E; w.mu[k] = a.mu && w.on[k] ? load_now_f(mu + k * kOneThreads) : 0.0f; }
+    w.g1 = load_now_f(a.g1); w.g2 = a.g2 ? load_now_f(a.g2) : 0.0f;
 }
-__device__ __forceinline__ void norm_one_row(const NormShiftArgs &a, const NormOne &w, const float (&x)[16], const float (&prev)[16], float *red) {
+template <int NK> __device__ __forceinline__ void norm_one_row(const NormShiftArgs &a, const NormOne<NK> &w, const float (&x)[NK], const float (&prev)[NK], float *red) {
     float s = 0.0f;
 #pragma unroll
-    for (uint32_t k = 0; k < 16u; k++) s = fmaf(x[k], x[k], s);
+    for (uint32_t k = 0; k < NK; k++) s = fmaf(x[k], x[k], s);
     s = block_sum(s, red);
     const float rinv = 1.0f / sqrtf(s / (float)a.E + a.eps);
+    float *hm = a.hm + threadIdx.x, *h2 = a.h2 + threadIdx.x, *state = a.state + threadIdx.x;
 #pragma unroll
-    for (uint32_t k = 0; k < 16u; k++) {
-        const uint32_t i = threadIdx.x + k * kOneThreads;
-        if (i >= a.E) break;
-        const float u = x[k] * rinv, n1 = u * w.g1;
-        a.hm[i] = a.mu ? n1 + (prev[k] - n1) * w.mu[k] : n1;
-        if (a.h2) a.h2[i] = u * w.g2;
-        a.state[i] = n1;
-    }
+    for (uint32_t k = 0; k < NK; k++)
+        if (w.on[k]) {
+            const float u = x[k] * rinv, n1 = u * w.g1;
+            hm[k * kOneThreads] = a.mu ? n1 + (prev[k] - n1) * w.mu[k] : n1;
+            if (a.h2) h2[k * kOneThreads] = u * w.g2;
+            state[k * kOneThreads] = n1;
+        }
 }
+template <int NK>
 __global__ void __launch_bounds__(kOneThreads) k_norm_shift_one(const NormShiftArgs a) {
     pdl_launch_next();
     __shared__ float red[32];
-    NormOne w;
+    NormOne<NK> w;
     norm_one_weights(a, w);
     pdl_wait();
-    float x[16], p[16];
+    float x[NK], p[NK];
+    const float *xt = a.x + threadIdx.x, *st = a.state + threadIdx.x;
 #pragma unroll
-    for (uint32_t k = 0; k < 16u; k++) { const uint32_t i = threadIdx.x + k * kOneThreads; x[k] = i < a.E ? a.x[i] : 0.0f; p[k] = i < a.E ? a.state[i] : 0.0f; }
+    for (uint32_t k = 0; k < NK; k++) { x[k] = w.on[k] ? xt[k * kOneThreads] : 0.0f; p[k] = w.on[k] ? st[k * kOneThreads] : 0.0f; }
     norm_one_row(a, w, x, p, red);
 }
 
 // k_combine of one token and k_norm_shift_one of the run that follows, in one link: the updated row stays in the registers of the block that norms it
 struct CombineNormArgs { CombineArgs c; NormShiftArgs n; };
+template <int NK>
 __global__ void __launch_bounds__(kOneThreads) k_combine_norm_one(const CombineNormArgs a) {
     pdl_launch_next();
     __shared__ float red[32];
     const CombineArgs &c = a.c;
-    NormOne w;
+    NormOne<NK> w;
     norm_one_weights(a.n, w);
     pdl_wait();
-    uint32_t slot[4]; float wt[4];
+    uint32_t slot[2]; float wt[2];
+    const bool routed = c.eo != nullptr;
 #pragma unroll
-    for (uint32_t j = 0; j < 4u; j++) { slot[j] = 0; wt[j] = 0.0f; if (c.eo && j < c.top) { slot[j] = c.slot[j]; wt[j] = c.wt[j]; } }
-    float x[16], p[16], d[16], sh[16];
+    for (uint32_t j = 0; j < 2u; j++) { const bool in = routed && j < c.top; slot[j] = in ? c.slot[j] : 0u; wt[j] = in ? c.wt[j] : 0.0f; }
+    float x[NK], p[NK], d[NK], sh[NK], f[NK];
+    const bool shared = routed && c.shared;
+    const float *xt = c.x + threadIdx.x, *st = a.n.state + threadIdx.x, *dt = c.d + threadIdx.x, *sht = c.shared + threadIdx.x;
 #pragma unroll
-    for (uint32_t k = 0; k < 16u; k++) {
-        const uint32_t i = threadIdx.x + k * kOneThreads;
-        x[k] = p[k] = d[k] = sh[k] = 0.0f;
-        if (i < c.E) { x[k] = c.x[i]; d[k] = c.d[i]; p[k] = a.n.state[i]; if (c.eo && c.shared) sh[k] = c.shared[i]; }
+    for (uint32_t k = 0; k < NK; k++) {
+        x[k] = p[k] = d[k] = sh[k] = f[k] = 0.0f;
+        if (w.on[k]) { x[k] = xt[k * kOneThreads]; d[k] = dt[k * kOneThreads]; p[k] = st[k * kOneThreads]; if (shared) sh[k] = sht[k * kOneThreads]; }
     }
+    if (routed) {          // the chosen experts' rows, two at a time (both rows' columns in flight), in their order
+#pragma unroll 1
+        for (uint32_t j = 0;;) {
+            const float *e0 = c.eo + (size_t)slot[0] * c.E + threadIdx.x, *e1 = c.eo + (size_t)slot[1] * c.E + threadIdx.x;
+            float v0[NK], v1[NK];
+            const bool two = j + 1u < c.top;
 #pragma unroll
-    for (uint32_t k = 0; k < 16u; k++) {
-        const uint32_t i = threadIdx.x + k * kOneThreads;
-        if (i >= c.E) break;
-        float delta = d[k];
-        if (c.eo) {
-            float f = 0.0f;
+            for (uint32_t k = 0; k < NK; k++) { v0[k] = w.on[k] ? e0[k * kOneThreads] : 0.0f; v1[k] = w.on[k] && two ? e1[k * kOneThreads] : 0.0f; }
 #pragma unroll
-            for (uint32_t j = 0; j < 4u; j++) if (j < c.top) f = fmaf(wt[j], c.eo[(size_t)slot[j] * c.E + i], f);
-            for (uint32_t j = 4u; j < c.top; j++) f = fmaf(c.wt[j], c.eo[(size_t)c.slot[j] * c.E + i], f);
-            if (c.shared) f += sh[k];
-            delta += f;
+            for (uint32_t k = 0; k < NK; k++) { f[k] = fmaf(wt[0], v0[k], f[k]); if (two) f[k] = fmaf(wt[1], v1[k], f[k]); }
+            j += 2u;
+            if (j >= c.top) break;
+#pragma unroll
+            for (uint32_t q = 0; q < 2u; q++) { const bool in = j + q < c.top; slot[q] = in ? c.slot[j + q] : 0u; wt[q] = in ? c.wt[j + q] : 0.0f; }
         }
-        x[k] += delta;
-        c.x[i] = x[k];
-        if (c.keep) c.keep[i] = x[k];
+    }
+    float *xo = c.x + threadIdx.x, *kp = c.keep + threadIdx.x;
+#pragma unroll
+    for (uint32_t k = 0; k < NK; k++) {
+        if (shared) f[k] += sh[k];
+        x[k] += routed ? d[k] + f[k] : d[k];
+        if (w.on[k]) { xo[k * kOneThreads] = x[k]; if (c.keep) kp[k * kOneThreads] = x[k]; }
     }
     norm_one_row(a.n, w, x, p, red);
 }

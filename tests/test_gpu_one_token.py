@@ -142,3 +142,15 @@ def test_delta_chunk_edges(tmp_path, n, dim, conv, f32):
     eng.seq_close(s)
     assert off(got, ref) < 5 * BOUND[f32]
     eng.close()
+
+
+# rows at the edges of the instances of the lone-row norms (256 threads with 4, 8 and 16 columns each, or a walk), with no expert, one, two and five
+@pytest.mark.parametrize("width,top", [(1020, 2), (1024, 1), (1028, 5), (2048, 0), (2052, 3), (4096, 2), (4100, 2)])
+def test_one_token_rows(tmp_path, width, top):
+    mlp = {"experts": max(top, 1), "top": top, "ff": 8, "shared_ff": 16 if top % 2 else None} if top else None
+    cfg = md.famudra_config(61, width, [("rglru", {"width": 32, "blocks": 2, "conv": 2}, mlp), ("rglru", {"width": 32, "blocks": 2, "conv": 2}, mlp)])
+    w = md.famudra_random(cfg, 3)
+    eng = E.Engine(md.write_model_dir(str(tmp_path / "m"), cfg, w), 64, flags=E.FLAG_F32)
+    toks = np.random.default_rng(1).integers(0, 61, size=5).astype(np.uint32)
+    assert off(one_by_one(eng, toks), A.forward(cfg, w, toks)) < BOUND[True]
+    eng.close()
