@@ -144,6 +144,32 @@ def test_delta_chunk_edges(tmp_path, n, dim, conv, f32):
     eng.close()
 
 
+# tokens at the edges of groups of eight keys, of pages and of the turns of a cluster's 64 warps; heads that share keys by one to five, blocks of positions that end inside a group,
+# norms of a head or of the whole row, a sink with and without a gate
+@pytest.mark.parametrize("design,heads,kv,dim,vdim,mask", [("fidatar", 2, 2, 4, 8, None), ("fidatar", 4, 2, 128, 100, None), ("fidatar", 10, 2, 64, 128, 21), ("fidatar", 3, 1, 36, 4, 8), ("kadesun", 6, 2, 128, 128, None), ("kadesun", 5, 1, 20, 64, None)])
+def test_one_token_keys(tmp_path, design, heads, kv, dim, vdim, mask):
+    a = {"heads": heads, "kv_heads": kv, "dim": dim, "vdim": vdim, "scale": dim ** -0.5, "rot": {"dims": dim // 4 * 2, "base": 100.0}}
+    if design == "fidatar":
+        if mask:
+            a["mask"] = {"size": mask}
+        cfg = md.fidatar_config(97, 64, [("attention", a, {"kind": "dense", "ff": 32})], alpha=2.0, scale=2.0)
+        w, O = md.fidatar_random(cfg, 5), F
+    else:
+        cfg = md.kadesun_config(97, 64, [("parallel", {"left": dict(a, softcap=20.0), "right": {"heads": 2, "kv_heads": 2, "dim": 8, "vdim": 8, "conv": 2}}, None)])
+        w, O = md.kadesun_random(cfg, 5, decay_rank=8, gate_rank=16), K
+    eng = E.Engine(md.write_model_dir(str(tmp_path / "m"), cfg, w), 640, flags=E.FLAG_F32)
+    toks = np.random.default_rng(4).integers(0, 97, size=530).astype(np.uint32)
+    ref = O.forward(cfg, w, toks)
+    for n, m in ((0, 34), (62, 4), (510, 5)):          # (a token behind n others, and the next ones)
+        s = eng.seq_open()
+        if n:
+            eng.step(s, toks[:n])
+        for i in range(n, n + m):
+            assert off(eng.step(s, toks[i:i + 1], [0])[0], ref[i]) < BOUND[True], i
+        eng.seq_close(s)
+    eng.close()
+
+
 # rows at the edges of the instances of the lone-row norms (256 threads with 4, 8 and 16 columns each, or a walk), with no expert, one, two and five
 @pytest.mark.parametrize("width,top", [(1020, 2), (1024, 1), (1028, 5), (2048, 0), (2052, 3), (4096, 2), (4100, 2)])
 def test_one_token_rows(tmp_path, width, top):
