@@ -7,6 +7,9 @@
 // k_gemv, which serves up to four rows and any alignment, reads the row in every warp, converts it there, and its epilogue starts a trip of its own.
 // A chain of 1024 x 1024 products from HBM, us a link: k_gemv 4.5, weights in registers 2.9, this 2.1 (with two
 // running sums; one, in k_gemv's order, makes a whole step of eight routed layers bit for bit that of the general kernels: 290 us a token, 265 with two, 364 before).
+// What is left of a link is then the instructions it passes, 620 a warp for a row of 1024, most of them for steps that such a row does not have: a warp leaves a run of steps at its own
+// last one, checks lanes only in rows that end inside a step, and loads an activation row of up to 8 KB at once.  Call to call, a token of eight Famudra layers of width 1024 249 -> 232 us, of two
+// Fidatar layers 84 -> 79 (width 1024), 147 -> 145 (2048).
 #pragma once
 #include "layered_kernels.cuh"
 #include "layered_mixers3.cuh"
@@ -59,17 +62,23 @@ __device__ __forceinline__ void one_stage(const GemmArgs &a, const float *row, f
     const float4 *src = reinterpret_cast<const float4 *>(row), *nw = reinterpret_cast<const float4 *>(a.a_norm_w);
     const bool poly = EXT == 2 && a.a_poly, raw = nw || poly;
     float s2 = 0.0f, s4 = 0.0f, s6 = 0.0f;
-#pragma unroll 4
-    for (uint32_t c = threadIdx.x; c < P4; c += kOneThreads) {
-        float4 v = make_float4(0, 0, 0, 0);
-        if (c < K4) v = src[c];
-        if (EXT == 2) s2 = sum_sq4(v, s2);
-        if (EXT == 2) {
-            const float q[4] = {v.x, v.y, v.z, v.w};
+    for (uint32_t c0 = threadIdx.x; c0 - threadIdx.x < P4; c0 += 2u * kOneThreads) {          // two loads at a time, also of a short row
+        float4 vs[2];
 #pragma unroll
-            for (int j = 0; j < 4; j++) { const float v2 = q[j] * q[j], v3 = v2 * q[j]; s4 = fmaf(v2, v2, s4); s6 = fmaf(v3, v3, s6); }
+        for (uint32_t j = 0; j < 2u; j++) vs[j] = c0 + j * kOneThreads < K4 ? src[c0 + j * kOneThreads] : make_float4(0, 0, 0, 0);
+#pragma unroll
+        for (uint32_t j = 0; j < 2u; j++) {
+            const uint32_t c = c0 + j * kOneThreads;
+            if (c - threadIdx.x >= P4) break;
+            float4 v = vs[j];
+            if (EXT == 2) s2 = sum_sq4(v, s2);
+            if (EXT == 2) {
+                const float q[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int j = 0; j < 4; j++) { const float v2 = q[j] * q[j], v3 = v2 * q[j]; s4 = fmaf(v2, v2, s4); s6 = fmaf(v3, v3, s6); }
+            }
+            if (c < P4) x[one_place<WT>(c)] = !raw && a.round_a ? round4(v) : v;
         }
-        x[one_place<WT>(c)] = !raw && a.round_a ? round4(v) : v;
     }
     if (raw) {
         float sc = 1.0f;
@@ -161,15 +170,19 @@ __device__ __forceinline__ void gemv_one(const GemmArgs &a, uint32_t bx, uint32_
     const uint32_t n0 = bx * rpb + (warp >> split);
     uint32_t n = n0;
     uint4 w[NW][PRE];
-    auto fetch = [&](uint32_t row, uint32_t s0) {
+    const bool ragged = a.K % STEP != 0;          // the last step's lanes past the row: zeros
+    auto fetch = [&](uint32_t row, uint32_t s0) {          // steps s0 .. of this warp's share (a row past the last: the last one, whose result nobody stores)
+        const WT *p = W + (size_t)min(row, a.N - 1u) * a.ldw + s0 * STEP + lane * VN;
+        const uint32_t left = a.K - s0 * STEP - lane * VN;
 #pragma unroll
-        for (uint32_t h = 0; h < NW; h++)
+        for (uint32_t i = 0; i < PRE; i++) {
+            if (s0 + i >= s_hi) break;
 #pragma unroll
-            for (uint32_t i = 0; i < PRE; i++) {
-                const uint32_t k = (s0 + i) * STEP + lane * VN;
-                w[h][i] = make_uint4(0, 0, 0, 0);
-                if (row < a.N && s0 + i < s_hi && k < a.K) w[h][i] = load_now(W + (size_t)(h * a.N + row) * a.ldw + k);
+            for (uint32_t h = 0; h < NW; h++) {
+                if (!ragged || (int32_t)(i * STEP) < (int32_t)left) w[h][i] = load_now(p + (size_t)(h * a.N) * a.ldw + i * STEP);
+                else w[h][i] = make_uint4(0, 0, 0, 0);
             }
+        }
     };
     if (fixed) {
         W += (uint64_t)gy * a.w_gstride;
@@ -241,11 +254,11 @@ __device__ __forceinline__ void gemv_one(const GemmArgs &a, uint32_t bx, uint32_
         for (uint32_t h = 0; h < NW; h++) acc[h] = 0.0f;
         for (uint32_t s0 = s_lo;;) {
 #pragma unroll
-            for (uint32_t i = 0; i < PRE; i++)
-                if (s0 + i < s_hi) {
+            for (uint32_t i = 0; i < PRE; i++) {
+                if (s0 + i >= s_hi) break;
 #pragma unroll
-                    for (uint32_t h = 0; h < NW; h++) one_fma<WT>(w[h][i], one_x, s0 + i, lane, acc[h]);
-                }
+                for (uint32_t h = 0; h < NW; h++) one_fma<WT>(w[h][i], one_x, s0 + i, lane, acc[h]);
+            }
             s0 += PRE;
             if (s0 >= s_hi) break;
             fetch(n, s0);
