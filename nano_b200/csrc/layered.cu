@@ -1030,6 +1030,7 @@ int attn_optin(int smem) {
 // ---------------- mixers: e->hm [T][E] -> e->d [T][E], from the cache pages and the state slot of the sequence ----------------
 struct Ctx { float *st; const uint32_t *table; uint32_t T, pos0; const uint32_t *pos_ptr; };
 
+constexpr size_t kSideMixBytes = 8u << 20;      // a recurrent mixer's weights up to which a single token's feed-forward keeps the norm's stream
 constexpr uint64_t kTcAttnWork = 128 * 128;      // tokens x keys, or keys, from which a portion's grouped-query attention goes to the tensor cores
 constexpr uint32_t kTcAttnKeys = 512, kTcLatentKeys = 128;      // ... and keys from which latents are multiplied out
 
@@ -1833,12 +1834,19 @@ int run_layers(LayeredEngine *e, uint32_t slot, uint32_t T, uint32_t pos0, const
             } else if ((r = launch<NormShiftArgs>(e, k_norm_shift, dim3(T > 1 ? T - 1 : 1), dim3(256), 0, a))) return r;
             if (L.has_mlp && e->branch_streams) CK(cudaEventRecord(e->ev_fork, e->stream));
         }
+        // A lone token's feed-forward (routing, then two products of the experts it chose) is a longer chain than a recurrent mixer of few bytes: it follows the norm on the norm's own
+        // stream, where its first kernel's weights are on the way before the norm ends, and the mixer is the branch.  Mixer of 6 MB (width 1024, eight layers) 224 us a token the other way round, 216 this
+        // way; of 12 MB (the same in 32 bits, two layers) 73.0 and 73.9, of 24 MB 112 and 116.  Latent attention is the longer chain in its layers.
+        const bool side_mix = T == 1 && L.has_mlp && e->branch_streams && L.type == MIX_RGLRU &&
+                              ((size_t)L.yx.rows * L.yx.cols + (size_t)L.o.rows * L.o.cols) * (e->f32 ? 4u : 2u) <= kSideMixBytes;
+        if (side_mix) { e->cur = e->side; CK(cudaStreamWaitEvent(e->side, e->ev_fork, 0)); }
         if ((r = mix(e, L, run, cx))) return r;
+        if (side_mix) { CK(cudaEventRecord(e->ev_join, e->side)); e->cur = e->stream; }
         CombineArgs c{e->x, e->d, nullptr, nullptr, nullptr, nullptr, keep, T, E, 0};
         if (L.has_mlp) {
             // The layer is parallel: the feed-forward reads h2 = norm2(x) of the SAME x and shares no buffer with the mixer, so its
             // kernels go to a second stream (a parallel branch of the captured decode graph) and join before the residual update.
-            if (e->branch_streams) { e->cur = e->side; CK(cudaStreamWaitEvent(e->side, e->ev_fork, 0)); }
+            if (e->branch_streams && !side_mix) { e->cur = e->side; CK(cudaStreamWaitEvent(e->side, e->ev_fork, 0)); }
             if ((r = ff_moe_relu2(e, L, T))) return r;
             if (L.has_shared) {      // a third branch: the shared expert depends on h2 only
                 if (e->branch_streams) { e->cur = e->side2; CK(cudaStreamWaitEvent(e->side2, e->ev_fork, 0)); }
@@ -1847,7 +1855,7 @@ int run_layers(LayeredEngine *e, uint32_t slot, uint32_t T, uint32_t pos0, const
             }
             c.eo = e->b_eo; c.slot = e->b_slot; c.wt = e->b_wt; c.shared = L.has_shared ? e->b_so : nullptr; c.top = L.top;
             e->cur = e->stream;
-            if (e->branch_streams) { CK(cudaEventRecord(e->ev_join, e->side)); CK(cudaStreamWaitEvent(e->stream, e->ev_join, 0)); }
+            if (e->branch_streams) { if (!side_mix) CK(cudaEventRecord(e->ev_join, e->side)); CK(cudaStreamWaitEvent(e->stream, e->ev_join, 0)); }
         }
         // a lone token: the update also norms the row for the run that follows (two links of 2.4 and 2.3 us, now one)
         const Run *nrun = ri + 1 < e->runs.size() && !e->runs[ri + 1].add_embed ? &e->runs[ri + 1] : nullptr;
