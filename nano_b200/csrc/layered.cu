@@ -1418,7 +1418,7 @@ int delta_branch(LayeredEngine *e, const Layer &L, const Run &run, const Ctx &cx
 #undef DELTA_STEP
         return r ? r : gemm(e, plain(e->b_ga, H * VD, L.d_o, dst, e->E, T), 1, T);
     }
-    if (L.ra && (r = gemm(e, plain(e->b_p + L.c_a, P, L.a2, e->b_gsp, H * D, T, L.d_bias, EPI_SOFTPLUS), 1, T))) return r;
+    if (L.ra && (r = gemm(e, plain(e->b_p + L.c_a, P, L.a2, e->b_gsp, H * D, T, L.d_bias), 1, T))) return r;
     if (L.rg && (r = gemm(e, plain(e->b_p + L.c_g, P, L.g2, e->b_gt, H * VD, T), 1, T))) return r;
     const uint32_t chunks = (T + kDeltaChunk - 1u) / kDeltaChunk;
     DeltaPrepArgs pa{e->b_p, P, L.c_conv, L.c_b, L.c_a, L.d_conv, cx.st + run.st_conv, L.d_taps, L.ra ? e->b_gsp : nullptr, L.d_bias, L.d_rate,

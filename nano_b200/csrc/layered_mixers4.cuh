@@ -588,7 +588,7 @@ __device__ __forceinline__ float delta_decay(float rate, float sp) { return (flo
 
 struct DeltaPrepArgs {
     const float *p; uint32_t ld, c0, b0, a0; const float *taps; const float *state; uint32_t K;      // c0: the first convolved channel's column
-    const float *sp;                       // per-channel decay: softplus already taken, [T][H D]; null: one decay per head from column a0 + h
+    const float *sp;                       // per-channel decay: the low-rank product with its bias, [T][H D]; null: one decay per head from column a0 + h
     const float *dt_bias, *rate;
     float *blk, *v;                        // blk [chunks][H][delta_block], v [T][H VD]
     uint32_t T, H, G, D, VD; float qscale;
@@ -661,7 +661,7 @@ __global__ void __launch_bounds__(kDeltaPrepThreads) k_delta_prep(const DeltaPre
 #pragma unroll 1
         for (uint32_t i = tid; i < CN * DP; i += NT) {
             const uint32_t t = t0 + i / DP, d = i % DP;
-            g_s[i] = t < a.T && d < D ? delta_decay(rate, a.sp[((size_t)t * a.H + h) * D + d]) : 1.0f;
+            g_s[i] = t < a.T && d < D ? delta_decay(rate, softplusf_(a.sp[((size_t)t * a.H + h) * D + d])) : 1.0f;          // (softplus here: as the product's epilogue, four warps a tile, it was 26 us of a product of 37)
         }
     } else {
         if (tid < CN) fac[tid] = t0 + tid < a.T ? delta_decay(rate, softplusf_(a.p[(size_t)(t0 + tid) * a.ld + a.a0 + h] + a.dt_bias[h])) : 1.0f;
