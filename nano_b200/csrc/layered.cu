@@ -972,8 +972,9 @@ int gemm(LayeredEngine *e, GemmArgs a, uint32_t groups, uint32_t maxM, bool wf32
     if (a.glu) return fail(NB200_EINVAL, "the gated-pair product is a matrix-vector instance (portions of at most %u tokens)", kGemvMaxM);
     const uint32_t rows = a.g_off && active ? active : a.M;
     if (!f32 && (!a.g_off || active) && tc_fits(&e->tc, a, rows)) {
-        e->launches += 2;
-        return tc_gemm(&e->tc, a, groups, maxM, rows, a.g_off ? std::max(1u, (active + groups - 1u) / groups) : maxM, e->cur == e->side ? 1u : e->cur == e->side2 ? 2u : 0u, e->cur, e->use_pdl);
+        const uint32_t each = a.g_off ? std::max(1u, (active + groups - 1u) / groups) : maxM;
+        e->launches += tc_raw_rows(a, groups, each) ? 1 : 2;
+        return tc_gemm(&e->tc, a, groups, maxM, rows, each, e->cur == e->side ? 1u : e->cur == e->side2 ? 2u : 0u, e->cur, e->use_pdl);
     }
     const dim3 grid((a.N + 63u) / 64u, (maxM + 63u) / 64u, groups);
     if (f32 && gemm_f32_fits(a)) {

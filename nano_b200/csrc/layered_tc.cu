@@ -1,7 +1,7 @@
 // layered_tc.cu -- matrix products of long portions on the fifth-generation tensor cores (layered.cu chooses them; layered_kernels.cuh has
 // the tile products for shapes that this path does not take).
 //
-//   k_rows_bf16   the product's fp32 activation rows, rounded once to bfloat16 (what every product of this family does to its operand) and
+//   k_rows_bf16   the product's fp32 activation rows, rounded once to bfloat16 (what every product of this family does to its operand; short portions round them in k_gemm_tc) and
 //                 gathered into expert order where a row list says so: a dense matrix that bulk copies can read
 //   k_gemm_tc     C^T = W A^T in tiles of 128 weight rows x TN tokens: tcgen05.mma (one issuing thread), operands by cp.async.bulk.tensor into a ring of
 //                 128-byte-swizzled stages, fp32 accumulators in tensor memory.  A tensor-memory lane is an output COLUMN of C, so a
@@ -152,9 +152,57 @@ __device__ __forceinline__ void gather(const TcArgs &ta, const GroupView &gv, ui
     }
 }
 
+// A tile's activations, rounded to bfloat16 and swizzled as a bulk copy would leave them, by the four warps that finish the tile later: a thread has 16 columns of every 32nd row of a
+// stage.  Short portions (TN 32 and 64), whose products are a chain of launches: a kernel of its own for the rows, and the wait for it, cost 2 to 4 us a product.
 template <int TN>
+__device__ __forceinline__ bool tc_rows(const GemmArgs &a, const GroupView &gv, uint32_t m0, uint32_t s0, uint32_t ns, uint32_t ring, uint32_t full, uint32_t empty) {
+    constexpr uint32_t ST = tc_stages(TN), SB = tc_stage_bytes(TN), NR = TN / 32;
+    const uint32_t t = threadIdx.x - 64u, r = t >> 2, c16 = (t & 3u) * 16u;
+    const float *src[NR];
+#pragma unroll
+    for (uint32_t h = 0; h < NR; h++) {
+        const uint32_t row = m0 + r + 32u * h;
+        src[h] = row < gv.rows ? a.A + (size_t)(a.a_rows ? a.a_rows[gv.r0 + row] : gv.r0 + row) * a.lda + gv.a0 : nullptr;
+    }
+    float4 v[NR][4];
+    auto load = [&](uint32_t i) {
+        const uint32_t k = (s0 + i) * kTcK + c16;
+#pragma unroll
+        for (uint32_t h = 0; h < NR; h++)
+#pragma unroll
+            for (uint32_t q = 0; q < 4u; q++) v[h][q] = src[h] && k + 4u * q < a.K ? *reinterpret_cast<const float4 *>(src[h] + k + 4u * q) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    };
+    if (ns) load(0);
+    for (uint32_t i = 0; i < ns; i++) {
+        const uint32_t st = i % ST, rows = ring + st * SB + kTcRows * kTcK * 2u;
+        uint4 o[NR][2];
+#pragma unroll
+        for (uint32_t h = 0; h < NR; h++)
+#pragma unroll
+            for (uint32_t q = 0; q < 4u; q++) {
+                __nv_bfloat162 *ob = reinterpret_cast<__nv_bfloat162 *>(&o[h][q >> 1]) + (q & 1u) * 2u;
+                ob[0] = __floats2bfloat162_rn(v[h][q].x, v[h][q].y); ob[1] = __floats2bfloat162_rn(v[h][q].z, v[h][q].w);
+            }
+        if (i + 1u < ns) load(i + 1u);
+        if (i >= ST && !mbar_wait_warp(empty + st * 8u, ((i / ST) - 1u) & 1u)) return false;
+#pragma unroll
+        for (uint32_t h = 0; h < NR; h++)
+#pragma unroll
+            for (uint32_t q = 0; q < 2u; q++) {
+                const uint32_t row = r + 32u * h, at = rows + row * 128u + ((((c16 >> 3) + q) ^ (row & 7u)) << 4);
+                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(o[h][q].x), "r"(o[h][q].y), "r"(o[h][q].z), "r"(o[h][q].w) : "memory");
+            }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");          // plain stores, read by the tensor core
+        __syncwarp();
+        if ((threadIdx.x & 31u) == 0) mbar_arrive(full + st * 8u);
+    }
+    return true;
+}
+
+// RAW: the activations are ta.g.A itself (fp32 rows of whole 16-byte pieces), not a rounded copy that bulk copies read
+template <int TN, bool RAW>
 __global__ void __launch_bounds__(192) k_gemm_tc(const __grid_constant__ TcArgs ta) {
-    constexpr uint32_t ST = tc_stages(TN), SB = tc_stage_bytes(TN), COLS = TN < 32 ? 32 : TN;
+    constexpr uint32_t ST = tc_stages(TN), SB = tc_stage_bytes(TN), COLS = TN < 32 ? 32 : TN, LOADED = RAW ? kTcRows * kTcK * 2u : SB;          // bytes of a stage that bulk copies bring
     extern __shared__ uint8_t tc_raw[];
     __shared__ __align__(8) uint64_t bars[2 * ST + 1];
     __shared__ uint32_t tmem_s, bad_s;
@@ -170,7 +218,7 @@ __global__ void __launch_bounds__(192) k_gemm_tc(const __grid_constant__ TcArgs 
         if (m0 >= a.g_off[group + 1] - a.g_off[group]) return;
     }
     if (threadIdx.x == 0) {
-        for (uint32_t i = 0; i < ST; i++) { mbar_init(full + i * 8u, 1); mbar_init(empty + i * 8u, 1); }
+        for (uint32_t i = 0; i < ST; i++) { mbar_init(full + i * 8u, RAW ? 5 : 1); mbar_init(empty + i * 8u, 1); }
         mbar_init(done, 1);
         bad_s = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -183,15 +231,15 @@ __global__ void __launch_bounds__(192) k_gemm_tc(const __grid_constant__ TcArgs 
     pdl_launch_next();
     const uint32_t tmem = tmem_s, npre = a.g_off ? 0u : min(ST, ns);
     if (warp == 0 && lane == 0)          // weights do not depend on the kernel before: their first tiles are on the way while it ends
-        for (uint32_t i = 0; i < npre; i++) { mbar_expect(full + i * 8u, SB); tma_3d(ring + i * SB, &ta.wmap, (s0 + i) % ta.wsteps * kTcK, n0, group, full + i * 8u); }
+        for (uint32_t i = 0; i < npre; i++) { mbar_expect(full + i * 8u, LOADED); tma_3d(ring + i * SB, &ta.wmap, (s0 + i) % ta.wsteps * kTcK, n0, group, full + i * 8u); }
     pdl_wait();
     const GroupView gv = group_view(a, group);
     if (warp == 0 && lane == 0) {
         for (uint32_t i = 0; i < ns; i++) {
             const uint32_t st = i % ST, bar = full + st * 8u, dst = ring + st * SB;
             if (i >= ST && !mbar_wait(empty + st * 8u, ((i / ST) - 1u) & 1u)) { bad_s = 1; break; }
-            if (i >= npre) { mbar_expect(bar, SB); tma_3d(dst, &ta.wmap, (s0 + i) % ta.wsteps * kTcK, n0, group, bar); }
-            tma_3d(dst + kTcRows * kTcK * 2u, &ta.amap, (s0 + i) * kTcK, group % a.a_gmod, gv.r0 + m0, bar);
+            if (i >= npre) { mbar_expect(bar, LOADED); tma_3d(dst, &ta.wmap, (s0 + i) % ta.wsteps * kTcK, n0, group, bar); }
+            if (!RAW) tma_3d(dst + kTcRows * kTcK * 2u, &ta.amap, (s0 + i) * kTcK, group % a.a_gmod, gv.r0 + m0, bar);
         }
     } else if (warp == 1 && lane == 0) {
         constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TN >> 3) << 17) | ((kTcRows >> 4) << 24);      // fp32 += bf16 x bf16, both K-major
@@ -213,6 +261,7 @@ __global__ void __launch_bounds__(192) k_gemm_tc(const __grid_constant__ TcArgs 
     bool live = true;
     const uint32_t quad = warp & 3u, n = n0 + quad * 32u + lane, rows = gv.rows;
     if (warp >= 2) {
+        if constexpr (RAW) { if (!tc_rows<TN>(a, gv, m0, s0, ns, ring, full, empty)) bad_s = 4; }
         live = mbar_wait_warp(done, 0);
         if (!live) bad_s = 3;
         tc_fence_after();
@@ -291,8 +340,8 @@ int launch(void (*k)(const A), dim3 grid, dim3 block, size_t smem, cudaStream_t 
     NB_CK(cudaLaunchKernelEx(&cfg, k, args));
     return 0;
 }
-template <int TN>
-int optin() { NB_CK(nb::smem_at_least((const void *)k_gemm_tc<TN>, (int)tc_smem(TN))); return 0; }
+template <int TN, bool RAW>
+int optin() { NB_CK(nb::smem_at_least((const void *)k_gemm_tc<TN, RAW>, (int)tc_smem(TN))); return 0; }
 }  // namespace
 
 int tc_setup(TcState *t, size_t elems, uint32_t sms) {
@@ -308,7 +357,7 @@ int tc_setup(TcState *t, size_t elems, uint32_t sms) {
     *t->err_host = 0;
     NB_CK(cudaHostGetDevicePointer(&t->err_dev, t->err_host, 0));
     int r;
-    if ((r = optin<32>()) || (r = optin<64>()) || (r = optin<128>())) return r;
+    if ((r = optin<32, true>()) || (r = optin<64, true>()) || (r = optin<32, false>()) || (r = optin<64, false>()) || (r = optin<128, false>())) return r;
     return 0;
 }
 void tc_free(TcState *t) {
@@ -333,18 +382,21 @@ bool tc_fits(const TcState *t, const GemmArgs &a, uint32_t rows) {
     return t->encode && a.K % 8u == 0 && a.ldw % 8u == 0 && a.w_gstride % 8u == 0 && (a.a_gmod == 1 || a.a_gcols % 8u == 0) && (reinterpret_cast<uintptr_t>(a.W) & 15u) == 0 && rows * width <= t->elems;
 }
 int tc_gemm(TcState *t, GemmArgs a, uint32_t groups, uint32_t maxM, uint32_t rows, uint32_t each, uint32_t buf, cudaStream_t stream, bool pdl) {
-    const uint32_t width = (a.a_gmod - 1) * a.a_gcols + a.K;
+    const uint32_t width = (a.a_gmod - 1) * a.a_gcols + a.K, tn = each <= 32 ? 32u : each <= 64 ? 64u : 128u;
+    const bool raw = tc_raw_rows(a, groups, each);
     __nv_bfloat16 *dst = t->rows[buf];
     int r;
-    const RowsArgs ra{a.A, a.lda, a.a_rows, dst, width, rows, width};
-    const size_t threads = (size_t)rows * width / 8u;
-    if ((r = launch<RowsArgs>(k_rows_bf16, dim3((uint32_t)((threads + 255u) / 256u < t->sms * 16u ? (threads + 255u) / 256u : t->sms * 16u)), dim3(256), 0, stream, pdl, ra))) return r;
-    a.A = nullptr; a.a_rows = nullptr;
-    const uint32_t tn = each <= 32 ? 32u : each <= 64 ? 64u : 128u;
     TcArgs ta{};
+    if (!raw) {
+        const RowsArgs ra{a.A, a.lda, a.a_rows, dst, width, rows, width};
+        const size_t threads = (size_t)rows * width / 8u;
+        if ((r = launch<RowsArgs>(k_rows_bf16, dim3((uint32_t)((threads + 255u) / 256u < t->sms * 16u ? (threads + 255u) / 256u : t->sms * 16u)), dim3(256), 0, stream, pdl, ra))) return r;
+        a.A = nullptr; a.a_rows = nullptr;
+        if (!tensor_map(t, &ta.amap, dst, a.K, a.a_gmod, rows, (uint64_t)(a.a_gmod > 1 ? a.a_gcols : width) * 2u, (uint64_t)width * 2u, kTcK, 1, tn))
+            return fail(NB200_ECUDA, "cuTensorMapEncodeTiled refused the rows of a product of %u x %u x %u", rows, a.N, a.K);
+    }
     ta.g = a; ta.err = t->err_dev;
-    if (!tensor_map(t, &ta.wmap, a.W, a.K, a.N, groups, (uint64_t)a.ldw * 2u, groups > 1 ? a.w_gstride * 2u : (uint64_t)a.ldw * 2u * a.N, kTcK, kTcRows, 1) ||
-        !tensor_map(t, &ta.amap, dst, a.K, a.a_gmod, rows, (uint64_t)(a.a_gmod > 1 ? a.a_gcols : width) * 2u, (uint64_t)width * 2u, kTcK, 1, tn))
+    if (!tensor_map(t, &ta.wmap, a.W, a.K, a.N, groups, (uint64_t)a.ldw * 2u, groups > 1 ? a.w_gstride * 2u : (uint64_t)a.ldw * 2u * a.N, kTcK, kTcRows, 1))
         return fail(NB200_ECUDA, "cuTensorMapEncodeTiled refused a product of %u x %u x %u", rows, a.N, a.K);
     // Blocks of a cluster share a tile's depth while fewer than 7 of 10 SMs have one, down to two stages each (two layers of width 2048: 200 tokens 644 us
     // before, 443 with it; up to two blocks per SM, ks = 2 for 128 tiles, was the same within the noise at 1024 tokens)
@@ -353,9 +405,9 @@ int tc_gemm(TcState *t, GemmArgs a, uint32_t groups, uint32_t maxM, uint32_t row
     while (ks < 8u && tiles * ks * 10u <= t->sms * 7u && steps >= ks * 4u) ks *= 2u;
     ta.ks = ks; ta.wsteps = steps;
     const dim3 grid((a.N + kTcRows - 1u) / kTcRows, (maxM + tn - 1u) / tn, groups * ks), block(192);
-    if (tn == 32) return launch<TcArgs>(k_gemm_tc<32>, grid, block, tc_smem(32), stream, pdl, ta, ks);
-    if (tn == 64) return launch<TcArgs>(k_gemm_tc<64>, grid, block, tc_smem(64), stream, pdl, ta, ks);
-    return launch<TcArgs>(k_gemm_tc<128>, grid, block, tc_smem(128), stream, pdl, ta, ks);
+    if (tn == 32) return launch<TcArgs>(raw ? k_gemm_tc<32, true> : k_gemm_tc<32, false>, grid, block, tc_smem(32), stream, pdl, ta, ks);
+    if (tn == 64) return launch<TcArgs>(raw ? k_gemm_tc<64, true> : k_gemm_tc<64, false>, grid, block, tc_smem(64), stream, pdl, ta, ks);
+    return launch<TcArgs>(k_gemm_tc<128, false>, grid, block, tc_smem(128), stream, pdl, ta, ks);
 }
 
 int tc_split_setup(TcState *t, size_t elems) {
@@ -377,7 +429,7 @@ int tc_gemm_split(TcState *t, const float *cache, const uint32_t *table, uint32_
     ta.err = t->err_dev; ta.ks = 1; ta.wsteps = width / 3u / kTcK;
     if (!tensor_map(t, &ta.wmap, W, K, N, 1, (uint64_t)K * 2u, (uint64_t)K * 2u * N, kTcK, kTcRows, 1) || !tensor_map(t, &ta.amap, t->planes, width, 1, rows, (uint64_t)width * 2u, (uint64_t)width * 2u, kTcK, 1, 128))
         return fail(NB200_ECUDA, "cuTensorMapEncodeTiled refused a product of %u x %u x %u", rows, N, width);
-    return launch<TcArgs>(k_gemm_tc<128>, dim3((N + kTcRows - 1u) / kTcRows, (rows + 127u) / 128u, 1), dim3(192), tc_smem(128), stream, pdl, ta);
+    return launch<TcArgs>(k_gemm_tc<128, false>, dim3((N + kTcRows - 1u) / kTcRows, (rows + 127u) / 128u, 1), dim3(192), tc_smem(128), stream, pdl, ta);
 }
 
 }  // namespace lm

@@ -8,6 +8,7 @@
 namespace nb {
 namespace lm {
 
+constexpr uint64_t kTcRawBytes = 32u << 20;
 // what an engine keeps for these products: rounded activation rows (one buffer for each of its three streams), the driver's tensor-map encoder,
 // the word a bounded wait reports to
 struct TcState {
@@ -22,7 +23,14 @@ void tc_free(TcState *t);
 int tc_check(TcState *t);
 // whether the product's layout allows it.  rows: all rows of A it reads (a routed product: tokens x choices)
 bool tc_fits(const TcState *t, const GemmArgs &a, uint32_t rows);
-// two launches on `stream` (with programmatic serialization when pdl).  buf: which of the row buffers is the stream's; maxM: the most rows of a group, each:
+// Does the product read its fp32 rows itself (one launch), or a rounded copy that a launch of its own makes before it.  each: as below.  Groups of at most 64 rows on average, whose tiles are
+// 32 or 64 tokens, and only while the tiles read less than 32 MB of them: every tile of weights reads the rows again.  Two layers, us a portion, copy / rows: Famudra width 1024 (eight layers) 5 tokens
+// 616 / 470, 11 535 / 490, 40 718 / 677, 64 783 / 708; Fidatar width 1024 5 162 / 147, 64 184 / 180; Kadesun width 2048 5 220 / 207, 40 257 / 245, but 64 (50 MB for 12288 columns) 254 / 260 and
+// Fidatar width 2048 64 (33 MB) 258 / 264.
+inline bool tc_raw_rows(const GemmArgs &a, uint32_t groups, uint32_t each) {
+    return each <= 64u && a.lda % 4u == 0 && (reinterpret_cast<uintptr_t>(a.A) & 15u) == 0 && (uint64_t)((a.N + 127u) / 128u) * groups * each * a.K * 4u <= kTcRawBytes;
+}
+// one or two launches on `stream` (with programmatic serialization when pdl).  buf: which of the row buffers is the stream's; maxM: the most rows of a group, each:
 // how many a group has on average
 int tc_gemm(TcState *t, GemmArgs a, uint32_t groups, uint32_t maxM, uint32_t rows, uint32_t each, uint32_t buf, cudaStream_t stream, bool pdl);
 
