@@ -43,7 +43,7 @@ UNITS = {
     "layered_tc.cu": ["layered_common.cuh", "layered_tc.h", "tc_ptx.cuh", "family.h"],
     "attn_tc.cu": ["attn_tc.h", "tc_ptx.cuh", "family.h"],
     "prefill.cu": ["prefill.h", "prompt_split.h", "attn_tc.h", "tc_ptx.cuh", "kernels.cuh", "expf_ref.cuh", "family.h"],
-    "engine.cu": ["prefill.h", "attn_tc.h", "kernels.cuh", "expf_ref.cuh", "stream_args.h", "stream_count.h", "stream_host.h", "sample_host.h", "family.h", "../../include/nano_b200.h"],
+    "engine.cu": ["prefill.h", "attn_tc.h", "kernels.cuh", "expf_ref.cuh", "stream_args.h", "stream_count.h", "stream_groups.h", "stream_host.h", "sample_host.h", "family.h", "../../include/nano_b200.h"],
     "stream.cu": ["kernels.cuh", "expf_ref.cuh", "stream_args.h", "stream_host.h", "stream.cuh"],
     "sample.cu": ["kernels.cuh", "expf_ref.cuh", "sample_host.h"],
 }

@@ -28,6 +28,7 @@
 #include "../../include/nano_b200.h"
 #include "kernels.cuh"
 #include "stream_count.h"
+#include "stream_groups.h"
 #include "stream_host.h"
 #include "sample_host.h"
 #include "family.h"
@@ -95,7 +96,8 @@ struct nb200_engine : nb::EngineBase {
     unsigned long long *trace_dev = nullptr;
     // grid-wide persistent streaming kernel (stream.cuh): the default path in fast mode on one GPU
     float calib_ms[2] = {0.0f, 0.0f};      // ms per token of {streaming, multi-kernel} measured by calibrate_paths (0 = not calibrated)
-    bool use_stream = false; const void *st_kern = nullptr; StreamArgs sa{}; uint32_t st_smem = 0, st_grid = 0;
+    bool use_stream = false; const void *st_kern[3] = {nullptr, nullptr, nullptr}; StreamArgs sa{};      // st_kern: by 1, 2, 4 query heads to an attention item (stream_groups.h)
+     uint32_t st_smem = 0, st_grid = 0;
     uint32_t *st_err_host = nullptr, *st_err_dev = nullptr;      // mapped pinned word: the code a device-side spin recorded before trapping
     nb::StreamCount st_count;                                    // exchange epochs and barrier arrivals used up so far (stream.cuh)
     float *logits_host = nullptr; bool logits_on_host = false;   // pinned copy of the logits that one-token calls of the streaming kernel write; whether it holds the last step's
@@ -386,27 +388,38 @@ int run_token(nb200_engine *e) {
     return run_classifier(e);
 }
 
-// n_steps tokens in ONE cooperative launch of the streaming kernel.  st: the state of its first step (null: what the launch before left on the device);
-// with_logits: the (last) step's logits also go to the pinned copy
-int launch_stream(nb200_engine *e, uint32_t n_steps, const DevState *st = nullptr, bool with_logits = false) {
+// n_steps tokens on the streaming kernel, the first at position pos: one cooperative launch, or one for each run of positions whose attention items have the same number of heads (a token
+// runs on the same kernel however it is asked for).  st: the state of the first step (null: what the launch before left on the device);
+// with_logits: the (last) step's logits also go to the pinned copy; causal 0: the token sees the whole context
+int launch_stream(nb200_engine *e, uint32_t n_steps, uint32_t pos, uint32_t causal = 1, const DevState *st = nullptr, bool with_logits = false) {
     e->logits_on_host = false;
-    if (n_steps == 0) return 0;
-    StreamArgs g = e->sa;
-    g.n_steps = n_steps; g.trace = e->trace_dev;
-    if (st) { g.st0 = *st; g.with_state = 1; g.next_host = e->tok_host; }
-    if (with_logits) g.logits_host = e->logits_host;
-    return e->st_count.run(n_steps * 5u * e->d.L, n_steps * e->st_grid, [&](uint32_t epoch, uint32_t bar) -> int {
-        g.epoch_base = epoch; g.bar_base = bar;
-        void *params[] = {&g};
-        CK(cudaLaunchCooperativeKernel(e->st_kern, dim3(e->st_grid), dim3(kThreads), params, e->st_smem, e->stream));
-        e->launches++;
-        return 0;
-    });
+    const Dims &d = e->d;
+    auto heads_at = [&](uint32_t p) { return nb::st_group_heads(d.KV, d.kv_mul, d.hd, d.quant == 0x42u, causal ? p + 1u : d.max_seq, e->st_grid); };
+    for (uint32_t done = 0; done < n_steps;) {
+        const uint32_t heads = heads_at(pos + done);
+        uint32_t n = 1;
+        while (done + n < n_steps && heads_at(pos + done + n) == heads) n++;
+        StreamArgs g = e->sa;
+        g.n_steps = n; g.trace = e->trace_dev;
+        g.group_div = d.kv_mul / heads; g.groups = d.KV * g.group_div; g.nsplit_max = nb::st_splits(g.groups, e->st_grid);
+        if (st && done == 0) { g.st0 = *st; g.with_state = 1; g.next_host = e->tok_host; }
+        if (with_logits) g.logits_host = e->logits_host;
+        const int r = e->st_count.run(n * 5u * d.L, n * e->st_grid, [&](uint32_t epoch, uint32_t bar) -> int {
+            g.epoch_base = epoch; g.bar_base = bar;
+            void *params[] = {&g};
+            CK(cudaLaunchCooperativeKernel(e->st_kern[heads >> 1], dim3(e->st_grid), dim3(kThreads), params, e->st_smem, e->stream));
+            e->launches++;
+            return 0;
+        });
+        if (r) return r;
+        done += n;
+    }
+    return 0;
 }
 
-int launch_token(nb200_engine *e) {
+int launch_token(nb200_engine *e, uint32_t pos, uint32_t causal = 1) {
     if (e->tp_size > 1 && !e->tp_attached) return fail(NB200_EINVAL, "tensor-parallel engine: attach the peer ranks first (nb200_tp_attach_*)");
-    if (e->use_stream) return launch_stream(e, 1);
+    if (e->use_stream) return launch_stream(e, 1, pos, causal);
     e->logits_on_host = false;
     if (e->graph) {
         CK(cudaGraphLaunch(e->graph, e->stream));
@@ -485,8 +498,9 @@ uint32_t env_u32(const char *name, uint32_t dflt) { const char *s = getenv(name)
 int setup_stream(nb200_engine *e) {
     const Dims &d = e->d;
     if (d.exact || e->tp_size > 1) return 0;
-    StreamKern k = pick_stream(d);
-    if (!k) return 0;
+    if (d.kv_mul != 1u && d.kv_mul != 2u && d.kv_mul != 4u) return 0;
+    const void *kerns[3] = {nullptr, nullptr, nullptr};
+    for (uint32_t h = 1; h <= d.kv_mul; h *= 2u) if (!(kerns[h >> 1] = (const void *)pick_stream(d, h))) return 0;
     uint32_t maxn = d.E; if (d.q_dim > maxn) maxn = d.q_dim; if (d.F > maxn) maxn = d.F;
     if (maxn > st_prep_max_n(d.quant, d.gs)) return 0;
     if (d.quant == 0x80u && (d.E % 16 || d.q_dim % 16 || d.F % 16)) return 0;
@@ -517,14 +531,12 @@ int setup_stream(nb200_engine *e) {
     // phase never waits for the slowest warp of the previous one before it writes its operand.  The ring stage is 16 KB by default and
     // shrinks in 1 KB steps (never below one row unit of the longest row) until kStSegTiles + 4 stages fit beside the fixed regions.
     auto al = [](uint32_t v) { return (v + 127u) & ~127u; };
-    const uint32_t nsplit_max = e->nsplit_max;          // num_sms / kv heads (<= 64), as the multi-kernel path
     const uint32_t act_b = al(act_region_bytes(d.quant, maxn, d.gs ? d.gs : 1));
     g.off_act = 0; g.off_act2 = act_b; g.off_xs = 2 * act_b; g.off_attn = g.off_xs + al(d.E * 4u);
     int max_optin = 0;
     CK(cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, e->device));
-    cudaFuncAttributes fattr;
-    CK(cudaFuncGetAttributes(&fattr, (const void *)k));
-    const uint32_t static_smem = al((uint32_t)fattr.sharedSizeBytes);   // mbarriers, row ranges, residual rows, reduction scratch
+    uint32_t static_smem = 0;
+    for (const void *k : kerns) if (k) { cudaFuncAttributes fattr; CK(cudaFuncGetAttributes(&fattr, k)); static_smem = std::max(static_smem, al((uint32_t)fattr.sharedSizeBytes)); }   // mbarriers, row ranges, residual rows, reduction scratch
     const uint32_t min_stage = (unit_b_max + 16u + 1023u) & ~1023u;
     uint32_t stage_bytes = env_u32("NB200_STAGE_KB", 16) * 1024u;
     if (stage_bytes < min_stage) stage_bytes = min_stage;
@@ -573,10 +585,13 @@ int setup_stream(nb200_engine *e) {
     g.cta_stride = (g.cls_off + (uint64_t)ntl[SK_CLS] * g.kind[SK_CLS].tile_stride + 127u) & ~(uint64_t)127u;
 
     const uint32_t smem = region0 + nst * stage_bytes;
-    cudaError_t ce = nb::smem_at_least((const void *)k, (int)smem);
-    int occ = 0;
-    if (ce == cudaSuccess) ce = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, (const void *)k, kThreads, smem);
-    if (ce != cudaSuccess || occ < 1) { cudaGetLastError(); return 0; }
+    for (const void *k : kerns) {
+        if (!k) continue;
+        cudaError_t ce = nb::smem_at_least(k, (int)smem);
+        int occ = 0;
+        if (ce == cudaSuccess) ce = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, kThreads, smem);
+        if (ce != cudaSuccess || occ < 1) { cudaGetLastError(); return 0; }
+    }
 
     // device objects: the stream copy of the weights
     uint8_t *stream = nullptr;
@@ -618,16 +633,19 @@ int setup_stream(nb200_engine *e) {
             g.rs[i] = ((ns[i] + 31u) & ~31u) + 32u;                 // replicas 256 bytes apart at least: different L2 slices
             if ((r = words(g.xv[i], (size_t)g.rs[i] * kStRep))) return r;
         }
-        if ((r = words(g.xws, (size_t)d.KV * nsplit_max * d.kv_mul * (d.hd + 2)))) return r;
+        size_t parts = 0;
+        for (uint32_t h = 1; h <= d.kv_mul; h *= 2u) { const uint32_t n = d.KV * (d.kv_mul / h); parts = std::max(parts, (size_t)n * nb::st_splits(n, NC) * h * (d.hd + 2)); }
+        if ((r = words(g.xws, parts))) return r;
     }
     g.cls_val = e->cls_val; g.cls_idx = e->cls_idx;
     g.st = e->st; g.ids = e->ids_dev; g.seen = e->seen; g.bar = e->bar; g.err = e->st_err_dev;
-    g.n_steps = 1; g.nsplit_max = nsplit_max;
+    g.n_steps = 1;
     uint32_t ct = 32768u / (d.hd * 8u); ct &= ~7u; if (ct < 32) ct = 32;      // measured: ~32 KB of K+V per (kv head, split) item
     g.chunk_target = env_u32("NB200_ATTN_CHUNK", ct);
     if (g.chunk_target < 8) g.chunk_target = 8;
     g.d = d;
-    e->st_kern = (const void *)k; e->st_smem = smem; e->st_grid = NC; e->use_stream = true; e->launches_per_token = 1;
+    for (int i = 0; i < 3; i++) e->st_kern[i] = kerns[i];
+    e->st_smem = smem; e->st_grid = NC; e->use_stream = true; e->launches_per_token = 1;
     return 0;
 }
 
@@ -978,8 +996,8 @@ static int calibrate_paths(nb200_engine *e) {
             CK(cudaMemsetAsync(e->ids_dev, 0, (size_t)(pos0 + 1) * 4, e->stream));
             if ((r = push_state(e, pos0, 1, pos0 + 1, 1, 1.0f, 0, 0))) return r;
             CK(cudaEventRecord(evs.ev[0], e->stream));
-            if (e->use_stream) { if ((r = launch_stream(e, n))) return r; }
-            else for (uint32_t i = 0; i < n; i++) if ((r = launch_token(e))) return r;
+            if (e->use_stream) { if ((r = launch_stream(e, n, pos0))) return r; }
+            else for (uint32_t i = 0; i < n; i++) if ((r = launch_token(e, pos0 + i))) return r;
             CK(cudaEventRecord(evs.ev[1], e->stream));
             CK(cudaStreamSynchronize(e->stream));
             CK(cudaEventElapsedTime(&ms[path], evs.ev[0], evs.ev[1]));
@@ -1168,11 +1186,11 @@ static int push_state(nb200_engine *e, uint32_t pos, uint32_t causal, uint32_t n
 // pinned memory that the kernel writes while it works: a copy in front of the kernel, one behind it and the waits between cost 45 us of a 134 us
 // call (four F32 layers of Nano's width), and 100 of 690 for the 608 KB of Qwen3's logits.
 static int run_one(nb200_engine *e, uint32_t pos, uint32_t causal, float penalty, uint32_t token, bool with_logits) {
-    if (!e->use_stream) { const int r = push_state(e, pos, causal, 0, 0, penalty, token, 1); return r ? r : launch_token(e); }
+    if (!e->use_stream) { const int r = push_state(e, pos, causal, 0, 0, penalty, token, 1); return r ? r : launch_token(e, pos, causal); }
     DevState st;
     memset(&st, 0, sizeof st);
     st.pos = pos; st.is_causal = causal; st.penalty = penalty; st.token = token; st.use_token = 1;
-    return launch_stream(e, 1, &st, with_logits);
+    return launch_stream(e, 1, pos, causal, &st, with_logits);
 }
 
 static int nano_forward(nb200_engine *e, uint32_t token, uint32_t pos, uint32_t is_causal) {
@@ -1243,7 +1261,7 @@ static int nano_next_sampled(nb200_engine *e, const uint32_t *ids, uint32_t pos,
     int r;
     if ((r = push_state(e, pos, 1, 0, 0, penalty, ids[pos], 1))) return r;
     if (penalty != 1.0f) { if ((r = sync_seen(e, ids, pos))) return r; }
-    if ((r = launch_token(e))) return r;
+    if ((r = launch_token(e, pos))) return r;
     uint32_t *out_dev = nullptr;
     CK(sample_top_p_launch(e->samp_ws, e->samp_cub, e->logits, e->d.V, temperature, top_p, coin, e->st, &out_dev, e->stream));
     e->launches += 3;
@@ -1284,11 +1302,11 @@ static int nano_decode_greedy(nb200_engine *e, uint32_t *ids, uint32_t n_prompt,
         CK(cudaGetLastError());
         e->launches++;
     }
-    if (e->use_stream) { if ((r = launch_stream(e, first - start))) return r; }
-    else for (uint32_t p = start; p < first; p++) if ((r = launch_token(e))) return r;
+    if (e->use_stream) { if ((r = launch_stream(e, first - start, start))) return r; }
+    else for (uint32_t p = start; p < first; p++) if ((r = launch_token(e, p))) return r;
     CK(cudaEventRecord(ev[1], e->stream));
-    if (e->use_stream) { if ((r = launch_stream(e, n_total - n_prompt))) return r; }
-    else for (uint32_t p = n_prompt - 1; p + 1 < n_total; p++) if ((r = launch_token(e))) return r;
+    if (e->use_stream) { if ((r = launch_stream(e, n_total - n_prompt, n_prompt - 1u))) return r; }
+    else for (uint32_t p = n_prompt - 1; p + 1 < n_total; p++) if ((r = launch_token(e, p))) return r;
     CK(cudaEventRecord(ev[2], e->stream));
     CK(cudaMemcpyAsync(ids, e->ids_dev, (size_t)n_total * 4, cudaMemcpyDeviceToHost, e->stream));
     CK(cudaStreamSynchronize(e->stream));
@@ -1407,7 +1425,7 @@ int nb200_trace_token(nb200_engine *e, uint32_t token, uint32_t pos, unsigned lo
     CK(cudaMemset(buf, 0, (size_t)n * 8));
     e->trace_dev = buf;
     int r = push_state(e, pos, 1, 0, 0, 1.0f, token, 1);
-    if (!r) r = launch_stream(e, 1);
+    if (!r) r = launch_stream(e, 1, pos);
     e->trace_dev = nullptr;
     cudaStreamSynchronize(e->stream);
     if (!r) { CK(cudaMemcpy(stamps, buf, (size_t)n * 8, cudaMemcpyDeviceToHost)); *count = n; }

@@ -44,14 +44,14 @@ static StreamKern pick_stream_kvm(uint32_t kvm) {
     }
 }
 template <int QUANT, int LPG>
-static StreamKern pick_stream_hd(const Dims &d) { return d.hd <= 64 ? pick_stream_kvm<QUANT, LPG, 64>(d.kv_mul) : pick_stream_kvm<QUANT, LPG, 128>(d.kv_mul); }
+static StreamKern pick_stream_hd(const Dims &d, uint32_t heads) { return d.hd <= 64 ? pick_stream_kvm<QUANT, LPG, 64>(heads) : pick_stream_kvm<QUANT, LPG, 128>(heads); }
 
-StreamKern pick_stream(const Dims &d) {
+StreamKern pick_stream(const Dims &d, uint32_t heads) {
     if (d.hd > 128 || (d.arch == 3u && (d.hd & (d.hd - 1)) != 0)) return nullptr;     // in-register half-split RoPE needs hd = 4 * 2^k
-    if (d.quant == 0x00u) return pick_stream_hd<0x00, 8>(d);
-    if (d.quant == 0x42u) return pick_stream_hd<0x42, 8>(d);
-    if (d.gs == 128) return pick_stream_hd<0x80, 8>(d);
-    if (d.gs == 64) return pick_stream_hd<0x80, 4>(d);
+    if (d.quant == 0x00u) return pick_stream_hd<0x00, 8>(d, heads);
+    if (d.quant == 0x42u) return pick_stream_hd<0x42, 8>(d, heads);
+    if (d.gs == 128) return pick_stream_hd<0x80, 8>(d, heads);
+    if (d.gs == 64) return pick_stream_hd<0x80, 4>(d, heads);
     return nullptr;
 }
 

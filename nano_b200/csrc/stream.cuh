@@ -132,7 +132,7 @@ __device__ __forceinline__ void st_attn_plan(uint32_t range, uint32_t nsplit_max
     nsplit = (range + c - 1) / c;
 }
 
-struct StPlan { uint32_t nsplit, kvh, sp, t0, t1; };          // this CTA's attention item of the token (kvh >= KV: none)
+struct StPlan { uint32_t nsplit, grp, sp, t0, t1; };          // this CTA's attention item of the token (grp >= groups: none)
 struct StSmem { float red[2][16]; float best_v[kConsWarps]; uint32_t best_i[kConsWarps]; DevState st; uint32_t target, ti, tj; StPlan plan; };
 
 struct StRing {
@@ -188,8 +188,8 @@ static __device__ void st_producer(const StreamArgs &g, const StRing &r, const S
         for (uint32_t l = 0; l < d.L; l++) {
             const uint8_t *lb = base + (uint64_t)l * g.layer_stride;
             st_issue_kind(g, r, c, issued, g.kind[SK_QKV], lb, own[SK_QKV].rows);
-            if (cta < d.KV * nsplit) {
-                const uint32_t kvh = cta / nsplit, sp = cta % nsplit;
+            if (cta < g.groups * nsplit) {
+                const uint32_t kvh = cta / nsplit / g.group_div, sp = cta % nsplit;
                 const uint32_t t0 = min(range, sp * chunk), t1 = min(range, t0 + chunk);
                 const float *kb = g.kc + l * kvl + (size_t)kvh * d.max_seq * d.hd;
                 const float *vb = g.vc + l * kvl + (size_t)kvh * d.max_seq * d.hd;
@@ -580,7 +580,7 @@ __device__ __forceinline__ void st_consume(const StreamArgs &g, const StRing &r,
 }
 
 // ---------------------------------------------------------------- attention item (infer.c:814-879) on K/V tiles from the ring
-// One CTA = one (kv head, split).  The item's rows are processed in segments of up to kStSegTiles ring tiles that are resident at the same time.  A cache
+// One CTA = one (group of KVM query heads of a key/value head, split).  The item's rows are processed in segments of up to kStSegTiles ring tiles that are resident at the same time.  A cache
 // row belongs to LPR lanes of a warp, each with NC of its 16-byte chunks for all KVM query heads: a score is log2(LPR) shuffles, and the weighted value row stays
 // in the lanes that have the weight, so there is no barrier and no shared memory between scores, softmax and values.  Every row slot keeps a running maximum, sum and
 // accumulators of its own (KVM * NC = 4 or 8 float4).  LPR is the least that fits them: what bounds an item of this size is the instructions that its
@@ -595,8 +595,9 @@ static __device__ void st_attention(const StreamArgs &g, const StRing &r, StCurs
                                     uint32_t e_in, uint32_t e_out, float *sm) {
     constexpr uint32_t LPR = KVM * HDC / 32 < HDC / 16 ? HDC / 16 : KVM * HDC / 32, NC = HDC / 4 / LPR, RP = 32 / LPR;          // lanes of a row, chunks of a lane, rows of a warp's pass
     const Dims &d = g.d;
-    const uint32_t nsplit = plan.nsplit, kvh = plan.kvh, sp = plan.sp, t0 = plan.t0, t1 = plan.t1;
-    if (kvh >= d.KV) return;
+    const uint32_t nsplit = plan.nsplit, grp = plan.grp, sp = plan.sp, t0 = plan.t0, t1 = plan.t1;
+    if (grp >= g.groups) return;
+    const uint32_t kvh = grp / g.group_div;
     const uint32_t hd = d.hd;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t kvr = g.kv_tile_rows, seg_max = (uint32_t)kStSegTiles * kvr;
@@ -620,13 +621,13 @@ static __device__ void st_attention(const StreamArgs &g, const StRing &r, StCurs
             rt = rope_tab_load(g.rope_cos + (size_t)pos * (hd / 2), g.rope_sin + (size_t)pos * (hd / 2), d, col, colon);
             if (d.arch == 3u && colon) gn = __ldg(reinterpret_cast<const float4 *>(gains + (size_t)layer * hd + col));
         }
-        const uint32_t at = warp < KVM ? (kvh * KVM + warp) * hd : d.q_dim + (warp == KVM ? 0u : d.kv_dim) + kvh * hd;
+        const uint32_t at = warp < KVM ? (grp * KVM + warp) * hd : d.q_dim + (warp == KVM ? 0u : d.kv_dim) + kvh * hd;
         if (colon) v4 = xw_poll4(g.xq + at + col, e_in, g.err);
         __syncwarp();
         if (warp <= KVM) v4 = norm_rope_apply(v4, gn, rt, d, lpr, col, colon);
         if (colon && lane < lpr) {
             *reinterpret_cast<float4 *>(q_s + warp * hd + col) = v4;               // krow follows q_s: row KVM is k, row KVM + 1 is v
-            if (warp == KVM)                                                       // K rows are cached post-RoPE
+            if (warp == KVM && grp == kvh * g.group_div)                           // K rows are cached post-RoPE, once
                 *reinterpret_cast<float4 *>(g.kc + ((size_t)(layer * d.KV + kvh) * d.max_seq + pos) * hd + col) = v4;
         }
     }
@@ -754,10 +755,10 @@ static __device__ void st_attention(const StreamArgs &g, const StRing &r, StCurs
     }
     cbar();
     const uint32_t pw = KVM * (hd + 2u);                               // words of one partial
-    unsigned long long *part_x = g.xws + (size_t)kvh * g.nsplit_max * pw;
+    unsigned long long *part_x = g.xws + (size_t)grp * g.nsplit_max * pw;
     const uint32_t slabs = (hd + 31u) / 32u, units = KVM * slabs;
     auto publish = [&](uint32_t m, uint32_t i, float v) {
-        unsigned long long *dst = g.xv[1] + (kvh * KVM + m) * hd + i;
+        unsigned long long *dst = g.xv[1] + (grp * KVM + m) * hd + i;
         const uint32_t rs = g.rs[1];
 #pragma unroll
         for (uint32_t rep = 0; rep < (uint32_t)kStRep; rep++) xw_st(dst + rep * rs, v, e_out);
@@ -923,8 +924,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_decode_stream(const __grid_cons
             const uint32_t range = ms.st.is_causal ? pos + 1u : d.max_seq;
             uint32_t nsplit, chunk;
             st_attn_plan(range, g.nsplit_max, g.chunk_target, nsplit, chunk);
-            const uint32_t kvh = cta / nsplit, sp = cta - kvh * nsplit, t0 = min(range, sp * chunk);
-            ms.plan = StPlan{nsplit, kvh, sp, t0, min(range, t0 + chunk)};
+            const uint32_t grp = cta / nsplit, sp = cta - grp * nsplit, t0 = min(range, sp * chunk);
+            ms.plan = StPlan{nsplit, grp, sp, t0, min(range, t0 + chunk)};
         }
         // embedding row (infer.c:987-988) into shared memory; the rows this CTA owns in the residual phases start from it
         embed_row<kConsThreads>(g.emb_w, g.emb_aux, x_s, tok, d);

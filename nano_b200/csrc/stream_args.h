@@ -36,7 +36,7 @@ struct StreamArgs {
     float *logits, *kc, *vc;
     // activation exchange: 64-bit words {fp32 value, 32-bit epoch}.  xq: QKV outputs [q_dim + 2 kv_dim] (one copy: read per head);
     // xv[0] = x, xv[1] = attention output, xv[2] = SwiGLU output: kStRep replicas each, rs[i] words apart;
-    // xws: split-KV partials [KV][nsplit_max][KVM * (hd + 2)]
+    // xws: split-KV partials [groups][nsplit_max][KVM * (hd + 2)]
     unsigned long long *xq, *xv[3], *xws;
     uint32_t rs[3];
     uint32_t epoch_base;                              // epochs handed out before this launch (host-maintained, monotonic)
@@ -48,6 +48,7 @@ struct StreamArgs {
     float *logits_host; uint32_t *next_host;          // pinned host copies of the logits and of the chosen token, or null
     uint32_t *err;                                    // set to a nonzero code before a spin gives up (and traps)
     uint32_t n_steps, nsplit_max, chunk_target;
+    uint32_t groups, group_div;                       // groups of query heads (as many as the kernel instance's KVM), and how many of them share a key/value head
     unsigned long long *trace;                        // optional: CTA 0 / thread 0 clock64() after every barrier of the LAST step
     Dims d;
 };

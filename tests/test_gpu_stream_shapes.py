@@ -45,6 +45,29 @@ def test_f32_shapes(arch, H, KV, hd, E_, F, chunk, stage, monkeypatch):
     assert np.linalg.norm(a - b) <= 1e-5 * np.linalg.norm(b)
 
 
+# contexts at the edge of the rule for the query heads of an attention item (640 keys of 32 where every query head's item has all keys): the tokens on both sides of it against the oracle,
+# and a device loop over the edge gives the bits of one call per token
+@pytest.mark.parametrize("H,KV,hd,edge", [(80, 40, 32, 640), (80, 20, 32, 640)])
+def test_heads_of_an_item(H, KV, hd, edge, monkeypatch):
+    monkeypatch.setenv("NB200_STREAM", "1")
+    n = edge + 6
+    spec = mf.ModelSpec("heads-%d-%d-%d" % (H, KV, hd), mf.ARCH_QWEN3, 1024, 97, 1, 64, H, KV, 64, hd)
+    path = mf.cached_model(spec, mf.QUANT_F32, 128)
+    eng, o = E.Engine(path, n + 2), ob.NanoOracle(path, n + 2)
+    assert eng.path.startswith("streaming"), eng.path
+    ids = np.zeros(n + 2, np.uint32)
+    ids[:4] = 5, 7, 9, 11
+    eng.decode_greedy(ids, 4, n + 1)
+    loop = eng.logits()
+    for pos in range(n):
+        a, b = eng.forward(int(ids[pos]), pos), o.forward(int(ids[pos]), pos)
+        if pos >= edge - 4:
+            assert np.linalg.norm(a - b) <= 1e-5 * np.linalg.norm(b), pos          # as above
+    assert np.array_equal(a, loop)
+    eng.close()
+    o.close()
+
+
 # widths of one quantisation group, of an odd number of them, of more than one 1024-byte step of a warp, and of more than one turn of the prologue's warps
 @pytest.mark.parametrize("E_,F,gs", [(64, 64, 64), (192, 320, 64), (640, 1152, 128), (128, 4224, 128), (3968, 128, 128)])
 def test_q80_rows(E_, F, gs, monkeypatch):
