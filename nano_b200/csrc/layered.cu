@@ -1832,7 +1832,10 @@ int run_layers(LayeredEngine *e, uint32_t slot, uint32_t T, uint32_t pos0, const
             else if (norm_one) {
                 const auto k = E <= 1024u ? k_norm_shift_one<4> : E <= 2048u ? k_norm_shift_one<8> : k_norm_shift_one<16>;
                 if ((r = launch<NormShiftArgs>(e, k, dim3(1), dim3(kOneThreads), 0, a))) return r;
-            } else if ((r = launch<NormShiftArgs>(e, k_norm_shift, dim3(T > 1 ? T - 1 : 1), dim3(256), 0, a))) return r;
+            } else {
+                const auto k = E <= 1024u ? k_norm_shift<4> : E <= 2048u ? k_norm_shift<8> : k_norm_shift<0>;
+                if ((r = launch<NormShiftArgs>(e, k, dim3(T > 1 ? T - 1 : 1), dim3(256), 0, a))) return r;
+            }
             if (L.has_mlp && e->branch_streams) CK(cudaEventRecord(e->ev_fork, e->stream));
         }
         // A lone token's feed-forward (routing, then two products of the experts it chose) is a longer chain than a recurrent mixer of few bytes: it follows the norm on the norm's own
