@@ -1035,6 +1035,14 @@ constexpr size_t kSideMixBytes = 8u << 20;      // a recurrent mixer's weights u
 constexpr uint64_t kTcAttnWork = 128 * 128;      // tokens x keys, or keys, from which a portion's grouped-query attention goes to the tensor cores
 constexpr uint32_t kTcAttnKeys = 512, kTcLatentKeys = 128;      // ... and keys from which latents are multiplied out
 
+int conv_launch(LayeredEngine *e, const ConvArgs &ca) {
+    int r;
+    if (ca.K == 4u && ca.T >= 3u) return launch<ConvArgs>(e, k_conv_four, dim3((ca.C + 127u) / 128u, (ca.T + kConvTokens - 1u) / kConvTokens), dim3(128), 0, ca);
+    if ((r = launch<ConvArgs>(e, k_conv, dim3(ew_grid((size_t)ca.T * ca.C)), dim3(256), 0, ca))) return r;
+    if (ca.K > 1 && (r = launch<ConvArgs>(e, k_conv_state, dim3((ca.C + 127) / 128), dim3(128), 0, ca))) return r;
+    return 0;
+}
+
 int mix_rglru(LayeredEngine *e, const Layer &L, const Run &run, const Ctx &cx) {
     const uint32_t E = e->E, T = cx.T; float *st = cx.st; int r;
     const uint32_t C = L.C, bs = C / L.blocks;
@@ -1052,15 +1060,15 @@ int mix_rglru(LayeredEngine *e, const Layer &L, const Run &run, const Ctx &cx) {
     } else {
         if ((r = gemm(e, plain(e->hm, E, L.yx, e->b_yx, 2 * C, T, L.yx_b, EPI_GELU_SPLIT, C), 1, T))) return r;
         ConvArgs ca{e->b_yx + C, 2 * C, L.conv, L.conv_b, st + run.st_conv, e->b_u, T, C, L.taps};
-        if ((r = launch<ConvArgs>(e, k_conv, dim3(ew_grid((size_t)T * C)), dim3(256), 0, ca))) return r;
-        if (L.taps > 1 && (r = launch<ConvArgs>(e, k_conv_state, dim3((C + 127) / 128), dim3(128), 0, ca))) return r;
+        if ((r = conv_launch(e, ca))) return r;
         GemmArgs g{};
         g.A = e->b_u; g.lda = C; g.W = L.gates.p; g.ldw = bs; g.C = e->b_g; g.ldc = 2 * C; g.bias = L.gates_b; g.M = T; g.N = bs; g.K = bs;
         g.a_gmod = L.blocks; g.a_gcols = bs; g.c_gcols = bs; g.b_gstride = bs; g.w_gstride = (uint64_t)bs * bs; g.epi = EPI_SIGMOID;
         if ((r = gemm(e, g, 2 * L.blocks, T))) return r;
         ScanArgs sa{e->b_g, 2 * C, e->b_u, e->b_yx, 2 * C, L.lam, st + run.st_S, e->b_sy, T, C, kRglruDecay};
-        if (T <= 32) { if ((r = launch<ScanArgs>(e, k_rglru_scan, dim3((C + 63) / 64), dim3(64), 0, sa))) return r; }
-        else if ((r = launch<ScanArgs>(e, k_rglru_scan_par, dim3((C + 31) / 32), dim3(32, T >= 256 ? 32 : 8), 0, sa))) return r;
+        const dim3 grid((C + 31u) / 32u);
+        const auto scan = T <= 32u ? k_rglru_scan<1> : T <= 64u ? k_rglru_scan<2> : T <= 128u ? k_rglru_scan<4> : T <= 256u ? k_rglru_scan<8> : k_rglru_scan_par;
+        if ((r = launch<ScanArgs>(e, scan, grid, dim3(32, T <= 32u ? T : 32u), 0, sa))) return r;
     }
     if ((r = gemm(e, plain(e->b_sy, C, L.o, e->d, E, T), 1, T))) return r;
     return 0;
@@ -1239,13 +1247,6 @@ int sel_scan_launch(LayeredEngine *e, const SelScanArgs &a) {
         return launch<SelScanArgs>(e, k_selective_scan_par<LG, false>, grid, block, 0, a);
     }
     return launch<SelScanArgs>(e, k_selective_scan<LG>, dim3(((size_t)a.C * LG + 255u) / 256u), dim3(256), 0, a);
-}
-
-int conv_launch(LayeredEngine *e, const ConvArgs &ca) {
-    int r;
-    if ((r = launch<ConvArgs>(e, k_conv, dim3(ew_grid((size_t)ca.T * ca.C)), dim3(256), 0, ca))) return r;
-    if (ca.K > 1 && (r = launch<ConvArgs>(e, k_conv_state, dim3((ca.C + 127) / 128), dim3(128), 0, ca))) return r;
-    return 0;
 }
 
 // window attention and selective scan on the same input: one product gives [q | k | x | g | z]; q, k pass their convolution (tail in

@@ -11,10 +11,10 @@
 //                        input against the previous token's input, carried in the sequence state), k_latent_norm (vector-gain RMS norm
 //                        of the query latent and of the key/value latent, the latter written into the paged cache; for short portions
 //                        k_gemv_latent does both inside the query up-projection), k_final_norm
-//   recurrence           k_conv / k_conv_state (causal per-channel convolution with its taps-1 tail in the state; for short portions it is
-//                        an epilogue of k_gemv), k_rglru_scan (real-gated linear recurrent unit: a = exp(-c r softplus(lam)),
-//                        S = a S + sqrt(1 - a^2) i u, fp32 state; token by token), k_rglru_scan_par (the same, parallel over time
-//                        segments, for long portions) and k_rglru_gates_scan (both gate products + the recurrence, short portions)
+//   recurrence           k_conv_four, k_conv / k_conv_state (causal per-channel convolution with its taps-1 tail in the state; for short
+//                        portions it is an epilogue of k_gemv), k_rglru_scan (real-gated linear recurrent unit: a = exp(-c r softplus(lam)),
+//                        S = a S + sqrt(1 - a^2) i u, fp32 state; 32 segments of up to 8 tokens in registers), k_rglru_scan_par (the same for
+//                        long portions, two walks) and k_rglru_gates_scan (both gate products + the recurrence, short portions)
 //   attention            k_latent_attn (softmax attention of absorbed queries directly over cached latents: the latent is key AND
 //                        value, positions-free, causal; split over the keys for decode, merged by the block that finishes last)
 //   mixture of experts   k_route (fp32 router logits -> top-k, softmax over the chosen), k_route_place (expert-sorted slots), k_route_small
@@ -688,6 +688,33 @@ __global__ void k_conv(const ConvArgs a) {
         a.u[(size_t)t * (a.ldu ? a.ldu : a.C) + c] = s;
     }
 }
+// the same with four taps for three or more tokens, and the tail in the same launch: a thread takes a channel through eight tokens, whose rows and the three before are asked for at once;
+// the first tokens' block, the only reader of the tail, writes it after.  Same products in the same order
+constexpr uint32_t kConvTokens = 8;
+__global__ void __launch_bounds__(128) k_conv_four(const ConvArgs a) {
+    pdl_launch_next();
+    const uint32_t c = blockIdx.x * 128u + threadIdx.x, t0 = blockIdx.y * kConvTokens;
+    if (c >= a.C) return;
+    const float *tp = a.taps + (size_t)c * 4u;
+    const float tap0 = __ldg(tp), tap1 = __ldg(tp + 1), tap2 = __ldg(tp + 2), tap3 = __ldg(tp + 3), bias = a.bias ? __ldg(a.bias + c) : 0.0f;
+    pdl_wait();
+    const float *v = a.v + c, *last = v + (size_t)(a.T - 3u) * a.ldv;
+    const uint32_t ldu = a.ldu ? a.ldu : a.C;
+    float w[kConvTokens + 3], e0, e1, e2;
+#pragma unroll
+    for (uint32_t i = 0; i < 3u; i++) w[i] = t0 ? v[(size_t)(t0 + i - 3u) * a.ldv] : a.state[(size_t)i * a.C + c];
+#pragma unroll
+    for (uint32_t i = 0; i < kConvTokens; i++) w[i + 3u] = t0 + i < a.T ? v[(size_t)(t0 + i) * a.ldv] : 0.0f;
+    if (t0 == 0) { e0 = last[0]; e1 = last[a.ldv]; e2 = last[2u * (size_t)a.ldv]; }
+#pragma unroll
+    for (uint32_t i = 0; i < kConvTokens; i++) {
+        if (t0 + i >= a.T) break;
+        float s = fmaf(tap3, w[i + 3u], fmaf(tap2, w[i + 2u], fmaf(tap1, w[i + 1u], fmaf(tap0, w[i], bias))));
+        if (a.act) s = s / (1.0f + expf(-s));
+        a.u[(size_t)(t0 + i) * ldu + c] = s;
+    }
+    if (t0 == 0) { a.state[c] = e0; a.state[a.C + c] = e1; a.state[2u * (size_t)a.C + c] = e2; }
+}
 // after k_conv: the tail becomes the last K-1 inputs, this portion included
 __global__ void k_conv_state(const ConvArgs a) {
     pdl_enter();
@@ -699,23 +726,57 @@ __global__ void k_conv_state(const ConvArgs a) {
     }
 }
 
-// real-gated linear recurrent unit, one thread per channel, tokens in order:
+// real-gated linear recurrent unit:
 //   a = exp(-c_decay * r * softplus(lam)),  S <- a S + sqrt(1 - a^2) * (i * u),  out = S * y
+// Portions of up to 32 NT tokens: NT tokens of a channel to a thread, 32 of them along the portion.  The tokens' inputs are asked for at once and their decays and increments stay in
+// registers; a thread composes its tokens' map S -> P S + Q, the first of the 32 chains the maps, each writes its outputs.  With one token to a thread the chain is the recurrence itself.
+// (Bound by the latency of its loads: width 1024, 24 tokens 6.8 us token by token, 2.0 now; eight layers with the convolution below, whole portions of 24 tokens 550 -> 483 us, 200, which
+// had eight segments with two walks each, 859 -> 730.  32 segments round less often than a chain over all tokens does: 0.8 of its error against 64 bits at 200 tokens.)
 struct ScanArgs { const float *gates; uint32_t ldg; const float *u; const float *y; uint32_t ldy; const float *lam; float *S; float *out; uint32_t T, C; float c_decay; };
-__global__ void k_rglru_scan(const ScanArgs a) {
-    pdl_enter();
-    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= a.C) return;
-    const float sp = softplusf_(a.lam[c]);
-    float S = a.S[c];
-    for (uint32_t t = 0; t < a.T; t++) {
-        const float r = a.gates[(size_t)t * a.ldg + c], i = a.gates[(size_t)t * a.ldg + a.C + c];
-        const float la = -a.c_decay * r * sp;
-        const float av = expf(la);
-        S = av * S + sqrtf(1.0f - av * av) * (i * a.u[(size_t)t * a.C + c]);
-        a.out[(size_t)t * a.C + c] = S * a.y[(size_t)t * a.ldy + c];
+template <int NT>
+__global__ void __launch_bounds__(1024) k_rglru_scan(const ScanArgs a) {
+    pdl_launch_next();
+    __shared__ float P[32][33], Q[32][33];
+    const uint32_t x = threadIdx.x, seg = threadIdx.y, nseg = blockDim.y, c = blockIdx.x * 32u + x, t0 = seg * NT;
+    const bool live = c < a.C;
+    const float sp = live ? softplusf_(__ldg(a.lam + c)) : 0.0f;
+    pdl_wait();
+    float av[NT], bv[NT], y[NT], s0 = 0.0f;
+    if (live && seg == 0) s0 = a.S[c];
+#pragma unroll
+    for (uint32_t k = 0; k < NT; k++) {
+        const uint32_t t = t0 + k;
+        const bool on = live && t < a.T;
+        av[k] = on ? a.gates[(size_t)t * a.ldg + c] : 0.0f;
+        bv[k] = on ? a.gates[(size_t)t * a.ldg + a.C + c] * a.u[(size_t)t * a.C + c] : 0.0f;
+        y[k] = on ? a.y[(size_t)t * a.ldy + c] : 0.0f;
     }
-    a.S[c] = S;
+    float p = 1.0f, q = 0.0f;
+#pragma unroll
+    for (uint32_t k = 0; k < NT; k++) {
+        if (t0 + k >= a.T) break;
+        av[k] = expf(-a.c_decay * av[k] * sp);
+        bv[k] = sqrtf(1.0f - av[k] * av[k]) * bv[k];
+        q = av[k] * q + bv[k];
+        p *= av[k];
+    }
+    P[seg][x] = p; Q[seg][x] = q;
+    __syncthreads();
+    if (seg == 0 && live) {
+        float s = s0;
+#pragma unroll 8
+        for (uint32_t g = 0; g < nseg; g++) { const float pg = P[g][x], qg = Q[g][x]; P[g][x] = s; s = pg * s + qg; }
+        a.S[c] = s;
+    }
+    __syncthreads();
+    if (!live) return;
+    float S = P[seg][x];
+#pragma unroll
+    for (uint32_t k = 0; k < NT; k++) {
+        if (t0 + k >= a.T) break;
+        S = av[k] * S + bv[k];
+        a.out[(size_t)(t0 + k) * a.C + c] = S * y[k];
+    }
 }
 
 // The same recurrence for long portions, parallel over time: the portion is cut into blockDim.y segments.  A thread (channel,

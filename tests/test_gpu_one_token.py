@@ -180,3 +180,22 @@ def test_one_token_rows(tmp_path, width, top):
     toks = np.random.default_rng(1).integers(0, 61, size=5).astype(np.uint32)
     assert off(one_by_one(eng, toks), A.forward(cfg, w, toks)) < BOUND[True]
     eng.close()
+
+
+# portions at the edges of the recurrence's 1, 2, 4 and 8 tokens a thread and of its long walk, of the eight tokens that a thread convolves (four taps or another number of them), of the
+# keys from which latents are multiplied out and of the tokens up to which the router's last block places the rows
+@pytest.mark.parametrize("conv,f32", [(4, True), (3, True), (4, False)])
+def test_portion_edges(tmp_path, conv, f32):
+    mlp = {"experts": 3, "top": 3, "ff": 24, "shared_ff": 32}
+    layers = [("rglru", {"width": 72, "blocks": 3, "conv": conv}, mlp), ("latent_attention", {"heads": 2, "dim": 64, "vdim": 64, "kv_rank": 32, "q_rank": 24, "scale": 0.125}, mlp)]
+    cfg = md.famudra_config(97, 64, layers)
+    w = md.famudra_random(cfg, 6)
+    eng = E.Engine(md.write_model_dir(str(tmp_path / "m"), cfg, w), 512, flags=E.FLAG_F32 if f32 else 0)
+    toks = np.random.default_rng(5).integers(0, 97, size=264).astype(np.uint32)
+    ref = A.forward(cfg, w, toks)
+    for n in (5, 8, 9, 31, 32, 33, 64, 65, 128, 129, 256, 257):
+        s = eng.seq_open()
+        got = np.concatenate([eng.step(s, toks[:n], range(n)), eng.step(s, toks[n:n + 6], range(6))])          # and the state behind it
+        eng.seq_close(s)
+        assert off(got, ref[:n + 6]) < 5 * BOUND[f32], n
+    eng.close()
