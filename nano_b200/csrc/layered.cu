@@ -1616,6 +1616,13 @@ int route_small(LayeredEngine *e, const RouteArgs &ra) {
     return launch<RouteArgs>(e, k_route_small, dim3(nb), dim3(kRouteThreads), route_small_smem(NL), ra, nb);
 }
 
+int route_many(LayeredEngine *e, const RouteArgs &ra) {
+    const size_t smem = route_smem(ra.NE + ra.extra, 256);
+    if (ra.T <= kRoutePlaceMax) return launch<RouteArgs>(e, k_route<true>, dim3(ra.T), dim3(256), smem, ra);
+    const int r = launch<RouteArgs>(e, k_route<false>, dim3(ra.T), dim3(256), smem, ra);
+    return r ? r : launch<RouteArgs>(e, k_route_place, dim3(1), dim3(1024), (size_t)ra.NE * 4u, ra);
+}
+
 // experts chosen by sigmoid scores: e->h2 -> the rows of e->b_eo (one per token and choice, in expert order) and, with a shared expert,
 // e->b_so and the gate logits e->b_sg; the residual kernel adds them up.  The score weights the expert's INPUT; the experts have no
 // bias, so act(s g) (s u) of the unweighted products g, u is the same number.  The shared expert runs on a second stream.
@@ -1627,7 +1634,7 @@ int ff_moe_scored(LayeredEngine *e, const Layer &L, uint32_t T) {
     float *wrow = L.score_in ? e->b_wrow : nullptr;
     RouteArgs ra{e->h2, L.router, e->b_idx, e->b_wt, e->b_cnt, e->b_off, e->b_fill, e->b_slot, e->b_rows, T, L.NE, L.top, E, L.route_mode, L.sh_gate ? 1u : 0u, e->b_sg, wrow};
     if (small) { ra.act = e->b_act; if ((r = route_small(e, ra))) return r; }
-    else if ((r = launch<RouteArgs>(e, k_route, dim3(T), dim3(256), route_smem(NL, 256), ra)) || (r = launch<RouteArgs>(e, k_route_place, dim3(1), dim3(1024), 0, ra))) return r;
+    else if ((r = route_many(e, ra))) return r;
     GemmArgs u{};
     u.A = e->h2; u.lda = E; u.W = L.up.p; u.ldw = E; u.M = T; u.K = E; u.a_gmod = 1;
     u.g_off = e->b_off; u.a_rows = e->b_rows; u.g_act = small ? e->b_act : nullptr; u.w_gstride = (uint64_t)2 * L.ff * E;
@@ -1721,8 +1728,7 @@ int ff_moe_relu2(LayeredEngine *e, const Layer &L, uint32_t T) {
     ra.groups = L.groups; ra.keep = L.keep_groups; ra.wscale = L.route_scale;
     const bool small = T <= kGemvMaxM;
     if (small) { ra.act = e->b_act; if ((r = route_small(e, ra))) return r; }
-    else if ((r = launch<RouteArgs>(e, k_route, dim3(T), dim3(256), route_smem(L.NE, 256), ra)) ||
-             (r = launch<RouteArgs>(e, k_route_place, dim3(1), dim3(1024), 0, ra))) return r;
+    else if ((r = route_many(e, ra))) return r;
     GemmArgs u{};
     u.A = e->h2; u.lda = E; u.W = L.up.p; u.ldw = E; u.C = e->b_hb; u.ldc = L.ff; u.M = T; u.N = L.ff; u.K = E; u.a_gmod = 1;
     u.g_off = e->b_off; u.a_rows = e->b_rows; u.g_act = small ? e->b_act : nullptr; u.w_gstride = (uint64_t)L.ff * E; u.epi = EPI_RELU2;
@@ -2817,7 +2823,7 @@ int create(LayeredEngine *e, const nb::ModelDir *dir, uint32_t max_tokens) {
     if (mNE) {
         DM(e->b_idx, T * mTop * 4); DM(e->b_wt, T * mTop * 4); DM(e->b_slot, T * mTop * 4); DM(e->b_rows, T * mTop * 4);
         DM(e->b_cnt, (size_t)mNE * 4); DM(e->b_off, ((size_t)mNE + 1) * 4); DM(e->b_fill, (size_t)mNE * 4); DM(e->b_act, (size_t)kGemvMaxM * mTop * 4);
-        CK(cudaMemset(e->b_cnt, 0, (size_t)mNE * 4));
+        CK(cudaMemset(e->b_cnt, 0, (size_t)mNE * 4)); CK(cudaMemset(e->b_fill, 0, (size_t)mNE * 4));
         DM(e->b_hb, T * mFF * 4); DM(e->b_eo, T * mTop * E * 4);
         if (mSFF) { DM(e->b_sh, T * std::max(mSFF, mSFF2) * 4); DM(e->b_so, T * E * 4); }
         if (mFF2) { DM(e->b_hg, T * mFF2 * 4); DM(e->b_wrow, T * mTop * 4); DM(e->b_sg, T * 4); }

@@ -1252,15 +1252,72 @@ __device__ __forceinline__ void route_pick(const RouteArgs &a, uint32_t t, float
     for (uint32_t j = 0; j < a.top; j++) { wt[j] = expf(wt[j] - mx); s += wt[j]; }
     for (uint32_t j = 0; j < a.top; j++) wt[j] /= s;
 }
+// Expert-sorted places, by one block: off[e] = rows before expert e (off[NE] = total), counters cleared for the next use; then slot[t][j] = the row of (token t, choice j) in that
+// order and rows[slot] = t.  cur: NE words of shared memory
+__device__ __forceinline__ void route_place(const RouteArgs &a, uint32_t *cur) {
+    if (threadIdx.x < 32u) {
+        const uint32_t lane = threadIdx.x;
+        uint32_t s = 0;
+        for (uint32_t e0 = 0; e0 < a.NE; e0 += 32u) {
+            const uint32_t e = e0 + lane, c = e < a.NE ? __ldcg(a.counts + e) : 0u;
+            uint32_t run = c;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) { const uint32_t v = __shfl_up_sync(0xffffffffu, run, o); if (lane >= (uint32_t)o) run += v; }
+            if (e < a.NE) { a.off[e] = cur[e] = s + run - c; a.counts[e] = 0; }
+            s += __shfl_sync(0xffffffffu, run, 31);
+        }
+        if (lane == 0) a.off[a.NE] = s;
+    }
+    __syncthreads();
+    for (uint32_t i0 = threadIdx.x; i0 < a.T * a.top; i0 += 8u * blockDim.x) {          // eight choices at a time
+        uint32_t e[8]; float w[8];
+#pragma unroll
+        for (uint32_t q = 0; q < 8u; q++) {
+            const uint32_t i = i0 + q * blockDim.x;
+            e[q] = i < a.T * a.top ? __ldcg(a.idx + i) : 0u;
+            w[q] = a.wrow && i < a.T * a.top ? __ldcg(a.wt + i) : 0.0f;
+        }
+#pragma unroll
+        for (uint32_t q = 0; q < 8u; q++) {
+            const uint32_t i = i0 + q * blockDim.x;
+            if (i >= a.T * a.top) break;
+            const uint32_t s = atomicAdd(cur + e[q], 1u);
+            a.slot[i] = s; a.rows[s] = i / a.top;
+            if (a.wrow) a.wrow[s] = w[q];
+        }
+    }
+}
+// A token a block.  PLACE: the block that draws the last ticket places the rows, which is a launch less; its 256 threads are the slower ones beyond a few hundred tokens
+// (width 2048, 4 of 16 experts, whole portions: 100 tokens 298 -> 293 us, 512 383 -> 378, 1024 533 -> 536, 1777 1017 -> 1027; 11 tokens of width 1024, eight layers 458 -> 447, but 300 807 -> 818)
+constexpr uint32_t kRoutePlaceMax = 256;
+template <bool PLACE>
 __global__ void __launch_bounds__(256) k_route(const RouteArgs a) {
     pdl_enter();
     extern __shared__ float z[];
+    __shared__ uint32_t last_s;
     route_logits(a, blockIdx.x, z, z + a.NE + a.extra);
     __syncthreads();
-    if (threadIdx.x >= 32u) return;
-    route_pick(a, blockIdx.x, z, z + a.NE + a.extra);
-    if (threadIdx.x) return;
-    for (uint32_t j = 0; j < a.top; j++) atomicAdd(a.counts + a.idx[(size_t)blockIdx.x * a.top + j], 1u);
+    if (threadIdx.x < 32u) {
+        route_pick(a, blockIdx.x, z, z + a.NE + a.extra);
+        if (threadIdx.x == 0) {
+            for (uint32_t j = 0; j < a.top; j++) atomicAdd(a.counts + a.idx[(size_t)blockIdx.x * a.top + j], 1u);
+        }
+    }
+    if constexpr (PLACE) {
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            __threadfence();
+            last_s = atomicAdd(a.fill, 1u) + 1u == gridDim.x;
+            if (last_s) { *a.fill = 0u; __threadfence(); }
+        }
+        __syncthreads();
+        if (last_s) route_place(a, reinterpret_cast<uint32_t *>(z));
+    }
+}
+__global__ void __launch_bounds__(1024) k_route_place(const RouteArgs a) {
+    pdl_enter();
+    extern __shared__ uint32_t cur[];
+    route_place(a, cur);
 }
 // Short portions: routing and placement of all T <= kGemvMaxM tokens in one launch.  A cluster of blocks shares the router's rows (a warp
 // sums a slice of a row for all tokens at once) and hands the logits to its first block, where a warp per token chooses.  Same outputs as
@@ -1347,32 +1404,6 @@ __global__ void __launch_bounds__(kRouteThreads) k_route_small(const RouteArgs a
     a.off[a.NE] = s;
     for (uint32_t i = 0; i < n; i++) { const uint32_t sl = cur[a.idx[i]]++; a.slot[i] = sl; a.rows[sl] = i / a.top; if (a.wrow) a.wrow[sl] = a.wt[i]; }
 }
-// One block: off[e] = rows before expert e (off[NE] = total), counters cleared for the next use; then slot[t][j] = the row of
-// (token t, choice j) in the expert-sorted order and rows[slot] = t
-__global__ void __launch_bounds__(1024) k_route_place(const RouteArgs a) {
-    pdl_enter();
-    if (threadIdx.x < 32u) {
-        const uint32_t lane = threadIdx.x;
-        uint32_t s = 0;
-        for (uint32_t e0 = 0; e0 < a.NE; e0 += 32u) {
-            const uint32_t e = e0 + lane, c = e < a.NE ? a.counts[e] : 0u;
-            uint32_t run = c;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) { const uint32_t v = __shfl_up_sync(0xffffffffu, run, o); if (lane >= (uint32_t)o) run += v; }
-            if (e < a.NE) { a.off[e] = s + run - c; a.counts[e] = 0; a.fill[e] = 0; }
-            s += __shfl_sync(0xffffffffu, run, 31);
-        }
-        if (lane == 0) a.off[a.NE] = s;
-    }
-    __syncthreads();
-    for (uint32_t i = threadIdx.x; i < a.T * a.top; i += blockDim.x) {
-        const uint32_t e = a.idx[i];
-        const uint32_t s = a.off[e] + atomicAdd(a.fill + e, 1u);
-        a.slot[i] = s; a.rows[s] = i / a.top;
-        if (a.wrow) a.wrow[s] = a.wt[i];
-    }
-}
-
 // x[t] += d[t] + ( sum_j wt[t][j] * eo[slot[t][j]]  (+ shared[t]) ),  the sum in the order of the choices; keep (optional) gets x
 struct CombineArgs { float *x; const float *d; const float *eo; const uint32_t *slot; const float *wt; const float *shared; float *keep; uint32_t T, E, top; };
 __global__ void k_combine(const CombineArgs a) {
