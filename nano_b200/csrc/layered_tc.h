@@ -23,12 +23,14 @@ void tc_free(TcState *t);
 int tc_check(TcState *t);
 // whether the product's layout allows it.  rows: all rows of A it reads (a routed product: tokens x choices)
 bool tc_fits(const TcState *t, const GemmArgs &a, uint32_t rows);
-// Does the product read its fp32 rows itself (one launch), or a rounded copy that a launch of its own makes before it.  each: as below.  Groups of at most 64 rows on average, whose tiles are
-// 32 or 64 tokens, and only while the tiles read less than 32 MB of them: every tile of weights reads the rows again.  Two layers, us a portion, copy / rows: Famudra width 1024 (eight layers) 5 tokens
-// 616 / 470, 11 535 / 490, 40 718 / 677, 64 783 / 708; Fidatar width 1024 5 162 / 147, 64 184 / 180; Kadesun width 2048 5 220 / 207, 40 257 / 245, but 64 (50 MB for 12288 columns) 254 / 260 and
-// Fidatar width 2048 64 (33 MB) 258 / 264.
+// Does the product read its fp32 rows itself (one launch), or a rounded copy that a launch of its own makes before it.  each: as below.  Groups of at most 384 rows on average, in tiles of 32
+// or 64 tokens (copies in up to 128), and only while the tiles read less than 32 MB of them, 16 beyond one tile: every tile of weights reads the rows again.  Whole portions, us, copy / rows:
+// Famudra width 1024 (eight layers) 5 tokens 616 / 470, 40 718 / 677, 64 783 / 708, 100 642 / 604, 200 734 / 649, 400 870 / 770; width 2048 (two) 100 252 / 220, 400 314 / 316, but 512
+// 325 / 332; Fidatar width 1024 5 162 / 147, 65 208 / 187, 256 239 / 230; Kadesun width 2048 40 257 / 245, 100 316 / 307, 400 485 / 476, 300 381 / 388, and without the line at 32 MB 64 (50 MB
+// for 12288 columns) 254 / 260; Fidatar width 2048 without the one at 16 MB 256 333 / 339.
 inline bool tc_raw_rows(const GemmArgs &a, uint32_t groups, uint32_t each) {
-    return each <= 64u && a.lda % 4u == 0 && (reinterpret_cast<uintptr_t>(a.A) & 15u) == 0 && (uint64_t)((a.N + 127u) / 128u) * groups * each * a.K * 4u <= kTcRawBytes;
+    return each <= 384u && a.lda % 4u == 0 && (reinterpret_cast<uintptr_t>(a.A) & 15u) == 0 &&
+           (uint64_t)((a.N + 127u) / 128u) * groups * each * a.K * 4u <= (each <= 64u ? kTcRawBytes : kTcRawBytes / 2u);
 }
 // one or two launches on `stream` (with programmatic serialization when pdl).  buf: which of the row buffers is the stream's; maxM: the most rows of a group, each:
 // how many a group has on average
