@@ -1427,24 +1427,17 @@ int delta_branch(LayeredEngine *e, const Layer &L, const Run &run, const Ctx &cx
     const uint32_t chunks = (T + kDeltaChunk - 1u) / kDeltaChunk;
     DeltaPrepArgs pa{e->b_p, P, L.c_conv, L.c_b, L.c_a, L.d_conv, cx.st + run.st_conv, L.d_taps, L.ra ? e->b_gsp : nullptr, L.d_bias, L.d_rate,
                      e->b_gblk, e->b_gv, T, H, G, D, VD, qscale};
-    {
-        const dim3 grid(chunks, H), block(kDeltaPrepThreads);
-        const size_t smem = delta_prep_smem(delta_dp(D));
-        if (D <= 32) r = launch<DeltaPrepArgs>(e, k_delta_prep<32>, grid, block, smem, pa);
-        else if (D <= 64) r = launch<DeltaPrepArgs>(e, k_delta_prep<64>, grid, block, smem, pa);
-        else if (D <= 128) r = launch<DeltaPrepArgs>(e, k_delta_prep<128>, grid, block, smem, pa);
-        else r = launch<DeltaPrepArgs>(e, k_delta_prep<256>, grid, block, smem, pa);
-        if (r) return r;
-    }
+    if ((r = launch<DeltaPrepArgs>(e, k_delta_prep, dim3(chunks, H), dim3(delta_dp(D)), 0, pa))) return r;
     if (L.d_taps > 1) {
         ConvArgs ca{e->b_p + L.c_conv, P, L.d_conv, nullptr, cx.st + run.st_conv, nullptr, T, C, L.d_taps, 0, 1};
         if ((r = launch<ConvArgs>(e, k_conv_state, dim3((C + 127u) / 128u), dim3(128), 0, ca))) return r;
     }
     DeltaScanArgs sa{e->b_gblk, e->b_gv, cx.st + run.st_S, e->b_go, T, H, D, VD};
-    const dim3 grid((VD + kDeltaCols - 1u) / kDeltaCols, H), block(256);
-#define DELTA_SCAN(DP) (e->f32 ? launch<DeltaScanArgs>(e, k_delta_scan<DP, DeltaStateFma>, grid, block, delta_scan_smem<DP>(), sa) : launch<DeltaScanArgs>(e, k_delta_scan<DP, DeltaStateMma>, grid, block, delta_scan_smem<DP>(), sa))
-    r = D <= 32 ? DELTA_SCAN(32) : D <= 64 ? DELTA_SCAN(64) : D <= 128 ? DELTA_SCAN(128) : DELTA_SCAN(256);
-#undef DELTA_SCAN
+    const dim3 grid((VD + 15u) / 16u, H), block(256);
+    if (D <= 32) r = launch<DeltaScanArgs>(e, k_delta_scan<1>, grid, block, 0, sa);
+    else if (D <= 64) r = launch<DeltaScanArgs>(e, k_delta_scan<2>, grid, block, 0, sa);
+    else if (D <= 128) r = launch<DeltaScanArgs>(e, k_delta_scan<4>, grid, block, 0, sa);
+    else r = launch<DeltaScanArgs>(e, k_delta_scan<8>, grid, block, 0, sa);
     if (r) return r;
     RetOutArgs oa{e->b_go, L.rg ? e->b_gt : e->b_p + L.c_g, L.rg ? H * VD : P, e->b_ga, T, H, VD, e->eps, L.d_gain, L.rg ? 1u : 0u};
     if ((r = launch<RetOutArgs>(e, k_retention_out, dim3((T * H + 7u) / 8u), dim3(256), 0, oa))) return r;
@@ -2736,10 +2729,6 @@ int create(LayeredEngine *e, const nb::ModelDir *dir, uint32_t max_tokens) {
     if (dC) {
         DM(e->b_gcv, (size_t)kGemvMaxM * dC * 4); DM(e->b_gv, T * dV * 4);
         DM(e->b_gblk, (T + kDeltaChunk - 1) / kDeltaChunk * dBlk * 4); DM(e->b_go, T * dV * 4); DM(e->b_ga, T * dV * 4);
-        CK(nb::smem_at_least((const void *)k_delta_prep<256>, (int)delta_prep_smem(256)));
-#define DELTA_SMEM(DP) CK(nb::smem_at_least((const void *)k_delta_scan<DP, DeltaStateFma>, (int)delta_scan_smem<DP>())); CK(nb::smem_at_least((const void *)k_delta_scan<DP, DeltaStateMma>, (int)delta_scan_smem<DP>()))
-        DELTA_SMEM(32); DELTA_SMEM(64); DELTA_SMEM(128); DELTA_SMEM(256);
-#undef DELTA_SMEM
         if (dSp) DM(e->b_gsp, T * dSp * 4);
         if (dGt) DM(e->b_gt, T * dGt * 4);
     }

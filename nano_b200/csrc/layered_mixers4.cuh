@@ -180,10 +180,6 @@ constexpr uint32_t kGqaM = 64, kGqaN = 64;
 __host__ __device__ inline uint32_t gqa_ld(uint32_t D) { const uint32_t Dp = (D + 3u) & ~3u; return ((Dp >> 2) & 1u) ? Dp : Dp + 4u; }      // rows of an odd number of 16-byte units
 __host__ __device__ inline uint32_t gqa_kwords(uint32_t D) { const uint32_t k = kGqaN * gqa_ld(D), p = kGqaM * (kGqaN + 4u); return k > p ? k : p; }
 inline size_t gqa_attn_smem(uint32_t D, int vj) { return ((size_t)kGqaM * gqa_ld(D) + gqa_kwords(D) + (size_t)kGqaN * vj * 64u) * 4; }
-__device__ __forceinline__ void cp_async4(float *dst, const float *src, bool ok) {      // 4 bytes into shared memory; zero when !ok
-    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst), n = ok ? 4u : 0u;
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
-}
 __device__ __forceinline__ void cp_async16(float *dst, const float *src, bool ok) {      // 16 bytes into shared memory; zeros when !ok
     const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst), n = ok ? 16u : 0u;
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
@@ -572,17 +568,14 @@ __global__ void __launch_bounds__(256) k_gqa_decode(const GqaArgs a) {
 //     p_i = S^T (Gm_i k_i) + sum_{j<i} A_ij u_j,    A_ij = sum_d k_i k_j prod_{j<l<=i} g_l,    u_i = beta_i (v_i - p_i)
 //     o_i = S^T (Gm_i q_i) + sum_{j<=i} B_ij u_j,   B_ij = sum_d q_i k_j prod_{j<l<=i} g_l
 //     S  <- Gm_C S + sum_j (prod_{l>j} g_l k_j) u_j^T
-// so  u = M_u w  and  o = S^T (Gm q) + M_o w  with  w_j = v_j - S^T (Gm_j k_j)  and two triangular matrices made of A, B and beta alone:
+// so  u = M_u w  and  o = S^T (Gm q) + M_o w  with  w_j = v_j - S^T (Gm_j k_j)  and two 4 x 4 triangular matrices made of A, B and beta alone:
 // a value column meets its state twice per chunk instead of twice per token, and the sums over the key coordinates of all its
 // tokens run side by side.  Every product of decays is a product of numbers in (0, 1], never a quotient.
 // ------------------------------------------------------------------------------------------------
-constexpr uint32_t kDeltaChunk = 16, kDeltaDim = 256, kDeltaPrepThreads = 256, kDeltaPitch = kDeltaChunk + 4;
-// What the scan reads of a chunk and head, in one run: 16 rows Gm_i k_i and 16 Gm_i q_i, 16 rows prod_{l>j} g_l k_j, Gm_C, each of `dp` coordinates, then the rows of M_u and M_o.  Rows are
-// as far apart as lets the fragments of a warp lie in different banks.
-__host__ __device__ constexpr uint32_t delta_kq(uint32_t dp) { return dp + 8u; }
-__host__ __device__ constexpr uint32_t delta_sk(uint32_t dp) { return dp + 4u; }
+constexpr uint32_t kDeltaChunk = 4, kDeltaDim = 256, kDeltaVecs = 3 * kDeltaChunk + 1, kDeltaMat = 2 * kDeltaChunk * kDeltaChunk;
+// what the scan reads of a chunk and head, in one run: Gm_i k_i (4), Gm_i q_i (4), prod_{l>j} g_l k_j (4), Gm_C, each `dp` coordinates; M_u, M_o
 __host__ __device__ inline uint32_t delta_dp(uint32_t D) { return D <= 32u ? 32u : D <= 64u ? 64u : D <= 128u ? 128u : 256u; }
-__host__ __device__ constexpr uint32_t delta_block(uint32_t dp) { return kDeltaChunk * (2u * delta_kq(dp) + delta_sk(dp) + 2u * kDeltaPitch) + dp; }
+__host__ __device__ inline uint32_t delta_block(uint32_t dp) { return kDeltaVecs * dp + kDeltaMat; }
 // exp(-rate sp), in double precision and rounded once: a state that forgets slowly takes thousands of these factors
 __device__ __forceinline__ float delta_decay(float rate, float sp) { return (float)exp(-(double)rate * (double)sp); }
 
@@ -593,405 +586,254 @@ struct DeltaPrepArgs {
     float *blk, *v;                        // blk [chunks][H][delta_block], v [T][H VD]
     uint32_t T, H, G, D, VD; float qscale;
 };
-// Shared memory of k_delta_prep: q, k and decays [16][dp] each
-inline size_t delta_prep_smem(uint32_t dp) { return (size_t)3u * kDeltaChunk * dp * 4u; }
-// The chunk's tokens of one convolved channel, silu taken, into the first `room` places of `to`, `step` floats apart (zeros past the portion).  Up to four taps: the inputs that the
-// chunk meets are loaded at once
-__device__ __forceinline__ void delta_conv(const DeltaPrepArgs &a, uint32_t t0, uint32_t c, uint32_t C, float *to, size_t step, uint32_t room) {
-    constexpr uint32_t CN = kDeltaChunk;
-    auto put = [&](uint32_t i, float y) { if (i < room) to[i * step] = y; };
-    const uint32_t K = a.K, left = a.T - t0;          // tokens of the portion from the chunk's first on
-    const float *p = a.p + (size_t)t0 * a.ld + a.c0 + c, *tap = a.taps + (size_t)c * K;
-    if (K <= 4u) {
-        float w[4], in[CN + 3u];
-        const bool inside = t0 >= 3u;
-#pragma unroll
-        for (uint32_t m = 0; m < 3u; m++) {          // the tokens before the chunk: rows of the portion, or of the tail in the state
-            const uint32_t back = 3u - m;
-            in[m] = back >= K ? 0.0f : inside || t0 >= back ? *(p - (size_t)back * a.ld) : a.state[(size_t)(K - 1u + t0 - back) * C + c];
-        }
-#pragma unroll
-        for (uint32_t m = 0; m < CN; m++) in[3u + m] = m < left ? p[(size_t)m * a.ld] : 0.0f;
-#pragma unroll
-        for (uint32_t m = 0; m < 4u; m++) w[m] = m + K >= 4u ? tap[m + K - 4u] : 0.0f;
-#pragma unroll
-        for (uint32_t i = 0; i < CN; i++) {
-            float v = 0.0f;
-            if (i < left) {          // (a short last chunk passes less code)
-#pragma unroll
-                for (uint32_t m = 0; m < 4u; m++) v = fmaf(w[m], in[i + m], v);
-                v = siluf_(v);
-            }
-            put(i, v);
-        }
-    } else {
-#pragma unroll 1
-        for (uint32_t i = 0; i < CN; i++) {
-            float v = 0.0f;
-#pragma unroll 4
-            for (uint32_t m = 0; m < K; m++) {
-                const int32_t src = (int32_t)(t0 + i + m) - (int32_t)(K - 1u);
-                v = fmaf(tap[m], src < 0 ? a.state[(size_t)((int32_t)(K - 1u) + src) * C + c] : src < (int32_t)a.T ? a.p[(size_t)src * a.ld + a.c0 + c] : 0.0f, v);
-            }
-            put(i, i < left ? siluf_(v) : 0.0f);
-        }
-    }
-}
-// grid = (chunks, heads).  A thread per channel of the head makes its convolution and silu.  Then warp w makes rows w and 15 - w of A and B, a lane with every 32nd key
-// coordinate: k_j, decayed step by step towards the row, meets k_i and q_i; 31 shuffles leave sum l of a row's 32 in lane l.  All sums over the coordinates -- squares, and
-// the products between tokens -- are taken of the vectors before they become unit vectors; their factors join afterwards.
-// What bounds it is the number of instructions, and for a few chunks how many come one after the other: 16 heads of 128, one chunk / 64 of them: a thread per coordinate with all rows
-// unrolled 40 / 78 us (143 KB of code, which each block passes once: fetching it), every warp walking all rows 25 / 68, this 12 / 32.
-template <int DPT>
-__global__ void __launch_bounds__(kDeltaPrepThreads) k_delta_prep(const DeltaPrepArgs a) {
+// grid = (chunks, heads), delta_dp(D) threads: a thread makes the chunk's tokens of its key coordinate (and of some value columns).  All sums
+// over the coordinates -- squares, and the products between tokens -- are taken of the vectors before they become unit vectors, in one
+// reduction; their factors join afterwards.
+__global__ void __launch_bounds__(kDeltaDim) k_delta_prep(const DeltaPrepArgs a) {
     pdl_enter();
-    constexpr uint32_t CN = kDeltaChunk, NT = kDeltaPrepThreads, DP = DPT, NPL = DP / 32u, PK = delta_kq(DP), PS = delta_sk(DP);
-    static_assert(NT == 32u * CN / 2u, "two rows a warp");
-    extern __shared__ __align__(16) float delta_pm[];
-    __shared__ __align__(16) float A_s[CN][CN], B_s[CN][CN];
-    __shared__ float fac[2 * CN], q2_s[CN], k2_s[CN], beta_s[CN];
-    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u, t0 = blockIdx.x * CN, h = blockIdx.y, g = h / (a.H / a.G);
-    const uint32_t D = a.D, GD = a.G * D, C = 2u * GD + a.H * a.VD;
-    float *q_s = delta_pm, *k_s = q_s + CN * DP, *g_s = k_s + CN * DP;
+    constexpr uint32_t C4 = kDeltaChunk;
+    __shared__ float red[8][32], tot[32], fac[2 * C4], beta_s[C4];
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u, nw = blockDim.x >> 5, DP = blockDim.x, t0 = blockIdx.x * C4, h = blockIdx.y, g = h / (a.H / a.G);
+    const uint32_t D = a.D, GD = a.G * D, C = 2u * GD + a.H * a.VD, K = a.K;
     float *blk = a.blk + ((size_t)blockIdx.x * a.H + h) * delta_block(DP);
+    // one row of channel c before (or in) the portion
+    auto input = [&](int32_t src, uint32_t c) {
+        return src >= 0 ? (src < (int32_t)a.T ? a.p[(size_t)src * a.ld + a.c0 + c] : 0.0f) : a.state[(size_t)((int32_t)(K - 1u) + src) * C + c];
+    };
+    float q[C4], k[C4], gv[C4];
+#pragma unroll
+    for (uint32_t i = 0; i < C4; i++) { q[i] = 0.0f; k[i] = 0.0f; gv[i] = 1.0f; }
     const float rate = a.rate[h];
-    // step sizes and decays; tokens past the portion: nothing is forgotten, nothing is written
-    if (tid >= NT - CN) { const uint32_t t = t0 + tid - (NT - CN); beta_s[tid - (NT - CN)] = t < a.T ? sigmoidf_(a.p[(size_t)t * a.ld + a.b0 + h]) : 0.0f; }
-    if (a.sp) {
-#pragma unroll 1
-        for (uint32_t i = tid; i < CN * DP; i += NT) {
-            const uint32_t t = t0 + i / DP, d = i % DP;
-            g_s[i] = t < a.T && d < D ? delta_decay(rate, softplusf_(a.sp[((size_t)t * a.H + h) * D + d])) : 1.0f;          // (softplus here: as the product's epilogue, four warps a tile, it was 26 us of a product of 37)
+    if (tid < D) {
+        const uint32_t cq = g * D + tid, ck = GD + cq;
+        float wq[C4], wk[C4];              // the taps that meet input m for tokens 0..3: taps[m - i]
+#pragma unroll
+        for (uint32_t i = 0; i < C4; i++) { wq[i] = 0.0f; wk[i] = 0.0f; }
+#pragma unroll 4
+        for (uint32_t m = 0; m < K + C4 - 1u; m++) {
+            const int32_t src = (int32_t)(t0 + m) - (int32_t)(K - 1u);
+            const float xq = input(src, cq), xk = input(src, ck);
+#pragma unroll
+            for (int i = (int)C4 - 1; i > 0; i--) { wq[i] = wq[i - 1]; wk[i] = wk[i - 1]; }
+            wq[0] = m < K ? a.taps[(size_t)cq * K + m] : 0.0f; wk[0] = m < K ? a.taps[(size_t)ck * K + m] : 0.0f;
+#pragma unroll
+            for (uint32_t i = 0; i < C4; i++) { q[i] = fmaf(wq[i], xq, q[i]); k[i] = fmaf(wk[i], xk, k[i]); }
         }
-    } else {
-        if (tid < CN) fac[tid] = t0 + tid < a.T ? delta_decay(rate, softplusf_(a.p[(size_t)(t0 + tid) * a.ld + a.a0 + h] + a.dt_bias[h])) : 1.0f;
-        __syncthreads();
-#pragma unroll 1
-        for (uint32_t i = tid; i < CN * DP; i += NT) g_s[i] = i % DP < D ? fac[i / DP] : 1.0f;
+#pragma unroll
+        for (uint32_t i = 0; i < C4; i++) {
+            const uint32_t t = t0 + i;
+            if (t < a.T) {
+                q[i] = siluf_(q[i]); k[i] = siluf_(k[i]);
+                // (softplus here: as the product's epilogue, four warps a tile, it was 26 us of a product of 37)
+                gv[i] = delta_decay(rate, softplusf_(a.sp ? a.sp[((size_t)t * a.H + h) * D + tid] : a.p[(size_t)t * a.ld + a.a0 + h] + a.dt_bias[h]));
+            } else { q[i] = 0.0f; k[i] = 0.0f; }      // tokens past the portion: nothing is forgotten, nothing is written
+        }
     }
-#pragma unroll 1
-    for (uint32_t n = tid; n < 2u * DP + a.VD; n += NT) {          // channels of q (padded to dp), k (the same), v
-        const uint32_t part = n < DP ? 0u : n < 2u * DP ? 1u : 2u, e = n - part * DP;
-        if (part < 2u && e >= D) { for (uint32_t i = 0; i < CN; i++) q_s[(part * CN + i) * DP + e] = 0.0f; continue; }
-        const uint32_t c = part == 2u ? 2u * GD + h * a.VD + e : part * GD + g * D + e;
-        float *to = part == 2u ? a.v + (size_t)t0 * a.H * a.VD + h * a.VD + e : q_s + part * CN * DP + e;
-        delta_conv(a, t0, c, C, to, part == 2u ? (size_t)a.H * a.VD : DP, part == 2u ? a.T - t0 : CN);
+    if (tid < C4) beta_s[tid] = t0 + tid < a.T ? sigmoidf_(a.p[(size_t)(t0 + tid) * a.ld + a.b0 + h]) : 0.0f;
+    // sums 0..3: q_i^2, 4..7: k_i^2, 8 + i (i - 1) / 2 + j: k_i k_j prod_{j<l<=i} g_l (j < i), 14 + i (i + 1) / 2 + j: q_i k_j prod (j <= i)
+    float x[32];
+#pragma unroll
+    for (int i = 0; i < 32; i++) x[i] = 0.0f;
+#pragma unroll
+    for (int i = 0; i < (int)C4; i++) {
+        x[i] = q[i] * q[i]; x[4 + i] = k[i] * k[i];
+        float dec = 1.0f;
+#pragma unroll
+        for (int j = i; j >= 0; j--) {
+            if (j < i) { dec *= gv[j + 1]; x[8 + i * (i - 1) / 2 + j] = k[i] * k[j] * dec; }
+            x[14 + i * (i + 1) / 2 + j] = q[i] * k[j] * dec;
+        }
+    }
+    // 32 sums over 32 lanes: lane l ends with sum l
+#pragma unroll
+    for (int half = 16; half > 0; half >>= 1) {
+        const bool up = lane & half;
+#pragma unroll
+        for (int i = 0; i < half; i++) {
+            const float keep = up ? x[i + half] : x[i], give = up ? x[i] : x[i + half];
+            x[i] = keep + __shfl_xor_sync(0xffffffffu, give, half);
+        }
+    }
+    red[warp][lane] = x[0];
+    // the value columns, meanwhile
+    for (uint32_t j = tid; j < a.VD; j += blockDim.x) {
+        const uint32_t cv = 2u * GD + h * a.VD + j;
+        float v[C4], wv[C4];
+#pragma unroll
+        for (uint32_t i = 0; i < C4; i++) { v[i] = 0.0f; wv[i] = 0.0f; }
+#pragma unroll 4
+        for (uint32_t m = 0; m < K + C4 - 1u; m++) {
+            const float xv = input((int32_t)(t0 + m) - (int32_t)(K - 1u), cv);
+#pragma unroll
+            for (int i = (int)C4 - 1; i > 0; i--) wv[i] = wv[i - 1];
+            wv[0] = m < K ? a.taps[(size_t)cv * K + m] : 0.0f;
+#pragma unroll
+            for (uint32_t i = 0; i < C4; i++) v[i] = fmaf(wv[i], xv, v[i]);
+        }
+#pragma unroll
+        for (uint32_t i = 0; i < C4; i++) if (t0 + i < a.T) a.v[(size_t)(t0 + i) * a.H * a.VD + h * a.VD + j] = siluf_(v[i]);
     }
     __syncthreads();
-#pragma unroll 1
-    for (uint32_t two = 0; two < 2u; two++) {
-        const uint32_t i = two ? CN - 1u - warp : warp;
-        if (t0 + i >= a.T) {          // past the portion: nothing to sum
-            if (lane < CN) A_s[i][lane] = 0.0f; else B_s[i][lane - CN] = 0.0f;
-            if (lane == 0) q2_s[i] = k2_s[i] = 0.0f;
-            continue;
-        }
-        float kv[NPL], qv[NPL], dec[NPL], x[32], q2 = 0.0f;
-#pragma unroll
-        for (uint32_t n = 0; n < NPL; n++) { kv[n] = k_s[i * DP + n * 32u + lane]; qv[n] = q_s[i * DP + n * 32u + lane]; dec[n] = 1.0f; q2 = fmaf(qv[n], qv[n], q2); }
-#pragma unroll
-        for (uint32_t r = 0; r < 32u; r++) x[r] = 0.0f;
-#pragma unroll
-        for (uint32_t b = 0; b < CN; b++) {          // token j = i - b: sums b (A; k_i^2 first) and 16 + b (B)
-            if (b > i) break;
-#pragma unroll
-            for (uint32_t n = 0; n < NPL; n++) {
-                const uint32_t at = (i - b) * DP + n * 32u + lane;
-                const float r = k_s[at] * dec[n];
-                x[b] = fmaf(kv[n], r, x[b]); x[CN + b] = fmaf(qv[n], r, x[CN + b]);
-                dec[n] *= g_s[at];
-            }
-        }
-#pragma unroll
-        for (int half = 16; half > 0; half >>= 1) {
-            const bool up = lane & half;
-#pragma unroll
-            for (int r = 0; r < half; r++) {
-                const float keep = up ? x[r + half] : x[r], give = up ? x[r] : x[r + half];
-                x[r] = keep + __shfl_xor_sync(0xffffffffu, give, half);
-            }
-        }
-        q2 = warp_sum(q2);
-        const uint32_t b = lane & (CN - 1u), j = (i - b) & (CN - 1u);
-        if (lane == 0) { q2_s[i] = q2; k2_s[i] = x[0]; }
-        if (lane < CN) A_s[i][j] = b && b <= i ? x[0] : 0.0f;
-        else B_s[i][j] = b <= i ? x[0] : 0.0f;
+    if (tid < 32u) {
+        float s = 0.0f;
+        for (uint32_t w = 0; w < nw; w++) s += red[w][tid];
+        tot[tid] = s;
+        if (tid < 2u * C4) fac[tid] = (tid < C4 ? a.qscale : 1.0f) / sqrtf(s + 1e-6f);      // the unit vectors' factors: q 0..3, k 4..7
     }
-    __syncthreads();
-    if (tid < 2u * CN) fac[tid] = (tid < CN ? a.qscale : 1.0f) / sqrtf((tid < CN ? q2_s[tid] : k2_s[tid - CN]) + 1e-6f);      // the unit vectors' factors: q 0..15, k 16..31
     __syncthreads();
     {
-        const uint32_t i = tid / CN, j = tid % CN;
-        A_s[i][j] *= fac[CN + i] * fac[CN + j];
-        B_s[i][j] *= fac[i] * fac[CN + j];
-    }
-    __syncthreads();
-    float *sk = blk + 2u * CN * PK, *mat = sk + CN * PS + DP;
-    // w = v - S^T (Gm k)  ->  u = M_u w with rows M_i = beta_i (e_i - sum_{j<i} A_ij M_j), and o = S^T (Gm q) + (B M_u) w: column lane % 16 of both, the second's even and odd rows in
-    // the warp's halves.  One warp's work, while the others write the rows
-    if (warp == 0) {
-        const uint32_t col = lane & (CN - 1u);
-        float M[CN];
+        float pre = 1.0f, suf = 1.0f;
 #pragma unroll
-        for (uint32_t i = 0; i < CN; i++) {
-            float v[2] = {i == col ? 1.0f : 0.0f, 0.0f};
-#pragma unroll
-            for (uint32_t j = 0; j < i; j++) v[j & 1u] = fmaf(-A_s[i][j], M[j], v[j & 1u]);
-            M[i] = beta_s[i] * (v[0] + v[1]);
-            if (lane < CN) mat[i * kDeltaPitch + col] = M[i];
+        for (uint32_t i = 0; i < C4; i++) {
+            pre *= gv[i];
+            k[i] *= fac[C4 + i];
+            blk[i * DP + tid] = pre * k[i];
+            blk[(C4 + i) * DP + tid] = pre * (q[i] * fac[i]);
         }
-#pragma unroll 1
-        for (uint32_t i = lane / CN; i < CN; i += 32u / CN) {
-            float v[2] = {0.0f, 0.0f};
 #pragma unroll
-            for (uint32_t j = 0; j < CN; j++) v[j & 1u] = fmaf(B_s[i][j], M[j], v[j & 1u]);
-            mat[(CN + i) * kDeltaPitch + col] = v[0] + v[1];
-        }
-        return;
+        for (int i = (int)C4 - 1; i >= 0; i--) { blk[(2u * C4 + i) * DP + tid] = suf * k[i]; suf *= gv[i]; }
+        blk[3u * C4 * DP + tid] = pre;
     }
-#pragma unroll 1
-    for (uint32_t n = tid - 32u; n < 2u * DP; n += NT - 32u) {          // a coordinate's rows from the first token on, or from the last one back
-        const uint32_t d = n & (DP - 1u);
-        float dec = 1.0f;
-        if (n < DP) {
-#pragma unroll 4
-            for (uint32_t i = 0; i < CN; i++) {
-                dec *= g_s[i * DP + d];
-                blk[i * PK + d] = dec * (k_s[i * DP + d] * fac[CN + i]);
-                blk[(CN + i) * PK + d] = dec * (q_s[i * DP + d] * fac[i]);
-            }
-            sk[CN * PS + d] = dec;
-        } else {
-#pragma unroll 4
-            for (uint32_t b = 0; b < CN; b++) { const uint32_t i = CN - 1u - b; sk[i * PS + d] = dec * (k_s[i * DP + d] * fac[CN + i]); dec *= g_s[i * DP + d]; }
+    // w = v - S^T (Gm k)  ->  u = M_u w with rows M_i = beta_i (e_i - sum_{j<i} A_ij M_j), and o = S^T (Gm q) + (B M_u) w: column `tid` of both
+    if (tid < C4) {
+        float M[C4], *mat = blk + kDeltaVecs * DP;
+#pragma unroll
+        for (int i = 0; i < (int)C4; i++) {
+            float v = i == (int)tid ? 1.0f : 0.0f;
+#pragma unroll
+            for (int j = 0; j < i; j++) v = fmaf(-tot[8 + i * (i - 1) / 2 + j] * fac[C4 + i] * fac[C4 + j], M[j], v);
+            M[i] = beta_s[i] * v;
+            mat[i * C4 + tid] = M[i];
+        }
+#pragma unroll
+        for (int i = 0; i < (int)C4; i++) {
+            float v = 0.0f;
+#pragma unroll
+            for (int j = 0; j <= i; j++) v = fmaf(tot[14 + i * (i + 1) / 2 + j] * fac[i] * fac[C4 + j], M[j], v);
+            mat[C4 * C4 + i * C4 + tid] = v;
         }
     }
 }
 
-// x, y (to 2^-25 of themselves) as three pairs of bfloat16, the large parts first
-__device__ __forceinline__ void split3(float x, float y, uint32_t &p0, uint32_t &p1, uint32_t &p2) {
-    auto pack = [&](uint32_t &p) {
-        const __nv_bfloat162 b = __floats2bfloat162_rn(x, y);
-        p = *reinterpret_cast<const uint32_t *>(&b);
-        x -= __uint_as_float(p << 16); y -= __uint_as_float(p & 0xffff0000u);
-    };
-    pack(p0); pack(p1); pack(p2);
-}
-// c += a b for operands in three parts each: the six products that are 2^-24 of the result or more, in two chains of three, small ones first
-__device__ __forceinline__ void mma_split3(float (&c)[4], const uint32_t (&a)[3][4], const uint32_t (&b)[3][2]) {
-    float s[4] = {};
-    mma_bf16(s, a[2], b[0]); mma_bf16(c, a[1], b[0]);
-    mma_bf16(s, a[0], b[2]); mma_bf16(c, a[0], b[1]);
-    mma_bf16(s, a[1], b[1]); mma_bf16(c, a[0], b[0]);
-#pragma unroll
-    for (int i = 0; i < 4; i++) c[i] += s[i];
-}
-
+// A block of 8 warps owns 16 value columns of head h = blockIdx.y, a warp two of them; the 32 lanes share the key coordinates.  A chunk
+// takes 8 sums over the coordinates per column (four S^T (Gm_i k_i), four S^T (Gm_i q_i)); the warp reduces its 16 sums with 16 shuffles
+// and no selection, because lane l keeps sum (i, column c) in the place (i ^ (l / 4), c ^ (l / 2 % 2)) from the start -- it reads the chunk
+// vectors in that order and its two columns of the state sit in that order.  Lanes 2 n and 2 n + 1 end with sum n.  Tiles of NCH chunks
+// travel two ahead (cp.async into a ring of three).
 struct DeltaScanArgs { const float *blk, *v; float *S; float *o; uint32_t T, H, D, VD; };
-constexpr uint32_t kDeltaRing = 3, kDeltaCols = 16, kDeltaPartCol = 52, kDeltaPart = kDeltaCols * kDeltaPartCol, kDeltaU = 24;          // a warp's part: columns 52 floats apart; u: columns 24 apart
-template <int DP> constexpr size_t delta_scan_smem() { return (kDeltaRing * delta_block(DP) + 8u * kDeltaPart + kDeltaCols * (kDeltaPitch + kDeltaU)) * 4u; }
 template <int VW> __device__ __forceinline__ void lds_vec(const float *p, float *v) {
     if constexpr (VW == 4) { const float4 f = *reinterpret_cast<const float4 *>(p); v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w; }
     else if constexpr (VW == 2) { const float2 f = *reinterpret_cast<const float2 *>(p); v[0] = f.x; v[1] = f.y; }
     else v[0] = *p;
 }
-// ---- the state of 16 value columns in the registers of a block's warps, and what a chunk does with it ----
-// bf16 models: accumulators of m16n8k16 (rows: columns of the state, eight coordinates each), which is at the same time the layout of the second operand of the next chunk's products;
-// every fp32 number goes in as three bfloat16 parts.  The fragments of a chunk's rows do not depend on the state: they are made while something else is waited for.
-template <int DP> struct DeltaStateMma {
-    static constexpr uint32_t CN = kDeltaChunk, PK = delta_kq(DP), PS = delta_sk(DP), NW = DP / 16u < 8u ? DP / 16u : 8u, KS = DP / 16u / NW;          // warps with coordinates, steps of 16 of each
-    uint32_t warp, fr, fc, A[KS][2][3][4], B[KS][2][3][2];
-    float S[KS][2][4];          // S[s][n][2 r + e]: column fr + 8 r, coordinate 16 (s NW + warp) + 8 n + fc + e
-    __device__ __forceinline__ DeltaStateMma(uint32_t w, uint32_t lane) : warp(w), fr(lane >> 2), fc((lane & 3u) * 2u) {}
-    template <typename F> __device__ __forceinline__ void each(F f) {          // (number, column, coordinate)
-#pragma unroll
-        for (uint32_t s = 0; s < KS; s++)
-#pragma unroll
-            for (uint32_t n = 0; n < 2u; n++)
-#pragma unroll
-                for (uint32_t i = 0; i < 4u; i++) f(S[s][n][i], fr + 8u * (i >> 1), warp < NW ? 16u * (s * NW + warp) + 8u * n + fc + (i & 1u) : (uint32_t)DP);
-    }
-    __device__ __forceinline__ void rows(const float *blk) {
-#pragma unroll
-        for (uint32_t s = 0; s < KS; s++)
-#pragma unroll
-            for (uint32_t m = 0; m < 2u; m++)
-#pragma unroll
-                for (uint32_t r = 0; r < 4u; r++) {
-                    const float2 f = *reinterpret_cast<const float2 *>(blk + (16u * m + fr + 8u * (r & 1u)) * PK + 16u * (s * NW + warp) + fc + 8u * (r >> 1));
-                    split3(f.x, f.y, A[s][m][0][r], A[s][m][1][r], A[s][m][2][r]);
-                }
-    }
-    // the chunk's 32 rows times the state -> this warp's part [column][row]; then the fragments of the writes' keys
-    __device__ __forceinline__ void parts(const float *blk, float *part) {
-        const float *sk = blk + 2u * CN * PK;
-        float x[2][2][4] = {};          // rows 16 m + fr (+ 8), columns 8 n + fc (+ 1)
-#pragma unroll
-        for (uint32_t s = 0; s < KS; s++)
-#pragma unroll
-            for (uint32_t n = 0; n < 2u; n++) {
-                uint32_t St[3][2];
-#pragma unroll
-                for (uint32_t r = 0; r < 2u; r++) split3(S[s][r][2u * n], S[s][r][2u * n + 1u], St[0][r], St[1][r], St[2][r]);
-#pragma unroll
-                for (uint32_t m = 0; m < 2u; m++) mma_split3(x[m][n], A[s][m], St);
-            }
-#pragma unroll
-        for (uint32_t m = 0; m < 2u; m++)
-#pragma unroll
-            for (uint32_t n = 0; n < 2u; n++)
-#pragma unroll
-                for (uint32_t i = 0; i < 4u; i++) part[(8u * n + fc + (i & 1u)) * kDeltaPartCol + 16u * m + fr + 8u * (i >> 1)] = x[m][n][i];
-#pragma unroll
-        for (uint32_t s = 0; s < KS; s++)
-#pragma unroll
-            for (uint32_t n = 0; n < 2u; n++) {
-                const float *k = sk + 16u * (s * NW + warp) + 8u * n + fr;
-#pragma unroll
-                for (uint32_t r = 0; r < 2u; r++) split3(k[(fc + 8u * r) * PS], k[(fc + 8u * r + 1u) * PS], B[s][n][0][r], B[s][n][1][r], B[s][n][2][r]);
-            }
-    }
-    __device__ __forceinline__ void update(const float *blk, const float *u_s) {
-        const float *sk = blk + 2u * CN * PK;
-        uint32_t U[3][4];          // u: rows are columns of the state, the depth is the chunk's tokens
-#pragma unroll
-        for (uint32_t r = 0; r < 4u; r++) {
-            const float2 f = *reinterpret_cast<const float2 *>(u_s + (fr + 8u * (r & 1u)) * kDeltaU + fc + 8u * (r >> 1));
-            split3(f.x, f.y, U[0][r], U[1][r], U[2][r]);
-        }
-#pragma unroll
-        for (uint32_t s = 0; s < KS; s++)
-#pragma unroll
-            for (uint32_t n = 0; n < 2u; n++) {
-                float c[4] = {};
-                mma_split3(c, U, B[s][n]);
-                const float2 gm = *reinterpret_cast<const float2 *>(sk + CN * PS + 16u * (s * NW + warp) + 8u * n + fc);
-#pragma unroll
-                for (uint32_t i = 0; i < 4u; i++) S[s][n][i] = fmaf(S[s][n][i], i & 1u ? gm.y : gm.x, c[i]);
-            }
-    }
-};
-// float32 models: fp32 multiply-adds, a lane with DP / 16 coordinates of one column.  Loads of operands into registers bound it (3050 wavefronts of 3900 cycles a chunk).  The split operands are
-// within 2^-24 too, but tensor cores cut their sums: logits of 650 positions of two layers were at 8.7e-7 of their size against 64 bits in one run and at 8.3e-7 before; here they are where they were.
-template <int DP> struct DeltaStateFma {
-    static constexpr uint32_t CN = kDeltaChunk, PK = delta_kq(DP), PS = delta_sk(DP), NW = 8u, DL = DP / 16u;
-    static constexpr int VW = DL < 4u ? (int)DL : 4, NB = (int)DL / VW;
-    uint32_t col, up, d0;
-    float S[DL];
-    __device__ __forceinline__ DeltaStateFma(uint32_t warp, uint32_t lane) : col(lane & 15u), up(lane >> 4), d0((warp * 2u + (lane >> 4)) * DL) {}
-    template <typename F> __device__ __forceinline__ void each(F f) {
-#pragma unroll
-        for (uint32_t e = 0; e < DL; e++) f(S[e], col, d0 + e);
-    }
-    __device__ __forceinline__ void rows(const float *) {}
-    __device__ __forceinline__ void parts(const float *blk, float *part) {
-        float x[2u * CN];
-#pragma unroll
-        for (uint32_t r = 0; r < 2u * CN; r++) {
-            float f[DL];
-#pragma unroll
-            for (int n = 0; n < NB; n++) lds_vec<VW>(blk + r * PK + d0 + n * VW, f + n * VW);
-            x[r] = S[0] * f[0];
-#pragma unroll
-            for (uint32_t e = 1; e < DL; e++) x[r] = fmaf(S[e], f[e], x[r]);
-        }
-#pragma unroll
-        for (uint32_t r = 0; r < CN; r++) {          // the lower half of the warp keeps the first 16 sums, the upper half the others
-            const float keep = up ? x[r + CN] : x[r], give = up ? x[r] : x[r + CN];
-            part[col * kDeltaPartCol + up * CN + r] = keep + __shfl_xor_sync(0xffffffffu, give, 16);
-        }
-    }
-    __device__ __forceinline__ void update(const float *blk, const float *u_s) {
-        const float *sk = blk + 2u * CN * PK;
-        float u[CN], f[DL];
-#pragma unroll
-        for (uint32_t j = 0; j < CN; j += 4u) lds_vec<4>(u_s + col * kDeltaU + j, u + j);
-#pragma unroll
-        for (int n = 0; n < NB; n++) lds_vec<VW>(sk + CN * PS + d0 + n * VW, f + n * VW);
-#pragma unroll
-        for (uint32_t e = 0; e < DL; e++) S[e] *= f[e];
-#pragma unroll
-        for (uint32_t j = 0; j < CN; j++) {
-#pragma unroll
-            for (int n = 0; n < NB; n++) lds_vec<VW>(sk + j * PS + d0 + n * VW, f + n * VW);
-#pragma unroll
-            for (uint32_t e = 0; e < DL; e++) S[e] = fmaf(f[e], u[j], S[e]);
-        }
-    }
-};
-
-// A block of 8 warps owns 16 value columns of head h = blockIdx.y, a warp a share of the key coordinates.  A chunk: 32 rows (Gm_i k_i, Gm_i q_i) times the state; the warps' sums meet
-// in shared memory, where a thread per token and column adds them up, solves for u (a warp has all tokens of two columns) and writes o; then the state's decay and the chunk's
-// writes.  Two barriers a chunk, chunks two ahead (cp.async into a ring of three).  What bounds it is that chain, 2800 cycles a chunk.  16 heads of 128, 1024 tokens: chunks of 4 with
-// a warp per two columns, which reads all of a chunk's vectors for them, 163 us; chunks of 16 on FMA 132, on tensor cores 94.
-template <int DP, template <int> class STATE>
-__global__ void __launch_bounds__(256) k_delta_scan(const DeltaScanArgs a) {
+__device__ __forceinline__ void cp_async4(float *dst, const float *src, bool ok) {      // 4 bytes into shared memory; zero when !ok
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst), n = ok ? 4u : 0u;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+}
+template <int DCH>
+__global__ void __launch_bounds__(256, 2) k_delta_scan(const DeltaScanArgs a) {
     pdl_enter();
-    constexpr uint32_t CN = kDeltaChunk, BLK = delta_block(DP), MAT = 2u * CN * delta_kq(DP) + CN * delta_sk(DP) + DP, NW = STATE<DP>::NW;
-    extern __shared__ __align__(16) float delta_sm[];
-    float *ring = delta_sm, *part = ring + kDeltaRing * BLK, *w_s = part + 8u * kDeltaPart, *u_s = w_s + kDeltaCols * kDeltaPitch;
-    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u, h = blockIdx.y, col0 = blockIdx.x * kDeltaCols;
-    const uint32_t HV = a.H * a.VD, chunks = (a.T + CN - 1u) / CN;
-    const uint32_t oc = warp * 2u + (lane >> 4), oj = lane & 15u;                 // this lane's column and token of the outputs
-    const bool ocol = col0 + oc < a.VD;
-    auto fetch = [&](uint32_t ch) {          // one group of copies per chunk, an empty one past the last
-        if (ch < chunks) {
-            const float *src = a.blk + ((size_t)ch * a.H + h) * BLK;
-            float *dst = ring + ch % kDeltaRing * BLK;
-            for (uint32_t i = tid * 4u; i < BLK; i += 1024u) cp_async16(dst + i, src + i, true);
+    constexpr uint32_t DP = DCH * 32u, NCH = DCH <= 4 ? 2u : 1u, BLK = kDeltaVecs * DP + kDeltaMat;
+    constexpr int VW = DCH < 4 ? DCH : 4, NB = DCH / VW;      // a lane's coordinates: NB runs of VW, at (run * 32 + lane) * VW
+    __shared__ __align__(16) float w_s[3][NCH][BLK];
+    __shared__ __align__(16) float v_s[3][NCH][4][16];
+    __shared__ __align__(16) float u_s[8][2][2][4];
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u, li = lane >> 2, lc = (lane >> 1) & 1u, h = blockIdx.y, col0 = blockIdx.x * 16u, jw = col0 + warp * 2u;
+    const uint32_t D = a.D, HV = a.H * a.VD, chunks = (a.T + kDeltaChunk - 1u) / kDeltaChunk, tiles = (chunks + NCH - 1u) / NCH;
+    auto fetch = [&](uint32_t tile) {          // one group of copies per tile, an empty one past the last
+        if (tile < tiles) {
+            const uint32_t st = tile % 3u, ch0 = tile * NCH;
+            for (uint32_t i = tid; i < NCH * (BLK / 4u); i += 256u) {
+                const uint32_t c = i / (BLK / 4u), e = (i % (BLK / 4u)) * 4u;
+                if (ch0 + c < chunks) cp_async16(&w_s[st][c][e], a.blk + ((size_t)(ch0 + c) * a.H + h) * BLK + e, true);
+            }
+            if (tid < NCH * 64u) {
+                const uint32_t c = tid / 64u, i = (tid / 16u) % 4u, j = tid % 16u, t = (ch0 + c) * kDeltaChunk + i;
+                const bool ok = t < a.T && col0 + j < a.VD;
+                cp_async4(&v_s[st][c][i][j], ok ? a.v + (size_t)t * HV + h * a.VD + col0 + j : a.v, ok);
+            }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    auto value = [&](uint32_t ch) { const uint32_t t = ch * CN + oj; return ocol && t < a.T ? a.v[(size_t)t * HV + h * a.VD + col0 + oc] : 0.0f; };
     fetch(0); fetch(1);
-    STATE<DP> state(warp, lane);
-    state.each([&](float &x, uint32_t c, uint32_t d) { x = col0 + c < a.VD && d < a.D ? a.S[((size_t)h * a.VD + col0 + c) * a.D + d] : 0.0f; });
-    float v = value(0);
-    asm volatile("cp.async.wait_group 1;" ::: "memory");
-    __syncthreads();
-    if (warp < NW) state.rows(ring);
-    for (uint32_t ch = 0; ch < chunks; ch++) {
-        const float *blk = ring + ch % kDeltaRing * BLK, *mat = blk + MAT;
-        if (warp < NW) state.parts(blk, part + warp * kDeltaPart);
-        float mu[CN], mo[CN];
+    float S[2][DCH];                           // S[c]: column jw + (c ^ lc)
 #pragma unroll
-        for (uint32_t j = 0; j < CN; j += 4u) { lds_vec<4>(mat + oj * kDeltaPitch + j, mu + j); lds_vec<4>(mat + (CN + oj) * kDeltaPitch + j, mo + j); }
-        const float vnext = ch + 1u < chunks ? value(ch + 1u) : 0.0f;
-        __syncthreads();                       // the parts are there
-        {
-            float qk[NW], qo[NW];
-            const float *mine = part + oc * kDeltaPartCol + oj;
+    for (uint32_t c = 0; c < 2; c++)
 #pragma unroll
-            for (uint32_t w = 0; w < NW; w++) { qk[w] = mine[w * kDeltaPart]; qo[w] = mine[w * kDeltaPart + CN]; }
-#pragma unroll
-            for (uint32_t n = NW / 2u; n > 0u; n >>= 1)
-#pragma unroll
-                for (uint32_t w = 0; w < n; w++) { qk[w] += qk[w + n]; qo[w] += qo[w + n]; }
-            w_s[oc * kDeltaPitch + oj] = v - qk[0];
-            __syncwarp();
-            float u4[4] = {}, o4[4] = {qo[0], 0.0f, 0.0f, 0.0f};
-#pragma unroll
-            for (uint32_t j = 0; j < CN; j += 4u) {
-                float wv[4];
-                lds_vec<4>(w_s + oc * kDeltaPitch + j, wv);
-#pragma unroll
-                for (uint32_t e = 0; e < 4u; e++) { u4[e] = fmaf(mu[j + e], wv[e], u4[e]); o4[e] = fmaf(mo[j + e], wv[e], o4[e]); }
-            }
-            u_s[oc * kDeltaU + oj] = (u4[0] + u4[1]) + (u4[2] + u4[3]);
-            const uint32_t t = ch * CN + oj;
-            if (ocol && t < a.T) a.o[(size_t)t * HV + h * a.VD + col0 + oc] = (o4[0] + o4[1]) + (o4[2] + o4[3]);
-            v = vnext;
+        for (int e = 0; e < DCH; e++) {
+            const uint32_t d = ((e / VW) * 32u + lane) * VW + e % VW, col = jw + (c ^ lc);
+            S[c][e] = (col < a.VD && d < D) ? a.S[((size_t)h * a.VD + col) * D + d] : 0.0f;
         }
-        asm volatile("cp.async.wait_group 0;" ::: "memory");          // the next chunk
-        __syncthreads();
-        fetch(ch + 2u);                        // into the place of the chunk before, which every thread is done with
-        if (warp < NW) {
-            state.update(blk, u_s);
-            if (ch + 1u < chunks) state.rows(ring + (ch + 1u) % kDeltaRing * BLK);
+    for (uint32_t tile = 0; tile < tiles; tile++) {
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();                       // this tile has landed for every thread, and the one before is done with: its place is free
+        fetch(tile + 2u);
+        const uint32_t st = tile % 3u;
+#pragma unroll
+        for (uint32_t c = 0; c < NCH; c++) {
+            if (tile * NCH + c >= chunks) break;
+            const float *w = &w_s[st][c][lane * VW], *mat = &w_s[st][c][kDeltaVecs * DP];
+            float x[8][2];
+#pragma unroll
+            for (uint32_t i = 0; i < 8; i++) {
+                float f[DCH];
+#pragma unroll
+                for (int n = 0; n < NB; n++) lds_vec<VW>(w + (i ^ li) * DP + n * 32 * VW, f + n * VW);
+#pragma unroll
+                for (int j = 0; j < 2; j++) {
+                    x[i][j] = S[j][0] * f[0];
+#pragma unroll
+                    for (int e = 1; e < DCH; e++) x[i][j] = fmaf(S[j][e], f[e], x[i][j]);
+                }
+            }
+#pragma unroll
+            for (int half = 4; half > 0; half >>= 1)
+#pragma unroll
+                for (int i = 0; i < half; i++)
+#pragma unroll
+                    for (int j = 0; j < 2; j++) x[i][j] += __shfl_xor_sync(0xffffffffu, x[i + half][j], half * 4);
+            float mine = x[0][0] + __shfl_xor_sync(0xffffffffu, x[0][1], 2);
+            mine += __shfl_xor_sync(0xffffffffu, mine, 1);      // lanes 0..15: S^T (Gm_i k_i), 16..31: S^T (Gm_i q_i), i = li % 4, column jw + lc
+            const float wj = v_s[st][c][li & 3u][warp * 2u + lc] - mine;
+            const float4 mr = *reinterpret_cast<const float4 *>(mat + li * 4u);
+            float y = li < 4u ? 0.0f : mine;
+            y = fmaf(mr.x, __shfl_sync(0xffffffffu, wj, lc * 2u), y); y = fmaf(mr.y, __shfl_sync(0xffffffffu, wj, 4u + lc * 2u), y);
+            y = fmaf(mr.z, __shfl_sync(0xffffffffu, wj, 8u + lc * 2u), y); y = fmaf(mr.w, __shfl_sync(0xffffffffu, wj, 12u + lc * 2u), y);
+            if ((lane & 1u) == 0) {
+                if (li < 4u) u_s[warp][c & 1u][lc][li] = y;
+                else {
+                    const uint32_t t = (tile * NCH + c) * kDeltaChunk + (li & 3u);
+                    if (t < a.T && jw + lc < a.VD) a.o[(size_t)t * HV + h * a.VD + jw + lc] = y;
+                }
+            }
+            float f[5][DCH];                   // the writes' keys, decayed to the chunk's end, and the chunk's whole decay
+#pragma unroll
+            for (int i = 0; i < 5; i++)
+#pragma unroll
+                for (int n = 0; n < NB; n++) lds_vec<VW>(w + (8 + i) * DP + n * 32 * VW, f[i] + n * VW);
+            __syncwarp();
+            float u[2][4];                     // u[c]: the four tokens' steps of column jw + (c ^ lc)
+#pragma unroll
+            for (uint32_t j = 0; j < 2; j++) lds_vec<4>(&u_s[warp][c & 1u][j ^ lc][0], u[j]);
+#pragma unroll
+            for (int j = 0; j < 2; j++)
+#pragma unroll
+                for (int e = 0; e < DCH; e++) {
+                    float v = S[j][e] * f[4][e];
+#pragma unroll
+                    for (int i = 0; i < 4; i++) v = fmaf(f[i][e], u[j][i], v);
+                    S[j][e] = v;
+                }
         }
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
-    state.each([&](float &x, uint32_t c, uint32_t d) { if (col0 + c < a.VD && d < a.D) a.S[((size_t)h * a.VD + col0 + c) * a.D + d] = x; });
+#pragma unroll
+    for (uint32_t c = 0; c < 2; c++)
+#pragma unroll
+        for (int e = 0; e < DCH; e++) {
+            const uint32_t d = ((e / VW) * 32u + lane) * VW + e % VW, col = jw + (c ^ lc);
+            if (col < a.VD && d < D) a.S[((size_t)h * a.VD + col) * D + d] = S[c][e];
+        }
 }
 
 // Short portions (T <= kGemvMaxM): a cluster of blocks per head, each with a share of its value columns, from the convolved channels (an

@@ -144,6 +144,24 @@ def test_delta_chunk_edges(tmp_path, n, dim, conv, f32):
     eng.close()
 
 
+# a token that is no number: it and those after it are lost, and of those before it the ones that the scan solves together with it (four from a multiple of four on), no others
+@pytest.mark.parametrize("f32", [True, False])
+@pytest.mark.parametrize("at", [13, 30, 32])
+def test_delta_no_number(tmp_path, at, f32):
+    delta = {"heads": 2, "kv_heads": 1, "dim": 64, "vdim": 40, "conv": 4}
+    cfg = md.kadesun_config(97, 64, [("delta", delta, None), ("delta", delta, None)])
+    w = md.kadesun_random(cfg, 7)
+    toks = np.random.default_rng(3).integers(0, 96, size=40).astype(np.uint32)
+    ref = K.forward(cfg, w, toks)
+    toks[at], w["embed"][96] = 96, np.inf
+    eng = E.Engine(md.write_model_dir(str(tmp_path / "m"), cfg, w), 64, flags=E.FLAG_F32 if f32 else 0)
+    got = eng.step(eng.seq_open(), toks, range(toks.size))
+    eng.close()
+    whole = at // 4 * 4
+    assert off(got[:whole], ref[:whole]) < 5 * BOUND[f32]          # as above
+    assert np.isnan(got[at:]).all()
+
+
 # tokens at the edges of groups of eight keys, of pages and of the turns of a cluster's 64 warps; heads that share keys by one to five, blocks of positions that end inside a group,
 # norms of a head or of the whole row, a sink with and without a gate
 @pytest.mark.parametrize("design,heads,kv,dim,vdim,mask", [("fidatar", 2, 2, 4, 8, None), ("fidatar", 4, 2, 128, 100, None), ("fidatar", 10, 2, 64, 128, 21), ("fidatar", 3, 1, 36, 4, 8), ("kadesun", 6, 2, 128, 128, None), ("kadesun", 5, 1, 20, 64, None)])
