@@ -1033,7 +1033,7 @@ struct Ctx { float *st; const uint32_t *table; uint32_t T, pos0; const uint32_t 
 
 constexpr size_t kSideMixBytes = 8u << 20;      // a recurrent mixer's weights up to which a single token's feed-forward keeps the norm's stream
 constexpr uint64_t kTcAttnWork = 128 * 128;      // tokens x keys, or keys, from which a portion's grouped-query attention goes to the tensor cores
-constexpr uint32_t kTcAttnKeys = 512, kTcLatentKeys = 32;      // ... and keys from which latents are multiplied out
+constexpr uint32_t kTcAttnKeys = 512, kTcLatentKeys = 128;      // ... and keys from which latents are multiplied out
 
 int conv_launch(LayeredEngine *e, const ConvArgs &ca) {
     int r;
@@ -1080,9 +1080,9 @@ int mix_latent_attn(LayeredEngine *e, const Layer &L, const Run &run, const Ctx 
     // Long portions multiply the latents out: keys and values of every position in sight, in 32-bit precision, then attention over head sizes instead of
     // the latent's rank.  Per token and key that is 2 (dim + vdim) multiply-adds a head instead of 4 R, for 3 R (dim + vdim) a head and key
     // once: the larger part of a short portion, but the absorbed kernel has a block per 4 or 8 queries then, which walks the keys alone (8 tokens behind
-    // 2000, four layers of 16 heads: 4283 us; 64 tokens with the keys multiplied out: 1369).  From a page of keys on, whole portions, us, absorbed / multiplied out: width 1024 (four such
-    // layers of eight) 32 tokens 492 / 454, 100 885 / 603, 5 behind 60 599 / 427, 12 behind 100 712 / 439, and already 20 468 / 444; width 2048 (one of two) 12 behind 60 171 / 163, 80
-    // tokens 231 / 216, but 32 188 / 191 and 12 160 / 173.
+    // 2000, four layers of 16 heads: 4283 us; 64 tokens with the keys multiplied out: 1369).  Fewer than 128 keys stay with the absorbed kernel, which is the slower one from 32 keys on (four
+    // layers of width 1024, 64 tokens 379 us and 304, 100 485 and 360; two of width 2048, 100 tokens 278 and 259): its sums are fp32 multiply-adds of fp32 numbers, where the other
+    // holds a tile's numbers in two f16 parts, small ones next to large ones in fewer bits, and a number that is none spoils a page of keys there, a tile of 128 here.
     const uint32_t QW0 = H * (L.dim + L.RD);
     nb::TcAttn ta{};
     ta.q = QR ? e->b_q : e->b_z; ta.ldq = QR ? H * L.dim : QW0 + R + L.RD + (L.has_gate ? H * L.vdim : 0u); ta.q_head = L.dim;

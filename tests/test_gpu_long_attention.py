@@ -93,3 +93,17 @@ def test_negative_scale(tmp_path, design):
     eng.close()
     assert np.sqrt(((got - one) ** 2).mean(-1) / (one ** 2).mean(-1)).max() < 1.2e-2
     assert np.linalg.norm(got - ref) < 2e-2 * np.linalg.norm(ref)
+
+
+def test_no_number_spoils_its_page(tmp_path):
+    """A token that is no number: of the tokens before it only those are lost that share its page of 32 keys, in portions with fewer than 128 keys in sight (bound as above)."""
+    cfg = md.famudra_config(97, 96, [("latent_attention", {"heads": 4, "dim": 64, "vdim": 64, "kv_rank": 64, "q_rank": 56, "scale": 0.125}, None)])
+    w = md.famudra_random(cfg, 5)
+    toks = np.random.default_rng(2).integers(0, 96, size=100).astype(np.uint32)
+    ref = A.forward(cfg, w, toks)
+    toks[70], w["embed"][96] = 96, np.inf
+    eng = E.Engine(md.write_model_dir(str(tmp_path / "m"), cfg, w), 128)
+    got = eng.step(eng.seq_open(), toks, range(toks.size))
+    eng.close()
+    assert np.linalg.norm(got[:64] - ref[:64]) < 2e-2 * np.linalg.norm(ref[:64])
+    assert np.isnan(got[70:]).all()
