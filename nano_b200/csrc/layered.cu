@@ -68,7 +68,6 @@
 #include "layered_mixers3.cuh"
 #include "layered_mixers4.cuh"
 #include "layered_mixers5.cuh"
-#include "layered_gqa_one.cuh"
 #include "layered_one.cuh"
 #include "layered_tc.h"
 #include "modeldir.h"
@@ -1469,12 +1468,7 @@ int gqa_branch(LayeredEngine *e, const Layer &L, const Run &run, const Ctx &cx, 
     GqaArgs a{e->b_p, P, 0u, H * D, H * D + G * D, L.c_hg, L.qn, L.kn, L.rot_tab, L.a_half, run.cache, cx.table, T, H, G, D, VD, L.RL, cx.pos0, cx.pos_ptr, e->eps,
               L.scale, L.softcap, L.sink, L.has_gate ? 1u : 0u, e->b_a, 1u, e->b_gpart, e->b_gtick, gqa_hb(L), L.block_size, L.head_norm ? 1u : 0u};
     int r;
-    if (T == 1 && ((D | VD | P | L.RL) & 3u) == 0 && D <= kGqaOneDim && VD <= kGqaOneDim) {      // a single token: whole 16-byte pieces, heads of up to 128
-        const uint32_t nh = std::min(H / G, kGqaOneHeads);
-        const dim3 grid(kGqaOneBlocks, G * ((H / G + nh - 1u) / nh)), block(256);
-        const auto k = nh == 2u ? k_gqa_one<2> : k_gqa_one<1>;
-        r = launch<GqaArgs>(e, k, grid, block, gqa_one_smem(D, VD), a, kGqaOneBlocks);
-    } else if (T <= kGemvMaxM) {      // a captured step does not know the position: blocks without a share of the keys leave at once
+    if (T <= kGemvMaxM) {      // a captured step does not know the position: blocks without a share of the keys leave at once
         uint32_t pages = ((cx.pos_ptr ? e->max_tokens : cx.pos0 + T) + kPage - 1u) / kPage;
         if (L.block_size) pages = std::min(pages, (L.block_size + kPage - 2u) / kPage + 1u);      // a block of positions may start inside a page
         a.nsplit = std::max(1u, std::min(kGqaSplitMax, pages));
@@ -2741,8 +2735,6 @@ int create(LayeredEngine *e, const nb::ModelDir *dir, uint32_t max_tokens) {
     if (dPart) {
         if (dC) DM(e->d2, T * E * 4); DM(e->b_gpart, (size_t)kGemvMaxM * kGqaSplitMax * dPart * 4); DM(e->b_gtick, (size_t)kGemvMaxM * dTick * 4);
         CK(cudaMemset(e->b_gtick, 0, (size_t)kGemvMaxM * dTick * 4));
-        CK(nb::smem_at_least((const void *)k_gqa_one<1>, (int)gqa_one_smem(kGqaOneDim, kGqaOneDim)));
-        CK(nb::smem_at_least((const void *)k_gqa_one<2>, (int)gqa_one_smem(kGqaOneDim, kGqaOneDim)));
         if (gqa_smem[1] > 48 * 1024) CK(nb::smem_at_least((const void *)k_gqa_attn<1>, (int)gqa_smem[1]));
         if (gqa_smem[2] > 48 * 1024) CK(nb::smem_at_least((const void *)k_gqa_attn<2>, (int)gqa_smem[2]));
         if (gqa_smem[4] > 48 * 1024) CK(nb::smem_at_least((const void *)k_gqa_attn<4>, (int)gqa_smem[4]));
