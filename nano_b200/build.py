@@ -39,8 +39,8 @@ def _newer(target: str, sources) -> bool:
 UNITS = {
     "api.cu": ["family.h", "modeldir.h", "../../include/nano_b200.h"],
     "modeldir.cu": ["modeldir.h"],
-    "layered.cu": ["layered_kernels.cuh", "layered_common.cuh", "f32_split.h", "layered_tc.h", "attn_tc.h", "layered_mixers.cuh", "layered_mixers2.cuh", "layered_mixers3.cuh", "layered_mixers4.cuh", "layered_mixers5.cuh", "layered_one.cuh", "family.h", "modeldir.h", "sample_host.h", "../../include/nano_b200.h"],
-    "layered_tc.cu": ["layered_common.cuh", "layered_tc.h", "tc_ptx.cuh", "family.h"],
+    "layered.cu": ["layered_kernels.cuh", "layered_common.cuh", "f32_split.h", "layered_tc.h", "tc_tiles.h", "attn_tc.h", "layered_mixers.cuh", "layered_mixers2.cuh", "layered_mixers3.cuh", "layered_mixers4.cuh", "layered_mixers5.cuh", "layered_one.cuh", "family.h", "modeldir.h", "sample_host.h", "../../include/nano_b200.h"],
+    "layered_tc.cu": ["layered_common.cuh", "layered_tc.h", "tc_tiles.h", "tc_ptx.cuh", "family.h"],
     "attn_tc.cu": ["attn_tc.h", "tc_ptx.cuh", "family.h"],
     "prefill.cu": ["prefill.h", "prompt_split.h", "attn_tc.h", "tc_ptx.cuh", "kernels.cuh", "expf_ref.cuh", "family.h"],
     "engine.cu": ["prefill.h", "attn_tc.h", "kernels.cuh", "expf_ref.cuh", "stream_args.h", "stream_count.h", "stream_groups.h", "stream_host.h", "sample_host.h", "family.h", "../../include/nano_b200.h"],

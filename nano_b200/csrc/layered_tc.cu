@@ -382,9 +382,8 @@ bool tc_fits(const TcState *t, const GemmArgs &a, uint32_t rows) {
     return t->encode && a.K % 8u == 0 && a.ldw % 8u == 0 && a.w_gstride % 8u == 0 && (a.a_gmod == 1 || a.a_gcols % 8u == 0) && (reinterpret_cast<uintptr_t>(a.W) & 15u) == 0 && rows * width <= t->elems;
 }
 int tc_gemm(TcState *t, GemmArgs a, uint32_t groups, uint32_t maxM, uint32_t rows, uint32_t each, uint32_t buf, cudaStream_t stream, bool pdl) {
-    const uint32_t width = (a.a_gmod - 1) * a.a_gcols + a.K;
+    const uint32_t width = (a.a_gmod - 1) * a.a_gcols + a.K, tn = tc_tile_tokens(each);
     const bool raw = tc_raw_rows(a, groups, each);
-    const uint32_t tn = each <= 32 ? 32u : each <= 64 || raw ? 64u : 128u;
     __nv_bfloat16 *dst = t->rows[buf];
     int r;
     TcArgs ta{};

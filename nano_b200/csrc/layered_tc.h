@@ -4,11 +4,11 @@
 #include <stddef.h>
 
 #include "layered_common.cuh"
+#include "tc_tiles.h"
 
 namespace nb {
 namespace lm {
 
-constexpr uint64_t kTcRawBytes = 32u << 20;
 // what an engine keeps for these products: rounded activation rows (one buffer for each of its three streams), the driver's tensor-map encoder,
 // the word a bounded wait reports to
 struct TcState {
@@ -23,14 +23,9 @@ void tc_free(TcState *t);
 int tc_check(TcState *t);
 // whether the product's layout allows it.  rows: all rows of A it reads (a routed product: tokens x choices)
 bool tc_fits(const TcState *t, const GemmArgs &a, uint32_t rows);
-// Does the product read its fp32 rows itself (one launch), or a rounded copy that a launch of its own makes before it.  each: as below.  Groups of at most 384 rows on average, in tiles of 32
-// or 64 tokens (copies in up to 128), and only while the tiles read less than 32 MB of them, 16 beyond one tile: every tile of weights reads the rows again.  Whole portions, us, copy / rows:
-// Famudra width 1024 (eight layers) 5 tokens 616 / 470, 40 718 / 677, 64 783 / 708, 100 642 / 604, 200 734 / 649, 400 870 / 770; width 2048 (two) 100 252 / 220, 400 314 / 316, but 512
-// 325 / 332; Fidatar width 1024 5 162 / 147, 65 208 / 187, 256 239 / 230; Kadesun width 2048 40 257 / 245, 100 316 / 307, 400 485 / 476, 300 381 / 388, and without the line at 32 MB 64 (50 MB
-// for 12288 columns) 254 / 260; Fidatar width 2048 without the one at 16 MB 256 333 / 339.
+// whether the product reads its fp32 rows itself (tc_tiles.h); they have to be whole 16-byte pieces
 inline bool tc_raw_rows(const GemmArgs &a, uint32_t groups, uint32_t each) {
-    return each <= 384u && a.lda % 4u == 0 && (reinterpret_cast<uintptr_t>(a.A) & 15u) == 0 &&
-           (uint64_t)((a.N + 127u) / 128u) * groups * each * a.K * 4u <= (each <= 64u ? kTcRawBytes : kTcRawBytes / 2u);
+    return a.lda % 4u == 0 && (reinterpret_cast<uintptr_t>(a.A) & 15u) == 0 && tc_reads_rows(a.N, groups, each, a.K);
 }
 // one or two launches on `stream` (with programmatic serialization when pdl).  buf: which of the row buffers is the stream's; maxM: the most rows of a group, each:
 // how many a group has on average

@@ -50,3 +50,22 @@ def test_portions_at_tile_edges(tmp_path, design, width, ff, vocab):
         assert rel(got, one[:n]) < 1.2e-2, n
         assert np.linalg.norm(got - ref[:n]) < 2e-2 * np.linalg.norm(ref[:n]), n
     eng.close()
+
+
+def test_wide_products(tmp_path):
+    """A head of 16392 x 2048, whose tiles would read 32 MB of rows from 32 rows on: on both sides of that line, in copies for tiles of 32 and of 64 tokens.  Bounds as above."""
+    cfg = md.kadesun_config(16392, 2048, [("delta", {"heads": 2, "kv_heads": 1, "dim": 24, "vdim": 40, "conv": 3}, None)])
+    w = md.kadesun_random(cfg, 3)
+    eng = E.Engine(md.write_model_dir(str(tmp_path / "m"), cfg, w), 128)
+    toks = np.random.default_rng(1).integers(0, 16392, size=64).astype(np.uint32)
+    ref = K.forward(cfg, w, toks)
+    s = eng.seq_open()
+    one = np.concatenate([eng.step(s, toks[i:i + 1], [0]) for i in range(toks.size)])
+    eng.seq_close(s)
+    for n in (31, 32, 33, 64):
+        s = eng.seq_open()
+        got = eng.step(s, toks[:n], range(n))
+        eng.seq_close(s)
+        assert rel(got, one[:n]) < 1.2e-2, n
+        assert np.linalg.norm(got - ref[:n]) < 2e-2 * np.linalg.norm(ref[:n]), n
+    eng.close()
