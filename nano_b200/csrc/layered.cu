@@ -977,7 +977,7 @@ int gemm(LayeredEngine *e, GemmArgs a, uint32_t groups, uint32_t maxM, bool wf32
     }
     const dim3 grid((a.N + 63u) / 64u, (maxM + 63u) / 64u, groups);
     if (f32 && gemm_f32_fits(a)) {
-        const uint32_t split = nb::f32_split(grid.x, a.g_off && active ? std::max(1u, (active + groups - 1u) / groups) : maxM, groups, a.K, 2u * (uint32_t)e->num_sms);
+        const uint32_t split = nb::f32_split(grid.x, a.g_off && active ? std::max(1u, (active + groups - 1u) / groups) : maxM, groups, a.K, (uint32_t)e->num_sms);
         return launch_split(e, k_gemm_f32_async, dim3(grid.x * split, grid.y, groups), dim3(kF32Threads), a, split);
     }
     return f32 ? launch<GemmArgs>(e, k_gemm_f32<float>, grid, dim3(256), 0, a) : launch<GemmArgs>(e, k_gemm_bf16, grid, dim3(128), 0, a);
