@@ -97,7 +97,7 @@ struct nb200_engine : nb::EngineBase {
     // grid-wide persistent streaming kernel (stream.cuh): the default path in fast mode on one GPU
     float calib_ms[2] = {0.0f, 0.0f};      // ms per token of {streaming, multi-kernel} measured by calibrate_paths (0 = not calibrated)
     bool use_stream = false; const void *st_kern[3] = {nullptr, nullptr, nullptr}; StreamArgs sa{};      // st_kern: by 1, 2, 4 query heads to an attention item (stream_groups.h)
-     uint32_t st_smem = 0, st_grid = 0;
+    uint32_t st_smem = 0, st_grid = 0;
     uint32_t *st_err_host = nullptr, *st_err_dev = nullptr;      // mapped pinned word: the code a device-side spin recorded before trapping
     nb::StreamCount st_count;                                    // exchange epochs and barrier arrivals used up so far (stream.cuh)
     float *logits_host = nullptr; bool logits_on_host = false;   // pinned copy of the logits that one-token calls of the streaming kernel write; whether it holds the last step's

@@ -1616,7 +1616,7 @@ int route_many(LayeredEngine *e, const RouteArgs &ra) {
 // e->b_so and the gate logits e->b_sg; the residual kernel adds them up.  The score weights the expert's INPUT; the experts have no
 // bias, so act(s g) (s u) of the unweighted products g, u is the same number.  The shared expert runs on a second stream.
 int ff_moe_scored(LayeredEngine *e, const Layer &L, uint32_t T) {
-    const uint32_t E = e->E, NL = L.NE + (L.sh_gate ? 1u : 0u);
+    const uint32_t E = e->E;
     const bool small = T <= kGemvMaxM;
     int r;
     if (L.has_shared && e->branch_streams) CK(cudaEventRecord(e->ev_fork, e->stream));
@@ -1961,7 +1961,7 @@ int decode_step(LayeredEngine *e, uint32_t slot) {
 }
 
 // A call of one token with logits: set_step, decode_step and the logits to e->stage_logits as ONE graph, whose first node's arguments are set anew for every call (a launch of its own
-// in front of the graph and a copy behind it: two Fidatar layers of width 1024 79 us a call, now 71; eight Famudra layers 232, now 224)
+// in front of the graph and a copy behind it: eight Famudra layers of width 1024 232 us a call, 224 so)
 int call_step(LayeredEngine *e, uint32_t slot, uint32_t pos, uint32_t token) {
     LayeredEngine::CallGraph &c = e->calls[slot];
     if (!c.exec) {

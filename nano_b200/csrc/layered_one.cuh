@@ -8,8 +8,7 @@
 // A chain of 1024 x 1024 products from HBM, us a link: k_gemv 4.5, weights in registers 2.9, this 2.1 (with two
 // running sums; one, in k_gemv's order, makes a whole step of eight routed layers bit for bit that of the general kernels: 290 us a token, 265 with two, 364 before).
 // What is left of a link is then the instructions it passes, 620 a warp for a row of 1024, most of them for steps that such a row does not have: a warp leaves a run of steps at its own
-// last one, checks lanes only in rows that end inside a step, and loads an activation row of up to 8 KB at once.  Call to call, a token of eight Famudra layers of width 1024 249 -> 232 us, of two
-// Fidatar layers 84 -> 79 (width 1024), 147 -> 145 (2048).
+// last one, checks lanes only in rows that end inside a step, and loads an activation row of up to 8 KB at once.  Call to call, a token of eight Famudra layers of width 1024 249 -> 232 us.
 #pragma once
 #include "layered_kernels.cuh"
 #include "layered_mixers3.cuh"

@@ -80,9 +80,9 @@ __global__ void __launch_bounds__(256) k_rows_split(const PlaneArgs a) {
     }
 }
 
-// g: the product (A and a_rows unused: the rows are in `amap`, gathered); wmap: [groups][N][K], amap: [rows][a_gmod][K], boxes of 128 weight rows / TN
-// tokens x 64; ks: blocks of a cluster that share one tile's depth (grid.z = groups * ks); wsteps: the stages after which W starts over (rows in several
-// parts; the whole depth otherwise)
+// g: the product; wmap: [groups][N][K], in boxes of 128 weight rows x 64.  Where a rounded copy is read, amap is that: [rows][a_gmod][K], gathered, boxes of TN tokens x 64, and A and
+// a_rows are unused; instances that read their rows themselves take them from A and a_rows, and amap is empty.  ks: blocks of a cluster that share one tile's depth (grid.z = groups * ks);
+// wsteps: the stages after which W starts over (rows in several parts; the whole depth otherwise)
 struct alignas(64) TcArgs { CUtensorMap wmap, amap; GemmArgs g; uint32_t ks, wsteps; uint32_t *err; };
 
 // Epilogue of NJ tokens of one output column: every option is looked at once for the NJ values (inside the loop over tokens the switch alone made a
