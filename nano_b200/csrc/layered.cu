@@ -1034,12 +1034,17 @@ constexpr size_t kSideMixBytes = 8u << 20;      // a recurrent mixer's weights u
 constexpr uint64_t kTcAttnWork = 128 * 128;      // tokens x keys, or keys, from which a portion's grouped-query attention goes to the tensor cores
 constexpr uint32_t kTcAttnKeys = 512, kTcLatentKeys = 128;      // ... and keys from which latents are multiplied out
 
-int conv_launch(LayeredEngine *e, const ConvArgs &ca) {
+// outputs, then the tail.  The two convolutions of a two-sided mixer stay with this: in one launch they end sooner, but which side's blocks then find the SMs free decides how long the layer takes
+// (eight Rakarax layers of width 2048, us a portion, two launches / one: 112 tokens 2030 / 1830, but 136 2020 / 2220 and 160 2180 / 2350)
+int conv_two(LayeredEngine *e, const ConvArgs &ca) {
     int r;
-    if (ca.K == 4u && ca.T >= 3u) return launch<ConvArgs>(e, k_conv_four, dim3((ca.C + 127u) / 128u, (ca.T + kConvTokens - 1u) / kConvTokens), dim3(128), 0, ca);
     if ((r = launch<ConvArgs>(e, k_conv, dim3(ew_grid((size_t)ca.T * ca.C)), dim3(256), 0, ca))) return r;
     if (ca.K > 1 && (r = launch<ConvArgs>(e, k_conv_state, dim3((ca.C + 127) / 128), dim3(128), 0, ca))) return r;
     return 0;
+}
+int conv_launch(LayeredEngine *e, const ConvArgs &ca) {
+    if (ca.K == 4u && ca.T >= 3u) return launch<ConvArgs>(e, k_conv_four, dim3((ca.C + 127u) / 128u, (ca.T + kConvTokens - 1u) / kConvTokens), dim3(128), 0, ca);
+    return conv_two(e, ca);
 }
 
 int mix_rglru(LayeredEngine *e, const Layer &L, const Run &run, const Ctx &cx) {
@@ -1267,7 +1272,7 @@ int mix_window_ssm(LayeredEngine *e, const Layer &L, const Run &run, const Ctx &
     // the two sides share nothing after the product: the scan side runs on a second stream and joins before the residual update
     if (e->branch_streams) { CK(cudaEventRecord(e->ev_fork, e->stream)); e->cur = e->side; CK(cudaStreamWaitEvent(e->side, e->ev_fork, 0)); }
     // right
-    if (!small && (r = conv_launch(e, ConvArgs{e->b_p + QK, P, L.m_conv, L.m_conv_b, cx.st + run.st_conv2, e->b_xc, T, C, L.m_taps, C, 1}))) return r;
+    if (!small && (r = conv_two(e, ConvArgs{e->b_p + QK, P, L.m_conv, L.m_conv_b, cx.st + run.st_conv2, e->b_xc, T, C, L.m_taps, C, 1}))) return r;
     if ((r = gemm(e, plain(e->b_xc, C, L.xw, e->b_dbc, R + 2 * N, T), 1, T))) return r;
     if (!small && (r = gemm(e, plain(e->b_dbc, R + 2 * N, L.dtw, e->b_dt, C, T, L.dt_b, EPI_SOFTPLUS), 1, T))) return r;
     SelScanArgs sa{e->b_dt, e->b_xc, e->b_dbc, R + 2 * N, R, R + N, L.A, L.Dv, e->b_p + z0, P, cx.st + run.st_S, e->b_y, T, C, N,
@@ -1284,7 +1289,7 @@ int mix_window_ssm(LayeredEngine *e, const Layer &L, const Run &run, const Ctx &
     if ((r = gemm(e, ro, 1, T))) return r;
     if (e->branch_streams) { CK(cudaEventRecord(e->ev_join, e->side)); e->cur = e->stream; }
     // left
-    if (!small && (r = conv_launch(e, ConvArgs{e->b_p, P, L.a_conv, nullptr, cx.st + run.st_conv, e->b_qk, T, QK, L.a_taps, QK, 0}))) return r;
+    if (!small && (r = conv_two(e, ConvArgs{e->b_p, P, L.a_conv, nullptr, cx.st + run.st_conv, e->b_qk, T, QK, L.a_taps, QK, 0}))) return r;
     QkPrepArgs qa{e->b_qk, QK, e->b_qk + H * D, QK, L.temp, L.scale, run.cache, cx.table, H, G, D, L.RL, cx.pos0, e->eps, cx.pos_ptr};
     if ((r = launch<QkPrepArgs>(e, k_qk_prepare, dim3(T), dim3(256), 0, qa))) return r;
     WinAttnArgs wa{e->b_qk, QK, run.cache, cx.table, e->b_p + g0, P, L.talk, L.slopes, e->b_a, T, H, G, D, L.RL, cx.pos0, L.window, L.softcap, cx.pos_ptr, 1u, e->b_wpart, e->b_wtick};
