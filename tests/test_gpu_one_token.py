@@ -129,7 +129,7 @@ def test_delta_scan_sizes(tmp_path, dim, vdim):
     eng.close()
 
 
-# chunks of four tokens: one short of full, full, one over, one more; convolutions of one tap, of as many as a chunk has tokens, of more, and of more than the scan's three tiles
+# chunks of four tokens: one short of full, full, one over, one more; convolutions of fewer taps than a chunk has tokens, of as many, of one more, and of five chunks
 @pytest.mark.parametrize("f32", [True, False])
 @pytest.mark.parametrize("n,dim,conv", [(15, 64, 4), (16, 128, 4), (17, 128, 1), (31, 20, 2), (33, 256, 4), (48, 128, 5), (37, 64, 21)])
 def test_delta_chunk_edges(tmp_path, n, dim, conv, f32):
